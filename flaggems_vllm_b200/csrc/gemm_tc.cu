@@ -301,8 +301,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
+      const bool leader = elect_lane();
       if constexpr (!GATHER) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
       uint32_t it = 0;
@@ -318,6 +319,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           MOE_TR(0, kb, 0);
           if (!mbar_wait(&aux->empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           MOE_TR(0, kb, 1);
+          if (!leader) continue;
           if constexpr (GATHER) {
             mbar_expect_tx(&aux->full[s], B_LOCAL_BYTES);  // A rows arrive by cp.async (warps 2-3)
           } else {
@@ -334,7 +336,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           MOE_TR(0, kb, 2);
         }
       }
-    } else if (warp == 1 && lane == 0 && cr == 0) {
+    } else if (warp == 1 && cr == 0 && (!PAIR || lane == 0)) {
       // ------------------------------------------------------------ MMA issuer (pair: leader only)
       constexpr uint32_t idesc = IDesc<FP8, AT, PAIR>::value;
       [[maybe_unused]] uint32_t it = 0;
@@ -347,6 +349,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // wait for it: stage index and phase are carried (no division), the descriptors are one
         // add away from a base, and the operands' barrier (which completed long before) is waited
         // for first.  After the release only the fence, the four MMAs and the commits remain.
+        const bool leader = elect_lane();
         const uint64_t adesc0 = make_smem_desc(smem_u32(sA));
         const uint64_t bdesc0 = make_smem_desc(smem_u32(sB));
         uint32_t s = 0, sph = 0;
@@ -370,6 +373,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             MOE_TR(1, kb, 2);
             tc_fence_after();
+            if (leader) {
 #pragma unroll
             for (int j = 0; j < RB; ++j) {
               const uint64_t aj = adesc + (uint64_t)(j * (A_STAGE_BYTES >> 4));
@@ -383,11 +387,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               for (int k4 = 1; k4 < 4; ++k4)  // 32 bytes of K per instruction: start address advances by 32 B >> 4
                 tc_mma_const<FP8, true>(d, aj + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc);
             }
-            if (FP8 || kb == KB - 1) {
-              tc_commit(&aux->tmem_full[a]);
-              ++acc_it;
-            }
+            if (FP8 || kb == KB - 1) tc_commit(&aux->tmem_full[a]);
             tc_commit(&aux->empty[s]);
+            }
+            if (FP8 || kb == KB - 1) ++acc_it;
             MOE_TR(1, kb, 3);
             if (kb == 0) MOE_TRN(1, 61, 2);
             if (kb == 1) MOE_TRN(1, 61, 3);

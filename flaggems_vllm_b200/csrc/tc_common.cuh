@@ -40,6 +40,21 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// One lane of a converged warp.  The warp that feeds the tensor core runs its loop with all 32
+// lanes and only predicates the instructions on this lane: under a divergent `lane == 0` branch
+// the compiler cannot keep descriptors and addresses in uniform registers and moves each of them
+// there in front of every tcgen05.mma, which costs a warp that shares its scheduler with busy
+// ones several hundred cycles per K block (e4m3 128x256 tile with the fp32 fold beside it,
+// operands streaming from L2: 880 -> 612 cycles per 128-wide K block).
+__device__ __forceinline__ bool elect_lane() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
