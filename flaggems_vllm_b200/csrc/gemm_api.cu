@@ -52,8 +52,8 @@ extern "C" int moe_gemm1_ex(int mode, int act_dtype, const void* a, int a_sorted
                             float beta, float limit, int32_t* status, void* stream) {
   using namespace moe;
   if (activation != MOE_ACT_SILU && activation != MOE_ACT_SWIGLUOAI) return fail(MOE_E_BADARG, "gemm1: unknown activation %d", activation);
-  if (use_tensor_cores && (activation != MOE_ACT_SILU || mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW))
-    return fail(MOE_E_SHAPE, "gemm1: the row-scaled modes and activations other than SiLU are served by the generic kernel");
+  if (use_tensor_cores && activation != MOE_ACT_SILU)
+    return fail(MOE_E_SHAPE, "gemm1: activations other than SiLU are served by the generic kernel");
   if (num_tokens < 0 || topk <= 0) return fail(MOE_E_BADARG, "gemm1: bad token count or topk");
   const int64_t numel = num_tokens * topk;
   int rc = check_common("gemm1", mode, a, a_scales_t, w1, w1_scale, expert_ids, sorted_ids, num_post_pad,
@@ -86,8 +86,6 @@ extern "C" int moe_gemm2(int mode, int act_dtype, const void* act_sorted, const 
                         route_weight, mul_weight, numel, rows_cap, block_m, E, H, I, y);
   if (rc) return rc;
   if (rows_cap == 0 || numel == 0) return 0;
-  if (use_tensor_cores && (mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW))
-    return fail(MOE_E_SHAPE, "gemm2: the row-scaled modes are served by the generic kernel");
   if (use_tensor_cores && mode == MOE_MODE_W8A16)
     return w8_gemm(false, act_dtype, act_sorted, w2, w2_scale, expert_ids, sorted_ids, num_post_pad, route_weight,
                    mul_weight, numel, rows_cap, 0, 1, block_m, E, I, H, y, status, (cudaStream_t)stream);
@@ -132,8 +130,8 @@ extern "C" int moe_gemm2_sorted(int mode, int act_dtype, const void* act_sorted,
                         num_post_pad, route_weight, mul_weight, numel, rows_cap, block_m, E, H, I, y_sorted);
   if (rc) return rc;
   if (!inv) return fail(MOE_E_BADARG, "gemm2 (sorted output): route index buffer missing");
-  if (mode != MOE_MODE_FP8_BLOCK && mode != MOE_MODE_HALF)
-    return fail(MOE_E_SHAPE, "gemm2 (sorted output): FP8 block-scale and half-precision modes only");
+  if (mode == MOE_MODE_W8A16)
+    return fail(MOE_E_SHAPE, "gemm2 (sorted output): not served for weight-only int8");
   if (rows_cap == 0 || numel == 0) return 0;
   return tc_gemm(false, mode, act_dtype, act_sorted, act_scales_t, w2, w2_scale, expert_ids, sorted_ids, num_post_pad,
                  route_weight, mul_weight, numel, rows_cap, 0, 1, block_m, E, I, H, y_sorted, nullptr, status,

@@ -168,8 +168,9 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
       // ------------------------------------------------------------ raw weight ring (TMA)
+      const bool leader = elect_lane();
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       uint32_t it = 0;
       bool alive = true;
@@ -180,6 +181,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % SR;
           if (!mbar_wait(&aux->r_empty[s], ((it / SR) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+          if (!leader) continue;
           mbar_expect_tx(&aux->r_full[s], RAW_BYTES);
 #pragma unroll
           for (int c = 0; c < RawBox<GEMM1>::COUNT; ++c)
@@ -187,8 +189,9 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         wrow0 + box_row<GEMM1>(nt, c, P.Nout));
         }
       }
-    } else if (warp == 1 && lane == 0) {
-      // ------------------------------------------------------------ MMA issuer
+    } else if (warp == 1) {
+      // ------------------------------------------------------------ MMA issuer (converged warp, one lane issues)
+      const bool leader = elect_lane();
       constexpr uint32_t idesc = IDesc<AT>::value;
       uint32_t it = 0, acc_it = 0;
       bool alive = true;
@@ -207,14 +210,15 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const uint64_t adesc = make_smem_desc(smem_u32(sA + (size_t)sa * A_BYTES));
           const uint64_t bdesc = make_smem_desc(smem_u32(sB + (size_t)sb * B_BYTES));
           const uint32_t d = tmem_base + a * BN;
+          if (!leader) continue;
 #pragma unroll
           for (int k4 = 0; k4 < 4; ++k4)  // 32 bytes (16 elements) of K per instruction
-            tc_mma<false>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
+            tc_mma<MMA_F16>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
           tc_commit(&aux->a_empty[sa]);
           tc_commit(&aux->b_empty[sb]);
         }
         if (!alive) break;
-        tc_commit(&aux->tmem_full[a]);
+        if (leader) tc_commit(&aux->tmem_full[a]);
         ++acc_it;
       }
     } else if (!GEMM1 && warp == 2 && lane == 0) {

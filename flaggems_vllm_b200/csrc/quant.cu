@@ -346,6 +346,86 @@ __global__ void __launch_bounds__(256) rowwise_quant_kernel(const T* __restrict_
   }
 }
 
+// The same for 2-byte inputs whose rows are whole 16-byte pieces: TPR threads per row (a warp, or the CTA for
+// long rows) hold the row in registers (CH pieces of 8 elements each), so it is read once, with all loads in
+// flight, and written with 8-byte stores.  The kernel above reads every row twice, 64 bytes per warp and
+// instruction (500 x 2048 and 4000 x 768: 29 us for both).
+template <typename T, int KIND, int TPR, int CH>
+__global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restrict__ x, int64_t rows, int cols,
+                                                                const float* __restrict__ scale_in,
+                                                                const int32_t* __restrict__ row_ids, int64_t valid_below,
+                                                                uint8_t* __restrict__ q, float* __restrict__ scale_out) {
+  constexpr int RPC = 256 / TPR;  // rows per CTA
+  __shared__ float s_amax[TPR > 32 ? 8 : 1], s_nan[TPR > 32 ? 8 : 1];
+  const int t = threadIdx.x % TPR, lane = threadIdx.x & 31;
+  const int pieces = cols / 8;
+  for (int64_t r = (int64_t)blockIdx.x * RPC + threadIdx.x / TPR; r < rows; r += (int64_t)gridDim.x * RPC) {
+    if (row_ids != nullptr) {  // uniform over the threads of a row
+      const int64_t id = row_ids[r];
+      if (id < 0 || id >= valid_below) continue;
+    }
+    uint4 raw[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (t + c * TPR < pieces) raw[c] = reinterpret_cast<const uint4*>(x + r * cols)[t + c * TPR];
+    float scale;
+    if constexpr (KIND == 0 || KIND == 1) {
+      float amax = 0.0f, nan_term = 0.0f;
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        if (t + c * TPR < pieces) {
+          const T* p = reinterpret_cast<const T*>(&raw[c]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float v = ToF32<T>::get(p[i]);
+            amax = fmaxf(amax, fabsf(v));
+            if (!(v == v)) nan_term = v;
+          }
+        }
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
+        nan_term += __shfl_xor_sync(0xFFFFFFFFu, nan_term, off);
+      }
+      if constexpr (TPR > 32) {
+        __syncthreads();  // the previous row's values have been read
+        if (lane == 0) { s_amax[threadIdx.x >> 5] = amax; s_nan[threadIdx.x >> 5] = nan_term; }
+        __syncthreads();
+        amax = 0.0f; nan_term = 0.0f;
+#pragma unroll
+        for (int w = 0; w < TPR / 32; ++w) { amax = fmaxf(amax, s_amax[w]); nan_term += s_nan[w]; }
+      }
+      if constexpr (KIND == 0) {
+        const float eps = ToF32<T>::get(from_f32<T>(1e-10f));
+        scale = (fmaxf(amax, eps) + nan_term) * (1.0f / 127.0f);
+      } else {
+        scale = fmaxf(fmaxf(amax, 1e-10f) / kFp8Max, 1.0f / (kFp8Max * 512.0f));
+      }
+      if (t == 0) scale_out[r] = scale;
+    } else {
+      scale = scale_in[0];
+    }
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (t + c * TPR < pieces) {
+        const T* p = reinterpret_cast<const T*>(&raw[c]);
+        uint32_t w[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float v = ToF32<T>::get(p[i]);
+          uint8_t o;
+          if constexpr (KIND == 0 || KIND == 4) o = (uint8_t)round_int8_even(__fdiv_rn(v, scale));
+          else if constexpr (KIND == 3) o = f32_to_fp8e4m3(fminf(fmaxf(v * (1.0f / scale), -kFp8Max), kFp8Max));
+          else o = f32_to_fp8e4m3(fminf(fmaxf(v / scale, -kFp8Max), kFp8Max));
+          w[i >> 2] |= (uint32_t)o << (8 * (i & 3));
+        }
+        reinterpret_cast<uint2*>(q + r * cols)[t + c * TPR] = make_uint2(w[0], w[1]);
+      }
+    }
+  }
+}
+
 // amax of the rows that count, as the bits of a non-negative float (atomicMax on the bits orders them)
 template <typename T>
 __global__ void __launch_bounds__(256) tensor_amax_kernel(const T* __restrict__ x, int64_t rows, int64_t cols,
@@ -391,7 +471,26 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
                                 const int32_t* row_ids, int64_t valid_below, void* q, float* scale_out, cudaStream_t st) {
   using namespace moe;
   const int grid = grid_for((rows + 7) / 8, 8);
-#define MOE_RQ(K, SIN) rowwise_quant_kernel<T, K><<<grid, 256, 0, st>>>((const T*)x, rows, cols, SIN, row_ids, valid_below, (uint8_t*)q, scale_out)
+  // whole 16-byte pieces: a warp holds up to 2048 columns of its row in registers, a CTA up to 8192
+  const bool vec = sizeof(T) == 2 && cols % 8 == 0 && cols <= 8192 && (((uintptr_t)x | (uintptr_t)q) & 15) == 0;
+#define MOE_RQ(K, SIN)                                                                                              \
+  do {                                                                                                              \
+    bool done = false;                                                                                              \
+    if constexpr (sizeof(T) == 2) {                                                                                 \
+      if (vec && cols <= 2048) {                                                                                    \
+        rowwise_quant_vec_kernel<T, K, 32, 8><<<grid, 256, 0, st>>>((const T*)x, rows, (int)cols, SIN, row_ids,     \
+                                                                    valid_below, (uint8_t*)q, scale_out);           \
+        done = true;                                                                                                \
+      } else if (vec) {                                                                                             \
+        rowwise_quant_vec_kernel<T, K, 256, 4><<<grid_for(rows, 8), 256, 0, st>>>(                                  \
+            (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, (uint8_t*)q, scale_out);                       \
+        done = true;                                                                                                \
+      }                                                                                                             \
+    }                                                                                                               \
+    if (!done)                                                                                                      \
+      rowwise_quant_kernel<T, K><<<grid, 256, 0, st>>>((const T*)x, rows, cols, SIN, row_ids, valid_below,          \
+                                                       (uint8_t*)q, scale_out);                                     \
+  } while (0)
   switch (kind) {
     case 0: MOE_RQ(0, nullptr); break;
     case 1: MOE_RQ(1, nullptr); break;

@@ -161,39 +161,30 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uin
         : "memory");
   }
 }
-template <bool FP8>
+// KIND of the single-CTA instructions: f16 / bf16 operands, e4m3 operands (fp32 accumulators), or
+// int8 operands with int32 accumulators
+constexpr int MMA_F16 = 0, MMA_F8 = 1, MMA_I8 = 2;
+#define MOE_MMA_ASM(KINDSTR, ACCC, ACCV)                                                  \
+  asm volatile(                                                                           \
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                  \
+      "tcgen05.mma.cta_group::1.kind::" KINDSTR " [%0], %1, %2, %3, p;\n\t}"              \
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), ACCC(ACCV)                       \
+      : "memory")
+template <int KIND>
 __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  if constexpr (FP8) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-        : "memory");
-  }
+  if constexpr (KIND == MMA_F8) MOE_MMA_ASM("f8f6f4", "r", acc);
+  else if constexpr (KIND == MMA_I8) MOE_MMA_ASM("i8", "r", acc);
+  else MOE_MMA_ASM("f16", "r", acc);
 }
 // The same with a compile-time accumulate flag: no predicate has to be computed at run time.
-template <bool FP8, bool ACC>
+template <int KIND, bool ACC>
 __device__ __forceinline__ void tc_mma_const(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
-  if constexpr (FP8) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0)
-        : "memory");
-  }
+  constexpr int acc = ACC ? 1 : 0;
+  if constexpr (KIND == MMA_F8) MOE_MMA_ASM("f8f6f4", "n", acc);
+  else if constexpr (KIND == MMA_I8) MOE_MMA_ASM("i8", "n", acc);
+  else MOE_MMA_ASM("f16", "n", acc);
 }
+#undef MOE_MMA_ASM
 // Packed fp32 pair FMA: d = a * b + d on two lanes of a 64-bit register pair.  Half the issue
 // slots of two scalar FMAs, which matters for warps that share a scheduler with the thread
 // that feeds the tensor core.

@@ -76,6 +76,8 @@ def _choose_kernel(mode, act_dtype, H, I, numel, num_experts):
         return KERNEL_GENERIC
     wide, pair = _policy("FLAGGEMS_B200_TC_WIDE"), _policy("FLAGGEMS_B200_TC_PAIR")
     pair_wide = _policy("FLAGGEMS_B200_TC_PAIR_WIDE")
+    if mode in (_lib.MODE_FP8_ROW, _lib.MODE_INT8_ROW):
+        return KERNEL_TC  # one-byte operands accumulated over the whole K loop, scales in the epilogue
     if mode == _lib.MODE_W8A16:
         return KERNEL_TC  # int8 weights widened in shared memory, one CTA per 128-row block
     if pair_wide == "on" and mode == _lib.MODE_HALF:
@@ -109,7 +111,7 @@ def _sorted_output(mode, kernel, numel, num_experts) -> bool:
     """GEMM2 of the 128-row tensor-core kernel writes its rows in sorted order through a staged tile and
     TMA stores (FP8 block scales and half precision) when experts own enough rows for the epilogue to
     matter: from 64 rows per expert on.  FLAGGEMS_B200_TMA_OUT = 0/1 forces it off/on."""
-    if kernel != KERNEL_TC or mode not in (_lib.MODE_FP8_BLOCK, _lib.MODE_HALF):
+    if kernel != KERNEL_TC or mode == _lib.MODE_W8A16:
         return False
     force = _policy("FLAGGEMS_B200_TMA_OUT")
     if force != "auto":
@@ -120,7 +122,7 @@ def _sorted_output(mode, kernel, numel, num_experts) -> bool:
 def _tc_eligible(mode: int, act_dtype: torch.dtype, H: int, I: int) -> bool:
     if act_dtype not in (torch.bfloat16, torch.float16):
         return False
-    if mode == _lib.MODE_FP8_BLOCK:
+    if mode in (_lib.MODE_FP8_BLOCK, _lib.MODE_FP8_ROW, _lib.MODE_INT8_ROW):
         return H % 128 == 0 and I % 128 == 0
     if mode in (_lib.MODE_HALF, _lib.MODE_W8A16):
         return H % 64 == 0 and I % 128 == 0
@@ -336,8 +338,8 @@ def route_pipeline(a_rows, a_scales_t, w1, w2, route_weight, topk_ids, *, mode, 
     act_code = _lib.dtype_code(act_dtype)
     if use_tensor_cores is None:
         kernel = _choose_kernel(mode, act_dtype, H, I, numel, global_num_experts)
-        if act_fn[0] != _lib.ACT_SILU or mode in (_lib.MODE_FP8_ROW, _lib.MODE_INT8_ROW):
-            # activations other than SiLU and the row-scaled W8A8 modes run on the generic kernel
+        if act_fn[0] != _lib.ACT_SILU:
+            # activations other than SiLU run on the generic kernel
             kernel = KERNEL_GENERIC
     else:
         kernel = int(use_tensor_cores)
@@ -395,14 +397,14 @@ def route_pipeline(a_rows, a_scales_t, w1, w2, route_weight, topk_ids, *, mode, 
     act_in = act
     if row_scaled:
         # quantise the intermediate (sorted rows) the way the mode says: one scale per row, or one for
-        # the whole tensor (dynamic: over the occupied rows only; padding rows hold stale bytes)
+        # the whole tensor; occupied rows only (padding rows hold stale bytes)
         kind, static = row_quant
         act_in = torch.empty((rows_cap, I), dtype=torch.int8 if mode == _lib.MODE_INT8_ROW else torch.float8_e4m3fn,
                              device=dev)
         per_row = kind in (0, 1)
         sc = torch.empty(rows_cap if per_row else 1, dtype=torch.float32, device=dev)
         _lib.check(L.moe_rowwise_quant(act.data_ptr(), act_code, rows_cap, I, kind, _lib.ptr(static),
-                                       sorted_ids.data_ptr() if kind == 3 else None, numel, act_in.data_ptr(),
+                                       sorted_ids.data_ptr(), numel, act_in.data_ptr(),
                                        sc.data_ptr(), st))
         act_scales = sc if per_row else sc.expand(rows_cap).contiguous()
         mark("quant2")

@@ -244,8 +244,8 @@ int moe_gemm1(int mode, int act_dtype, const void* a, int a_sorted, const float*
  * (min(gate, limit) * sigmoid(alpha * gate) * (clamp(up, -limit, limit) + beta) on the gate | up halves,
  * src/flaggems_vllm/ops/fused_moe.py:733-773).  The row-scaled modes MOE_MODE_FP8_ROW / MOE_MODE_INT8_ROW
  * (per-tensor and per-token W8A8, src/flaggems_vllm/ops/fused_moe.py:853-1010, scales applied to the
- * finished dot product as in :1894-1925) and every activation other than SiLU are served by the
- * generic kernel (use_tensor_cores = 0): a [num_tokens, H] in e4m3 / int8, a_scales_t [num_tokens]
+ * finished dot product as in :1894-1925) take kernels 0 and 1 (1: H and I multiples of 128); every activation
+ * other than SiLU takes the generic kernel (use_tensor_cores = 0).  Row-scaled: a [num_tokens, H] in e4m3 / int8, a_scales_t [num_tokens]
  * (one per row), w1_scale [E, 2I]; the intermediate is written in the activation dtype, unquantised.
  * In moe_gemm2 the same modes take act_scales_t [rows_cap] and w2_scale [E, H].
  */

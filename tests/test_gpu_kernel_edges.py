@@ -1,0 +1,58 @@
+"""The newer kernels at the sizes where they can go wrong: edges of tiles, remainders, the smallest and the
+largest of the range that their dispatch rule sends them."""
+
+import pytest
+import torch
+
+import flaggems_vllm_b200 as fg
+from flaggems_vllm_b200 import _lib, testing as T
+from oracle import moe_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _route(M, E, k, seed=5):
+    logits, _ = T.make_router_inputs(M, E, DEV, seed=seed)
+    w, ids = torch.topk(torch.softmax(logits, -1), k, dim=-1)
+    return (w / w.sum(-1, keepdim=True)).contiguous(), ids.to(torch.int32).contiguous()
+
+
+def _parity(out, ref, what):
+    assert _lib.read_status() == 0
+    assert O.rel_l2(out.float(), ref) < 1e-2 and O.cosine(out.float(), ref) > 0.9999, what
+
+
+@pytest.mark.parametrize("fmt", ["fp8", "int8"])
+@pytest.mark.parametrize("M,E,k,H,I", [(1, 8, 2, 256, 128), (129, 4, 2, 1152, 384), (700, 4, 2, 256, 640)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_row_scaled_tensor_core_layer(fmt, M, E, k, H, I, dtype):
+    x = T.make_activations(M, H, DEV, dtype=dtype)
+    w1f = torch.randn(E, 2 * I, H, device=DEV) * H**-0.5
+    w2f = torch.randn(E, H, I, device=DEV) * I**-0.5
+    tw, ti = _route(M, E, k)
+    top = 448.0 if fmt == "fp8" else 127.0
+    s1, s2 = w1f.abs().amax(-1) / top, w2f.abs().amax(-1) / top
+    cast = (lambda w: w.to(torch.float8_e4m3fn)) if fmt == "fp8" else (lambda w: w.round().to(torch.int8))
+    w1, w2 = cast(w1f / s1[..., None]), cast(w2f / s2[..., None])
+    kw = {"use_fp8_w8a8": True} if fmt == "fp8" else {"use_int8_w8a8": True}
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti, per_channel_quant=True, w1_scale=s1, w2_scale=s2, **kw)
+    _parity(out, O.fused_moe_row_scaled_oracle(x, w1, w2, s1, s2, tw, ti, fmt=fmt, per_token=True), (fmt, M))
+
+
+@pytest.mark.parametrize("cols", [8, 768, 2048, 2056, 7168, 8192, 8200])
+def test_rowwise_quant_widths(cols):
+    """A warp per row up to 2048 columns, a CTA per row up to 8192, the scalar kernel beyond; padding rows skipped."""
+    x = (torch.randn(11, cols, device=DEV) * 3).to(torch.bfloat16)
+    x[4] = 0
+    ids = torch.arange(11, dtype=torch.int32, device=DEV)
+    ids[7] = 11
+    for kind, oracle in ((0, O.int8_per_token_quant_oracle), (1, O.fp8_per_token_quant_oracle)):
+        q = torch.full(x.shape, 77, dtype=torch.uint8, device=DEV)
+        sc = torch.full((11,), -1.0, device=DEV)
+        _lib.check(_lib.lib().moe_rowwise_quant(x.data_ptr(), _lib.dtype_code(x.dtype), 11, cols, kind, None,
+                                                ids.data_ptr(), 11, q.data_ptr(), sc.data_ptr(), _lib.stream_of(x)))
+        oq, os_ = oracle(x.cpu())
+        rows = [r for r in range(11) if r != 7]
+        assert torch.equal(q.cpu()[rows], oq.view(torch.uint8)[rows]) and torch.equal(sc.cpu()[rows], os_.reshape(-1)[rows])
+        assert bool((q[7] == 77).all()) and float(sc[7]) == -1.0
