@@ -239,6 +239,12 @@ __device__ __forceinline__ void tmem_wait64(uint32_t* a, uint32_t* b) {
                : MOE_RW8(a, 0), MOE_RW8(a, 8), MOE_RW8(a, 16), MOE_RW8(a, 24), MOE_RW8(b, 0), MOE_RW8(b, 8), MOE_RW8(b, 16),
                  MOE_RW8(b, 24)::"memory");
 }
+// One 32-column load and its wait.
+__device__ __forceinline__ void tmem_ld32_sync(uint32_t taddr, uint32_t* a) {
+  tmem_ld32_async(taddr, a);
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : MOE_RW8(a, 0), MOE_RW8(a, 8), MOE_RW8(a, 16), MOE_RW8(a, 24)::"memory");
+}
 #undef MOE_R8
 #undef MOE_RW8
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
@@ -355,13 +361,13 @@ static inline EncodeTiledFn get_encode() {
 // 2-D row-major [rows, cols] tensor, box = `box_bytes` of a row x box_rows rows.  128-byte
 // boxes use the 128-byte swizzle (tensor-core operand layout); narrower boxes land unswizzled.
 static inline int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t rows,
-                           uint64_t cols, uint32_t box_rows, bool weights, int box_bytes = 128) {
+                           uint64_t cols, uint32_t box_rows, bool weights, int box_bytes = 128, uint64_t ld = 0) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return fail(MOE_E_DRIVER, "cuTensorMapEncodeTiled is not available from the driver");
   if (((uintptr_t)base & 15) != 0) return fail(MOE_E_BADARG, "tensor-core GEMM: operand not 16-byte aligned");
-  if ((cols * elem_bytes) % 16 != 0) return fail(MOE_E_SHAPE, "tensor-core GEMM: row pitch must be a multiple of 16 bytes");
+  if (((ld != 0 ? ld : cols) * elem_bytes) % 16 != 0) return fail(MOE_E_SHAPE, "tensor-core GEMM: row pitch must be a multiple of 16 bytes");
   cuuint64_t gdim[2] = {cols, rows};
-  cuuint64_t gstr[1] = {cols * (uint64_t)elem_bytes};
+  cuuint64_t gstr[1] = {(ld != 0 ? ld : cols) * (uint64_t)elem_bytes};  // ld: row pitch in elements
   cuuint32_t box[2] = {(cuuint32_t)(box_bytes / elem_bytes), box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(m, dt, 2, const_cast<void*>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -5,7 +5,7 @@ Mirrors ``router_gemm`` (src/flaggems_vllm/ops/router_gemm.py:207-237) and
 (src/flaggems_vllm/ops/fp32_router_gemm.py:17-145): same names, argument meaning
 and error behaviour.  Both kernels of ``csrc/router_gemm.cu`` are deterministic: a
 row-streaming fp32 kernel for decode-sized batches (and for every dtype pair), a
-tensor-core (warp MMA, fp32 accumulate) kernel for half-precision batches above 320 rows.
+tcgen05 kernel (fp32 accumulate, K split over a cluster) for half-precision batches above 4 rows.
 No library GEMM is called.  ``router_gemm_grouped_topk`` fuses the GEMM with the
 group-limited routing for decode batches (no counterpart in the reference, which runs the
 two ops back to back).
@@ -18,11 +18,12 @@ import logging
 import torch
 
 from . import _lib
+from .routing import grouped_topk
 
 logger = logging.getLogger(__name__)
 
-# up to this many rows the fused GEMM + routing kernel (one CTA per token) beats two launches
-FUSED_MAX_ROWS = 64
+# half-precision batches above this many rows go through the tcgen05 router GEMM (kRowStreamMax of csrc/router_gemm.cu)
+ROW_STREAM_MAX = 4
 
 
 def _launch(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -33,8 +34,9 @@ def _launch(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         return out
     xc = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
     wc = weight if weight.is_contiguous() else weight.contiguous()
-    _lib.check(_lib.lib().moe_router_gemm(xc.data_ptr(), _lib.dtype_code(xc.dtype), xc.stride(0), wc.data_ptr(),
-                                          _lib.dtype_code(wc.dtype), M, N, K, out.data_ptr(), _lib.stream_of(x)))
+    _lib.check(_lib.lib().moe_router_gemm_ex(
+        xc.data_ptr(), _lib.dtype_code(xc.dtype), xc.stride(0), wc.data_ptr(), _lib.dtype_code(wc.dtype), M, N, K,
+        out.data_ptr(), _lib.status_word(x.device).data_ptr(), _lib.stream_of(x)))
     return out
 
 
@@ -56,10 +58,11 @@ def router_gemm(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 def router_gemm_grouped_topk(x: torch.Tensor, weight: torch.Tensor, n_group: int, topk_group: int, topk: int,
                              renormalize: bool, routed_scaling_factor: float, bias: torch.Tensor,
                              scoring_func: int = 0, return_logits: bool = False):
-    """``grouped_topk(router_gemm(x, weight), ...)`` in one launch: hidden states [M, K] and router
-    weight [E, K] in, (topk_weights fp32 [M, topk], topk_ids int32 [M, topk]) out; the logits stay on
-    chip (``return_logits=True`` also returns a copy).  Results equal the two separate calls bit for
-    bit.  Meant for decode batches (one CTA per token); any M is accepted."""
+    """``grouped_topk(router_gemm(x, weight), ...)``: hidden states [M, K] and router weight [E, K] in,
+    (topk_weights fp32 [M, topk], topk_ids int32 [M, topk]) out (``return_logits=True`` also returns the
+    logits).  Results equal the two separate calls bit for bit.  Up to ``ROW_STREAM_MAX`` tokens it is one
+    launch (one CTA per token, the logits stay on chip); half-precision batches beyond take the two
+    kernels of the separate calls, whose GEMM reads the weights once per 128 tokens instead of per token."""
     logger.debug("GEMS ROUTER GEMM + GROUPED TOPK")
     if x.ndim != 2 or weight.ndim != 2 or x.shape[1] != weight.shape[1]:
         raise ValueError("router_gemm_grouped_topk expects x [M, K] and weight [E, K]")
@@ -70,6 +73,11 @@ def router_gemm_grouped_topk(x: torch.Tensor, weight: torch.Tensor, n_group: int
     E = weight.shape[0]
     if bias.numel() != E:
         raise ValueError(f"bias length {bias.numel()} does not match the expert count {E}")
+    if M > ROW_STREAM_MAX and x.dtype == weight.dtype and x.dtype in (torch.bfloat16, torch.float16) and K % 8 == 0:
+        logits = _launch(x, weight)
+        tw, ti = grouped_topk(logits, n_group, topk_group, topk, renormalize, routed_scaling_factor, bias.float(),
+                              scoring_func)
+        return (tw, ti, logits) if return_logits else (tw, ti)
     xc = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
     wc = weight if weight.is_contiguous() else weight.contiguous()
     b = bias.to(torch.float32).contiguous()

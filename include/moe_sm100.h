@@ -166,6 +166,9 @@ int moe_widen_int8(const void* src, void* dst, int dst_dtype, int64_t n, void* s
  */
 int moe_router_gemm(const void* x, int x_dtype, int64_t x_ld, const void* w, int w_dtype, int64_t M, int N, int K,
                     float* out, void* stream);
+/* The same with the device status word of the kernels that wait on barriers (may be NULL). */
+int moe_router_gemm_ex(const void* x, int x_dtype, int64_t x_ld, const void* w, int w_dtype, int64_t M, int N, int K,
+                       float* out, int32_t* status, void* stream);
 
 /*
  * Router GEMM fused with the group-limited routing, for decode batches: one launch takes the hidden

@@ -56,3 +56,29 @@ def test_rowwise_quant_widths(cols):
         rows = [r for r in range(11) if r != 7]
         assert torch.equal(q.cpu()[rows], oq.view(torch.uint8)[rows]) and torch.equal(sc.cpu()[rows], os_.reshape(-1)[rows])
         assert bool((q[7] == 77).all()) and float(sc[7]) == -1.0
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 256, 7168), (65, 256, 7168), (128, 8, 64), (129, 33, 72), (200, 256, 7168), (257, 40, 520),
+                                   (4097, 128, 2048), (640, 1024, 512)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_router_gemm_tensor_core_tiles(M, N, K, dtype):
+    """Row, column and K remainders of the tcgen05 tiles, every split of K over a cluster that the rule picks."""
+    x = T.make_activations(M, K, DEV, seed=M, dtype=dtype)
+    w = torch.randn((N, K), generator=torch.Generator(device=DEV).manual_seed(N), device=DEV).to(dtype)
+    out = fg.router_gemm(x, w)
+    ref = x.double() @ w.double().t()
+    assert float((out.double() - ref).norm() / ref.norm()) < 4e-6 and _lib.read_status() == 0
+    assert torch.equal(out, fg.router_gemm(x, w))
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+def test_router_gemm_row_tiles_share_one_order(M):
+    """The decode kernel's tiles differ in shape only: row m of a batch equals the one-row call, bit for bit."""
+    x = T.make_activations(M, 2048, DEV, seed=M)
+    w = torch.randn((130, 2048), device=DEV).to(torch.bfloat16)
+    out = fg.router_gemm(x, w)
+    for m in range(M):
+        assert torch.equal(out[m:m + 1], fg.router_gemm(x[m:m + 1], w))
+    x32 = T.make_activations(37, 2048, DEV, seed=M, dtype=torch.float32)  # 8-row tiles, 1 and 4 columns wide
+    out = fg.router_gemm(x32, w)
+    assert torch.equal(out[:9], fg.router_gemm(x32[:9], w)) and torch.equal(out[36:], fg.router_gemm(x32[36:], w))
