@@ -349,7 +349,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           MOE_TR(0, kb, 2);
         }
       }
-    } else if (warp == 1 && cr == 0 && (!PAIR || lane == 0)) {
+    } else if (warp == 1 && cr == 0) {
       // ------------------------------------------------------------ MMA issuer (pair: leader only)
       constexpr uint32_t idesc = IDesc<FMT, AT, PAIR>::value;
       [[maybe_unused]] uint32_t it = 0;
@@ -412,6 +412,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       } else {
+      const bool leader = elect_lane();
       for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
         MOE_TILE_COORDS(tile)
         if (e < 0 || e >= P.E) continue;
@@ -430,6 +431,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if constexpr (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async writes -> tensor core reads
           tc_fence_after();
           const uint64_t bdesc = make_smem_desc(smem_u32(sB + (size_t)s * B_LOCAL_BYTES));
+          if (leader) {
 #pragma unroll
           for (int j = 0; j < RB; ++j) {
             const uint64_t adesc = make_smem_desc(smem_u32(sA + (size_t)s * A_LOCAL_BYTES + j * A_STAGE_BYTES));
@@ -442,10 +444,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
           }
           tc_commit_pair(&aux->empty[s]);
-          if (FP8 || kb == KB - 1) {
-            tc_commit_pair(&aux->tmem_full[a]);
-            ++acc_it;
+          if (FP8 || kb == KB - 1) tc_commit_pair(&aux->tmem_full[a]);
           }
+          if (FP8 || kb == KB - 1) ++acc_it;
         }
       }
       }
@@ -736,7 +737,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           amax = fmaxf(amax, x[(1 - h) * BM + row]);
           const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
           const float inv_s = 1.0f / s;  // one reciprocal per row instead of 64 divisions
-          if (row_ok) {
+          if (row_ok || SORTED) {
             uint4 pieces[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {

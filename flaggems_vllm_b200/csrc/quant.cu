@@ -276,9 +276,12 @@ __global__ void gather_rows_kernel(const uint4* __restrict__ x, const int32_t* _
   const int64_t npp = min((int64_t)num_post_pad[0], rows_cap);
   for (int64_t p = warp; p < npp; p += warps) {
     const int64_t sid = sorted_ids[p];
-    if (sid < 0 || sid >= numel) continue;
-    const uint4* src = x + (sid / topk) * row_vec;
     uint4* dst = out + p * row_vec;
+    if (sid < 0 || sid >= numel) {
+      for (int64_t c = lane; c < row_vec; c += 32) dst[c] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    const uint4* src = x + (sid / topk) * row_vec;
     int64_t c = lane;
     for (; c + 96 < row_vec; c += 128) {  // four loads in flight
       const uint4 v0 = src[c], v1 = src[c + 32], v2 = src[c + 64], v3 = src[c + 96];
