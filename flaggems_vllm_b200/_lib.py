@@ -77,6 +77,11 @@ SYMBOLS = {
                                  c_void_p, c_void_p]),
     "moe_sum": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int, c_int64, c_void_p, c_int, c_int, c_void_p,
                         c_void_p, c_void_p]),
+    "moe_layer_workspace": (c_int, [c_int, c_int, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "moe_layer": (c_int, [c_int, c_int, c_void_p, c_int64, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                          c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                          c_float, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                          c_void_p]),
     "moe_silu_and_mul": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_void_p]),
     "moe_silu_and_mul_grad": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_void_p]),
     "moe_sum_ld": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int64, c_int, c_int64, c_void_p, c_int, c_int, c_void_p,
@@ -87,7 +92,7 @@ _lib = None
 _status = {}
 # calls of entry points that enqueue a kernel (bench.py reports the count of its timed region)
 LAUNCHES = 0
-_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_set_wait_limit_ns")
+_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_set_wait_limit_ns")
 
 
 class _Counted:

@@ -2,9 +2,40 @@
 #include <cstdarg>
 #include <cstdio>
 
+#include <atomic>
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "moe_common.cuh"
 
 namespace moe {
+
+int allow_smem(const void* kernel, int bytes) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;  // one entry per kernel and device
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({kernel, dev})) return 0;
+  const cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (ce != cudaSuccess) return fail((int)ce, "shared memory attribute (%d bytes): %s", bytes, cudaGetErrorString(ce));
+  done.insert({kernel, dev});
+  return 0;
+}
+
+int sm_count() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 static thread_local char g_err[512] = "";
 static unsigned long long g_wait_limit_ns = 2000000000ull;
 unsigned long long wait_limit_ns() { return g_wait_limit_ns; }

@@ -109,6 +109,8 @@ struct Params {
   const uint8_t* a_rows;    // GEMM1: activations [tokens, K] in token order (gathered by cp.async)
   const float* a_scales_t;  // [K/128, a_scale_ld]        (FP8)
   const float* w_scale;     // FP8: [E, rows_w/128, K/128]; half mode: optional per-row scale [E, rows_w]
+  const int4* tiles;        // route plan (plan.cu): one entry {row0, rows | occupied rows << 16, expert, -} per 128-row block;
+                            // null: the blocks are described by expert_ids and sorted_ids
   const int32_t* expert_ids;
   const int32_t* sorted_ids;
   const int32_t* num_post_pad;
@@ -130,6 +132,7 @@ struct Params {
   int n_tiles;  // column tiles per align block
   int group_m;  // align blocks per group of the tile order
   int w_row0;   // GEMM2 over a window of the output columns: first weight row (output column) of the window
+  bool all_rows;    // route plan: fetch whole 128-row blocks of A (their padding rows are zero) instead of the occupied rows
   bool wide_store;  // the output is 32-byte aligned: rows are written with 32-byte stores
 #ifdef MOE_TC_TRACE
   long long* trace;  // [4 roles][64 K blocks][8 events] cycle stamps of CTA 0, third tile (experiment builds)
@@ -211,7 +214,8 @@ __device__ __forceinline__ int box_row(int nt, int c, int cr, int Nout) {
 template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_out, const Params P) {
+               const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_a16,
+               const __grid_constant__ CUtensorMap map_a8, const Params P) {
   constexpr bool FP8 = FMT == FMT_FP8, ROW = FMT == FMT_FP8ROW || FMT == FMT_I8ROW;
   constexpr bool BYTE = FMT != FMT_HALF;  // one-byte operands
   constexpr int KIND = FMT == FMT_HALF ? MMA_F16 : (FMT == FMT_I8ROW ? MMA_I8 : MMA_F8);
@@ -258,6 +262,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     nt = within / gsz;
     blk = first + within - nt * gsz;
   };
+  auto expert_of = [&](int blk) -> int { return P.tiles != nullptr ? P.tiles[blk].z : P.expert_ids[blk]; };
   // tile -> expert_ids index (blk), this CTA's 128-row block (mb), column tile (nt).  The expert of
   // the NEXT tile is fetched while the current one is worked on: a tile starts without waiting
   // for a global load (every role walks the same tile list with its own copy of e_next).
@@ -270,18 +275,26 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if ((tile) + tile_step < total_tiles) {                 \
     int blk2, nt2;                                        \
     tile_blk_nt((tile) + tile_step, blk2, nt2);           \
-    e_next = P.expert_ids[blk2];                          \
+    e_next = expert_of(blk2);                             \
   }
   int e_next = -1;
   if (tile0 < total_tiles) {
     int blk0, nt0;
     tile_blk_nt(tile0, blk0, nt0);
-    e_next = P.expert_ids[blk0];
+    e_next = expert_of(blk0);
   }
 
 #ifdef MOE_TC_TRACE
   if (threadIdx.x == 0 && blockIdx.x == 0 && P.trace) { P.trace[2048] = clock64(); P.trace[2049] = (long long)now_ns(); P.trace[2052] = total_tiles; }
 #endif
+  if constexpr (!GATHER && !PAIR && RB == 1) {
+    // Route plan, occupied rows only: the other rows of a stage are multiplied all the same.  They start as zeros and
+    // stay zeros until a larger tile comes by, and zeros cost the tensor cores less energy than stale bytes.
+    if (P.tiles != nullptr && !P.all_rows) {
+      for (int i = threadIdx.x; i < STAGES * A_LOCAL_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(sA)[i] = make_uint4(0, 0, 0, 0);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&aux->full[s], GATHER ? 1 + GATHER_THREADS : (FP8 ? 1 + SCALE_THREADS : 1));
@@ -326,6 +339,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (e < 0 || e >= P.E) continue;
         [[maybe_unused]] const int row0 = mb * BM;
         const int wrow0 = e * P.rows_w + P.w_row0;
+        [[maybe_unused]] int a_rows = RB * BM;
+        if constexpr (!GATHER && !PAIR && RB == 1) {
+          if (P.tiles != nullptr && !P.all_rows) a_rows = ((P.tiles[blk].y >> 16) + 7) & ~7;
+        }
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -336,7 +353,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if constexpr (GATHER) {
             mbar_expect_tx(&aux->full[s], B_LOCAL_BYTES);  // A rows arrive by cp.async (warps 2-3)
           } else {
-            mbar_expect_tx(&aux->full[s], A_LOCAL_BYTES + B_LOCAL_BYTES);
+            mbar_expect_tx(&aux->full[s], (uint32_t)a_rows * 128 + B_LOCAL_BYTES);
+            if (a_rows < RB * BM) {  // route plan, few rows: the rest of the stage keeps stale bytes, its results are never stored
+              uint8_t* dst = sA + (size_t)s * A_LOCAL_BYTES;
+              int r = 0;
+              for (; a_rows - r >= 16; r += 16) tma_load_2d(&map_a16, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
+              if (r < a_rows) tma_load_2d(&map_a8, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
+            } else
 #pragma unroll
             for (int j = 0; j < RB; ++j)
               tma_load_2d(&map_a, &aux->full[s], sA + (size_t)s * A_LOCAL_BYTES + j * A_STAGE_BYTES, kb * KBE,
@@ -440,7 +463,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int k4 = 0; k4 < 4; ++k4) {
               // 32 bytes of K per instruction: start address advances by 32 B >> 4
               const uint32_t accum = FP8 ? (k4 > 0) : (kb > 0 || k4 > 0);
-              tc_mma_pair<FP8>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, accum);
+              tc_mma_pair<KIND>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, accum);
             }
           }
           tc_commit_pair(&aux->empty[s]);
@@ -586,9 +609,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       nx_sid = P.numel;
       if (t < total_tiles) {
         tile_blk_nt(t, nx_blk, nx_nt);
-        nx_e = P.expert_ids[nx_blk];
         const int64_t pn = (int64_t)(UNIT * nx_blk + RB * cr) * BM + row;
-        if (pn < P.rows_cap) nx_sid = (int64_t)P.sorted_ids[pn];
+        if (P.tiles != nullptr) {  // rows leave in sorted order, weighted by the combine
+          const int4 d = P.tiles[nx_blk];
+          nx_e = d.z;
+          if (row < (d.y >> 16)) nx_sid = pn;
+        } else {
+          nx_e = P.expert_ids[nx_blk];
+          if (pn < P.rows_cap) nx_sid = (int64_t)P.sorted_ids[pn];
+        }
       }
     };
     prefetch_tile(tile0);
@@ -737,7 +766,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           amax = fmaxf(amax, x[(1 - h) * BM + row]);
           const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
           const float inv_s = 1.0f / s;  // one reciprocal per row instead of 64 divisions
-          if (row_ok || SORTED) {
+          if (row_ok || (SORTED && P.tiles != nullptr && P.all_rows)) {  // zero rows stay zero for GEMM2
             uint4 pieces[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
@@ -778,7 +807,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           uint8_t* dst = s_out + (size_t)(2 * h + (c >> 3)) * (BM * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4);
           *reinterpret_cast<uint4*>(dst) = piece;
         }
-        if (row_ok && h == 0) P.inv[sid] = (int32_t)p;
+        if (row_ok && h == 0 && P.inv != nullptr) P.inv[sid] = (int32_t)p;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> TMA reads
         asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory");
         if (threadIdx.x == 128) {
@@ -838,18 +867,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // ------------------------------------------------------------------ host side
 template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P, int grid, cudaStream_t st,
-                  const CUtensorMap* mo = nullptr) {
+                  const CUtensorMap* mo = nullptr, const CUtensorMap* ms = nullptr) {
   auto kern = tc_gemm_kernel<FMT, AT, GEMM1, PAIR, RB, SORTED, TMAOUT>;
   constexpr size_t smem = smem_bytes<PAIR, RB, TMAOUT>();
-  cudaFuncAttributes fa;
-  cudaError_t ce = cudaFuncGetAttributes(&fa, kern);
-  if (ce != cudaSuccess) return fail((int)ce, "tensor-core GEMM: cudaFuncGetAttributes: %s", cudaGetErrorString(ce));
+  static const int regs = [&] {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : 0;
+  }();
   // see LAUNCH_REGS: refuse to launch rather than let setmaxnreg.inc wait for registers that do not exist
-  if ((THREADS - EPI_THREADS) * PRODUCER_REGS + EPI_THREADS * CONSUMER_REGS > THREADS * fa.numRegs)
-    return fail(MOE_E_DRIVER, "tensor-core GEMM: kernel was built with %d registers per thread, %d needed",
-                fa.numRegs, LAUNCH_REGS);
-  ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (ce != cudaSuccess) return fail((int)ce, "tensor-core GEMM: shared memory attribute: %s", cudaGetErrorString(ce));
+  if ((THREADS - EPI_THREADS) * PRODUCER_REGS + EPI_THREADS * CONSUMER_REGS > THREADS * regs)
+    return fail(MOE_E_DRIVER, "tensor-core GEMM: kernel was built with %d registers per thread, %d needed", regs, LAUNCH_REGS);
+  const int rc = allow_smem((const void*)kern, (int)smem);
+  if (rc) return rc;
+  cudaError_t ce;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(THREADS);
@@ -862,7 +892,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P,
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ce = cudaLaunchKernelEx(&cfg, kern, ma, mb, mo != nullptr ? *mo : ma, P);
+  ce = cudaLaunchKernelEx(&cfg, kern, ma, mb, mo != nullptr ? *mo : ma, ms != nullptr ? ms[0] : ma, ms != nullptr ? ms[1] : ma, P);
   if (ce != cudaSuccess) return fail((int)ce, "tensor-core GEMM launch: %s", cudaGetErrorString(ce));
   return check_launch(GEMM1 ? "gemm1 (tcgen05)" : "gemm2 (tcgen05)");
 }
@@ -935,6 +965,7 @@ int tc_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
 
   Params P;
   if (sorted && (topk <= 0 || a_tokens * topk != numel)) return fail(MOE_E_BADARG, "tensor-core GEMM1: tokens * topk != numel");
+  P.tiles = nullptr; P.all_rows = true;
   P.a_rows = (const uint8_t*)a; P.a_scale_ld = (gemm1 && !sorted) ? a_tokens : rows_cap; P.topk = gemm1 ? topk : 1;
   P.a_scales_t = a_scales_t; P.w_scale = w_scale; P.expert_ids = expert_ids; P.sorted_ids = sorted_ids;
   P.num_post_pad = npp; P.route_weight = route_weight; P.out = out; P.out_scales_t = out_scales_t; P.inv = nullptr;
@@ -1012,6 +1043,48 @@ int tc_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
   return act_dtype == MOE_BF16 ? MOE_TC_LAUNCH(FMT_HALF, __nv_bfloat16) : MOE_TC_LAUNCH(FMT_HALF, __half);
 #undef MOE_TC_LAUNCH
 #undef MOE_TC_LAUNCH2
+}
+
+// The same GEMMs over the blocks of a route plan made with 128-row tiles (plan.cu): A rows (GEMM1: scattered token
+// rows, GEMM2: the intermediate) in sorted order, results in sorted order.  all_rows: the padding rows of A are zero,
+// fetch whole blocks.
+int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
+                 const void* tiles, const int32_t* rows, int64_t numel, int64_t rows_cap, int E, int K, int Nout, void* out,
+                 float* out_scales_t, const float* row_weight, bool all_rows, bool staged, int32_t* status, cudaStream_t st) {
+  using namespace tc;
+  const bool fp8 = mode == MOE_MODE_FP8_BLOCK;
+  const int eb = fp8 ? 1 : 2, rows_w = gemm1 ? 2 * Nout : Nout;
+  if ((int64_t)E * rows_w >= (1ll << 31) || rows_cap >= (1ll << 31)) return fail(MOE_E_TOOBIG, "tensor-core GEMM: extent exceeds int32 coordinates");
+  const CUtensorMapDataType half_t = act_dtype == MOE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const CUtensorMapDataType dt = fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : half_t;
+  CUtensorMap ma, mb, mo, ms[2];
+  int rc = make_map(&ma, a, dt, eb, (uint64_t)rows_cap, (uint64_t)K, BM, false);
+  if (!rc) rc = make_map(&ms[0], a, dt, eb, (uint64_t)rows_cap, (uint64_t)K, 16, false);
+  if (!rc) rc = make_map(&ms[1], a, dt, eb, (uint64_t)rows_cap, (uint64_t)K, 8, false);
+  if (!rc) rc = make_map(&mb, w, dt, eb, (uint64_t)E * rows_w, (uint64_t)K, gemm1 ? 128 : 256, true);
+  if (!rc && staged) rc = make_map(&mo, out, half_t, 2, (uint64_t)rows_cap, (uint64_t)Nout, BM, false);
+  if (rc) return rc;
+  Params P = {};
+  P.a_rows = (const uint8_t*)a; P.a_scale_ld = rows_cap; P.topk = 1;
+  P.a_scales_t = a_scales_t; P.w_scale = w_scale; P.tiles = (const int4*)tiles; P.all_rows = all_rows;
+  P.route_weight = row_weight; P.mul_weight = row_weight != nullptr;  // sorted order: row p's weight
+  P.num_post_pad = rows; P.out = out; P.out_scales_t = out_scales_t; P.status = status; P.wait_ns = wait_limit_ns();
+  P.numel = rows_cap; P.rows_cap = rows_cap; P.E = E; P.K = K; P.Nout = Nout; P.rows_w = rows_w;
+  P.n_tiles = gemm1 ? Nout / 128 : (Nout + BN - 1) / BN;
+  const int64_t gm = numel / E / BM + 1;
+  P.group_m = (int)(gm > 16 ? 16 : gm);
+  P.wide_store = ((uintptr_t)out & 31) == 0;
+  const int64_t cap_tiles = (rows_cap / BM) * (int64_t)P.n_tiles;
+  const int sms = sm_count();
+  const int grid = (int)(cap_tiles < sms ? cap_tiles : sms);
+#define MOE_TCP(F, T)                                                                                             \
+  (gemm1 ? launch<F, T, true, false, 1, true>(ma, mb, P, grid, st, nullptr, ms)                                   \
+         : (staged ? launch<F, T, false, false, 1, false, true>(ma, mb, P, grid, st, &mo, ms)                     \
+                   : launch<F, T, false, false, 1>(ma, mb, P, grid, st, nullptr, ms)))
+  if (fp8) return act_dtype == MOE_BF16 ? MOE_TCP(FMT_FP8, __nv_bfloat16) : MOE_TCP(FMT_FP8, __half);
+  if (mode == MOE_MODE_HALF) return act_dtype == MOE_BF16 ? MOE_TCP(FMT_HALF, __nv_bfloat16) : MOE_TCP(FMT_HALF, __half);
+#undef MOE_TCP
+  return fail(MOE_E_SHAPE, "tensor-core GEMM over a route plan: FP8 block scales and half precision");
 }
 
 }  // namespace moe

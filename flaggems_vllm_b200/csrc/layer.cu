@@ -1,0 +1,191 @@
+// The whole expert layer behind one call: route plan -> scatter -> GEMM1 -> GEMM2 -> combine.
+//
+// The launches of a decode step take a few microseconds each; made one by one from Python (a dozen allocations, a
+// ctypes call per launch) they cost the host more than the device.  Here the caller passes the workspaces and the
+// launches follow each other in native code.  No state is kept between calls.
+#include "moe_common.cuh"
+
+namespace moe {
+void plan_caps(int64_t numel, int E_local, int gran, int tile_rows, int64_t* rows_cap, int64_t* tiles_cap);
+bool plan_serves(int64_t numel, int E, int E_local);
+int plan_routes(const void* ids, int ids64, int64_t numel, int E, const int32_t* emap, int E_local, int gran, int tile_rows,
+                int32_t* row_index, int64_t rows_cap, void* tiles, int64_t tiles_cap, int32_t* counts, int32_t* status,
+                cudaStream_t st);
+int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,
+                        float* scales_t, cudaStream_t st);
+int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st);
+int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, cudaStream_t st);
+int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
+                 const void* tiles, const int32_t* rows, int64_t numel, int64_t rows_cap, int E, int K, int Nout, void* out,
+                 float* out_scales_t, const float* row_weight, bool all_rows, bool staged, int32_t* status, cudaStream_t st);
+int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_index, float* dst, cudaStream_t st);
+int combine_rows(const void* y, int dtype, const float* weight, const int32_t* row_index, int64_t M, int k, int64_t H, void* out,
+                 cudaStream_t st);
+int rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, const float* scale_in,
+                  const int32_t* row_ids, int64_t valid_below, const int32_t* indirect, void* q, float* scale_out, cudaStream_t st);
+bool wt_serves(int mode, int act_dtype, int H, int I);
+int wt_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
+            const void* tiles, int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K,
+            int Nout, void* out, int act_kind, float alpha, float beta, float limit, int32_t* status,
+            cudaStream_t st);
+
+namespace {
+// Which grouped GEMM serves the call and how the plan cuts the rows for it.
+struct Choice {
+  bool pair;        // gemm_wt.cu: weights as the M operand of a CTA pair; else gemm_tc.cu: 128 tokens as M
+  int gran, tile;   // row granule and most rows of a tile
+  bool zero_pad;    // gemm_tc.cu: zero the padding rows and fetch whole blocks
+  bool staged;      // gemm_tc.cu: GEMM2 leaves through staged TMA stores of whole tiles
+};
+
+bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
+  if (mode == MOE_MODE_FP8_BLOCK)
+    return act_kind == MOE_ACT_SILU && (act_dtype == MOE_BF16 || act_dtype == MOE_F16) && H % 128 == 0 && I % 128 == 0;
+  return wt_serves(mode, act_dtype, H, I);
+}
+
+Choice choose(int mode, int act_kind, int64_t numel, int E) {
+  const int64_t per_expert = numel / (E > 0 ? E : 1);
+  Choice c = {};
+  // FP8 block scales: tokens as M (gemm_wt.cu says why).  Half precision: up to 96 rows per expert the weights are
+  // streamed and both kernels wait for memory (the single-CTA kernel is a few per cent ahead); above, the pair's finer
+  // row padding counts (Mixtral shape, 1024 tokens: 1047 -> 887 us).
+  c.pair = mode != MOE_MODE_FP8_BLOCK && !(mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && per_expert < 96);
+  if (c.pair) {
+    c.gran = mode == MOE_MODE_INT8_ROW ? 32 : 16;  // kind::i8 on a pair takes multiples of 32
+    c.tile = 256;
+  } else {
+    c.gran = c.tile = 128;
+    c.zero_pad = per_expert >= 128;
+    c.staged = per_expert >= 64;
+  }
+  return c;
+}
+
+bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
+
+// Pieces of the four workspaces (plan; rows of GEMM1; intermediate; rows behind GEMM2), 256-byte aligned.
+struct Piece { int ws; int64_t at; };
+struct Layout {
+  int64_t rows_cap, tiles_cap;
+  Piece row_index, tiles, counts, row_weight, tmp_scales, x_rows, x_scales, tmp_q, act, act_q, act_scales, y;
+  int64_t bytes[4];
+};
+
+Layout layout(int mode, const Choice& c, int64_t M, int k, int E_local, int H, int I) {
+  Layout L = {};
+  const int64_t numel = M * k;
+  plan_caps(numel, E_local, c.gran, c.tile, &L.rows_cap, &L.tiles_cap);
+  auto take = [&](int ws, int64_t bytes) {
+    const Piece p = {ws, L.bytes[ws]};
+    L.bytes[ws] += (bytes + 255) / 256 * 256;
+    return p;
+  };
+  const bool byte = mode != MOE_MODE_HALF, row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
+  L.row_index = take(0, numel * 4);
+  L.tiles = take(0, L.tiles_cap * 16);
+  L.counts = take(0, 8);
+  L.row_weight = take(0, L.rows_cap * 4);
+  L.tmp_scales = take(0, row ? M * 4 : 0);
+  L.x_rows = take(1, L.rows_cap * H * (byte ? 1 : 2));
+  L.x_scales = take(1, block ? L.rows_cap * (H / 128) * 4 : (row ? L.rows_cap * 4 : 0));
+  L.tmp_q = take(1, row ? M * H : 0);
+  L.act = take(2, L.rows_cap * I * (block ? 1 : 2));
+  L.act_q = take(2, row ? L.rows_cap * I : 0);
+  L.act_scales = take(2, block ? L.rows_cap * (I / 128) * 4 : (row ? L.rows_cap * 4 : 0));
+  L.y = take(3, L.rows_cap * H * 2);
+  return L;
+}
+}  // namespace
+}  // namespace moe
+
+extern "C" int moe_layer_workspace(int mode, int act_dtype, int64_t num_tokens, int topk, int num_experts, int E_local, int H,
+                                   int I, int activation, int64_t* bytes) {
+  using namespace moe;
+  if (num_tokens <= 0 || num_tokens > 65535 || topk <= 0 || topk > 32 || E_local <= 0 || H <= 0 || I <= 0 || !bytes ||
+      !plan_serves(num_tokens * topk, num_experts, E_local) || !sizes_served(mode, act_dtype, H, I, activation))
+    return fail(MOE_E_SHAPE, "layer: mode, type or sizes are not served by this call");
+  const Layout L = layout(mode, choose(mode, activation, num_tokens * topk, num_experts), num_tokens, topk, E_local, H, I);
+  for (int i = 0; i < 4; ++i) bytes[i] = L.bytes[i];
+  return 0;
+}
+
+extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tokens, int topk, const void* topk_ids, int ids_int64,
+                         const float* topk_weights, const void* w1, const float* w1_scale, const void* w2, const float* w2_scale,
+                         void* out, int num_experts, const int32_t* expert_map, int E_local, int H, int I, int weight_on_input,
+                         int activation, float alpha, float beta, float limit, int quant_kind1, const float* quant_scale1,
+                         int quant_kind2, const float* quant_scale2, void* ws_plan, void* ws_x, void* ws_act, void* ws_y, int stages,
+                         int32_t* status, void* stream) {
+  using namespace moe;
+  const int64_t M = num_tokens, numel = M * topk;
+  int64_t bytes[4];
+  int rc = moe_layer_workspace(mode, act_dtype, M, topk, num_experts, E_local, H, I, activation, bytes);
+  if (rc) return rc;
+  if (!x || !topk_ids || !topk_weights || !w1 || !w2 || !out || !ws_plan || !ws_x || !ws_act || !ws_y)
+    return fail(MOE_E_BADARG, "layer: null pointer");
+  if (((uintptr_t)x | (uintptr_t)out | (uintptr_t)ws_plan | (uintptr_t)ws_x | (uintptr_t)ws_act | (uintptr_t)ws_y) & 15)
+    return fail(MOE_E_BADARG, "layer: rows and workspaces must be 16-byte aligned");
+  const bool row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
+  if ((row || block) && (!w1_scale || !w2_scale)) return fail(MOE_E_BADARG, "layer: weight scales missing");
+  cudaStream_t st = (cudaStream_t)stream;
+  const Choice c = choose(mode, activation, numel, num_experts);
+  const Layout L = layout(mode, c, M, topk, E_local, H, I);
+  void* const base[4] = {ws_plan, ws_x, ws_act, ws_y};
+  auto at = [&](const Piece& p) -> void* { return (uint8_t*)base[p.ws] + p.at; };
+  int32_t* row_index = (int32_t*)at(L.row_index);
+  int32_t* counts = (int32_t*)at(L.counts);
+  void* tiles = at(L.tiles);
+  float* x_scales = (float*)at(L.x_scales);
+  float* act_scales = (float*)at(L.act_scales);
+  float* row_weight = weight_on_input ? (float*)at(L.row_weight) : nullptr;
+  if (stages & 1) {
+    rc = plan_routes(topk_ids, ids_int64, numel, num_experts, expert_map, E_local, c.gran, c.tile,
+                     row_index, L.rows_cap, tiles, L.tiles_cap, counts, status, st);
+    if (rc) return rc;
+  }
+  if (stages & 2) {
+    if (block) {
+      rc = scatter_quant_group(x, act_dtype, M, H, topk, row_index, L.rows_cap, at(L.x_rows), x_scales, st);
+    } else if (row) {
+      const bool per_row = quant_kind1 == 0 || quant_kind1 == 1;
+      float* sc = (float*)at(L.tmp_scales);
+      rc = rowwise_quant(x, act_dtype, M, H, quant_kind1, quant_scale1, nullptr, 0, nullptr, at(L.tmp_q), sc, st);
+      if (!rc) rc = scatter_rows(at(L.tmp_q), M, H, topk, row_index, at(L.x_rows), st);
+      if (!rc) rc = scatter_floats(sc, numel, per_row ? topk : (int)numel, row_index, x_scales, st);
+    } else {
+      rc = scatter_rows(x, M, (int64_t)H * 2, topk, row_index, at(L.x_rows), st);
+    }
+    if (!rc && c.zero_pad) rc = zero_padding(tiles, L.tiles_cap, counts, (int64_t)H * (block ? 1 : 2), at(L.x_rows), st);
+    if (!rc && row_weight != nullptr) rc = scatter_floats(topk_weights, numel, 1, row_index, row_weight, st);
+    if (rc) return rc;
+  }
+  if (stages & 4) {
+    rc = c.pair ? wt_gemm(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
+                          L.rows_cap, E_local, H, I, at(L.act), activation, alpha, beta, limit, status, st)
+                : tc_gemm_plan(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, counts + 1, numel, L.rows_cap,
+                               E_local, H, I, at(L.act), act_scales, row_weight, c.zero_pad, c.staged, status, st);
+    if (rc) return rc;
+  }
+  const void* act = at(L.act);
+  if (row) {
+    act = at(L.act_q);
+    if (stages & 8) {
+      const bool per_row = quant_kind2 == 0 || quant_kind2 == 1;
+      float* sc = (float*)at(L.tmp_scales);
+      rc = rowwise_quant(at(L.act), act_dtype, numel, I, quant_kind2, quant_scale2, nullptr, 0, row_index, at(L.act_q),
+                         per_row ? act_scales : sc, st);
+      if (!rc && !per_row) rc = scatter_floats(sc, numel, (int)numel, row_index, act_scales, st);
+      if (rc) return rc;
+    }
+  }
+  if (stages & 16) {
+    rc = c.pair ? wt_gemm(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
+                          E_local, I, H, at(L.y), MOE_ACT_SILU, 0.0f, 0.0f, 0.0f, status, st)
+                : tc_gemm_plan(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, counts + 1, numel, L.rows_cap, E_local,
+                               I, H, at(L.y), nullptr, nullptr, c.zero_pad, c.staged, status, st);
+    if (rc) return rc;
+  }
+  if (stages & 32)
+    rc = combine_rows(at(L.y), act_dtype, weight_on_input ? nullptr : topk_weights, row_index, M, topk, H, out, st);
+  return rc;
+}

@@ -19,6 +19,10 @@ int check_launch(const char* what);
 // Limit, in nanoseconds, of every bounded barrier wait of the kernels launched from now on
 // (moe_set_wait_limit_ns; 2 s unless changed).
 unsigned long long wait_limit_ns();
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device (set once per device, remembered).
+int allow_smem(const void* kernel, int bytes);
+// Multiprocessors of the current device (remembered).
+int sm_count();
 
 template <typename T> struct ToF32;
 template <> struct ToF32<float> {

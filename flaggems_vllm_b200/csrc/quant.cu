@@ -276,12 +276,9 @@ __global__ void gather_rows_kernel(const uint4* __restrict__ x, const int32_t* _
   const int64_t npp = min((int64_t)num_post_pad[0], rows_cap);
   for (int64_t p = warp; p < npp; p += warps) {
     const int64_t sid = sorted_ids[p];
-    uint4* dst = out + p * row_vec;
-    if (sid < 0 || sid >= numel) {
-      for (int64_t c = lane; c < row_vec; c += 32) dst[c] = make_uint4(0, 0, 0, 0);
-      continue;
-    }
+    if (sid < 0 || sid >= numel) continue;
     const uint4* src = x + (sid / topk) * row_vec;
+    uint4* dst = out + p * row_vec;
     int64_t c = lane;
     for (; c + 96 < row_vec; c += 128) {  // four loads in flight
       const uint4 v0 = src[c], v1 = src[c + 32], v2 = src[c + 64], v3 = src[c + 96];
@@ -299,16 +296,19 @@ __device__ __forceinline__ int8_t round_int8_even(float v) {
   return (int8_t)__float2int_rn(v);
 }
 
-// One warp per row.  KIND as in moe_rowwise_quant.
+// One warp per row.  KIND as in moe_rowwise_quant; `indirect`: the i-th row is row indirect[i] (negative: none).
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256) rowwise_quant_kernel(const T* __restrict__ x, int64_t rows, int64_t cols,
                                                             const float* __restrict__ scale_in,
                                                             const int32_t* __restrict__ row_ids, int64_t valid_below,
+                                                            const int32_t* __restrict__ indirect,
                                                             uint8_t* __restrict__ q, float* __restrict__ scale_out) {
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = warp0; r < rows; r += warps) {
+  for (int64_t idx = warp0; idx < rows; idx += warps) {
+    const int64_t r = indirect != nullptr ? (int64_t)indirect[idx] : idx;
+    if (r < 0) continue;
     if (row_ids != nullptr) {
       const int64_t id = row_ids[r];
       if (id < 0 || id >= valid_below) continue;
@@ -357,12 +357,15 @@ template <typename T, int KIND, int TPR, int CH>
 __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restrict__ x, int64_t rows, int cols,
                                                                 const float* __restrict__ scale_in,
                                                                 const int32_t* __restrict__ row_ids, int64_t valid_below,
+                                                                const int32_t* __restrict__ indirect,
                                                                 uint8_t* __restrict__ q, float* __restrict__ scale_out) {
   constexpr int RPC = 256 / TPR;  // rows per CTA
   __shared__ float s_amax[TPR > 32 ? 8 : 1], s_nan[TPR > 32 ? 8 : 1];
   const int t = threadIdx.x % TPR, lane = threadIdx.x & 31;
   const int pieces = cols / 8;
-  for (int64_t r = (int64_t)blockIdx.x * RPC + threadIdx.x / TPR; r < rows; r += (int64_t)gridDim.x * RPC) {
+  for (int64_t idx = (int64_t)blockIdx.x * RPC + threadIdx.x / TPR; idx < rows; idx += (int64_t)gridDim.x * RPC) {
+    const int64_t r = indirect != nullptr ? (int64_t)indirect[idx] : idx;
+    if (r < 0) continue;
     if (row_ids != nullptr) {  // uniform over the threads of a row
       const int64_t id = row_ids[r];
       if (id < 0 || id >= valid_below) continue;
@@ -433,12 +436,15 @@ __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(256) tensor_amax_kernel(const T* __restrict__ x, int64_t rows, int64_t cols,
                                                           const int32_t* __restrict__ row_ids, int64_t valid_below,
+                                                          const int32_t* __restrict__ indirect,
                                                           unsigned int* __restrict__ amax_bits) {
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   float amax = 0.0f;
-  for (int64_t r = warp0; r < rows; r += warps) {
+  for (int64_t idx = warp0; idx < rows; idx += warps) {
+    const int64_t r = indirect != nullptr ? (int64_t)indirect[idx] : idx;
+    if (r < 0) continue;
     if (row_ids != nullptr) {
       const int64_t id = row_ids[r];
       if (id < 0 || id >= valid_below) continue;
@@ -471,7 +477,7 @@ __global__ void gather_scales_kernel(const float* __restrict__ scales_t, int gro
 
 template <typename T>
 static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int kind, const float* scale_in,
-                                const int32_t* row_ids, int64_t valid_below, void* q, float* scale_out, cudaStream_t st) {
+                                const int32_t* row_ids, int64_t valid_below, const int32_t* indirect, void* q, float* scale_out, cudaStream_t st) {
   using namespace moe;
   const int grid = grid_for((rows + 7) / 8, 8);
   // whole 16-byte pieces: a warp holds up to 2048 columns of its row in registers, a CTA up to 8192
@@ -482,17 +488,17 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
     if constexpr (sizeof(T) == 2) {                                                                                 \
       if (vec && cols <= 2048) {                                                                                    \
         rowwise_quant_vec_kernel<T, K, 32, 8><<<grid, 256, 0, st>>>((const T*)x, rows, (int)cols, SIN, row_ids,     \
-                                                                    valid_below, (uint8_t*)q, scale_out);           \
+                                                                    valid_below, indirect, (uint8_t*)q, scale_out);           \
         done = true;                                                                                                \
       } else if (vec) {                                                                                             \
         rowwise_quant_vec_kernel<T, K, 256, 4><<<grid_for(rows, 8), 256, 0, st>>>(                                  \
-            (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, (uint8_t*)q, scale_out);                       \
+            (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect, (uint8_t*)q, scale_out);                       \
         done = true;                                                                                                \
       }                                                                                                             \
     }                                                                                                               \
     if (!done)                                                                                                      \
       rowwise_quant_kernel<T, K><<<grid, 256, 0, st>>>((const T*)x, rows, cols, SIN, row_ids, valid_below,          \
-                                                       (uint8_t*)q, scale_out);                                     \
+                                                       indirect, (uint8_t*)q, scale_out);                                     \
   } while (0)
   switch (kind) {
     case 0: MOE_RQ(0, nullptr); break;
@@ -502,7 +508,7 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
     case 3: {
       cudaError_t ce = cudaMemsetAsync(scale_out, 0, sizeof(float), st);
       if (ce != cudaSuccess) return fail((int)ce, "rowwise_quant: %s", cudaGetErrorString(ce));
-      tensor_amax_kernel<T><<<grid, 256, 0, st>>>((const T*)x, rows, cols, row_ids, valid_below, (unsigned int*)scale_out);
+      tensor_amax_kernel<T><<<grid, 256, 0, st>>>((const T*)x, rows, cols, row_ids, valid_below, indirect, (unsigned int*)scale_out);
       amax_to_scale_kernel<<<1, 1, 0, st>>>(scale_out);
       MOE_RQ(3, scale_out);
       break;
@@ -513,25 +519,31 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
   return check_launch("rowwise_quant");
 }
 
-extern "C" int moe_rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, const float* scale_in,
-                                 const int32_t* row_ids, int64_t valid_below, void* q, float* scale_out, void* stream) {
-  using namespace moe;
+namespace moe {
+int rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, const float* scale_in,
+                                 const int32_t* row_ids, int64_t valid_below, const int32_t* indirect, void* q, float* scale_out, cudaStream_t st) {
   if (rows < 0 || cols <= 0) return fail(MOE_E_BADARG, "rowwise_quant: bad extent");
   if (rows == 0) return 0;
   if (!x || !q) return fail(MOE_E_BADARG, "rowwise_quant: null pointer");
   if ((kind == 2 || kind == 4) && !scale_in) return fail(MOE_E_BADARG, "rowwise_quant: static scale missing");
   if ((kind == 0 || kind == 1 || kind == 3) && !scale_out) return fail(MOE_E_BADARG, "rowwise_quant: scale output missing");
-  cudaStream_t st = (cudaStream_t)stream;
   if ((kind == 2 || kind == 4) && scale_out && scale_out != scale_in) {
     cudaError_t ce = cudaMemcpyAsync(scale_out, scale_in, sizeof(float), cudaMemcpyDeviceToDevice, st);
     if (ce != cudaSuccess) return fail((int)ce, "rowwise_quant: %s", cudaGetErrorString(ce));
   }
   switch (x_dtype) {
-    case MOE_F32: return rowwise_quant_launch<float>(x, rows, cols, kind, scale_in, row_ids, valid_below, q, scale_out, st);
-    case MOE_F16: return rowwise_quant_launch<__half>(x, rows, cols, kind, scale_in, row_ids, valid_below, q, scale_out, st);
-    case MOE_BF16: return rowwise_quant_launch<__nv_bfloat16>(x, rows, cols, kind, scale_in, row_ids, valid_below, q, scale_out, st);
+    case MOE_F32: return rowwise_quant_launch<float>(x, rows, cols, kind, scale_in, row_ids, valid_below, indirect, q, scale_out, st);
+    case MOE_F16: return rowwise_quant_launch<__half>(x, rows, cols, kind, scale_in, row_ids, valid_below, indirect, q, scale_out, st);
+    case MOE_BF16: return rowwise_quant_launch<__nv_bfloat16>(x, rows, cols, kind, scale_in, row_ids, valid_below, indirect, q, scale_out, st);
     default: return fail(MOE_E_DTYPE, "rowwise_quant: unsupported dtype %d", x_dtype);
   }
+}
+}  // namespace moe
+
+extern "C" int moe_rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, const float* scale_in,
+                                 const int32_t* row_ids, int64_t valid_below, void* q, float* scale_out, void* stream) {
+  return moe::rowwise_quant(x, x_dtype, rows, cols, kind, scale_in, row_ids, valid_below, nullptr, q, scale_out,
+                            (cudaStream_t)stream);
 }
 
 extern "C" int moe_gather_scales_t(const float* scales_t, int groups, int64_t num_tokens, int topk,

@@ -131,6 +131,23 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* ba
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
       : "memory");
 }
+// The loads of a CTA pair: the data lands in this CTA, the bytes are counted on the barrier at this
+// offset in the pair's leader (clearing the peer bit of a shared-memory address names the even CTA).
+constexpr uint32_t LEADER_BAR_MASK = 0xFEFFFFFFu;
+__device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint64_t* bar, void* dst, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar) & LEADER_BAR_MASK), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(const CUtensorMap* map, uint64_t* bar, void* dst, int c0, int c1, int c2,
+                                                 int c3, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar) & LEADER_BAR_MASK), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
@@ -144,26 +161,23 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
       ::"r"(smem_u32(bar)), "h"((uint16_t)3)
       : "memory");
 }
-// One instruction for the pair: M = 256 (128 rows from each CTA), N = 256 (128 B rows from each CTA)
-template <bool FP8>
-__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  if constexpr (FP8) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-        : "memory");
-  }
-}
-// KIND of the single-CTA instructions: f16 / bf16 operands, e4m3 operands (fp32 accumulators), or
+// KIND of the instructions: f16 / bf16 operands, e4m3 operands (fp32 accumulators), or
 // int8 operands with int32 accumulators
 constexpr int MMA_F16 = 0, MMA_F8 = 1, MMA_I8 = 2;
+// One instruction for the pair: M = 256 (128 rows from each CTA), B rows half from each CTA
+template <int KIND>
+__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+#define MOE_MMA2_ASM(KINDSTR)                                                             \
+  asm volatile(                                                                           \
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                  \
+      "tcgen05.mma.cta_group::2.kind::" KINDSTR " [%0], %1, %2, %3, p;\n\t}"              \
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)                         \
+      : "memory")
+  if constexpr (KIND == MMA_F8) MOE_MMA2_ASM("f8f6f4");
+  else if constexpr (KIND == MMA_I8) MOE_MMA2_ASM("i8");
+  else MOE_MMA2_ASM("f16");
+#undef MOE_MMA2_ASM
+}
 #define MOE_MMA_ASM(KINDSTR, ACCC, ACCV)                                                  \
   asm volatile(                                                                           \
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"                                  \
@@ -239,11 +253,24 @@ __device__ __forceinline__ void tmem_wait64(uint32_t* a, uint32_t* b) {
                : MOE_RW8(a, 0), MOE_RW8(a, 8), MOE_RW8(a, 16), MOE_RW8(a, 24), MOE_RW8(b, 0), MOE_RW8(b, 8), MOE_RW8(b, 16),
                  MOE_RW8(b, 24)::"memory");
 }
+// 16 accumulator lanes x 32 columns in the fragment layout of the warp MMAs: for the 8-column chunk c,
+// a[4c], a[4c+1] = lane t/4, columns 8c + 2 (t mod 4) and the next; a[4c+2], a[4c+3] = lane t/4 + 8.
+__device__ __forceinline__ void tmem_ld_frag32_async(uint32_t taddr, uint32_t* a) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : MOE_R8(a, 0), MOE_R8(a, 8)
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait32(uint32_t* a) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : MOE_RW8(a, 0), MOE_RW8(a, 8), MOE_RW8(a, 16), MOE_RW8(a, 24)::"memory");
+}
 // One 32-column load and its wait.
 __device__ __forceinline__ void tmem_ld32_sync(uint32_t taddr, uint32_t* a) {
   tmem_ld32_async(taddr, a);
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : MOE_RW8(a, 0), MOE_RW8(a, 8), MOE_RW8(a, 16), MOE_RW8(a, 24)::"memory");
+  tmem_wait32(a);
 }
 #undef MOE_R8
 #undef MOE_RW8
@@ -375,6 +402,26 @@ static inline int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType
                    weights ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(MOE_E_DRIVER, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return 0;
+}
+
+// Gate | up weights [E, 2I, K] as five dimensions, so that one box of 128 rows is eight times {8 gate rows, the
+// up rows of the same 8 outputs}: (K, 8 rows, gate/up, I/8, E).  In the fragment layout of
+// tmem_ld_frag32_async a thread then holds gate and up of the same output and token.
+static inline int make_gate_up_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t E,
+                                   uint64_t I, uint64_t K) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return fail(MOE_E_DRIVER, "cuTensorMapEncodeTiled is not available from the driver");
+  if (((uintptr_t)base & 15) != 0) return fail(MOE_E_BADARG, "tensor-core GEMM: weights not 16-byte aligned");
+  if ((K * elem_bytes) % 16 != 0 || I % 8 != 0) return fail(MOE_E_SHAPE, "tensor-core GEMM: weight shape");
+  const uint64_t row = K * (uint64_t)elem_bytes;
+  cuuint64_t gdim[5] = {K, 8, 2, I / 8, E};
+  cuuint64_t gstr[4] = {row, I * row, 8 * row, 2 * I * row};
+  cuuint32_t box[5] = {(cuuint32_t)(128 / elem_bytes), 8, 2, 8, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = enc(m, dt, 5, const_cast<void*>(base), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(MOE_E_DRIVER, "cuTensorMapEncodeTiled (gate | up) failed with CUresult %d", (int)r);
   return 0;
 }
 

@@ -474,12 +474,67 @@ def combine_routes(y, out, topk_ids, global_num_experts, expert_map=None, row_in
                                      _lib.ptr(emap), _lib.ptr(row_index), _lib.stream_of(out)))
 
 
+# switches that pin one of the kernels behind route_pipeline / run_chunk_small (tests and experiments)
+_KERNEL_SWITCHES = ("FLAGGEMS_B200_GENERIC_GEMM", "FLAGGEMS_B200_TC_WIDE", "FLAGGEMS_B200_TC_PAIR",
+                    "FLAGGEMS_B200_TC_PAIR_WIDE", "FLAGGEMS_B200_PRESORT", "FLAGGEMS_B200_TMA_OUT",
+                    "FLAGGEMS_B200_SMALL_M")
+_workspace_sizes = {}
+
+
+def _workspace_bytes(*key):
+    """Workspaces of the native layer call for these sizes, None when it does not serve them (a pure function of the
+    sizes: remembered)."""
+    if key not in _workspace_sizes:
+        sizes = (ctypes.c_int64 * 4)()
+        rc = _lib.lib().moe_layer_workspace(*key, ctypes.addressof(sizes))
+        if len(_workspace_sizes) > 4096:
+            _workspace_sizes.clear()
+        _workspace_sizes[key] = None if rc != 0 else tuple(sizes)
+    return _workspace_sizes[key]
+
+
+def run_chunk_native(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w2_scale, global_num_experts, expert_map,
+                     apply_router_weight_on_input, mark, act_fn, row_quant) -> bool:
+    """One chunk through the native layer call (csrc/layer.cu); False when it does not serve the sizes."""
+    M, H = x.shape
+    k = topk_ids.shape[1]
+    E_local, N2, _ = w1.shape
+    act_code = _lib.dtype_code(x.dtype)
+    need = _workspace_bytes(mode, act_code, M, k, global_num_experts, E_local, H, N2 // 2, act_fn[0])
+    if need is None:
+        return False
+    dev = x.device
+    ids = topk_ids if topk_ids.is_contiguous() else topk_ids.contiguous()
+    rw = topk_weights if topk_weights.dtype == torch.float32 else topk_weights.float()
+    rw = rw if rw.is_contiguous() else rw.contiguous()
+    emap = expert_map
+    if emap is not None:
+        emap = emap if emap.dtype == torch.int32 else emap.to(torch.int32)
+        emap = emap if emap.is_contiguous() else emap.contiguous()
+    (q1, qs1), (q2, qs2) = row_quant if row_quant is not None else ((0, None), (0, None))
+    ws = [torch.empty(n, dtype=torch.uint8, device=dev) for n in need]
+    args = (mode, act_code, x.data_ptr(), M, k, ids.data_ptr(), int(ids.dtype == torch.int64), rw.data_ptr(),
+            w1.data_ptr(), _lib.ptr(w1_scale), w2.data_ptr(), _lib.ptr(w2_scale), out.data_ptr(), global_num_experts,
+            _lib.ptr(emap), E_local, H, N2 // 2, int(apply_router_weight_on_input), act_fn[0], act_fn[1], act_fn[2],
+            act_fn[3], q1, _lib.ptr(qs1), q2, _lib.ptr(qs2), *[w.data_ptr() for w in ws])
+    tail = (_lib.status_word(dev).data_ptr(), _lib.stream_of(x))
+    call = _lib.lib().moe_layer
+    if mark is None:
+        _lib.check(call(*args, 63, *tail))
+    else:  # stage by stage, so that the caller can time them
+        for bits, name in ((1, "align"), (2, "quant"), (4, "gemm1"), (8, "quant2"), (16, "gemm2"), (32, "sum")):
+            _lib.check(call(*args, bits, *tail))
+            mark(name)
+    return True
+
+
 def run_chunk(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w2_scale, global_num_experts,
               expert_map, apply_router_weight_on_input, use_tensor_cores=None, keep=None, mark=None,
               act_fn=(0, 0.0, 0.0, 0.0), row_quant=None):
     """One chunk of the layer.  ``keep`` (a dict) receives the intermediates for
     tests; ``mark(name)`` is called after each stage has been enqueued (bench.py
     records CUDA events there)."""
+    native_mark = mark or STAGE_HOOK
     if mark is None:
         mark = STAGE_HOOK or _no_mark
     # (half-precision weights with per-channel scales -- the widened int8 experiment -- stay on the tile kernels)
@@ -489,6 +544,13 @@ def run_chunk(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w2_scal
         run_chunk_small(x, w1, w2, topk_weights, topk_ids, out, mode=mode, w1_scale=w1_scale, w2_scale=w2_scale,
                         global_num_experts=global_num_experts, expert_map=expert_map,
                         apply_router_weight_on_input=apply_router_weight_on_input, keep=keep, mark=mark)
+        return
+    if use_tensor_cores is None and keep is None and not (mode == _lib.MODE_HALF and w1_scale is not None) \
+            and not any(v in os.environ for v in _KERNEL_SWITCHES) and run_chunk_native(
+                x, w1, w2, topk_weights, topk_ids, out, mode=mode, w1_scale=w1_scale, w2_scale=w2_scale,
+                global_num_experts=global_num_experts, expert_map=expert_map,
+                apply_router_weight_on_input=apply_router_weight_on_input, mark=native_mark, act_fn=act_fn,
+                row_quant=row_quant):
         return
     row_quant2 = None
     if mode == _lib.MODE_FP8_BLOCK:

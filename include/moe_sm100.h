@@ -426,6 +426,27 @@ int moe_ep_pack(const void* rows, int64_t row_bytes, const float* scales, int gr
 int moe_ep_unpack(const float* side, int64_t rows, int groups, int k, int rank, int experts_per_rank,
                   float* scales_t, int32_t* slot_ids, float* slot_w, void* stream);
 
+/*
+ * The whole expert layer in one call: route plan, scatter (with the activation quantiser of the mode), GEMM1,
+ * GEMM2, weighted sum over a token's routes (src/flaggems_vllm/ops/fused_moe.py:2314-2737).  Serves the modes
+ * MOE_MODE_HALF (H % 64 == 0), MOE_MODE_FP8_BLOCK (SiLU), MOE_MODE_FP8_ROW and MOE_MODE_INT8_ROW (H % 128 == 0), f16 / bf16
+ * activations, I % 128 == 0, topk <= 32, at most 1024 experts and 2^20 routes; moe_layer_workspace
+ * writes the sizes in bytes of the four workspaces, or returns MOE_E_SHAPE for anything else.
+ *   x, out [num_tokens, H]; topk_ids, topk_weights [num_tokens, topk]; weights and scales as in moe_gemm1_ex /
+ *   moe_gemm2; expert_map [num_experts] or NULL: local index of every expert, negative = not local;
+ *   quant_kind1 / 2, quant_scale1 / 2: row-scaled modes, how the input and the intermediate are quantised
+ *   (moe_rowwise_quant); stages: bit mask of the steps to enqueue (1 plan, 2 scatter, 4 GEMM1, 8 intermediate
+ *   quantiser, 16 GEMM2, 32 sum), 63 = the layer.  `out` may be `x`.
+ */
+int moe_layer_workspace(int mode, int act_dtype, int64_t num_tokens, int topk, int num_experts, int E_local, int H, int I,
+                        int activation, int64_t bytes[4]);
+int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tokens, int topk, const void* topk_ids, int ids_int64,
+              const float* topk_weights, const void* w1, const float* w1_scale, const void* w2, const float* w2_scale,
+              void* out, int num_experts, const int32_t* expert_map, int E_local, int H, int I, int weight_on_input,
+              int activation, float alpha, float beta, float limit, int quant_kind1, const float* quant_scale1,
+              int quant_kind2, const float* quant_scale2, void* ws_plan, void* ws_x, void* ws_act, void* ws_y, int stages,
+              int32_t* status, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

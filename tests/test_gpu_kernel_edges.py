@@ -82,3 +82,56 @@ def test_router_gemm_row_tiles_share_one_order(M):
     x32 = T.make_activations(37, 2048, DEV, seed=M, dtype=torch.float32)  # 8-row tiles, 1 and 4 columns wide
     out = fg.router_gemm(x32, w)
     assert torch.equal(out[:9], fg.router_gemm(x32[:9], w)) and torch.equal(out[36:], fg.router_gemm(x32[36:], w))
+
+
+def _half_layer(M, E, k, H, I, dtype, **kw):
+    x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
+    w1 = T.make_half_weights(E, 2 * I, H, DEV, seed=1, dtype=dtype, std=H**-0.5)
+    w2 = T.make_half_weights(E, H, I, DEV, seed=2, dtype=dtype, std=I**-0.5)
+    tw, ti = _route(M, E, k)
+    return x, w1, w2, tw, ti
+
+
+@pytest.mark.parametrize("M,E,k,H,I", [
+    (16, 4, 1, 192, 128), (50, 8, 2, 320, 256),      # tokens as M: a few rows per block, K of an odd number of stages
+    (290, 3, 1, 256, 128), (1000, 4, 2, 448, 384),   # CTA pair: tiles of 96 / 112 .. rows, last 256-column tile half empty
+    (2100, 4, 2, 128, 128), (513, 1, 1, 576, 256)])  # several tiles per expert, one expert
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_half_layer_tiles(M, E, k, H, I, dtype):
+    x, w1, w2, tw, ti = _half_layer(M, E, k, H, I, dtype)
+    _parity(fg.fused_experts_impl(x, w1, w2, tw, ti), O.fused_moe_half_oracle(x, w1, w2, tw, ti), (M, E))
+
+
+@pytest.mark.parametrize("M,E,k", [(2, 8, 2), (40, 8, 2), (520, 4, 2), (1100, 4, 2)])
+def test_fp8_block_layer_tiles(M, E, k):
+    """Occupied rows only, whole blocks, row stores and staged stores of the 128-row kernel over a route plan."""
+    H, I = 384, 256
+    x = T.make_activations(M, H, DEV, seed=M)
+    w1, s1 = T.make_fp8_block_weights(E, 2 * I, H, DEV, seed=1)
+    w2, s2 = T.make_fp8_block_weights(E, H, I, DEV, seed=2)
+    tw, ti = _route(M, E, k)
+    kw = dict(use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+    _parity(out, O.fused_moe_fp8_block_oracle(x, w1, w2, s1, s2, tw, ti), M)
+    x2 = x.clone()
+    assert torch.equal(fg.fused_experts_impl(x2, w1, w2, tw, ti, inplace=True, **kw), out)
+
+
+@pytest.mark.parametrize("M", [7, 300, 2500])
+def test_layer_with_local_experts_and_weights_on_the_input(M):
+    """expert_map (routes of other ranks get no rows), ids out of range, route weights applied on the input."""
+    E, k, H, I = 12, 3, 256, 128
+    x, w1, w2, tw, ti = _half_layer(M, E, k, H, I, torch.bfloat16)
+    emap = torch.full((E,), -1, dtype=torch.int32, device=DEV)
+    emap[4:8] = torch.arange(4, dtype=torch.int32, device=DEV)
+    ti[M // 2, 1] = -1
+    keep = (ti >= 4) & (ti < 8)
+    ref = O.fused_moe_half_oracle(x, w1, w2, tw * keep, ti.clamp(min=0))
+    out = fg.fused_experts_impl(x, w1[4:8].contiguous(), w2[4:8].contiguous(), tw, ti, global_num_experts=E, expert_map=emap)
+    _parity(out, ref, M)
+    assert bool((out[~keep.any(1)] == 0).all())
+    if M > 100:
+        full = ti.clamp(min=0)
+        out = fg.fused_experts_impl(x, w1, w2, tw, full, apply_router_weight_on_input=True)
+        ref = O.fused_moe_half_oracle(x, w1, w2, tw, full, apply_router_weight_on_input=True)
+        _parity(out, ref, M)
