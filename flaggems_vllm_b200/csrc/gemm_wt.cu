@@ -26,19 +26,17 @@
 // (make_gate_up_map), so those two lanes are gate and up of one output, and SiLU(gate) * up needs no exchange.
 // Results are transposed on their way to shared memory by stmatrix.trans and leave as whole rows.
 //
-//
 // Formats: half precision, and e4m3 / int8 with one scale per row and per output channel, which the epilogue applies
 // to the finished sums.  FP8 with block scales stays with tokens as M: its sums leave the tensor core every
 // 128 elements of K and are folded with one scale per token.  With tokens along the columns that is a scale per
 // register (a shared-memory load each) and twice as many rounds between MMA and fold per byte of weights; it
 // measured 1.3 to 1.5 times slower than gemm_tc.cu from one token to 8192.
-#include "tc_common.cuh"
+#include "wt_common.cuh"
 
 namespace moe {
 namespace wt {
 using namespace tc;
 
-constexpr int FMT_HALF = 0, FMT_FP8ROW = 2, FMT_I8ROW = 3;
 constexpr int WROWS = 128;   // weight rows per CTA
 constexpr int NTOK = 256;    // most tokens of a tile
 constexpr int A_BYTES = WROWS * 128;
@@ -52,9 +50,7 @@ static_assert(128 * PRODUCER_REGS + CONS_THREADS * CONSUMER_REGS <= THREADS * LA
 
 template <bool GEMM1> struct Cfg {
   static constexpr int STAGES = GEMM1 ? 5 : 4;
-  static constexpr int OUT_COLS = GEMM1 ? 64 : 128;            // output columns per CTA
-  static constexpr int OUT_PITCH = OUT_COLS * 2 + 16;          // bytes; the 16 spread stmatrix rows over the banks
-  static constexpr int OUT_BYTES = NTOK * OUT_PITCH;
+  static constexpr int OUT_BYTES = NTOK * ((GEMM1 ? 64 : 128) * 2 + 16);  // staged rows, see drain_tile
 };
 struct Aux {
   uint64_t full[6], empty[6];
@@ -67,45 +63,11 @@ template <bool GEMM1> constexpr size_t smem_bytes() {
 }
 static_assert(smem_bytes<true>() <= 232448 && smem_bytes<false>() <= 232448, "shared memory of one SM");
 
-struct Params {
-  const int4* tiles;        // {first row, rows | occupied rows << 16, expert, first tile of the expert | its tile count << 16}
-  const int32_t* counts;    // [0] = number of tiles
-  const float* a_scales;    // row-scaled: [rows_cap]
-  const float* w_scale;     // row-scaled: [E, rows_w]
-  const float* row_weight;  // GEMM1 with the route weight on the input: [rows_cap], else null
-  void* out;                // GEMM1: [rows_cap, I]; GEMM2: [rows_cap, H]
-  int32_t* status;
-  unsigned long long wait_ns;
-  int E, K, Nout, R;        // R = row tiles per expert: I/128 (GEMM1), ceil(H/256) (GEMM2)
-  float alpha, beta, limit;
-};
-
-// tile list entry of one work item and its row tile
-struct Item {
-  int row0, n, e, rt;
-};
-
-__device__ __forceinline__ void stmatrix_x2_trans(uint32_t addr, uint32_t a, uint32_t b) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x2.trans.shared.b16 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
-}
-__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c),
-               "r"(d)
-               : "memory");
-}
-// the other activation; its clamps let NaN through (src/flaggems_vllm/ops/fused_moe.py:733-773)
-__device__ __forceinline__ float swigluoai(float g, float u, float alpha, float beta, float limit) {
-  g = (g != g) ? g : fminf(g, limit);
-  u = (u != u) ? u : fminf(fmaxf(u, -limit), limit);
-  return g * (1.0f / (1.0f + expf(-alpha * g))) * (u + beta);
-}
-
 // SILU: the activation of GEMM1 (false: swigluoai, which reads GEMM1's result rounded to the activation type)
 template <int FMT, typename AT, bool GEMM1, bool SILU>
 __global__ void __launch_bounds__(THREADS, 1)
 wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_b64,
                const __grid_constant__ CUtensorMap map_b16, const __grid_constant__ CUtensorMap map_b8, const Params P) {
-  constexpr bool ROW = FMT == FMT_FP8ROW || FMT == FMT_I8ROW;
   constexpr int KIND = FMT == FMT_HALF ? MMA_F16 : (FMT == FMT_I8ROW ? MMA_I8 : MMA_F8);
   constexpr int KBE = FMT == FMT_HALF ? 64 : 128;  // elements of K per stage
   using C = Cfg<GEMM1>;
@@ -120,20 +82,7 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const int cr = (int)cluster_ctarank();  // 0 leads
   const int item0 = blockIdx.x / 2, step = gridDim.x / 2;
   const int total = P.counts[0] * P.R;
-  // Work items, expert by expert; inside an expert the token tile runs fastest, so the pairs that
-  // run at the same time read the same weight tile.
-  auto fetch = [&](int item) -> Item {
-    Item it;
-    const int t0 = item / P.R;
-    int4 d = P.tiles[t0];
-    const int first = d.w & 0xFFFF, q = (int)((uint32_t)d.w >> 16);
-    const int within = item - first * P.R;
-    it.rt = within / q;
-    const int t = first + within - it.rt * q;
-    if (t != t0) d = P.tiles[t];
-    it.row0 = d.x; it.n = d.y & 0xFFFF; it.e = d.z;
-    return it;
-  };
+  auto fetch = [&](int item) { return fetch_item(P, item); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&aux->full[s], 1); mbar_init(&aux->empty[s], 1); }
@@ -230,7 +179,6 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // -------------------------------------------------------------- consumers
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CONSUMER_REGS));
     const int h = (warp - 4) >> 2, wq = warp & 3;
-    const int tr = lane >> 2, tq = lane & 3;
     const int et = threadIdx.x - 128;
     const uint32_t t_lane = tmem_base + ((uint32_t)(wq << 5) << 16);
     const uint32_t out_base = smem_u32(s_out);
@@ -244,9 +192,6 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         else mbar_arrive(&aux->tmem_empty[a]);
       }
     };
-    // rows of this thread: 16-lane block rh (0, 1) of the warp's 32 lanes, lanes tr and tr + 8
-    // GEMM1: output 64 cr + 8 (2 wq + rh) + tr of the row tile (gate in lane tr, up in lane tr + 8)
-    // GEMM2: output columns 128 cr + 32 wq + 16 rh + tr and + 8
     Item nx = {};
     if (item0 < total) nx = fetch(item0);
     // The tile loop runs to its end even after a wait has timed out: every consumer thread reaches
@@ -254,120 +199,16 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     for (int item = item0; item < total; item += step) {
       const Item it = nx;
       if (item + step < total) nx = fetch(item + step);
-      const int nh = it.n >> 1, tok0 = h * nh;      // this group's tokens [tok0, tok0 + nh) of the tile
-      const int nst = (nh + 31) >> 5;               // steps of 32 tokens
-
-      // (a) what is in the fragment registers r of step st, chunk c, block rh -> staged 16-bit values
-      auto stage_chunk = [&](int st, int c, const float (&lo)[2][2], const float (&hi)[2][2]) {
-        // lo[rh][j] / hi[rh][j]: lanes tr / tr + 8, token j of the pair (already final fp32 values)
-        const int tok = tok0 + st * 32 + c * 8;
-        if constexpr (GEMM1) {
-          (void)hi;
-          const uint32_t addr = out_base + (uint32_t)(tok + (lane & 7)) * C::OUT_PITCH + (uint32_t)((2 * wq + ((lane >> 3) & 1)) * 16);
-          stmatrix_x2_trans(addr, pack2<AT>(lo[0][0], lo[0][1]), pack2<AT>(lo[1][0], lo[1][1]));
-        } else {
-          const uint32_t addr = out_base + (uint32_t)(tok + (lane & 7)) * C::OUT_PITCH + (uint32_t)(wq * 64 + (lane >> 3) * 16);
-          stmatrix_x4_trans(addr, pack2<AT>(lo[0][0], lo[0][1]), pack2<AT>(hi[0][0], hi[0][1]), pack2<AT>(lo[1][0], lo[1][1]),
-                            pack2<AT>(hi[1][0], hi[1][1]));
-        }
-      };
-      // GEMM1: gate and up of (output, token) -> the staged activation value
-      auto activate = [&](float g, float u, float rw) -> float {
-        g *= rw; u *= rw;
-        if constexpr (ROW || !SILU) { g = round_act<AT>(g); u = round_act<AT>(u); }
-        if constexpr (SILU) return silu_mul_fast(g, u);
-        else return swigluoai(g, u, P.alpha, P.beta, P.limit);
-      };
-
-      // ---------------------------------------------------------- tile epilogue
+      const uint32_t a = acc_it & 1;
       asm volatile("bar.sync 2, %0;" ::"n"(CONS_THREADS) : "memory");  // the staging tile has been read
-      {
-        const uint32_t a = acc_it & 1;
-        if (alive && !mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) alive = false;
-        if (alive) {
-          tc_fence_after();
-          // channel scales of this thread's rows: [rh][lane tr / tr + 8]
-          float cs[2][2] = {{1.0f, 1.0f}, {1.0f, 1.0f}};
-          if constexpr (ROW) {
-            const float* ws = P.w_scale + (int64_t)it.e * (GEMM1 ? 2 * P.Nout : P.Nout);
-#pragma unroll
-            for (int rh = 0; rh < 2; ++rh) {
-              if constexpr (GEMM1) {
-                const int o = it.rt * 128 + cr * 64 + (2 * wq + rh) * 8 + tr;
-                cs[rh][0] = __ldg(ws + o);
-                cs[rh][1] = __ldg(ws + P.Nout + o);
-              } else {
-                const int o = it.rt * 256 + cr * 128 + wq * 32 + rh * 16 + tr;
-                cs[rh][0] = o < P.Nout ? __ldg(ws + o) : 0.0f;
-                cs[rh][1] = o + 8 < P.Nout ? __ldg(ws + o + 8) : 0.0f;
-              }
-            }
-          }
-          const uint32_t t0 = t_lane + a * NTOK + (uint32_t)tok0;
-#pragma unroll 1
-          for (int st = 0; st < nst; ++st) {
-            uint32_t r[32];
-            tmem_ld_frag32_async(t0 + (uint32_t)st * 32, r);
-            tmem_ld_frag32_async(t0 + (uint32_t)st * 32 + (16u << 16), r + 16);
-            float2 as[4], rw[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const bool in = st * 32 + c * 8 < nh;
-              const int64_t p = (int64_t)it.row0 + tok0 + st * 32 + c * 8 + 2 * tq;
-              if constexpr (ROW) as[c] = in ? *reinterpret_cast<const float2*>(P.a_scales + p) : make_float2(0.0f, 0.0f);
-              rw[c] = GEMM1 && in && P.row_weight != nullptr ? *reinterpret_cast<const float2*>(P.row_weight + p) : make_float2(1.0f, 1.0f);
-            }
-            tmem_wait32(r);
-            if (st == nst - 1) release_acc(a);  // everything of this tile is in registers or staged
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              if (st * 32 + c * 8 < nh) {
-                float lo[2][2], hi[2][2];
-#pragma unroll
-                for (int rh = 0; rh < 2; ++rh) {
-                  float v[2][2];  // [lane tr / tr + 8][token]
-#pragma unroll
-                  for (int l = 0; l < 2; ++l)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                      const uint32_t raw = r[rh * 16 + 4 * c + 2 * l + j];
-                      v[l][j] = FMT == FMT_I8ROW ? (float)(int)raw : __uint_as_float(raw);
-                      if constexpr (ROW) v[l][j] = v[l][j] * (j == 0 ? as[c].x : as[c].y) * cs[rh][l];
-                    }
-                  if constexpr (GEMM1) {
-                    lo[rh][0] = activate(v[0][0], v[1][0], rw[c].x);
-                    lo[rh][1] = activate(v[0][1], v[1][1], rw[c].y);
-                  } else {
-                    lo[rh][0] = v[0][0]; lo[rh][1] = v[0][1];
-                    hi[rh][0] = v[1][0]; hi[rh][1] = v[1][1];
-                  }
-                }
-                stage_chunk(st, c, lo, hi);
-              }
-            }
-          }
-          ++acc_it;
-        }
+      if (alive && !mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) alive = false;
+      if (alive) {
+        tc_fence_after();
+        drain_tile<FMT, AT, GEMM1, SILU, 2, 2>(P, it, cr, t_lane + a * NTOK, h, wq, lane, out_base, [&] { release_acc(a); });
+        ++acc_it;
       }
       asm volatile("bar.sync 2, %0;" ::"n"(CONS_THREADS) : "memory");  // the tile is staged
-
-      if constexpr (GEMM1) {
-        const int sub = et & 7, tl = et >> 3;  // eight lanes per token: 16 bytes each
-        const int64_t col = (int64_t)it.rt * 128 + cr * 64 + sub * 8;
-        if (alive) {
-          for (int tok = tl; tok < it.n; tok += 32)
-            *reinterpret_cast<uint4*>(reinterpret_cast<AT*>(P.out) + ((int64_t)it.row0 + tok) * P.Nout + col) =
-                *reinterpret_cast<const uint4*>(s_out + (size_t)tok * C::OUT_PITCH + sub * 16);
-        }
-      } else if (alive) {
-        const int sub = et & 15;  // sixteen lanes per token
-        const int col = it.rt * 256 + cr * 128 + sub * 8;
-        if (col < P.Nout) {
-          for (int tok = et >> 4; tok < it.n; tok += 16)
-            *reinterpret_cast<uint4*>(reinterpret_cast<AT*>(P.out) + ((int64_t)it.row0 + tok) * P.Nout + col) =
-                *reinterpret_cast<const uint4*>(s_out + (size_t)tok * C::OUT_PITCH + sub * 16);
-        }
-      }
+      if (alive) store_rows<AT, GEMM1, 2, CONS_THREADS>(P, it, cr, s_out, et);
     }
   }
 

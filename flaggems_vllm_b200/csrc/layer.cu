@@ -28,11 +28,17 @@ int wt_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
             const void* tiles, int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K,
             int Nout, void* out, int act_kind, float alpha, float beta, float limit, int32_t* status,
             cudaStream_t st);
+bool w8t_serves(int act_dtype, int H, int I);
+int w8t_tile(bool wide);
+int w8t_gemm(bool gemm1, bool wide, int act_dtype, const void* a, const void* w, const float* w_scale, const void* tiles,
+             int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K, int Nout, void* out,
+             int32_t* status, cudaStream_t st);
 
 namespace {
 // Which grouped GEMM serves the call and how the plan cuts the rows for it.
 struct Choice {
   bool pair;        // gemm_wt.cu: weights as the M operand of a CTA pair; else gemm_tc.cu: 128 tokens as M
+  bool wide;        // weight-only int8 (gemm_w8t.cu): tiles of up to 160 tokens instead of 64
   int gran, tile;   // row granule and most rows of a tile
   bool zero_pad;    // gemm_tc.cu: zero the padding rows and fetch whole blocks
   bool staged;      // gemm_tc.cu: GEMM2 leaves through staged TMA stores of whole tiles
@@ -41,12 +47,20 @@ struct Choice {
 bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
   if (mode == MOE_MODE_FP8_BLOCK)
     return act_kind == MOE_ACT_SILU && (act_dtype == MOE_BF16 || act_dtype == MOE_F16) && H % 128 == 0 && I % 128 == 0;
+  if (mode == MOE_MODE_W8A16) return act_kind == MOE_ACT_SILU && w8t_serves(act_dtype, H, I);
   return wt_serves(mode, act_dtype, H, I);
 }
 
 Choice choose(int mode, int act_kind, int64_t numel, int E) {
   const int64_t per_expert = numel / (E > 0 ? E : 1);
   Choice c = {};
+  if (mode == MOE_MODE_W8A16) {
+    // Qwen3 shape: at 32 rows per expert the narrow tile is 3 % ahead, at 64 the wide one 15 %
+    c.wide = per_expert > 40;
+    c.gran = 16;
+    c.tile = w8t_tile(c.wide);
+    return c;
+  }
   // FP8 block scales: tokens as M (gemm_wt.cu says why).  Half precision: up to 96 rows per expert the weights are
   // streamed and both kernels wait for memory (the single-CTA kernel is a few per cent ahead); above, the pair's finer
   // row padding counts (Mixtral shape, 1024 tokens: 1047 -> 887 us).
@@ -81,7 +95,7 @@ Layout layout(int mode, const Choice& c, int64_t M, int k, int E_local, int H, i
     L.bytes[ws] += (bytes + 255) / 256 * 256;
     return p;
   };
-  const bool byte = mode != MOE_MODE_HALF, row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
+  const bool byte = mode != MOE_MODE_HALF && mode != MOE_MODE_W8A16, row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
   L.row_index = take(0, numel * 4);
   L.tiles = take(0, L.tiles_cap * 16);
   L.counts = take(0, 8);
@@ -126,7 +140,7 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
   if (((uintptr_t)x | (uintptr_t)out | (uintptr_t)ws_plan | (uintptr_t)ws_x | (uintptr_t)ws_act | (uintptr_t)ws_y) & 15)
     return fail(MOE_E_BADARG, "layer: rows and workspaces must be 16-byte aligned");
   const bool row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
-  if ((row || block) && (!w1_scale || !w2_scale)) return fail(MOE_E_BADARG, "layer: weight scales missing");
+  if (mode != MOE_MODE_HALF && (!w1_scale || !w2_scale)) return fail(MOE_E_BADARG, "layer: weight scales missing");
   cudaStream_t st = (cudaStream_t)stream;
   const Choice c = choose(mode, activation, numel, num_experts);
   const Layout L = layout(mode, c, M, topk, E_local, H, I);
@@ -160,7 +174,9 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
     if (rc) return rc;
   }
   if (stages & 4) {
-    rc = c.pair ? wt_gemm(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
+    rc = mode == MOE_MODE_W8A16 ? w8t_gemm(true, c.wide, act_dtype, at(L.x_rows), w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
+                                           L.rows_cap, E_local, H, I, at(L.act), status, st)
+         : c.pair ? wt_gemm(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
                           L.rows_cap, E_local, H, I, at(L.act), activation, alpha, beta, limit, status, st)
                 : tc_gemm_plan(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, counts + 1, numel, L.rows_cap,
                                E_local, H, I, at(L.act), act_scales, row_weight, c.zero_pad, c.staged, status, st);
@@ -179,7 +195,9 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
     }
   }
   if (stages & 16) {
-    rc = c.pair ? wt_gemm(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
+    rc = mode == MOE_MODE_W8A16 ? w8t_gemm(false, c.wide, act_dtype, act, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
+                                           E_local, I, H, at(L.y), status, st)
+         : c.pair ? wt_gemm(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
                           E_local, I, H, at(L.y), MOE_ACT_SILU, 0.0f, 0.0f, 0.0f, status, st)
                 : tc_gemm_plan(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, counts + 1, numel, L.rows_cap, E_local,
                                I, H, at(L.y), nullptr, nullptr, c.zero_pad, c.staged, status, st);

@@ -135,3 +135,16 @@ def test_layer_with_local_experts_and_weights_on_the_input(M):
         out = fg.fused_experts_impl(x, w1, w2, tw, full, apply_router_weight_on_input=True)
         ref = O.fused_moe_half_oracle(x, w1, w2, tw, full, apply_router_weight_on_input=True)
         _parity(out, ref, M)
+
+
+@pytest.mark.parametrize("M,E,k,H,I", [
+    (20, 4, 2, 192, 128), (90, 3, 1, 256, 384),      # 64-token tiles: a last K block of 64, several tiles of one expert
+    (200, 2, 1, 320, 256), (1300, 4, 2, 128, 128)])  # 160-token tiles: even splits with remainders
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_int8_weight_layer_tiles(M, E, k, H, I, dtype):
+    x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
+    w1, s1 = T.make_int8_channel_weights(E, 2 * I, H, DEV, seed=1, std=H**-0.5)
+    w2, s2 = T.make_int8_channel_weights(E, H, I, DEV, seed=2, std=I**-0.5)
+    tw, ti = _route(M, E, k)
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti, use_int8_w8a16=True, per_channel_quant=True, w1_scale=s1, w2_scale=s2)
+    _parity(out, O.fused_moe_w8a16_oracle(x, w1, w2, s1, s2, tw, ti), (M, E))
