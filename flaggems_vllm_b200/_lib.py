@@ -90,8 +90,9 @@ SYMBOLS = {
 
 _lib = None
 _status = {}
-# calls of entry points that enqueue a kernel (bench.py reports the count of its timed region)
-LAUNCHES = 0
+# calls of entry points that enqueue a kernel; LAUNCHES adds those of the native host path (bench.py reports the
+# count of its timed region)
+_ctypes_launches = 0
 _NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_set_wait_limit_ns")
 
 
@@ -106,8 +107,8 @@ class _Counted:
     @staticmethod
     def _wrap(fn):
         def call(*args):
-            global LAUNCHES
-            LAUNCHES += 1
+            global _ctypes_launches
+            _ctypes_launches += 1
             return fn(*args)
 
         return call
@@ -132,6 +133,29 @@ def lib():
             fn.argtypes = args
         _lib = _Counted(handle)
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host_ext.cpp).  Its functions return None for whatever they do not serve."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host_ext
+        except ImportError as e:
+            raise RuntimeError(f"{os.path.join(HERE, '_host_ext.so')} has not been built or does not load ({e}); "
+                               "run `python -m flaggems_vllm_b200.build`.") from None
+        _host = _host_ext
+    return _host
+
+
+def __getattr__(name):
+    if name == "LAUNCHES":
+        return _ctypes_launches + (_host.launches() if _host is not None else 0)
+    raise AttributeError(name)
 
 
 def dtype_code(dt: torch.dtype) -> int:
@@ -160,7 +184,9 @@ def status_word(device) -> torch.Tensor:
     if key is None:
         key = torch.cuda.current_device()
     if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
+        word = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
+        host().set_status(key, word.data_ptr())
+        _status[key] = word
     return _status[key]
 
 

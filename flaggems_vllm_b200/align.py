@@ -72,8 +72,13 @@ def moe_align_block_size(
     max_num_tokens_padded = topk_ids.numel() + num_experts * (block_size - 1)
     if pad_sorted_ids:
         max_num_tokens_padded = round_up(max_num_tokens_padded, block_size)
-    sorted_ids, expert_ids, num_tokens_post_pad = _alloc(topk_ids, max_num_tokens_padded, block_size)
-    moe_align_block_size_triton(topk_ids, num_experts, block_size, sorted_ids, expert_ids, num_tokens_post_pad)
+    out = None
+    if topk_ids.is_cuda:
+        out = _lib.host().align(topk_ids, num_experts, block_size, max_num_tokens_padded)
+    if out is None:
+        out = _alloc(topk_ids, max_num_tokens_padded, block_size)
+        moe_align_block_size_triton(topk_ids, num_experts, block_size, *out)
+    sorted_ids, expert_ids, num_tokens_post_pad = out
     if expert_map is not None:
         expert_ids = expert_map[expert_ids]
     return sorted_ids, expert_ids, num_tokens_post_pad
@@ -96,8 +101,13 @@ def moe_align_block_size_no_tle(
         max_num_tokens_padded = round_up(max_num_tokens_padded, block_size)
     if topk_ids.numel() < num_experts:
         max_num_tokens_padded = min(topk_ids.numel() * block_size, max_num_tokens_padded)
-    sorted_ids, expert_ids, num_tokens_post_pad = _alloc(topk_ids, max_num_tokens_padded, block_size)
-    moe_align_block_size_triton(topk_ids, num_experts, block_size, sorted_ids, expert_ids, num_tokens_post_pad)
+    out = None
+    if topk_ids.is_cuda:
+        out = _lib.host().align(topk_ids, num_experts, block_size, max_num_tokens_padded)
+    if out is None:
+        out = _alloc(topk_ids, max_num_tokens_padded, block_size)
+        moe_align_block_size_triton(topk_ids, num_experts, block_size, *out)
+    sorted_ids, expert_ids, num_tokens_post_pad = out
     if expert_map is not None:
         expert_ids = expert_map[expert_ids]
     return sorted_ids, expert_ids, num_tokens_post_pad

@@ -10,13 +10,16 @@ import hashlib
 import os
 import shutil
 import subprocess
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmoe_sm100.so")
+# CPython extension over torch's C++ API and LIB: the native host path of the operators (csrc/host_ext.cpp)
+HOST_EXT = os.path.join(HERE, "_host_ext.so")
 STAMP = LIB + ".srchash"
-SOURCES = ["common.cu", "grouped_topk.cu", "topk_route.cu", "align.cu", "quant.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_wt.cu", "gemm_w8t.cu", "plan.cu", "route_rows.cu", "layer.cu",
-           "gemm_w8.cu", "gemm_small.cu", "gemm_api.cu", "router_gemm.cu", "ep_pack.cu"]
+SOURCES = ["common.cu", "grouped_topk.cu", "topk_route.cu", "align.cu", "quant.cu", "gemm_simt.cu", "gemm_tc.cu",
+           "gemm_wt.cu", "gemm_w8t.cu", "plan.cu", "route_rows.cu", "layer.cu", "gemm_w8.cu", "gemm_small.cu", "gemm_api.cu", "router_gemm.cu", "ep_pack.cu"]
 
 
 def _nvcc() -> str:
@@ -39,10 +42,24 @@ def _source_digest() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(STAMP):
+    if not os.path.exists(LIB) or not os.path.exists(HOST_EXT) or not os.path.exists(STAMP):
         return True
     with open(STAMP) as fh:
         return fh.read().strip() != _source_digest()
+
+
+def _host_ext_cmd() -> list:
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
+            os.path.join(CSRC, "host_ext.cpp"), "-o", HOST_EXT, "-L" + HERE, "-l:libmoe_sm100.so",
+            "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+            "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -70,6 +87,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}")
+    r = subprocess.run(_host_ext_cmd(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on host_ext.cpp:\n{r.stdout}")
     with open(STAMP, "w") as fh:
         fh.write(_source_digest())
     return LIB

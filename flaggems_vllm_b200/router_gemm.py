@@ -43,6 +43,10 @@ def _launch(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 def router_gemm(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """bf16 x bf16 -> fp32 GEMM for the MoE router gate: ``x`` [M, K], ``weight`` [N, K]."""
     logger.debug("GEMS ROUTER GEMM")
+    if x.is_cuda:
+        out = _lib.host().router_gemm(x, weight)
+        if out is not None:
+            return out
     if x.ndim != 2 or weight.ndim != 2:
         raise ValueError("router_gemm expects 2D x and weight tensors")
     if x.shape[1] != weight.shape[1]:

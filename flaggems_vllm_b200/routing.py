@@ -57,6 +57,11 @@ def grouped_topk(
 
     Returns (topk_weights fp32 [M, topk], topk_ids int32 [M, topk])."""
     logger.debug("GEMS GROUPED TOPK")
+    if is_padding is None and scores.is_cuda:
+        out = _lib.host().grouped_topk(scores, n_group, topk_group, topk, renormalize, routed_scaling_factor, bias,
+                                       scoring_func)
+        if out is not None:
+            return out
     if scores.ndim != 2:
         raise ValueError("scores must be a 2D Tensor")
     num_tokens, num_experts = scores.shape
@@ -99,6 +104,10 @@ def grouped_topk(
 
 def _launch_topk_route(topk_weights, topk_indices, token_expert_indices, gating_output, renormalize,
                        e_score_correction_bias, is_padding, *, sigmoid: bool, scale: float) -> None:
+    if is_padding is None and gating_output.is_cuda and _lib.host().topk_route(
+            topk_weights, topk_indices, token_expert_indices, gating_output, renormalize, e_score_correction_bias, sigmoid,
+            scale):
+        return
     # argument contract of the reference (src/flaggems_vllm/ops/topk_sigmoid.py:86-126)
     assert gating_output.ndim == 2 and topk_weights.ndim == 2
     if gating_output.device.type != "cuda":
