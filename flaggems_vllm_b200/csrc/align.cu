@@ -26,7 +26,7 @@
 // single-CTA kernel.
 #include <cooperative_groups.h>
 
-#include "moe_common.cuh"
+#include "sort_ids.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -303,6 +303,94 @@ align_cluster_kernel(const IdT* __restrict__ ids, int numel, int E, int block_si
   }
 }
 
+// The usual sizes (at most 1024 experts, 262144 ids): one pass over the ids with the ranks in registers, padding slots
+// written by a warp per expert and the unused tail by everybody, so no slot is written twice and the only
+// barriers are those of the scan.  B200, 256 experts, block 128, graph replay, kernels above: 65536 ids 26 us
+// (uniform) and 20 us (half of them on four experts).
+template <typename IdT, int CTAS, int ROUNDS>
+__device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int numel, int E, int block_size,
+                                                int32_t* __restrict__ sorted_ids, int sorted_cap,
+                                                int32_t* __restrict__ expert_ids, int expert_cap,
+                                                int32_t* __restrict__ num_post_pad, int32_t* __restrict__ status) {
+  using namespace sorting;
+  extern __shared__ __align__(16) int32_t sort_smem[];
+  const Shared sh = carve(sort_smem, E);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int rank = 0;
+  if constexpr (CTAS > 1) rank = (int)cg::this_cluster().block_rank();
+  bool bad = false;
+  int packed[ROUNDS], first, end;
+  rank_ids<CTAS, ROUNDS>(numel, E, sh, [&](int i) -> int {
+    const long long e = (long long)ids[i];
+    if (e >= E) bad = true;  // negative ids mean "no route" (padding rows, other ranks' slots)
+    return e >= 0 && e < E ? (int)e : -1;
+  }, packed, first, end);
+  if (bad) set_status(status, MOE_ST_BAD_EXPERT_ID);
+  int before = 0, all = 0, padded = 0;
+  if (tid < E) {
+    all = count_all<CTAS>(sh, tid, before);
+    padded = (all + block_size - 1) / block_size * block_size;
+  }
+  if constexpr (CTAS > 1) cg::this_cluster().barrier_arrive();  // this CTA has read its peers' totals
+  unsigned long long sum;
+  const int start = (int)scan_cta((unsigned long long)padded, sum);
+  const int total = (int)sum;
+  if (tid < E) {
+    sh.base[tid] = start;
+    sh.count[tid] = all;
+    sh.place[tid] = start + before;
+  }
+  if (tid == 0) sh.base[E] = total;
+  __syncthreads();
+  if (rank == 0 && tid == 0) num_post_pad[0] = total;
+  // the ids
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    if (packed[r] == kNone) continue;
+    const int e = packed[r] & 0x7FF;
+    const int pos = sh.place[e] + sh.hist[(size_t)warp * E + e] + (packed[r] >> 11);
+    if (pos < sorted_cap) sorted_ids[pos] = first + 32 * r + lane;
+  }
+  // padding slots and block ids of the experts: a warp per expert
+  for (int e = rank * kWarps + warp; e < E; e += CTAS * kWarps) {
+    const int s0 = sh.base[e], s1 = sh.base[e + 1];
+    if (s0 == s1) continue;
+    for (int p = s0 + sh.count[e] + lane; p < s1; p += 32)
+      if (p < sorted_cap) sorted_ids[p] = numel;
+    for (int b = s0 / block_size + lane; b < s1 / block_size; b += 32)
+      if (b < expert_cap) expert_ids[b] = e;
+  }
+  // what no expert uses
+  const int quads = min((total + 3) & ~3, sorted_cap);  // up to the first 16-byte boundary, then four at a time
+  if (rank == 0 && tid < quads - total) sorted_ids[total + tid] = numel;
+  const int whole = ((uintptr_t)sorted_ids & 15) == 0 ? (sorted_cap - quads) / 4 : 0;
+  for (int i = rank * kThreads + tid; i < whole; i += CTAS * kThreads)
+    reinterpret_cast<int4*>(sorted_ids + quads)[i] = make_int4(numel, numel, numel, numel);
+  for (int p = quads + 4 * whole + rank * kThreads + tid; p < sorted_cap; p += CTAS * kThreads) sorted_ids[p] = numel;
+  for (int b = total / block_size + rank * kThreads + tid; b < expert_cap; b += CTAS * kThreads) expert_ids[b] = -1;
+  if constexpr (CTAS > 1) cg::this_cluster().barrier_wait();  // no CTA leaves while its totals may still be read
+}
+template <typename IdT, int CTAS, int ROUNDS>
+__global__ void __launch_bounds__(sorting::kThreads)
+align_sort_kernel(const IdT* ids, int numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
+                  int expert_cap, int32_t* npp, int32_t* status) {
+  align_sort_body<IdT, CTAS, ROUNDS>(ids, numel, E, block_size, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status);
+}
+
+// a cluster at any size: even a call of a few ids writes tens of thousands of sentinels
+template <typename IdT>
+int launch_align_sort(const void* ids, int numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
+                      int expert_cap, int32_t* npp, int32_t* status, cudaStream_t st) {
+  using namespace sorting;
+#define MOE_ALIGN(C, R)                                                                                              \
+  launch_cluster(align_sort_kernel<IdT, C, R>, C, E, st, "align (sort)", (const IdT*)ids, numel, E, block_size, sorted_ids, \
+                 sorted_cap, expert_ids, expert_cap, npp, status)
+  if (numel <= capacity(kSmall, 2)) return MOE_ALIGN(kSmall, 2);
+  if (numel <= capacity(kLarge, 4)) return MOE_ALIGN(kLarge, 4);
+  return MOE_ALIGN(kLarge, 16);
+#undef MOE_ALIGN
+}
+
 }  // namespace
 }  // namespace moe
 
@@ -322,6 +410,11 @@ extern "C" int moe_align_block_size(const void* topk_ids, int ids_int64, int64_t
   // (numel + E*(bs-1) is the reference's bound); the kernel clips writes anyway.
   const int E = num_experts;
   cudaStream_t st = (cudaStream_t)stream;
+  if (E <= sorting::kMaxExperts && numel <= sorting::capacity(sorting::kLarge, 16))
+    return ids_int64 ? launch_align_sort<int64_t>(topk_ids, (int)numel, E, block_size, sorted_ids, (int)sorted_cap, expert_ids,
+                                                  (int)expert_cap, num_post_pad, status, st)
+                     : launch_align_sort<int32_t>(topk_ids, (int)numel, E, block_size, sorted_ids, (int)sorted_cap, expert_ids,
+                                                  (int)expert_cap, num_post_pad, status, st);
   cudaError_t ce;
   if (numel >= 4096 && E <= 1024) {
     // cluster of 8 CTAs; hist[W][E] + cta_tot[E] + blk_start[E+1] + 33 words per CTA

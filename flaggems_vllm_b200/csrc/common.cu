@@ -11,7 +11,7 @@
 
 namespace moe {
 
-int allow_smem(const void* kernel, int bytes) {
+int allow_smem(const void* kernel, int bytes, bool large_cluster) {
   int dev = 0;
   cudaGetDevice(&dev);
   static std::mutex mu;
@@ -20,6 +20,10 @@ int allow_smem(const void* kernel, int bytes) {
   if (done.count({kernel, dev})) return 0;
   const cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (ce != cudaSuccess) return fail((int)ce, "shared memory attribute (%d bytes): %s", bytes, cudaGetErrorString(ce));
+  if (large_cluster) {
+    const cudaError_t cl = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (cl != cudaSuccess) return fail((int)cl, "cluster size attribute: %s", cudaGetErrorString(cl));
+  }
   done.insert({kernel, dev});
   return 0;
 }

@@ -19,10 +19,41 @@ int check_launch(const char* what);
 // Limit, in nanoseconds, of every bounded barrier wait of the kernels launched from now on
 // (moe_set_wait_limit_ns; 2 s unless changed).
 unsigned long long wait_limit_ns();
-// Lets `kernel` use `bytes` of dynamic shared memory on the current device (set once per device, remembered).
-int allow_smem(const void* kernel, int bytes);
+// Lets `kernel` use `bytes` of dynamic shared memory (and clusters of more than 8 CTAs) on the current device (set once
+// per device, remembered).
+int allow_smem(const void* kernel, int bytes, bool large_cluster = false);
 // Multiprocessors of the current device (remembered).
 int sm_count();
+
+// Programmatic dependent launch.  The kernels of a layer are launched so that each may start while its predecessor
+// drains: what it does before pdl_wait() touches nothing the predecessor writes (barriers, TMEM, weights, and the
+// route plan, which is two kernels old for a GEMM; read past L1).  pdl_wait() returns when the predecessor has
+// completed and is visible; only then does a kernel let its own successor start, so whatever is older than the
+// predecessor is complete too.  Both are no-ops in a kernel launched the ordinary way.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launch with a cluster size (1 = none) and the programmatic dependency on what precedes it in the stream.
+template <typename Kernel, typename... Args>
+int launch_pdl(Kernel kern, dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, const char* what, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (ce != cudaSuccess) return fail((int)ce, "%s: %s", what, cudaGetErrorString(ce));
+  return check_launch(what);
+}
 
 template <typename T> struct ToF32;
 template <> struct ToF32<float> {

@@ -148,3 +148,16 @@ def test_int8_weight_layer_tiles(M, E, k, H, I, dtype):
     tw, ti = _route(M, E, k)
     out = fg.fused_experts_impl(x, w1, w2, tw, ti, use_int8_w8a16=True, per_channel_quant=True, w1_scale=s1, w2_scale=s2)
     _parity(out, O.fused_moe_w8a16_oracle(x, w1, w2, s1, s2, tw, ti), (M, E))
+
+
+@pytest.mark.parametrize("numel", [1, 31, 2048, 2049, 16384, 16385, 65536, 65537, 262144, 262145])
+@pytest.mark.parametrize("E,bs", [(5, 16), (256, 128), (1024, 7)])
+def test_align_slices(numel, E, bs):
+    """Clusters of 8 and 16, 2 to 16 rounds of ids per warp; ids without a place; every slot written."""
+    ids = T.make_align_ids(numel, 1, E, DEV, skewed=E > 5, seed=numel)
+    if numel > 40:
+        ids[7], ids[numel // 2] = -1, -3
+    got = fg.moe_align_block_size(ids, bs, E)
+    ref = O.moe_align_block_size_oracle(ids.cpu(), bs, E)
+    for g, r in zip(got, ref):
+        assert torch.equal(g.cpu(), torch.as_tensor(r))
