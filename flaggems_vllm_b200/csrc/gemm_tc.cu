@@ -238,7 +238,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int KBE = BYTE ? 128 : 64;  // elements of K per stage
   const int KB = (P.K + KBE - 1) / KBE;
-  const int npp = min((int64_t)P.num_post_pad[0], P.rows_cap);
+  const int npp = min((int64_t)__ldcg(P.num_post_pad), P.rows_cap);
   // work unit: one CTA and a 128-row align block; a CTA pair and a 256-row block; or one
   // CTA and a 256-row block (RB = 2).  UNIT = 128-row blocks per align block.
   constexpr int UNIT = PAIR ? 2 * RB : RB;
@@ -262,7 +262,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     nt = within / gsz;
     blk = first + within - nt * gsz;
   };
-  auto expert_of = [&](int blk) -> int { return P.tiles != nullptr ? P.tiles[blk].z : P.expert_ids[blk]; };
+  auto expert_of = [&](int blk) -> int { return P.tiles != nullptr ? __ldcg(&P.tiles[blk].z) : P.expert_ids[blk]; };
   // tile -> expert_ids index (blk), this CTA's 128-row block (mb), column tile (nt).  The expert of
   // the NEXT tile is fetched while the current one is worked on: a tile starts without waiting
   // for a global load (every role walks the same tile list with its own copy of e_next).
@@ -324,6 +324,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = aux->tmem_base;
+  // launched with a programmatic dependency over a route plan only (tc_gemm_plan)
+  if (warp != 0) {
+    pdl_wait();
+    pdl_trigger();
+  }
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
@@ -334,15 +339,37 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
       uint32_t it = 0;
       bool alive = true;
+      constexpr bool EARLY = !GATHER && !PAIR && RB == 1;
+      auto occupied_rows = [&](int blk) -> int {  // rows of A to fetch
+        if (EARLY && P.tiles != nullptr && !P.all_rows) return ((__ldcg(&P.tiles[blk].y) >> 16) + 7) & ~7;
+        return RB * BM;
+      };
+      // the stage's byte count and its weight tile
+      auto load_weights = [&](int kb, int s, int a_rows, int wrow0, int nt) {
+        mbar_expect_tx(&aux->full[s], (GATHER ? 0u : (uint32_t)a_rows * 128) + B_LOCAL_BYTES);  // GATHER: A rows arrive by cp.async (warps 2-3)
+#pragma unroll
+        for (int c = 0; c < BBox<GEMM1, PAIR>::COUNT; ++c)
+          tma_load_2d(&map_b, &aux->full[s], sB + (size_t)s * B_LOCAL_BYTES + c * (BBox<GEMM1, PAIR>::ROWS * 128),
+                      kb * KBE, wrow0 + box_row<GEMM1, PAIR>(nt, c, cr, P.Nout));
+      };
+      // route plan: the weights of the first stages do not wait for the kernel in front
+      int early = 0;
+      if constexpr (EARLY) {
+        if (P.tiles != nullptr && tile0 < total_tiles) {
+          int blk, nt;
+          tile_blk_nt(tile0, blk, nt);
+          const int a_rows = occupied_rows(blk), wrow0 = e_next * P.rows_w + P.w_row0;
+          for (; early < STAGES && early < KB; ++early)
+            if (leader) load_weights(early, early, a_rows, wrow0, nt);
+        }
+      }
+      pdl_wait();
       for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
         MOE_TILE_COORDS(tile)
         if (e < 0 || e >= P.E) continue;
         [[maybe_unused]] const int row0 = mb * BM;
         const int wrow0 = e * P.rows_w + P.w_row0;
-        [[maybe_unused]] int a_rows = RB * BM;
-        if constexpr (!GATHER && !PAIR && RB == 1) {
-          if (P.tiles != nullptr && !P.all_rows) a_rows = ((P.tiles[blk].y >> 16) + 7) & ~7;
-        }
+        [[maybe_unused]] const int a_rows = occupied_rows(blk);
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -350,25 +377,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (!mbar_wait(&aux->empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           MOE_TR(0, kb, 1);
           if (!leader) continue;
-          if constexpr (GATHER) {
-            mbar_expect_tx(&aux->full[s], B_LOCAL_BYTES);  // A rows arrive by cp.async (warps 2-3)
-          } else {
-            mbar_expect_tx(&aux->full[s], (uint32_t)a_rows * 128 + B_LOCAL_BYTES);
+          if (early > 0) --early;
+          else load_weights(kb, s, a_rows, wrow0, nt);
+          if constexpr (!GATHER) {
+            uint8_t* dst = sA + (size_t)s * A_LOCAL_BYTES;
             if (a_rows < RB * BM) {  // route plan, few rows: the rest of the stage keeps stale bytes, its results are never stored
-              uint8_t* dst = sA + (size_t)s * A_LOCAL_BYTES;
               int r = 0;
               for (; a_rows - r >= 16; r += 16) tma_load_2d(&map_a16, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
               if (r < a_rows) tma_load_2d(&map_a8, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
-            } else
+            } else {
 #pragma unroll
-            for (int j = 0; j < RB; ++j)
-              tma_load_2d(&map_a, &aux->full[s], sA + (size_t)s * A_LOCAL_BYTES + j * A_STAGE_BYTES, kb * KBE,
-                          row0 + j * BM);
+              for (int j = 0; j < RB; ++j) tma_load_2d(&map_a, &aux->full[s], dst + j * A_STAGE_BYTES, kb * KBE, row0 + j * BM);
+            }
           }
-#pragma unroll
-          for (int c = 0; c < BBox<GEMM1, PAIR>::COUNT; ++c)
-            tma_load_2d(&map_b, &aux->full[s], sB + (size_t)s * B_LOCAL_BYTES + c * (BBox<GEMM1, PAIR>::ROWS * 128),
-                        kb * KBE, wrow0 + box_row<GEMM1, PAIR>(nt, c, cr, P.Nout));
           MOE_TR(0, kb, 2);
         }
       }
@@ -611,7 +632,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tile_blk_nt(t, nx_blk, nx_nt);
         const int64_t pn = (int64_t)(UNIT * nx_blk + RB * cr) * BM + row;
         if (P.tiles != nullptr) {  // rows leave in sorted order, weighted by the combine
-          const int4 d = P.tiles[nx_blk];
+          const int4 d = __ldcg(P.tiles + nx_blk);
           nx_e = d.z;
           if (row < (d.y >> 16)) nx_sid = pn;
         } else {
@@ -879,7 +900,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P,
     return fail(MOE_E_DRIVER, "tensor-core GEMM: kernel was built with %d registers per thread, %d needed", regs, LAUNCH_REGS);
   const int rc = allow_smem((const void*)kern, (int)smem);
   if (rc) return rc;
-  cudaError_t ce;
+  const CUtensorMap &m_out = mo != nullptr ? *mo : ma, &m16 = ms != nullptr ? ms[0] : ma, &m8 = ms != nullptr ? ms[1] : ma;
+  const char* what = GEMM1 ? "gemm1 (tcgen05)" : "gemm2 (tcgen05)";
+  if (P.tiles != nullptr) return launch_pdl(kern, dim3((unsigned)grid), THREADS, smem, 1, st, what, ma, mb, m_out, m16, m8, P);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(THREADS);
@@ -892,9 +915,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P,
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ce = cudaLaunchKernelEx(&cfg, kern, ma, mb, mo != nullptr ? *mo : ma, ms != nullptr ? ms[0] : ma, ms != nullptr ? ms[1] : ma, P);
+  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, ma, mb, m_out, m16, m8, P);
   if (ce != cudaSuccess) return fail((int)ce, "tensor-core GEMM launch: %s", cudaGetErrorString(ce));
-  return check_launch(GEMM1 ? "gemm1 (tcgen05)" : "gemm2 (tcgen05)");
+  return check_launch(what);
 }
 
 }  // namespace tc

@@ -94,7 +94,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KB = (P.K + 127) / 128;
   const int item0 = blockIdx.x, step = gridDim.x;
-  const int total = P.counts[0] * P.R;
+  const int total = __ldcg(P.counts) * P.R;  // the route plan is older than the predecessor
   auto fetch = [&](int item) { return fetch_item(P, item); };
 
   if (threadIdx.x == 0) {
@@ -113,6 +113,12 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = aux->tmem_base;
 
+  // the weights, their widening and the tensor core do not wait for the kernel in front; the token rows and the
+  // results do
+  if (warp >= 3 && warp < 8) {
+    pdl_wait();
+    pdl_trigger();
+  }
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
     bool alive = true;
@@ -295,8 +301,8 @@ static int launch(const CUtensorMap& mw, const CUtensorMap (&mb)[3], const Param
   const int rc = allow_smem((const void*)kern, (int)smem);
   if (rc) return rc;
   const int sms = sm_count();
-  kern<<<(unsigned)(items < sms ? items : sms), THREADS, smem, st>>>(mw, mb[0], mb[1], mb[2], P);
-  return check_launch(GEMM1 ? "gemm1 (int8 weights, TMEM)" : "gemm2 (int8 weights, TMEM)");
+  return launch_pdl(kern, dim3((unsigned)(items < sms ? items : sms)), THREADS, smem, 1, st,
+                    GEMM1 ? "gemm1 (int8 weights, TMEM)" : "gemm2 (int8 weights, TMEM)", mw, mb[0], mb[1], mb[2], P);
 }
 
 }  // namespace w8t

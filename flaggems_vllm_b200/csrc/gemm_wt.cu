@@ -81,7 +81,7 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const int KB = (P.K + KBE - 1) / KBE;
   const int cr = (int)cluster_ctarank();  // 0 leads
   const int item0 = blockIdx.x / 2, step = gridDim.x / 2;
-  const int total = P.counts[0] * P.R;
+  const int total = __ldcg(P.counts) * P.R;  // the route plan is older than the predecessor
   auto fetch = [&](int item) { return fetch_item(P, item); };
 
   if (threadIdx.x == 0) {
@@ -101,6 +101,10 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across
   tc_fence_after();
   const uint32_t tmem_base = aux->tmem_base;
+  if (warp != 0) {
+    pdl_wait();
+    pdl_trigger();
+  }
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
@@ -115,21 +119,30 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       bool alive = true;
       Item nx = {};
       if (item0 < total) nx = fetch(item0);
+      auto load_weights = [&](const Item& it, int kb, uint32_t st) {
+        if (cr == 0) mbar_expect_tx(&aux->full[st], 2 * (A_BYTES + (uint32_t)(it.n >> 1) * 128));  // the peer's bytes may already have been counted
+        uint8_t* sA = smem + (size_t)st * STAGE_BYTES;
+        if constexpr (GEMM1) tma_load_5d_pair(&map_w, &aux->full[st], sA, kb * KBE, 0, 0, it.rt * 16 + cr * 8, it.e);
+        else tma_load_2d_pair(&map_w, &aux->full[st], sA, kb * KBE, it.e * P.Nout + it.rt * 256 + cr * 128);
+      };
+      // the weights of the first stages do not wait for the kernel in front
+      int early = 0;
+      if (item0 < total) {
+        for (; early < STAGES && early < KB; ++early)
+          if (leader) load_weights(nx, early, (uint32_t)early);
+      }
+      pdl_wait();
       for (int item = item0; item < total && alive; item += step) {
         const Item it = nx;
         if (item + step < total) nx = fetch(item + step);
         const int nh = it.n >> 1;                 // this CTA's share of the token rows
         const int brow = it.row0 + cr * nh;
-        const int wrow = GEMM1 ? it.rt * 16 + cr * 8 : it.e * P.Nout + it.rt * 256 + cr * 128;  // GEMM1: in groups of 8 outputs
-        const uint32_t pair_bytes = 2 * (A_BYTES + (uint32_t)nh * 128);
         for (int kb = 0; kb < KB; ++kb) {
           if (!mbar_wait(&aux->empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           if (leader) {
-            if (cr == 0) mbar_expect_tx(&aux->full[s], pair_bytes);  // the peer's bytes may already have been counted
-            uint8_t* sA = smem + (size_t)s * STAGE_BYTES;
-            if constexpr (GEMM1) tma_load_5d_pair(&map_w, &aux->full[s], sA, kb * KBE, 0, 0, wrow, it.e);
-            else tma_load_2d_pair(&map_w, &aux->full[s], sA, kb * KBE, wrow);
-            uint8_t* sB = sA + A_BYTES;
+            if (early > 0) --early;
+            else load_weights(it, kb, s);
+            uint8_t* sB = smem + (size_t)s * STAGE_BYTES + A_BYTES;
             int r = 0;
             for (; nh - r >= 64; r += 64) tma_load_2d_pair(&map_b64, &aux->full[s], sB + r * 128, kb * KBE, brow + r);
             for (; nh - r >= 16; r += 16) tma_load_2d_pair(&map_b16, &aux->full[s], sB + r * 128, kb * KBE, brow + r);
@@ -236,21 +249,8 @@ static int launch(const CUtensorMap& mw, const CUtensorMap (&mb)[3], const Param
     return fail(MOE_E_DRIVER, "grouped GEMM: kernel was built with %d registers per thread, %d needed", regs, LAUNCH_REGS);
   const int rc = allow_smem((const void*)kern, (int)smem);
   if (rc) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, mw, mb[0], mb[1], mb[2], P);
-  if (ce != cudaSuccess) return fail((int)ce, "grouped GEMM launch: %s", cudaGetErrorString(ce));
-  return check_launch(GEMM1 ? "gemm1 (pair, weights as M)" : "gemm2 (pair, weights as M)");
+  return launch_pdl(kern, dim3((unsigned)grid), THREADS, smem, 2, st, GEMM1 ? "gemm1 (pair, weights as M)" : "gemm2 (pair, weights as M)",
+                    mw, mb[0], mb[1], mb[2], P);
 }
 
 }  // namespace wt

@@ -183,6 +183,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps) grouped_topk_g32_kernel(
   __shared__ float s_group[kGroupWarps];
   __shared__ float s_w[32];
   __shared__ int32_t s_id[32];
+  pdl_wait();
+  pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, g = tid >> 5;
   const int64_t token = blockIdx.x;
   float* w_row = out_w + token * topk;
@@ -405,9 +407,8 @@ int launch_vpt(const ST* scores, int64_t s0, int64_t s1, const BT* bias, const u
   }
   // groups of exactly 32 experts whose candidates fit the CTA
   if (E == 32 * n_group && n_group <= kGroupWarps && topk * n_group <= E && M < (1ll << 31)) {
-    grouped_topk_g32_kernel<ST, BT><<<(unsigned)M, E, 0, st>>>(scores, s0, s1, bias, pad, n_group, topk_group, topk, renorm,
-                                                               scaling, scoring, w, ids);
-    return check_launch("grouped_topk (warp per group)");
+    return launch_pdl(grouped_topk_g32_kernel<ST, BT>, dim3((unsigned)M), E, 0, 1, st, "grouped_topk (warp per group)", scores, s0,
+                      s1, bias, pad, n_group, topk_group, topk, renorm, scaling, scoring, w, ids);
   }
   const int warps = 4;
   dim3 grid((unsigned)((M + warps - 1) / warps)), block(warps * 32);

@@ -359,6 +359,8 @@ __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restr
                                                                 const int32_t* __restrict__ row_ids, int64_t valid_below,
                                                                 const int32_t* __restrict__ indirect,
                                                                 uint8_t* __restrict__ q, float* __restrict__ scale_out) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int RPC = 256 / TPR;  // rows per CTA
   __shared__ float s_amax[TPR > 32 ? 8 : 1], s_nan[TPR > 32 ? 8 : 1];
   const int t = threadIdx.x % TPR, lane = threadIdx.x & 31;
@@ -487,12 +489,15 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
     bool done = false;                                                                                              \
     if constexpr (sizeof(T) == 2) {                                                                                 \
       if (vec && cols <= 2048) {                                                                                    \
-        rowwise_quant_vec_kernel<T, K, 32, 8><<<grid, 256, 0, st>>>((const T*)x, rows, (int)cols, SIN, row_ids,     \
-                                                                    valid_below, indirect, (uint8_t*)q, scale_out);           \
+        const int rc = launch_pdl(rowwise_quant_vec_kernel<T, K, 32, 8>, dim3(grid), 256, 0, 1, st, "rowwise_quant",   \
+                                  (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect, (uint8_t*)q, scale_out); \
+        if (rc) return rc;                                                                                          \
         done = true;                                                                                                \
       } else if (vec) {                                                                                             \
-        rowwise_quant_vec_kernel<T, K, 256, 4><<<grid_for(rows, 8), 256, 0, st>>>(                                  \
-            (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect, (uint8_t*)q, scale_out);                       \
+        const int rc = launch_pdl(rowwise_quant_vec_kernel<T, K, 256, 4>, dim3(grid_for(rows, 8)), 256, 0, 1, st,      \
+                                  "rowwise_quant", (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect,    \
+                                  (uint8_t*)q, scale_out);                                                             \
+        if (rc) return rc;                                                                                          \
         done = true;                                                                                                \
       }                                                                                                             \
     }                                                                                                               \

@@ -19,6 +19,8 @@ constexpr int kThreads = 256;
 constexpr int kPadParts = 8;
 __global__ void __launch_bounds__(kThreads) zero_padding_kernel(const int4* __restrict__ tiles, const int32_t* __restrict__ counts,
                                                                 int row_vec, uint4* __restrict__ rows) {
+  pdl_wait();
+  pdl_trigger();
   if ((int)blockIdx.x >= counts[0]) return;
   const int4 d = tiles[blockIdx.x];
   for (int r = (d.y >> 16) + blockIdx.y; r < (d.y & 0xFFFF); r += kPadParts) {
@@ -34,6 +36,8 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
                                                                        const int32_t* __restrict__ row_index,
                                                                        int64_t rows_cap, uint8_t* __restrict__ q,
                                                                        float* __restrict__ scales_t) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t m = blockIdx.y;
   const int g = (blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
@@ -71,6 +75,8 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
 __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint4* __restrict__ x, int vec, int k,
                                                                 const int32_t* __restrict__ row_index,
                                                                 uint4* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t m = blockIdx.y;
   const int c = blockIdx.x * 2 * kThreads + threadIdx.x;
   uint4 v[2];
@@ -89,6 +95,8 @@ __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint4* __r
 // dst[row_index[i]] = src[i / div] (one float per route: route weights, or a token's activation scale)
 __global__ void scatter_floats_kernel(const float* __restrict__ src, int64_t numel, int div,
                                       const int32_t* __restrict__ row_index, float* __restrict__ dst) {
+  pdl_wait();
+  pdl_trigger();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += (int64_t)gridDim.x * blockDim.x) {
     const int r = row_index[i];
     if (r >= 0) dst[r] = src[i / div];
@@ -101,6 +109,8 @@ template <typename T, bool WEIGHTED>
 __global__ void __launch_bounds__(kThreads) combine_kernel(const T* __restrict__ y, const float* __restrict__ weight,
                                                            const int32_t* __restrict__ row_index, int k, int vec,
                                                            T* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int V = 16 / sizeof(T);
   const int64_t m = blockIdx.y;
   const int c = blockIdx.x * kThreads + threadIdx.x;
@@ -138,9 +148,8 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const T* __restrict__
 
 // M <= 65535 for all of these (the second grid dimension): the layer call checks it.
 int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, cudaStream_t st) {
-  zero_padding_kernel<<<dim3((unsigned)tiles_cap, kPadParts), kThreads, 0, st>>>((const int4*)tiles, counts, (int)(row_bytes / 16),
-                                                                                 (uint4*)rows);
-  return check_launch("zero padding rows");
+  return launch_pdl(zero_padding_kernel, dim3((unsigned)tiles_cap, kPadParts), kThreads, 0, 1, st, "zero padding rows",
+                    (const int4*)tiles, counts, (int)(row_bytes / 16), (uint4*)rows);
 }
 
 int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,
@@ -148,38 +157,33 @@ int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const
   const int groups = H / 128;
   const dim3 grid((unsigned)((groups + 15) / 16), (unsigned)M);
   if (dtype == MOE_BF16)
-    scatter_quant_group_kernel<__nv_bfloat16><<<grid, kThreads, 0, st>>>((const __nv_bfloat16*)x, groups, k, row_index, rows_cap,
-                                                                        (uint8_t*)q, scales_t);
-  else
-    scatter_quant_group_kernel<__half><<<grid, kThreads, 0, st>>>((const __half*)x, groups, k, row_index, rows_cap, (uint8_t*)q,
-                                                                 scales_t);
-  return check_launch("scatter (1x128 quantised)");
+    return launch_pdl(scatter_quant_group_kernel<__nv_bfloat16>, grid, kThreads, 0, 1, st, "scatter (1x128 quantised)",
+                      (const __nv_bfloat16*)x, groups, k, row_index, rows_cap, (uint8_t*)q, scales_t);
+  return launch_pdl(scatter_quant_group_kernel<__half>, grid, kThreads, 0, 1, st, "scatter (1x128 quantised)", (const __half*)x,
+                    groups, k, row_index, rows_cap, (uint8_t*)q, scales_t);
 }
 
 int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st) {
   const int vec = (int)(row_bytes / 16);
-  scatter_rows_kernel<<<dim3((unsigned)((vec + 2 * kThreads - 1) / (2 * kThreads)), (unsigned)M), kThreads, 0, st>>>(
-      (const uint4*)x, vec, k, row_index, (uint4*)out);
-  return check_launch("scatter");
+  return launch_pdl(scatter_rows_kernel, dim3((unsigned)((vec + 2 * kThreads - 1) / (2 * kThreads)), (unsigned)M), kThreads, 0, 1, st,
+                    "scatter", (const uint4*)x, vec, k, row_index, (uint4*)out);
 }
 
 int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_index, float* dst, cudaStream_t st) {
   const int64_t blocks = (numel + 255) / 256;
-  scatter_floats_kernel<<<(unsigned)(blocks < 1024 ? blocks : 1024), 256, 0, st>>>(src, numel, div, row_index, dst);
-  return check_launch("scatter (floats)");
+  return launch_pdl(scatter_floats_kernel, dim3((unsigned)(blocks < 1024 ? blocks : 1024)), 256, 0, 1, st, "scatter (floats)", src,
+                    numel, div, row_index, dst);
 }
 
 int combine_rows(const void* y, int dtype, const float* weight, const int32_t* row_index, int64_t M, int k, int64_t H, void* out,
                  cudaStream_t st) {
   const int vec = (int)(H / 8);
   const dim3 grid((unsigned)((vec + kThreads - 1) / kThreads), (unsigned)M);
-#define MOE_COMBINE(T)                                                                                               \
-  (weight != nullptr ? combine_kernel<T, true><<<grid, kThreads, 0, st>>>((const T*)y, weight, row_index, k, vec, (T*)out) \
-                     : combine_kernel<T, false><<<grid, kThreads, 0, st>>>((const T*)y, weight, row_index, k, vec, (T*)out))
-  if (dtype == MOE_BF16) MOE_COMBINE(__nv_bfloat16);
-  else MOE_COMBINE(__half);
+#define MOE_COMBINE(T, W) \
+  launch_pdl(combine_kernel<T, W>, grid, kThreads, 0, 1, st, "combine", (const T*)y, weight, row_index, k, vec, (T*)out)
+  if (dtype == MOE_BF16) return weight != nullptr ? MOE_COMBINE(__nv_bfloat16, true) : MOE_COMBINE(__nv_bfloat16, false);
+  return weight != nullptr ? MOE_COMBINE(__half, true) : MOE_COMBINE(__half, false);
 #undef MOE_COMBINE
-  return check_launch("combine");
 }
 
 }  // namespace moe

@@ -25,13 +25,11 @@ __device__ __forceinline__ uint32_t tr_ordered_bits(float v) {
 __device__ __forceinline__ uint64_t tr_key(float v, uint32_t idx) {
   return ((uint64_t)tr_ordered_bits(v) << 32) | (uint64_t)(0xFFFFFFFFu - idx);
 }
+// two 32-bit reductions: the largest high word, then the largest low word among the lanes that hold it
 __device__ __forceinline__ uint64_t tr_warp_max(uint64_t k) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    uint64_t o = __shfl_xor_sync(0xFFFFFFFFu, k, off);
-    k = o > k ? o : k;
-  }
-  return k;
+  const uint32_t hi = (uint32_t)(k >> 32), lo = (uint32_t)k;
+  const uint32_t mh = __reduce_max_sync(0xFFFFFFFFu, hi);
+  return ((uint64_t)mh << 32) | __reduce_max_sync(0xFFFFFFFFu, hi == mh ? lo : 0u);
 }
 
 template <typename LT, typename IT, int VPT>
@@ -39,6 +37,8 @@ __global__ void __launch_bounds__(128) topk_route_kernel(
     const LT* __restrict__ logits, const float* __restrict__ bias, const uint8_t* __restrict__ is_padding,
     int64_t M, int E, int topk, int sigmoid, int renormalize, float scale, float* __restrict__ out_w,
     IT* __restrict__ out_ids, int32_t* __restrict__ out_src) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t token = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= M) return;
@@ -127,17 +127,17 @@ template <typename LT, typename IT>
 int launch_vpt(const LT* logits, const float* bias, const uint8_t* pad, int64_t M, int E, int topk, int sigmoid,
                int renorm, float scale, float* w, IT* ids, int32_t* src, cudaStream_t st) {
   const int warps = 4;
-  dim3 grid((unsigned)((M + warps - 1) / warps)), block(warps * 32);
+  dim3 grid((unsigned)((M + warps - 1) / warps));
 #define MOE_TR_LAUNCH(V) \
-  topk_route_kernel<LT, IT, V><<<grid, block, 0, st>>>(logits, bias, pad, M, E, topk, sigmoid, renorm, scale, w, ids, src)
-  if (E <= 32) MOE_TR_LAUNCH(1);
-  else if (E <= 64) MOE_TR_LAUNCH(2);
-  else if (E <= 128) MOE_TR_LAUNCH(4);
-  else if (E <= 256) MOE_TR_LAUNCH(8);
-  else if (E <= 512) MOE_TR_LAUNCH(16);
-  else MOE_TR_LAUNCH(32);
+  launch_pdl(topk_route_kernel<LT, IT, V>, grid, warps * 32, 0, 1, st, "topk_route", logits, bias, pad, M, E, topk, sigmoid, renorm, \
+             scale, w, ids, src)
+  if (E <= 32) return MOE_TR_LAUNCH(1);
+  if (E <= 64) return MOE_TR_LAUNCH(2);
+  if (E <= 128) return MOE_TR_LAUNCH(4);
+  if (E <= 256) return MOE_TR_LAUNCH(8);
+  if (E <= 512) return MOE_TR_LAUNCH(16);
+  return MOE_TR_LAUNCH(32);
 #undef MOE_TR_LAUNCH
-  return check_launch("topk_route");
 }
 
 template <typename LT>

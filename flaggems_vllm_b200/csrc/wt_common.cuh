@@ -49,12 +49,12 @@ __device__ __forceinline__ float swigluoai(float g, float u, float alpha, float 
 __device__ __forceinline__ Item fetch_item(const Params& P, int item) {
   Item it;
   const int t0 = item / P.R;
-  int4 d = P.tiles[t0];
+  int4 d = __ldcg(P.tiles + t0);  // past L1: this may run before pdl_wait()
   const int first = d.w & 0xFFFF, q = (int)((uint32_t)d.w >> 16);
   const int within = item - first * P.R;
   it.rt = within / q;
   const int t = first + within - it.rt * q;
-  if (t != t0) d = P.tiles[t];
+  if (t != t0) d = __ldcg(P.tiles + t);
   it.row0 = d.x; it.n = d.y & 0xFFFF; it.e = d.z;
   return it;
 }
