@@ -134,9 +134,6 @@ PyObject* fused_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   } else if (w1.scalar_type() != x.scalar_type() || w2.scalar_type() != x.scalar_type()) {
     MOE_NONE;
   }
-  // the small-batch schedule of gemm_small.cu (fused_moe._use_small_path)
-  const int64_t numel = M * k;
-  if ((mode == MOE_MODE_HALF && numel <= 8) || (mode == MOE_MODE_W8A16 && numel <= 16)) MOE_NONE;
   const int32_t* emap = nullptr;
   const int64_t experts = ng == -1 ? E : ng;
   if (a[14] != Py_None) {

@@ -18,6 +18,14 @@ int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, in
 int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
                  const void* tiles, const int32_t* rows, int64_t numel, int64_t rows_cap, int E, int K, int Nout, void* out,
                  float* out_scales_t, const float* row_weight, bool all_rows, bool staged, int32_t* status, cudaStream_t st);
+int small_align(const void* ids, int ids64, int numel, int E, int32_t* sorted_ids, int rows_cap, int32_t* expert_ids, int32_t* npp,
+                int32_t* counters, int ncounters, int32_t* status, cudaStream_t st);
+int small_slices(int mode, bool gemm1, int K, int N, int blocks);
+int small_gemm(bool pdl, int gemm1, int mode, int act_dtype, const void* a, int64_t num_tokens, int topk, const void* w,
+               const float* w_scale, const int32_t* expert_ids, const int32_t* sorted_ids, const int32_t* num_post_pad,
+               const int32_t* expert_map, int num_experts_global, const float* route_weight, int mul_weight, const void* topk_ids,
+               int ids_int64, int64_t rows_cap, int E, int K, int Nout, void* out, void* final_out, int k_slices, float* partial,
+               int32_t* unit_counters, int32_t* token_counters, int32_t* status, cudaStream_t st);
 int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_index, float* dst, cudaStream_t st);
 int combine_rows(const void* y, int dtype, const float* weight, const int32_t* row_index, int64_t M, int k, int64_t H, void* out,
                  cudaStream_t st);
@@ -37,6 +45,7 @@ int w8t_gemm(bool gemm1, bool wide, int act_dtype, const void* a, const void* w,
 namespace {
 // Which grouped GEMM serves the call and how the plan cuts the rows for it.
 struct Choice {
+  bool small;       // gemm_small.cu: blocks of 8 routes, K split over the chip; no scatter, the sum inside GEMM2
   bool pair;        // gemm_wt.cu: weights as the M operand of a CTA pair; else gemm_tc.cu: 128 tokens as M
   bool wide;        // weight-only int8 (gemm_w8t.cu): tiles of up to 160 tokens instead of 64
   int gran, tile;   // row granule and most rows of a tile
@@ -51,7 +60,14 @@ bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
   return wt_serves(mode, act_dtype, H, I);
 }
 
-Choice choose(int mode, int act_kind, int64_t numel, int E) {
+// The split-K weight streaming of gemm_small.cu: three launches instead of five, every SM busy however few tiles there
+// are, but one CTA needs more instructions per byte than the tile kernels.  So it is for calls whose launches count: up to
+// 8 routes that read up to 1 GB of weights (Mixtral shape: one token, 2 routes, 0.7 GB, 143 against 171 us with the tile
+// kernels; two tokens 230 against 225; four tokens 394 against 334; E8 H1024 I2048: four tokens 29 against 38).
+constexpr int kSmallRoutes = 8;
+constexpr int64_t kSmallBytes = 1000000000;
+
+Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
   const int64_t per_expert = numel / (E > 0 ? E : 1);
   Choice c = {};
   if (mode == MOE_MODE_W8A16) {
@@ -59,6 +75,11 @@ Choice choose(int mode, int act_kind, int64_t numel, int E) {
     c.wide = per_expert > 40;
     c.gran = 16;
     c.tile = w8t_tile(c.wide);
+    return c;
+  }
+  if (mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && numel <= kSmallRoutes && numel * 6 * H * I <= kSmallBytes &&
+      H % 128 == 0 && I % 64 == 0) {
+    c.small = true;
     return c;
   }
   // FP8 block scales: tokens as M (gemm_wt.cu says why).  Half precision: up to 96 rows per expert the weights are
@@ -82,20 +103,40 @@ bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_IN
 struct Piece { int ws; int64_t at; };
 struct Layout {
   int64_t rows_cap, tiles_cap;
-  Piece row_index, tiles, counts, row_weight, tmp_scales, x_rows, x_scales, tmp_q, act, act_q, act_scales, y;
+  Piece row_index, tiles, counts, row_weight, tmp_scales, x_rows, x_scales, tmp_q, act, act_q, act_scales, y, small_counters;
   int64_t bytes[4];
+  int slices[2];         // gemm_small.cu: K slices of GEMM1, GEMM2
+  int64_t ncounters[3];  // and its counters: units of GEMM1, of GEMM2, tokens of GEMM2
 };
 
-Layout layout(int mode, const Choice& c, int64_t M, int k, int E_local, int H, int I) {
+Layout layout(int mode, const Choice& c, int64_t M, int k, int E, int E_local, int H, int I) {
   Layout L = {};
   const int64_t numel = M * k;
-  plan_caps(numel, E_local, c.gran, c.tile, &L.rows_cap, &L.tiles_cap);
   auto take = [&](int ws, int64_t bytes) {
     const Piece p = {ws, L.bytes[ws]};
     L.bytes[ws] += (bytes + 255) / 256 * 256;
     return p;
   };
   const bool byte = mode != MOE_MODE_HALF && mode != MOE_MODE_W8A16, row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
+  if (c.small) {
+    const int64_t used = numel < E ? numel : E;
+    L.rows_cap = (numel + used * 7 + 7) / 8 * 8;
+    int64_t part[2] = {0, 0}, units[2] = {0, 0}, toks = 0;
+    for (int g = 0; g < 2; ++g) {
+      L.slices[g] = small_slices(mode, g == 0, g == 0 ? H : I, g == 0 ? I : H, (int)used);
+      moe_small_m_plan(g == 0, mode, g == 0 ? H : I, g == 0 ? I : H, L.rows_cap, M, L.slices[g], &part[g], &units[g], &toks);
+    }
+    L.ncounters[0] = units[0]; L.ncounters[1] = units[1]; L.ncounters[2] = toks;
+    L.row_index = take(0, L.rows_cap * 4);   // sorted_ids
+    L.tiles = take(0, L.rows_cap / 8 * 4);   // expert_ids
+    L.counts = take(0, 8);                   // num_post_pad
+    L.small_counters = take(0, (units[0] + units[1] + toks) * 4);
+    L.x_rows = take(1, (part[0] > part[1] ? part[0] : part[1]) * 4 + 16);  // partial sums
+    L.act = take(2, L.rows_cap * I * 2);
+    L.y = take(3, numel * H * 2);
+    return L;
+  }
+  plan_caps(numel, E_local, c.gran, c.tile, &L.rows_cap, &L.tiles_cap);
   L.row_index = take(0, numel * 4);
   L.tiles = take(0, L.tiles_cap * 16);
   L.counts = take(0, 8);
@@ -119,7 +160,7 @@ extern "C" int moe_layer_workspace(int mode, int act_dtype, int64_t num_tokens, 
   if (num_tokens <= 0 || num_tokens > 65535 || topk <= 0 || topk > 32 || E_local <= 0 || H <= 0 || I <= 0 || !bytes ||
       !plan_serves(num_tokens * topk, num_experts, E_local) || !sizes_served(mode, act_dtype, H, I, activation))
     return fail(MOE_E_SHAPE, "layer: mode, type or sizes are not served by this call");
-  const Layout L = layout(mode, choose(mode, activation, num_tokens * topk, num_experts), num_tokens, topk, E_local, H, I);
+  const Layout L = layout(mode, choose(mode, activation, num_tokens * topk, num_experts, H, I), num_tokens, topk, num_experts, E_local, H, I);
   for (int i = 0; i < 4; ++i) bytes[i] = L.bytes[i];
   return 0;
 }
@@ -142,8 +183,8 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
   const bool row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
   if (mode != MOE_MODE_HALF && (!w1_scale || !w2_scale)) return fail(MOE_E_BADARG, "layer: weight scales missing");
   cudaStream_t st = (cudaStream_t)stream;
-  const Choice c = choose(mode, activation, numel, num_experts);
-  const Layout L = layout(mode, c, M, topk, E_local, H, I);
+  const Choice c = choose(mode, activation, numel, num_experts, H, I);
+  const Layout L = layout(mode, c, M, topk, num_experts, E_local, H, I);
   void* const base[4] = {ws_plan, ws_x, ws_act, ws_y};
   auto at = [&](const Piece& p) -> void* { return (uint8_t*)base[p.ws] + p.at; };
   int32_t* row_index = (int32_t*)at(L.row_index);
@@ -152,6 +193,23 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
   float* x_scales = (float*)at(L.x_scales);
   float* act_scales = (float*)at(L.act_scales);
   float* row_weight = weight_on_input ? (float*)at(L.row_weight) : nullptr;
+  if (c.small) {
+    int32_t* cnt = (int32_t*)at(L.small_counters);
+    int32_t* experts = (int32_t*)tiles;
+    const int64_t* n = L.ncounters;
+    if (stages & 1)
+      rc = small_align(topk_ids, ids_int64, (int)numel, num_experts, row_index, (int)L.rows_cap, experts, counts, cnt,
+                       (int)(n[0] + n[1] + n[2]), status, st);
+    if (!rc && (stages & 4))
+      rc = small_gemm(true, 1, mode, act_dtype, x, M, topk, w1, w1_scale, experts, row_index, counts, expert_map, num_experts,
+                      topk_weights, weight_on_input, topk_ids, ids_int64, L.rows_cap, E_local, H, I, at(L.act), nullptr, L.slices[0],
+                      (float*)at(L.x_rows), cnt, nullptr, status, st);
+    if (!rc && (stages & 16))
+      rc = small_gemm(true, 0, mode, act_dtype, at(L.act), M, topk, w2, w2_scale, experts, row_index, counts, expert_map, num_experts,
+                      topk_weights, !weight_on_input, topk_ids, ids_int64, L.rows_cap, E_local, I, H, at(L.y), out, L.slices[1],
+                      (float*)at(L.x_rows), cnt + n[0], cnt + n[0] + n[1], status, st);
+    return rc;
+  }
   if (stages & 1) {
     rc = plan_routes(topk_ids, ids_int64, numel, num_experts, expert_map, E_local, c.gran, c.tile,
                      row_index, L.rows_cap, tiles, L.tiles_cap, counts, status, st);

@@ -167,7 +167,9 @@ def _small_eligible(mode, act_dtype, H, I, k) -> bool:
 
 
 def _use_small_path(mode, act_dtype, H, I, numel, k) -> bool:
-    """The weight-streaming split-K schedule serves the smallest decode batches.  Measured under
+    """Which calls of the staged pipeline (intermediates kept, kernels pinned by a switch) take the
+    weight-streaming split-K schedule; ordinary calls go through the native layer call, whose own
+    rule stands in csrc/layer.cu.  Measured under
     CUDA-graph replay it beats the 128-row tensor-core tiles for half precision up to 8 routes
     per call (Mixtral shape, one token: 0.162 against 0.193 ms) and for weight-only int8 up to
     16 routes (Qwen3 shape, one token: 0.049 against 0.054 ms); for FP8 block scales the tile
@@ -539,6 +541,13 @@ def run_chunk(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w2_scal
     native_mark = mark or STAGE_HOOK
     if mark is None:
         mark = STAGE_HOOK or _no_mark
+    if use_tensor_cores is None and keep is None and not (mode == _lib.MODE_HALF and w1_scale is not None) \
+            and not any(v in os.environ for v in _KERNEL_SWITCHES) and run_chunk_native(
+                x, w1, w2, topk_weights, topk_ids, out, mode=mode, w1_scale=w1_scale, w2_scale=w2_scale,
+                global_num_experts=global_num_experts, expert_map=expert_map,
+                apply_router_weight_on_input=apply_router_weight_on_input, mark=native_mark, act_fn=act_fn,
+                row_quant=row_quant):
+        return
     # (half-precision weights with per-channel scales -- the widened int8 experiment -- stay on the tile kernels)
     if use_tensor_cores is None and act_fn[0] == _lib.ACT_SILU and not (
             mode == _lib.MODE_HALF and w1_scale is not None) and _use_small_path(
@@ -546,13 +555,6 @@ def run_chunk(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w2_scal
         run_chunk_small(x, w1, w2, topk_weights, topk_ids, out, mode=mode, w1_scale=w1_scale, w2_scale=w2_scale,
                         global_num_experts=global_num_experts, expert_map=expert_map,
                         apply_router_weight_on_input=apply_router_weight_on_input, keep=keep, mark=mark)
-        return
-    if use_tensor_cores is None and keep is None and not (mode == _lib.MODE_HALF and w1_scale is not None) \
-            and not any(v in os.environ for v in _KERNEL_SWITCHES) and run_chunk_native(
-                x, w1, w2, topk_weights, topk_ids, out, mode=mode, w1_scale=w1_scale, w2_scale=w2_scale,
-                global_num_experts=global_num_experts, expert_map=expert_map,
-                apply_router_weight_on_input=apply_router_weight_on_input, mark=native_mark, act_fn=act_fn,
-                row_quant=row_quant):
         return
     row_quant2 = None
     if mode == _lib.MODE_FP8_BLOCK:

@@ -117,6 +117,24 @@ def test_fp8_block_layer_tiles(M, E, k):
     assert torch.equal(fg.fused_experts_impl(x2, w1, w2, tw, ti, inplace=True, **kw), out)
 
 
+@pytest.mark.parametrize("M,E,k,H,I", [
+    (1, 1, 1, 128, 64), (1, 8, 8, 256, 192), (8, 2, 1, 2176, 128), (4, 8, 2, 1024, 2048),
+    (3, 4, 3, 128, 64)])  # nine routes: the tile kernels
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_half_layer_few_routes(M, E, k, H, I, dtype):
+    """One to eight routes (one K slice and several), a repeated call on the same stream, int64 ids, no route at all."""
+    x, w1, w2, tw, ti = _half_layer(M, E, k, H, I, dtype)
+    ref = O.fused_moe_half_oracle(x, w1, w2, tw, ti)
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti)
+    _parity(out, ref, (M, E))
+    assert torch.equal(fg.fused_experts_impl(x, w1, w2, tw, ti.long()), out)
+    ti[0] = -1
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti)
+    assert bool((out[0] == 0).all())
+    if M > 1:
+        _parity(out[1:], ref[1:], (M, E))
+
+
 @pytest.mark.parametrize("M", [7, 300, 2500])
 def test_layer_with_local_experts_and_weights_on_the_input(M):
     """expert_map (routes of other ranks get no rows), ids out of range, route weights applied on the input."""
