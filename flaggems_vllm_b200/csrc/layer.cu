@@ -31,6 +31,9 @@ int combine_rows(const void* y, int dtype, const float* weight, const int32_t* r
                  cudaStream_t st);
 int rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, const float* scale_in,
                   const int32_t* row_ids, int64_t valid_below, const int32_t* indirect, void* q, float* scale_out, cudaStream_t st);
+bool rowwise_scatter_serves(int kind, int64_t cols);
+int rowwise_scatter(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, int k, const int32_t* row_index, void* q,
+                    float* scales, cudaStream_t st);
 bool wt_serves(int mode, int act_dtype, int H, int I);
 int wt_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
             const void* tiles, int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K,
@@ -220,10 +223,14 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
       rc = scatter_quant_group(x, act_dtype, M, H, topk, row_index, L.rows_cap, at(L.x_rows), x_scales, st);
     } else if (row) {
       const bool per_row = quant_kind1 == 0 || quant_kind1 == 1;
-      float* sc = (float*)at(L.tmp_scales);
-      rc = rowwise_quant(x, act_dtype, M, H, quant_kind1, quant_scale1, nullptr, 0, nullptr, at(L.tmp_q), sc, st);
-      if (!rc) rc = scatter_rows(at(L.tmp_q), M, H, topk, row_index, at(L.x_rows), st);
-      if (!rc) rc = scatter_floats(sc, numel, per_row ? topk : (int)numel, row_index, x_scales, st);
+      if (rowwise_scatter_serves(quant_kind1, H)) {
+        rc = rowwise_scatter(x, act_dtype, M, H, quant_kind1, topk, row_index, at(L.x_rows), x_scales, st);
+      } else {
+        float* sc = (float*)at(L.tmp_scales);
+        rc = rowwise_quant(x, act_dtype, M, H, quant_kind1, quant_scale1, nullptr, 0, nullptr, at(L.tmp_q), sc, st);
+        if (!rc) rc = scatter_rows(at(L.tmp_q), M, H, topk, row_index, at(L.x_rows), st);
+        if (!rc) rc = scatter_floats(sc, numel, per_row ? topk : (int)numel, row_index, x_scales, st);
+      }
     } else {
       rc = scatter_rows(x, M, (int64_t)H * 2, topk, row_index, at(L.x_rows), st);
     }

@@ -353,12 +353,13 @@ __global__ void __launch_bounds__(256) rowwise_quant_kernel(const T* __restrict_
 // long rows) hold the row in registers (CH pieces of 8 elements each), so it is read once, with all loads in
 // flight, and written with 8-byte stores.  The kernel above reads every row twice, 64 bytes per warp and
 // instruction (500 x 2048 and 4000 x 768: 29 us for both).
-template <typename T, int KIND, int TPR, int CH>
+// SCATTER: row r goes to the rows `indirect`[r k + j], j < k (negative: none), its scale with it.
+template <typename T, int KIND, int TPR, int CH, bool SCATTER = false>
 __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restrict__ x, int64_t rows, int cols,
                                                                 const float* __restrict__ scale_in,
                                                                 const int32_t* __restrict__ row_ids, int64_t valid_below,
                                                                 const int32_t* __restrict__ indirect,
-                                                                uint8_t* __restrict__ q, float* __restrict__ scale_out) {
+                                                                uint8_t* __restrict__ q, float* __restrict__ scale_out, int k = 1) {
   pdl_wait();
   pdl_trigger();
   constexpr int RPC = 256 / TPR;  // rows per CTA
@@ -366,11 +367,16 @@ __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restr
   const int t = threadIdx.x % TPR, lane = threadIdx.x & 31;
   const int pieces = cols / 8;
   for (int64_t idx = (int64_t)blockIdx.x * RPC + threadIdx.x / TPR; idx < rows; idx += (int64_t)gridDim.x * RPC) {
-    const int64_t r = indirect != nullptr ? (int64_t)indirect[idx] : idx;
+    const int64_t r = !SCATTER && indirect != nullptr ? (int64_t)indirect[idx] : idx;
     if (r < 0) continue;
     if (row_ids != nullptr) {  // uniform over the threads of a row
       const int64_t id = row_ids[r];
       if (id < 0 || id >= valid_below) continue;
+    }
+    int dst = -1;
+    if constexpr (SCATTER) {
+      if (lane < k) dst = indirect[idx * k + lane];
+      if (__ballot_sync(0xFFFFFFFFu, dst >= 0) == 0) continue;  // no route of this token is local
     }
     uint4 raw[CH];
 #pragma unroll
@@ -410,10 +416,15 @@ __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restr
       } else {
         scale = fmaxf(fmaxf(amax, 1e-10f) / kFp8Max, 1.0f / (kFp8Max * 512.0f));
       }
-      if (t == 0) scale_out[r] = scale;
+      if constexpr (SCATTER) {
+        if (t < 32 && dst >= 0) scale_out[dst] = scale;
+      } else {
+        if (t == 0) scale_out[r] = scale;
+      }
     } else {
       scale = scale_in[0];
     }
+    [[maybe_unused]] uint2 out[CH];
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (t + c * TPR < pieces) {
@@ -428,7 +439,17 @@ __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restr
           else o = f32_to_fp8e4m3(fminf(fmaxf(v / scale, -kFp8Max), kFp8Max));
           w[i >> 2] |= (uint32_t)o << (8 * (i & 3));
         }
-        reinterpret_cast<uint2*>(q + r * cols)[t + c * TPR] = make_uint2(w[0], w[1]);
+        if constexpr (SCATTER) out[c] = make_uint2(w[0], w[1]);
+        else reinterpret_cast<uint2*>(q + r * cols)[t + c * TPR] = make_uint2(w[0], w[1]);
+      }
+    }
+    if constexpr (SCATTER) {
+      for (int j = 0; j < k; ++j) {
+        const int64_t d = __shfl_sync(0xFFFFFFFFu, dst, j);
+        if (d < 0) continue;
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+          if (t + c * TPR < pieces) reinterpret_cast<uint2*>(q + d * cols)[t + c * TPR] = out[c];
       }
     }
   }
@@ -490,13 +511,13 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
     if constexpr (sizeof(T) == 2) {                                                                                 \
       if (vec && cols <= 2048) {                                                                                    \
         const int rc = launch_pdl(rowwise_quant_vec_kernel<T, K, 32, 8>, dim3(grid), 256, 0, 1, st, "rowwise_quant",   \
-                                  (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect, (uint8_t*)q, scale_out); \
+                                  (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect, (uint8_t*)q, scale_out, 1); \
         if (rc) return rc;                                                                                          \
         done = true;                                                                                                \
       } else if (vec) {                                                                                             \
         const int rc = launch_pdl(rowwise_quant_vec_kernel<T, K, 256, 4>, dim3(grid_for(rows, 8)), 256, 0, 1, st,      \
                                   "rowwise_quant", (const T*)x, rows, (int)cols, SIN, row_ids, valid_below, indirect,    \
-                                  (uint8_t*)q, scale_out);                                                             \
+                                  (uint8_t*)q, scale_out, 1);                                                          \
         if (rc) return rc;                                                                                          \
         done = true;                                                                                                \
       }                                                                                                             \
@@ -542,6 +563,27 @@ int rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int ki
     case MOE_BF16: return rowwise_quant_launch<__nv_bfloat16>(x, rows, cols, kind, scale_in, row_ids, valid_below, indirect, q, scale_out, st);
     default: return fail(MOE_E_DTYPE, "rowwise_quant: unsupported dtype %d", x_dtype);
   }
+}
+// Tokens quantised per row (KIND 0 / 1) straight into the sorted rows of their k routes: a CTA per token.  One launch
+// for what were three (quantise, copy the rows, copy the scales), and the quantised rows are not read back (Qwen3 shape,
+// e4m3 per token: layer 41 -> 36.5 us for one token, 152 -> 145 us for 500).
+bool rowwise_scatter_serves(int kind, int64_t cols) { return (kind == 0 || kind == 1) && cols % 8 == 0 && cols <= 8192; }
+
+template <typename T>
+static int rowwise_scatter_launch(const void* x, int64_t rows, int cols, int kind, int k, const int32_t* row_index, void* q,
+                                  float* scales, cudaStream_t st) {
+#define MOE_RS(K, CH)                                                                                                       \
+  launch_pdl(rowwise_quant_vec_kernel<T, K, 256, CH, true>, dim3((unsigned)rows), 256, 0, 1, st, "scatter (row quantised)", \
+             (const T*)x, rows, cols, (const float*)nullptr, (const int32_t*)nullptr, (int64_t)0, row_index, (uint8_t*)q, scales, k)
+  if (cols <= 2048) return kind == 0 ? MOE_RS(0, 1) : MOE_RS(1, 1);
+  return kind == 0 ? MOE_RS(0, 4) : MOE_RS(1, 4);
+#undef MOE_RS
+}
+
+int rowwise_scatter(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, int k, const int32_t* row_index, void* q,
+                    float* scales, cudaStream_t st) {
+  return x_dtype == MOE_BF16 ? rowwise_scatter_launch<__nv_bfloat16>(x, rows, (int)cols, kind, k, row_index, q, scales, st)
+                             : rowwise_scatter_launch<__half>(x, rows, (int)cols, kind, k, row_index, q, scales, st);
 }
 }  // namespace moe
 

@@ -29,9 +29,9 @@ __global__ void __launch_bounds__(kThreads) zero_padding_kernel(const int4* __re
   }
 }
 
-// Block (c, m): 2048 columns of token m, a warp per two neighbouring 128-groups, 8 elements per lane.  The arithmetic
+// Block (c, m): P x 2048 columns of token m, a warp per two neighbouring 128-groups, 8 elements per lane.  The arithmetic
 // is that of the stand-alone quantiser (quant.cu), bit for bit.
-template <typename T>
+template <typename T, int P>
 __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* __restrict__ x, int groups, int k,
                                                                        const int32_t* __restrict__ row_index,
                                                                        int64_t rows_cap, uint8_t* __restrict__ q,
@@ -40,34 +40,51 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
   pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t m = blockIdx.y;
-  const int g = (blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
   const int row = lane < k ? row_index[m * k + lane] : -1;
   if (__ballot_sync(0xFFFFFFFFu, row >= 0) == 0) return;  // no route of this token is local
   const int64_t K = (int64_t)groups * 128;
-  const bool in = g < groups;
-  uint4 raw = make_uint4(0, 0, 0, 0);
-  if (in) raw = *reinterpret_cast<const uint4*>(x + m * K + (int64_t)g * 128 + (lane & 15) * 8);
-  const T* pv = reinterpret_cast<const T*>(&raw);
-  float v[8], amax = 0.0f;
+  const int g0 = (blockIdx.x * P * (kThreads / 32) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
+  constexpr int STEP = kThreads / 16;  // groups of one pass of the block
+  uint4 raw[P];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    v[i] = ToF32<T>::get(pv[i]);
-    amax = fmaxf(amax, fabsf(v[i]));
+  for (int u = 0; u < P; ++u) {
+    raw[u] = make_uint4(0, 0, 0, 0);
+    if (g0 + u * STEP < groups) raw[u] = *reinterpret_cast<const uint4*>(x + m * K + (int64_t)(g0 + u * STEP) * 128 + (lane & 15) * 8);
   }
+  uint2 packed[P];
+  float scale[P];
 #pragma unroll
-  for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
-  const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
-  uint32_t lo = 0, hi = 0;
+  for (int u = 0; u < P; ++u) {
+    const T* pv = reinterpret_cast<const T*>(&raw[u]);
+    float v[8], amax = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    lo |= (uint32_t)f32_to_fp8e4m3(fminf(fmaxf(v[i] / s, -kFp8Max), kFp8Max)) << (8 * i);
-    hi |= (uint32_t)f32_to_fp8e4m3(fminf(fmaxf(v[4 + i] / s, -kFp8Max), kFp8Max)) << (8 * i);
+    for (int i = 0; i < 8; ++i) {
+      v[i] = ToF32<T>::get(pv[i]);
+      amax = fmaxf(amax, fabsf(v[i]));
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
+    const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      lo |= (uint32_t)f32_to_fp8e4m3(fminf(fmaxf(v[i] / s, -kFp8Max), kFp8Max)) << (8 * i);
+      hi |= (uint32_t)f32_to_fp8e4m3(fminf(fmaxf(v[4 + i] / s, -kFp8Max), kFp8Max)) << (8 * i);
+    }
+    packed[u] = make_uint2(lo, hi);
+    scale[u] = s;
   }
   for (int j = 0; j < k; ++j) {
     const int r = __shfl_sync(0xFFFFFFFFu, row, j);
-    if (r < 0 || !in) continue;
-    *reinterpret_cast<uint2*>(q + (int64_t)r * K + (int64_t)g * 128 + (lane & 15) * 8) = make_uint2(lo, hi);
-    if ((lane & 15) == 0) scales_t[(int64_t)g * rows_cap + r] = s;
+    if (r < 0) continue;
+#pragma unroll
+    for (int u = 0; u < P; ++u) {
+      const int g = g0 + u * STEP;
+      if (g < groups) {
+        *reinterpret_cast<uint2*>(q + (int64_t)r * K + (int64_t)g * 128 + (lane & 15) * 8) = packed[u];
+        if ((lane & 15) == 0) scales_t[(int64_t)g * rows_cap + r] = scale[u];
+      }
+    }
   }
 }
 
@@ -103,9 +120,9 @@ __global__ void scatter_floats_kernel(const float* __restrict__ src, int64_t num
   }
 }
 
-// Block (c, m): 256 16-byte pieces of token m's output row, one per thread, eight route rows in flight.  No loop over
-// tokens and no division: the loads of enough blocks are in flight to fill HBM whatever k is.
-template <typename T, bool WEIGHTED>
+// Block (c, m): blockDim x P 16-byte pieces of token m's output row, P per thread, P x U route rows in flight.  The slots
+// without a row are skipped before the loads, so a token with one local route of eight costs one round.
+template <typename T, bool WEIGHTED, int P, int U>
 __global__ void __launch_bounds__(kThreads) combine_kernel(const T* __restrict__ y, const float* __restrict__ weight,
                                                            const int32_t* __restrict__ row_index, int k, int vec,
                                                            T* __restrict__ out) {
@@ -113,37 +130,61 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const T* __restrict__
   pdl_trigger();
   constexpr int V = 16 / sizeof(T);
   const int64_t m = blockIdx.y;
-  const int c = blockIdx.x * kThreads + threadIdx.x;
-  if (c >= vec) return;
-  const int32_t* rows = row_index + m * k;
-  const float* w = weight + m * k;
-  float acc[V];
+  const int lane = threadIdx.x & 31, c0 = blockIdx.x * P * blockDim.x + threadIdx.x;
+  const int row = lane < k ? row_index[m * k + lane] : -1;
+  const float wl = WEIGHTED && lane < k ? weight[m * k + lane] : 1.0f;
+  uint32_t left = __ballot_sync(0xFFFFFFFFu, row >= 0);
+  float acc[P][V];
 #pragma unroll
-  for (int i = 0; i < V; ++i) acc[i] = 0.0f;
-  for (int j0 = 0; j0 < k; j0 += 8) {
-    uint4 raw[8];
-    int r[8];
+  for (int u = 0; u < P; ++u)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      r[u] = j0 + u < k ? rows[j0 + u] : -1;
-      if (r[u] >= 0) raw[u] = reinterpret_cast<const uint4*>(y)[(int64_t)r[u] * vec + c];
+    for (int i = 0; i < V; ++i) acc[u][i] = 0.0f;
+  while (left != 0) {  // slots in order
+    uint4 raw[U][P];
+    float w[U];
+    int n = 0;
+#pragma unroll
+    for (int s = 0; s < U; ++s) {
+      if (left != 0) {
+        const int j = __ffs(left) - 1;
+        left &= left - 1;
+        w[s] = __shfl_sync(0xFFFFFFFFu, wl, j);
+        const uint4* src = reinterpret_cast<const uint4*>(y) + (int64_t)__shfl_sync(0xFFFFFFFFu, row, j) * vec;
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+          if (c0 + u * (int)blockDim.x < vec) raw[s][u] = src[c0 + u * blockDim.x];
+        n = s + 1;
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      if (r[u] >= 0) {
-        const float wj = WEIGHTED ? w[j0 + u] : 1.0f;
-        const T* p = reinterpret_cast<const T*>(&raw[u]);
+    for (int s = 0; s < U; ++s) {
+      if (s < n) {
 #pragma unroll
-        for (int i = 0; i < V; ++i) acc[i] = WEIGHTED ? fmaf(wj, ToF32<T>::get(p[i]), acc[i]) : acc[i] + ToF32<T>::get(p[i]);
+        for (int u = 0; u < P; ++u) {
+          const T* p = reinterpret_cast<const T*>(&raw[s][u]);
+#pragma unroll
+          for (int i = 0; i < V; ++i)
+            acc[u][i] = WEIGHTED ? fmaf(w[s], ToF32<T>::get(p[i]), acc[u][i]) : acc[u][i] + ToF32<T>::get(p[i]);
+        }
       }
     }
   }
-  uint4 o;
-  T* p = reinterpret_cast<T*>(&o);
 #pragma unroll
-  for (int i = 0; i < V; ++i) p[i] = from_f32<T>(acc[i]);
-  reinterpret_cast<uint4*>(out)[m * vec + c] = o;
+  for (int u = 0; u < P; ++u) {
+    if (c0 + u * (int)blockDim.x < vec) {
+      uint4 o;
+      T* p = reinterpret_cast<T*>(&o);
+#pragma unroll
+      for (int i = 0; i < V; ++i) p[i] = from_f32<T>(acc[u][i]);
+      reinterpret_cast<uint4*>(out)[m * vec + c0 + u * blockDim.x] = o;
+    }
+  }
 }
+
+// From four tokens per SM on, a block takes a whole row: its dependent chain (row index, rows, store) is walked once per
+// token instead of once per quarter of it (DSV3 FP8, one of 8 ranks, 2000 tokens: layer 308 -> 300 us; 8192 tokens, where
+// HBM is the limit, the same).  Below, quarters spread a token over more SMs.
+bool whole_rows(int64_t M) { return M >= 4 * sm_count(); }
 }  // namespace
 
 // M <= 65535 for all of these (the second grid dimension): the layer call checks it.
@@ -155,12 +196,15 @@ int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, in
 int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,
                         float* scales_t, cudaStream_t st) {
   const int groups = H / 128;
-  const dim3 grid((unsigned)((groups + 15) / 16), (unsigned)M);
-  if (dtype == MOE_BF16)
-    return launch_pdl(scatter_quant_group_kernel<__nv_bfloat16>, grid, kThreads, 0, 1, st, "scatter (1x128 quantised)",
-                      (const __nv_bfloat16*)x, groups, k, row_index, rows_cap, (uint8_t*)q, scales_t);
-  return launch_pdl(scatter_quant_group_kernel<__half>, grid, kThreads, 0, 1, st, "scatter (1x128 quantised)", (const __half*)x,
-                    groups, k, row_index, rows_cap, (uint8_t*)q, scales_t);
+  const bool whole = whole_rows(M);
+  const int per_block = whole ? 64 : 16;
+  const dim3 grid((unsigned)((groups + per_block - 1) / per_block), (unsigned)M);
+#define MOE_SCATTER(T, P)                                                                                                     \
+  launch_pdl(scatter_quant_group_kernel<T, P>, grid, kThreads, 0, 1, st, "scatter (1x128 quantised)", (const T*)x, groups, k, \
+             row_index, rows_cap, (uint8_t*)q, scales_t)
+  if (dtype == MOE_BF16) return whole ? MOE_SCATTER(__nv_bfloat16, 4) : MOE_SCATTER(__nv_bfloat16, 1);
+  return whole ? MOE_SCATTER(__half, 4) : MOE_SCATTER(__half, 1);
+#undef MOE_SCATTER
 }
 
 int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st) {
@@ -178,11 +222,17 @@ int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_
 int combine_rows(const void* y, int dtype, const float* weight, const int32_t* row_index, int64_t M, int k, int64_t H, void* out,
                  cudaStream_t st) {
   const int vec = (int)(H / 8);
-  const dim3 grid((unsigned)((vec + kThreads - 1) / kThreads), (unsigned)M);
-#define MOE_COMBINE(T, W) \
-  launch_pdl(combine_kernel<T, W>, grid, kThreads, 0, 1, st, "combine", (const T*)y, weight, row_index, k, vec, (T*)out)
+  const int P = whole_rows(M) ? 4 : 1;
+  // equal blocks of whole warps: H = 7168 is 4 x 224 pieces, not 3.5 x 256
+  const int blocks = (vec + P * kThreads - 1) / (P * kThreads);
+  const int threads = ((vec + P * blocks - 1) / (P * blocks) + 31) / 32 * 32;
+  const dim3 grid((unsigned)blocks, (unsigned)M);
+#define MOE_COMBINE_P(T, W, P, U) \
+  launch_pdl(combine_kernel<T, W, P, U>, grid, threads, 0, 1, st, "combine", (const T*)y, weight, row_index, k, vec, (T*)out)
+#define MOE_COMBINE(T, W) (P == 4 ? MOE_COMBINE_P(T, W, 4, 4) : MOE_COMBINE_P(T, W, 1, 8))
   if (dtype == MOE_BF16) return weight != nullptr ? MOE_COMBINE(__nv_bfloat16, true) : MOE_COMBINE(__nv_bfloat16, false);
   return weight != nullptr ? MOE_COMBINE(__half, true) : MOE_COMBINE(__half, false);
+#undef MOE_COMBINE_P
 #undef MOE_COMBINE
 }
 
