@@ -135,6 +135,29 @@ def test_half_layer_few_routes(M, E, k, H, I, dtype):
         _parity(out[1:], ref[1:], (M, E))
 
 
+@pytest.mark.parametrize("M,k", [(1, 12), (4, 8), (32, 1), (33, 1), (11, 3)])
+@pytest.mark.parametrize("spread", [1, 12])
+def test_plan_of_few_routes(M, k, spread):
+    """Up to 32 routes (one warp) and just above: all on one expert or spread, local experts only, ids out of range."""
+    E, H, I = 12, 256, 128
+    x = T.make_activations(M, H, DEV, seed=M)
+    w1, s1 = T.make_int8_channel_weights(E, 2 * I, H, DEV, seed=1)
+    w2, s2 = T.make_int8_channel_weights(E, H, I, DEV, seed=2)
+    tw, ti = _route(M, E, k)
+    if spread == 1:
+        ti = torch.full_like(ti, 5)
+    emap = torch.full((E,), -1, dtype=torch.int32, device=DEV)
+    emap[4:9] = torch.arange(5, dtype=torch.int32, device=DEV).flip(0)
+    ti[M // 2, k - 1] = -1
+    keep = (ti >= 4) & (ti < 9)
+    ref = O.fused_moe_w8a16_oracle(x, w1, w2, s1, s2, tw * keep, ti.clamp(min=0))
+    loc = lambda w: w[4:9].flip(0).contiguous()
+    out = fg.fused_experts_impl(x, loc(w1), loc(w2), tw, ti, use_int8_w8a16=True, per_channel_quant=True, w1_scale=loc(s1),
+                                w2_scale=loc(s2), global_num_experts=E, expert_map=emap)
+    _parity(out, ref, (M, k))
+    assert bool((out[~keep.any(1)] == 0).all())
+
+
 @pytest.mark.parametrize("M", [7, 300, 2500])
 def test_layer_with_local_experts_and_weights_on_the_input(M):
     """expert_map (routes of other ranks get no rows), ids out of range, route weights applied on the input."""
