@@ -440,7 +440,9 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const Params P) {
       const int64_t pr = (int64_t)b * ROWS + 2 * q;  // sorted row of route 2q
       if (P.S > 1) {
         float* mine = P.partial + ((int64_t)s * P.rows_cap + pr) * tile_ld + (int64_t)nt * TILE_W;
-        mine[rowA] = v[0]; mine[tile_ld + rowA] = v[1]; mine[rowB] = v[2]; mine[tile_ld + rowB] = v[3];
+        const bool ok0 = aux->sid[2 * q] >= 0, ok1 = aux->sid[2 * q + 1] >= 0;  // padding routes leave nothing
+        if (ok0) { mine[rowA] = v[0]; mine[rowB] = v[2]; }
+        if (ok1) { mine[tile_ld + rowA] = v[1]; mine[tile_ld + rowB] = v[3]; }
         __syncwarp();  // the warp's partial sums are written; lane 0 publishes them with its release
         int last = 0;
         if (lane == 0) {
@@ -451,10 +453,23 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const Params P) {
         last = __shfl_sync(0xFFFFFFFFu, last, 0);
         if (!last) continue;  // the warp of another slice finishes these rows
         v[0] = v[1] = v[2] = v[3] = 0.0f;
-        for (int s2 = 0; s2 < P.S; ++s2) {  // slice order, whoever came last
-          const float* part = P.partial + ((int64_t)s2 * P.rows_cap + pr) * tile_ld + (int64_t)nt * TILE_W;
-          v[0] += ldcg_f(part + rowA); v[1] += ldcg_f(part + tile_ld + rowA);
-          v[2] += ldcg_f(part + rowB); v[3] += ldcg_f(part + tile_ld + rowB);
+        // slice order, whoever came last; the loads of eight slices are in flight together (slice after slice, they were
+        // 6 of the 145 us of the Mixtral shape's one-token layer)
+        for (int s0 = 0; s0 < P.S; s0 += 8) {
+          float part[8][4];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float* src = P.partial + ((int64_t)(s0 + i) * P.rows_cap + pr) * tile_ld + (int64_t)nt * TILE_W;
+            const bool in = s0 + i < P.S;
+            part[i][0] = in && ok0 ? ldcg_f(src + rowA) : 0.0f;
+            part[i][1] = in && ok1 ? ldcg_f(src + tile_ld + rowA) : 0.0f;
+            part[i][2] = in && ok0 ? ldcg_f(src + rowB) : 0.0f;
+            part[i][3] = in && ok1 ? ldcg_f(src + tile_ld + rowB) : 0.0f;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] += part[i][j];
         }
       }
       // weight row (inside the expert) behind tile rows A and B
@@ -507,8 +522,15 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const Params P) {
           if (lane < 16) {
             const int col = nt * TILE_W + 16 * warp + lane;
             float sum = 0.0f;
-            for (int j = 0; j < P.topk; ++j)
-              if ((mk >> j) & 1u) sum += ToF32<AT>::get(ldcg_at<AT>(y + (tok * P.topk + j) * P.Nout + col));
+            for (int j0 = 0; j0 < P.topk; j0 += 8) {  // slot order, eight loads in flight
+              float add[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                add[i] = j0 + i < P.topk && ((mk >> (j0 + i)) & 1u)
+                             ? ToF32<AT>::get(ldcg_at<AT>(y + (tok * P.topk + j0 + i) * P.Nout + col)) : 0.0f;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) sum += add[i];
+            }
             reinterpret_cast<AT*>(P.final_out)[tok * P.Nout + col] = from_f32<AT>(sum);
           }
         }
