@@ -10,7 +10,7 @@
 // At prefill sizes the board runs at its power limit, so operands not moved and padding not multiplied are
 // clock as well as cycles.
 //
-// Both operands arrive by TMA: token rows were put into sorted order by the scatter kernels (quant.cu).  Every load
+// Both operands arrive by TMA: token rows were put into sorted order by the scatter kernels (route_rows.cu, quant.cu).  Every load
 // of both CTAs counts its bytes on the leader's barrier of the stage; the leader's MMA thread needs no other
 // signal from its peer.
 //

@@ -1,4 +1,4 @@
-// Row movement on both sides of the grouped GEMMs of gemm_wt.cu: tokens into expert-sorted order (quantised on
+// Row movement on both sides of the grouped GEMMs of the layer call: tokens into expert-sorted order (quantised on
 // the way where the mode wants it), route rows back into tokens.
 //
 //   scatter   every token row is read ONCE and written to the sorted rows of its k routes (row_index of the route
