@@ -41,6 +41,10 @@ template <bool WIDE> struct Cfg {
   static constexpr int SUB_BYTES = TILE * 128;     // 64 elements of K of the token rows
   static constexpr int TOK_BYTES = 2 * SUB_BYTES;
   static constexpr int RSTAGES = WIDE ? 3 : 6, TSTAGES = WIDE ? 3 : 4;
+  // Every raw stage belongs to ONE converter group (as every A buffer does), which has seen the use before the one it waits
+  // for.  With five stages a group could wait two uses ahead of a late load: the parity wait lets it pass, it hands the
+  // stage back too early, and the launch fails, about once in a thousand layers.
+  static_assert(RSTAGES % GROUPS == 0, "raw stages per converter group");
 };
 struct Aux {
   uint64_t r_full[6], r_empty[6];
