@@ -23,6 +23,9 @@
 //                q the 32 weight rows = TMEM lanes 32 q...  A thread widens one row of 128 bytes; the 128-byte
 //                swizzle of the raw tile makes its 16-byte loads conflict-free.
 // TMEM columns hold two elements of K each, so an MMA (16 elements) takes 8 columns of A.
+//
+// Bound at prefill (Qwen3 shape, 4096 tokens): L2 -> SM traffic, 10.8 TB/s in GEMM1 with the tensor pipe at 52 %; at decode
+// HBM, less the last partial wave.  Against gemm_w8.cu: 33 tokens 191 -> 146 us per layer, 4096 tokens 591 -> 465.
 #include "wt_common.cuh"
 
 namespace moe {
