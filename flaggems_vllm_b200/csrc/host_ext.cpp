@@ -76,6 +76,16 @@ PyObject* set_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
+// The interpreter lock is given back for as long as a function allocates and launches: cudaMalloc may wait for the
+// device, and a launch waits when the stream's queue is full, while the work it waits for may need another thread
+// of the process (another stream's, another rank's).  Nothing between the braces of its scope touches a Python object.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 int32_t* status_of(int dev) { return dev >= 0 && dev < 64 ? g_status[dev].load(std::memory_order_relaxed) : nullptr; }
 
 // fused_experts(hidden, w1, w2, topk_weights, topk_ids, inplace, activation, apply_router_weight_on_input, use_fp8_w8a8,
@@ -147,19 +157,25 @@ PyObject* fused_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (status == nullptr || experts <= 0 || experts > (1 << 20) ||
       moe_layer_workspace(mode, code, M, (int)k, (int)experts, (int)E, (int)H, (int)I, MOE_ACT_SILU, bytes) != 0)
     MOE_NONE;
-  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-  const at::Tensor out = truth(a[5]) ? x : at::empty_like(x);
-  at::Tensor ws[4];
-  for (int i = 0; i < 4; ++i) ws[i] = bytes_on(bytes[i], x);
-  const int rc = moe_layer(mode, code, x.const_data_ptr(), M, (int)k, ti.const_data_ptr(), ids64, tw.const_data_ptr<float>(),
-                           w1.const_data_ptr(), s1 ? s1->const_data_ptr<float>() : nullptr, w2.const_data_ptr(),
-                           s2 ? s2->const_data_ptr<float>() : nullptr, out.mutable_data_ptr(), (int)experts, emap, (int)E, (int)H,
-                           (int)I, truth(a[7]), MOE_ACT_SILU, 0.0f, 0.0f, 0.0f, kind, nullptr, kind, nullptr, ws[0].mutable_data_ptr(),
-                           ws[1].mutable_data_ptr(), ws[2].mutable_data_ptr(), ws[3].mutable_data_ptr(), 63, status,
-                           c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  const bool inplace = truth(a[5]), weight_on_input = truth(a[7]);
+  at::Tensor out;
+  int rc;
+  {
+    Unlocked unlocked;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    out = inplace ? x : at::empty_like(x);
+    at::Tensor ws[4];
+    for (int i = 0; i < 4; ++i) ws[i] = bytes_on(bytes[i], x);
+    rc = moe_layer(mode, code, x.const_data_ptr(), M, (int)k, ti.const_data_ptr(), ids64, tw.const_data_ptr<float>(),
+                   w1.const_data_ptr(), s1 ? s1->const_data_ptr<float>() : nullptr, w2.const_data_ptr(),
+                   s2 ? s2->const_data_ptr<float>() : nullptr, out.mutable_data_ptr(), (int)experts, emap, (int)E, (int)H,
+                   (int)I, weight_on_input, MOE_ACT_SILU, 0.0f, 0.0f, 0.0f, kind, nullptr, kind, nullptr, ws[0].mutable_data_ptr(),
+                   ws[1].mutable_data_ptr(), ws[2].mutable_data_ptr(), ws[3].mutable_data_ptr(), 63, status,
+                   c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  }
   if (rc != 0) MOE_NONE;
   g_launches += 5;
-  if (truth(a[5])) {
+  if (inplace) {
     Py_INCREF(a[0]);
     return a[0];
   }
@@ -180,12 +196,19 @@ PyObject* grouped_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (sc < 0 || bc < 0 || !cuda_dense(b, dev) || b.numel() != E || M <= 0 || groups <= 0 || groups > 32 || E % groups != 0 || k <= 0 ||
       k > 32 || (func != 0 && func != 1))
     MOE_NONE;
-  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-  at::Tensor w = at::empty({M, k}, s.options().dtype(at::kFloat)), ids = at::empty({M, k}, s.options().dtype(at::kInt));
-  if (moe_grouped_topk(s.const_data_ptr(), sc, s.stride(0), s.stride(1), b.const_data_ptr(), bc, nullptr, M, (int)E, (int)groups,
-                       (int)keep, (int)k, truth(a[4]), (float)scale, (int)func, w.mutable_data_ptr<float>(),
-                       ids.mutable_data_ptr<int32_t>(), c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream()) != 0)
-    MOE_NONE;
+  const bool renormalize = truth(a[4]);
+  at::Tensor w, ids;
+  int rc;
+  {
+    Unlocked unlocked;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    w = at::empty({M, k}, s.options().dtype(at::kFloat));
+    ids = at::empty({M, k}, s.options().dtype(at::kInt));
+    rc = moe_grouped_topk(s.const_data_ptr(), sc, s.stride(0), s.stride(1), b.const_data_ptr(), bc, nullptr, M, (int)E, (int)groups,
+                          (int)keep, (int)k, renormalize, (float)scale, (int)func, w.mutable_data_ptr<float>(),
+                          ids.mutable_data_ptr<int32_t>(), c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  }
+  if (rc != 0) MOE_NONE;
   ++g_launches;
   PyObject* r = PyTuple_New(2);
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(w));
@@ -216,11 +239,16 @@ PyObject* topk_route(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!cuda_dense(b, dev) || b.scalar_type() != at::kFloat || b.dim() != 1 || b.numel() != E) MOE_NONE;
     bias = b.const_data_ptr<float>();
   }
-  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-  if (moe_topk_route(g.const_data_ptr(), gc, bias, nullptr, M, (int)E, (int)k, truth(a[6]), truth(a[4]), (float)scale,
-                     w.mutable_data_ptr<float>(), ids.mutable_data_ptr(), kind, rows.mutable_data_ptr<int32_t>(),
-                     c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream()) != 0)
-    MOE_NONE;
+  const bool sigmoid = truth(a[6]), renormalize = truth(a[4]);
+  int rc;
+  {
+    Unlocked unlocked;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    rc = moe_topk_route(g.const_data_ptr(), gc, bias, nullptr, M, (int)E, (int)k, sigmoid, renormalize, (float)scale,
+                        w.mutable_data_ptr<float>(), ids.mutable_data_ptr(), kind, rows.mutable_data_ptr<int32_t>(),
+                        c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  }
+  if (rc != 0) MOE_NONE;
   ++g_launches;
   Py_RETURN_TRUE;
 }
@@ -236,11 +264,16 @@ PyObject* router_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (xc < 0 || wc < 0 || !status || !cuda_dense(w, dev) || w.size(1) != K || M <= 0 || K % 8 != 0 || x.stride(1) != 1 ||
       x.stride(0) % 8 != 0 || ((uintptr_t)x.const_data_ptr() & 15) || N > (1 << 30) || K > (1 << 30))
     MOE_NONE;
-  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-  at::Tensor out = at::empty({M, N}, x.options().dtype(at::kFloat));
-  if (moe_router_gemm_ex(x.const_data_ptr(), xc, x.stride(0), w.const_data_ptr(), wc, M, (int)N, (int)K,
-                         out.mutable_data_ptr<float>(), status, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream()) != 0)
-    MOE_NONE;
+  at::Tensor out;
+  int rc;
+  {
+    Unlocked unlocked;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    out = at::empty({M, N}, x.options().dtype(at::kFloat));
+    rc = moe_router_gemm_ex(x.const_data_ptr(), xc, x.stride(0), w.const_data_ptr(), wc, M, (int)N, (int)K,
+                            out.mutable_data_ptr<float>(), status, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  }
+  if (rc != 0) MOE_NONE;
   ++g_launches;
   return THPVariable_Wrap(out);
 }
@@ -255,14 +288,21 @@ PyObject* align(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool ids64 = ids.scalar_type() == at::kLong;
   int32_t* status = status_of(dev);
   if ((!ids64 && ids.scalar_type() != at::kInt) || !status) MOE_NONE;
-  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-  const auto opt = ids.options().dtype(at::kInt);
   const int64_t blocks = (cap + bs - 1) / bs;
-  at::Tensor sorted = at::empty({cap}, opt), experts = at::empty({blocks}, opt), npp = at::empty({1}, opt);
-  if (moe_align_block_size(ids.const_data_ptr(), ids64, ids.numel(), (int)E, (int)bs, sorted.mutable_data_ptr<int32_t>(), cap,
-                           experts.mutable_data_ptr<int32_t>(), blocks, npp.mutable_data_ptr<int32_t>(), status,
-                           c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream()) != 0)
-    MOE_NONE;
+  at::Tensor sorted, experts, npp;
+  int rc;
+  {
+    Unlocked unlocked;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    const auto opt = ids.options().dtype(at::kInt);
+    sorted = at::empty({cap}, opt);
+    experts = at::empty({blocks}, opt);
+    npp = at::empty({1}, opt);
+    rc = moe_align_block_size(ids.const_data_ptr(), ids64, ids.numel(), (int)E, (int)bs, sorted.mutable_data_ptr<int32_t>(), cap,
+                              experts.mutable_data_ptr<int32_t>(), blocks, npp.mutable_data_ptr<int32_t>(), status,
+                              c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
+  }
+  if (rc != 0) MOE_NONE;
   ++g_launches;
   PyObject* r = PyTuple_New(3);
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(sorted));
