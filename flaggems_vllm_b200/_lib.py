@@ -33,6 +33,8 @@ SYMBOLS = {
     "moe_map_expert_ids": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_void_p]),
     "moe_align_block_size": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
                                      c_int64, c_void_p, c_void_p, c_void_p]),
+    "moe_align_block_size_ex": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
+                                        c_int64, c_void_p, c_int, c_void_p, c_void_p]),
     "moe_per_token_group_quant_fp8": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_void_p, c_void_p,
                                               c_int, c_int64, c_void_p]),
     "moe_per_token_group_quant_fp8_ex": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_float, c_int, c_void_p,
@@ -44,6 +46,7 @@ SYMBOLS = {
     "moe_ep_unpack": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                               c_void_p]),
     "moe_router_gemm": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p]),
+    "moe_router_gemm_tile": (c_int, [c_int64, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "moe_router_gemm_ex": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p,
                                    c_void_p]),
     "moe_router_gemm_grouped_topk": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_int,
@@ -93,7 +96,7 @@ _status = {}
 # calls of entry points that enqueue a kernel; LAUNCHES adds those of the native host path (bench.py reports the
 # count of its timed region)
 _ctypes_launches = 0
-_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_set_wait_limit_ns")
+_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_router_gemm_tile", "moe_set_wait_limit_ns")
 
 
 class _Counted:

@@ -1,7 +1,11 @@
 // moe_align_block_size: stable counting sort of the flat expert-id array with
 // each expert's run padded to a multiple of block_size.
 //
-// One CTA does the whole job in a single launch, entirely in shared memory:
+// The usual sizes run align_sort_kernel (below; the sort itself is sort_ids.cuh) in a cluster of 8 or 16 CTAs.  More
+// than 1024 experts or 262144 ids, and devices or partitions that hold no such cluster, run the two
+// kernels described here.
+//
+// align_kernel: one CTA does the whole job in a single launch, entirely in shared memory:
 //   phase 0  fill both output buffers with their sentinels (numel / -1)
 //   phase 1  per-warp histograms: warp w owns a contiguous slice of the ids
 //   phase 2  per expert: exclusive prefix over warps, padded count;
@@ -18,7 +22,7 @@
 // Ids outside [0, num_experts) are skipped; ids >= num_experts are also flagged in the
 // status word (negative ids are the conventional "no route" marker and stay silent).
 //
-// Large inputs (thousands of ids) use the same algorithm spread over a
+// align_cluster_kernel, from 4096 ids on: the same algorithm spread over a
 // thread-block cluster of 8 CTAs: each CTA owns a contiguous eighth of the ids,
 // the per-CTA expert totals are exchanged through distributed shared memory
 // (plain remote loads, two cluster barriers), every CTA derives the same
@@ -377,18 +381,58 @@ align_sort_kernel(const IdT* ids, int numel, int E, int block_size, int32_t* sor
   align_sort_body<IdT, CTAS, ROUNDS>(ids, numel, E, block_size, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status);
 }
 
-// a cluster at any size: even a call of a few ids writes tens of thousands of sentinels
+// A cluster at any size: even a call of a few ids writes tens of thousands of sentinels.  False where no such cluster can
+// run (or `limit` forbids it): the kernels above serve the call.
 template <typename IdT>
-int launch_align_sort(const void* ids, int numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
-                      int expert_cap, int32_t* npp, int32_t* status, cudaStream_t st) {
+bool launch_align_sort(const void* ids, int numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
+                       int expert_cap, int32_t* npp, int32_t* status, int limit, cudaStream_t st, int* rc) {
   using namespace sorting;
-#define MOE_ALIGN(C, R)                                                                                              \
-  launch_cluster(align_sort_kernel<IdT, C, R>, C, E, st, "align (sort)", (const IdT*)ids, numel, E, block_size, sorted_ids, \
-                 sorted_cap, expert_ids, expert_cap, npp, status)
-  if (numel <= capacity(kSmall, 2)) return MOE_ALIGN(kSmall, 2);
-  if (numel <= capacity(kLarge, 4)) return MOE_ALIGN(kLarge, 4);
-  return MOE_ALIGN(kLarge, 16);
-#undef MOE_ALIGN
+  auto launch = [&](auto kern, int ctas) {
+    if (ctas > limit || !cluster_fits(kern, ctas, E)) return false;
+    *rc = launch_cluster(kern, ctas, E, st, "align (sort)", (const IdT*)ids, numel, E, block_size, sorted_ids, sorted_cap, expert_ids,
+                         expert_cap, npp, status);
+    return true;
+  };
+  if (numel <= capacity(kSmall, 2)) return launch(align_sort_kernel<IdT, kSmall, 2>, kSmall);
+  if (numel <= capacity(kLarge, 4)) return launch(align_sort_kernel<IdT, kLarge, 4>, kLarge);
+  return launch(align_sort_kernel<IdT, kLarge, 16>, kLarge);
+}
+
+template <typename IdT>
+int align_any(const IdT* ids, int64_t numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
+              int expert_cap, int32_t* npp, int32_t* status, int limit, cudaStream_t st) {
+  int rc = 0;
+  if (E <= sorting::kMaxExperts && numel <= sorting::capacity(sorting::kLarge, 16) &&
+      launch_align_sort<IdT>(ids, (int)numel, E, block_size, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status, limit, st, &rc))
+    return rc;
+  if (numel >= 4096 && E <= 1024 && limit >= kClusterSize) {
+    // cluster of 8 CTAs; hist[W][E] + cta_tot[E] + blk_start[E+1] + 33 words per CTA
+    auto kern = align_cluster_kernel<IdT>;
+    int W = kAlignThreads / 32;
+    while (W > 1 && ((size_t)W * E + 2 * (size_t)E + 34) * 4 > 96 * 1024) W >>= 1;
+    const size_t smem = ((size_t)W * E + 2 * (size_t)E + 34) * 4;
+    const cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ce != cudaSuccess) return fail((int)ce, "align: smem attribute: %s", cudaGetErrorString(ce));
+    if (max_clusters((const void*)kern, kClusterSize, kAlignThreads, smem) != 0) {
+      kern<<<kClusterSize, kAlignThreads, smem, st>>>(ids, (int)numel, E, block_size, W, sorted_ids, sorted_cap, expert_ids, expert_cap,
+                                                      npp, status);
+      return check_launch("align (cluster)");
+    }
+  }
+  // one slice (and one histogram) per 64 ids: a decode-sized call clears and scans one or two
+  // histograms instead of 32
+  auto kern = align_kernel<IdT>;
+  int n_warps = kAlignThreads / 32;
+  const int64_t slices = (numel + 63) / 64;
+  if (slices < n_warps) n_warps = slices < 1 ? 1 : (int)slices;
+  const size_t budget = 200 * 1024;
+  while (n_warps > 1 && ((size_t)n_warps * E + E + 1 + 33) * 4 > budget) n_warps >>= 1;
+  const size_t smem = ((size_t)n_warps * E + E + 1 + 33) * 4;
+  const cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (ce != cudaSuccess) return fail((int)ce, "align: smem attribute: %s", cudaGetErrorString(ce));
+  kern<<<1, kAlignThreads, smem, st>>>(ids, (int)numel, E, block_size, n_warps, sorted_ids, sorted_cap, expert_ids, expert_cap, npp,
+                                       status);
+  return check_launch("align");
 }
 
 }  // namespace
@@ -398,8 +442,15 @@ extern "C" int moe_align_block_size(const void* topk_ids, int ids_int64, int64_t
                                     int num_experts, int block_size, int32_t* sorted_ids,
                                     int64_t sorted_cap, int32_t* expert_ids, int64_t expert_cap,
                                     int32_t* num_post_pad, int32_t* status, void* stream) {
+  return moe_align_block_size_ex(topk_ids, ids_int64, numel, num_experts, block_size, sorted_ids, sorted_cap, expert_ids, expert_cap,
+                                 num_post_pad, 0, status, stream);
+}
+
+extern "C" int moe_align_block_size_ex(const void* topk_ids, int ids_int64, int64_t numel, int num_experts, int block_size,
+                                       int32_t* sorted_ids, int64_t sorted_cap, int32_t* expert_ids, int64_t expert_cap,
+                                       int32_t* num_post_pad, int cluster_limit, int32_t* status, void* stream) {
   using namespace moe;
-  if (numel < 0 || num_experts <= 0 || block_size <= 0 || sorted_cap < 0 || expert_cap < 0)
+  if (numel < 0 || num_experts <= 0 || block_size <= 0 || sorted_cap < 0 || expert_cap < 0 || cluster_limit < 0)
     return fail(MOE_E_BADARG, "align: negative or zero extent");
   if (num_experts > 4096) return fail(MOE_E_TOOBIG, "align: at most 4096 experts");
   if (numel >= (1ll << 31) - 1 || sorted_cap >= (1ll << 31) - 1)
@@ -408,58 +459,12 @@ extern "C" int moe_align_block_size(const void* topk_ids, int ids_int64, int64_t
     return fail(MOE_E_BADARG, "align: null pointer");
   // worst case padded total must fit the buffers the caller gave
   // (numel + E*(bs-1) is the reference's bound); the kernel clips writes anyway.
-  const int E = num_experts;
+  const int limit = cluster_limit > 0 ? cluster_limit : 16;
   cudaStream_t st = (cudaStream_t)stream;
-  if (E <= sorting::kMaxExperts && numel <= sorting::capacity(sorting::kLarge, 16))
-    return ids_int64 ? launch_align_sort<int64_t>(topk_ids, (int)numel, E, block_size, sorted_ids, (int)sorted_cap, expert_ids,
-                                                  (int)expert_cap, num_post_pad, status, st)
-                     : launch_align_sort<int32_t>(topk_ids, (int)numel, E, block_size, sorted_ids, (int)sorted_cap, expert_ids,
-                                                  (int)expert_cap, num_post_pad, status, st);
-  cudaError_t ce;
-  if (numel >= 4096 && E <= 1024) {
-    // cluster of 8 CTAs; hist[W][E] + cta_tot[E] + blk_start[E+1] + 33 words per CTA
-    int W = kAlignThreads / 32;
-    while (W > 1 && ((size_t)W * E + 2 * (size_t)E + 34) * 4 > 96 * 1024) W >>= 1;
-    const size_t smem = ((size_t)W * E + 2 * (size_t)E + 34) * 4;
-    if (ids_int64) {
-      ce = cudaFuncSetAttribute(align_cluster_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (ce != cudaSuccess) return fail((int)ce, "align: smem attribute: %s", cudaGetErrorString(ce));
-      align_cluster_kernel<int64_t><<<kClusterSize, kAlignThreads, smem, st>>>(
-          (const int64_t*)topk_ids, (int)numel, E, block_size, W, sorted_ids, (int)sorted_cap, expert_ids,
-          (int)expert_cap, num_post_pad, status);
-    } else {
-      ce = cudaFuncSetAttribute(align_cluster_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (ce != cudaSuccess) return fail((int)ce, "align: smem attribute: %s", cudaGetErrorString(ce));
-      align_cluster_kernel<int32_t><<<kClusterSize, kAlignThreads, smem, st>>>(
-          (const int32_t*)topk_ids, (int)numel, E, block_size, W, sorted_ids, (int)sorted_cap, expert_ids,
-          (int)expert_cap, num_post_pad, status);
-    }
-    return check_launch("align (cluster)");
-  }
-  // one slice (and one histogram) per 64 ids: a decode-sized call clears and scans one or two
-  // histograms instead of 32
-  int n_warps = kAlignThreads / 32;
-  const int64_t slices = (numel + 63) / 64;
-  if (slices < n_warps) n_warps = slices < 1 ? 1 : (int)slices;
-  const size_t budget = 200 * 1024;
-  while (n_warps > 1 && ((size_t)n_warps * E + E + 1 + 33) * 4 > budget) n_warps >>= 1;
-  const size_t smem = ((size_t)n_warps * E + E + 1 + 33) * 4;
-  if (ids_int64) {
-    ce = cudaFuncSetAttribute(align_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem);
-    if (ce != cudaSuccess) return fail((int)ce, "align: smem attribute: %s", cudaGetErrorString(ce));
-    align_kernel<int64_t><<<1, kAlignThreads, smem, st>>>(
-        (const int64_t*)topk_ids, (int)numel, E, block_size, n_warps, sorted_ids, (int)sorted_cap,
-        expert_ids, (int)expert_cap, num_post_pad, status);
-  } else {
-    ce = cudaFuncSetAttribute(align_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem);
-    if (ce != cudaSuccess) return fail((int)ce, "align: smem attribute: %s", cudaGetErrorString(ce));
-    align_kernel<int32_t><<<1, kAlignThreads, smem, st>>>(
-        (const int32_t*)topk_ids, (int)numel, E, block_size, n_warps, sorted_ids, (int)sorted_cap,
-        expert_ids, (int)expert_cap, num_post_pad, status);
-  }
-  return check_launch("align");
+  return ids_int64 ? align_any((const int64_t*)topk_ids, numel, num_experts, block_size, sorted_ids, (int)sorted_cap, expert_ids,
+                               (int)expert_cap, num_post_pad, status, limit, st)
+                   : align_any((const int32_t*)topk_ids, numel, num_experts, block_size, sorted_ids, (int)sorted_cap, expert_ids,
+                               (int)expert_cap, num_post_pad, status, limit, st);
 }
 
 

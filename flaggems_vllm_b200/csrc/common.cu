@@ -28,6 +28,24 @@ int allow_smem(const void* kernel, int bytes, bool large_cluster) {
   return 0;
 }
 
+int max_clusters(const void* kernel, int ctas, int threads, size_t smem) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess) return n;
+  cudaGetLastError();
+  return -1;
+}
+
 int sm_count() {
   static std::atomic<int> cached[64];
   int dev = 0;

@@ -154,6 +154,7 @@ PyObject* fused_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   int32_t* status = status_of(dev);
   int64_t bytes[4];
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);  // what is served depends on the device
   if (status == nullptr || experts <= 0 || experts > (1 << 20) ||
       moe_layer_workspace(mode, code, M, (int)k, (int)experts, (int)E, (int)H, (int)I, MOE_ACT_SILU, bytes) != 0)
     MOE_NONE;
@@ -162,7 +163,6 @@ PyObject* fused_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int rc;
   {
     Unlocked unlocked;
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
     out = inplace ? x : at::empty_like(x);
     at::Tensor ws[4];
     for (int i = 0; i < 4; ++i) ws[i] = bytes_on(bytes[i], x);

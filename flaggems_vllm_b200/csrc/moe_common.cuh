@@ -24,6 +24,10 @@ unsigned long long wait_limit_ns();
 int allow_smem(const void* kernel, int bytes, bool large_cluster = false);
 // Multiprocessors of the current device (remembered).
 int sm_count();
+// Clusters of `ctas` CTAs of this kernel that the device, or the part of it this context has, runs at once: 0 = such a
+// cluster never starts (a partition without a GPC that holds it), -1 = there is no device to ask.  Asked on every
+// call, 0.2 us: what a context has of a device can change.
+int max_clusters(const void* kernel, int ctas, int threads, size_t smem);
 
 // Programmatic dependent launch.  The kernels of a layer are launched so that each may start while its predecessor
 // drains: what it does before pdl_wait() touches nothing the predecessor writes (barriers, TMEM, weights, and the

@@ -151,8 +151,15 @@ void plan_caps(int64_t numel, int E_local, int gran, int tile_rows, int64_t* row
   *tiles_cap = *rows_cap / tile_rows + used + 1;
 }
 
+// Not served where the device (or the partition of it) holds no cluster of the size that `numel` ids take: the layer then
+// goes through moe_align_block_size, which has kernels without clusters.
 bool plan_serves(int64_t numel, int E, int E_local) {
-  return E > 0 && E_local > 0 && E_local <= sorting::kMaxExperts && numel > 0 && numel <= sorting::capacity(sorting::kLarge, 16);
+  using namespace sorting;
+  if (E <= 0 || E_local <= 0 || E_local > kMaxExperts || numel <= 0 || numel > capacity(kLarge, 16)) return false;
+  if (numel <= capacity(1, 2)) return true;
+  if (numel <= capacity(kSmall, 2)) return cluster_fits(plan_kernel<int32_t, kSmall, 2>, kSmall, E_local);
+  if (numel <= capacity(kLarge, 4)) return cluster_fits(plan_kernel<int32_t, kLarge, 4>, kLarge, E_local);
+  return cluster_fits(plan_kernel<int32_t, kLarge, 16>, kLarge, E_local);
 }
 
 int plan_routes(const void* ids, int ids64, int64_t numel, int E, const int32_t* emap, int E_local, int gran, int tile_rows,

@@ -239,8 +239,8 @@ int launch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int 
   rc = tc::make_map(&mw, w, dt, 2, (uint64_t)N, (uint64_t)K, BN, true);
   if (rc) return rc;
   auto kern = router_tc_kernel<T, BN>;
-  cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-  if (ce != cudaSuccess) return fail((int)ce, "router_gemm: shared memory attribute: %s", cudaGetErrorString(ce));
+  rc = allow_smem((const void*)kern, (int)C::SMEM);
+  if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((N + BN - 1) / BN * split), (unsigned)((M + RBM - 1) / RBM));
   cfg.blockDim = dim3(RTHREADS);
@@ -253,7 +253,7 @@ int launch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ce = cudaLaunchKernelEx(&cfg, kern, mx, mw, M, N, (K + 63) / 64, split, out, status, wait_limit_ns());
+  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, mx, mw, M, N, (K + 63) / 64, split, out, status, wait_limit_ns());
   if (ce != cudaSuccess) return fail((int)ce, "router_gemm (tcgen05): %s", cudaGetErrorString(ce));
   return check_launch("router_gemm (tcgen05)");
 }
@@ -262,16 +262,18 @@ int launch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int 
 // per clock out of L2) and its tensor-core time per 64-element step; the fixed part stands for launch, pipeline
 // fill, epilogue and (split) the cluster sum.  `reach` = SMs that clusters of that size fill before a second
 // round starts (128 CTAs in clusters of 8, one per SM, took two rounds); narrow tiles run two CTAs per SM, which
-// then share its bandwidth.
-void pick_tc(int64_t M, int N, int K, int& bn, int& split) {
+// then share its bandwidth.  Of a whole GPU's 148 SMs it is 112 and 132 and not what the occupancy query gives (120 and
+// 132 on one GPU; which SMs are fused off differs), so that the order of the sums is one on every B200; a
+// partition has its share.  `largest`: most CTAs of a cluster.
+void pick_tc(int64_t M, int N, int K, int sms, int largest, int& bn, int& split) {
   const int kb = (K + 63) / 64;
   const int64_t mt = (M + RBM - 1) / RBM;
   double best = 0.0;
   bn = 0;
   for (int b = 32; b <= 256; b *= 2) {
     if (b > 32 && b / 2 >= N) break;
-    for (int s = 1; s <= 8 && s <= kb; s *= 2) {
-      const double reach = s == 8 ? 112.0 : (s == 4 ? 132.0 : 148.0);
+    for (int s = 1; s <= 8 && s <= kb && s <= largest; s *= 2) {
+      const double reach = (s == 8 ? 112.0 : (s == 4 ? 132.0 : 148.0)) * sms / 148.0;
       double load = (double)(mt * ((N + b - 1) / b) * s) / reach;
       if (load < 1.0) load = 1.0;
       else if (b > 64 || load > 2.0) load = (double)(int64_t)(load + 0.999);
@@ -282,10 +284,28 @@ void pick_tc(int64_t M, int N, int K, int& bn, int& split) {
   }
 }
 
+template <typename T, int BN>
+bool split_fits(int split) {
+  const void* kern = (const void*)router_tc_kernel<T, BN>;
+  return allow_smem(kern, (int)RCfg<BN>::SMEM) != 0 || max_clusters(kern, split, RTHREADS, RCfg<BN>::SMEM) != 0;
+}
+template <typename T>
+bool split_fits(int bn, int split) {
+  switch (bn) {
+    case 32: return split_fits<T, 32>(split);
+    case 64: return split_fits<T, 64>(split);
+    case 128: return split_fits<T, 128>(split);
+    default: return split_fits<T, 256>(split);
+  }
+}
+
 template <typename T>
 int dispatch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int K, float* out, int32_t* status, cudaStream_t st) {
-  int bn, split;
-  pick_tc(M, N, K, bn, split);
+  int bn = 0, split = 1;
+  for (int largest = 8; largest >= 1; largest /= 2) {  // the largest cluster that a partition holds
+    pick_tc(M, N, K, sm_count(), largest, bn, split);
+    if (split == 1 || split_fits<T>(bn, split)) break;
+  }
   switch (bn) {
     case 32: return launch_tc<T, 32>(x, x_ld, w, M, N, K, split, out, status, st);
     case 64: return launch_tc<T, 64>(x, x_ld, w, M, N, K, split, out, status, st);
@@ -326,6 +346,14 @@ int launch_w(const void* x, int64_t x_ld, const void* w, int w_dtype, int64_t M,
 
 }  // namespace
 }  // namespace moe
+
+extern "C" int moe_router_gemm_tile(int64_t M, int N, int K, int sms, int largest_cluster, int* columns, int* split) {
+  using namespace moe;
+  if (M <= 0 || N <= 0 || K <= 0 || sms <= 0 || largest_cluster <= 0 || !columns || !split)
+    return fail(MOE_E_BADARG, "router_gemm_tile: bad extent");
+  pick_tc(M, N, K, sms, largest_cluster, *columns, *split);
+  return 0;
+}
 
 extern "C" int moe_router_gemm(const void* x, int x_dtype, int64_t x_ld, const void* w, int w_dtype, int64_t M, int N,
                                int K, float* out, void* stream) {

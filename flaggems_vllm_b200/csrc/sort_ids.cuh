@@ -151,6 +151,13 @@ __device__ __forceinline__ unsigned long long scan_cta(unsigned long long v, uns
   return before + incl - v;
 }
 
+// Whether a cluster of this size can run at all; the callers have another way where it cannot.
+template <typename Kernel>
+bool cluster_fits(Kernel kern, int ctas, int E) {
+  if (ctas == 1 || allow_smem((const void*)kern, (int)smem_bytes(kMaxExperts), ctas > 8) != 0) return true;
+  return max_clusters((const void*)kern, ctas, kThreads, smem_bytes(E)) != 0;
+}
+
 template <typename Kernel, typename... Args>
 int launch_cluster(Kernel kern, int ctas, int E, cudaStream_t st, const char* what, Args... args) {
   int rc = allow_smem((const void*)kern, (int)smem_bytes(kMaxExperts), ctas > 8);

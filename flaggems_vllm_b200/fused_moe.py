@@ -482,19 +482,12 @@ def combine_routes(y, out, topk_ids, global_num_experts, expert_map=None, row_in
 _KERNEL_SWITCHES = ("FLAGGEMS_B200_GENERIC_GEMM", "FLAGGEMS_B200_TC_WIDE", "FLAGGEMS_B200_TC_PAIR",
                     "FLAGGEMS_B200_TC_PAIR_WIDE", "FLAGGEMS_B200_PRESORT", "FLAGGEMS_B200_TMA_OUT",
                     "FLAGGEMS_B200_SMALL_M")
-_workspace_sizes = {}
 
 
-def _workspace_bytes(*key):
-    """Workspaces of the native layer call for these sizes, None when it does not serve them (a pure function of the
-    sizes: remembered)."""
-    if key not in _workspace_sizes:
-        sizes = (ctypes.c_int64 * 4)()
-        rc = _lib.lib().moe_layer_workspace(*key, ctypes.addressof(sizes))
-        if len(_workspace_sizes) > 4096:
-            _workspace_sizes.clear()
-        _workspace_sizes[key] = None if rc != 0 else tuple(sizes)
-    return _workspace_sizes[key]
+def _workspace_bytes(*sizes):
+    """Workspaces of the native layer call for these sizes, None when it does not serve them on the current device."""
+    need = (ctypes.c_int64 * 4)()
+    return tuple(need) if _lib.lib().moe_layer_workspace(*sizes, ctypes.addressof(need)) == 0 else None
 
 
 def run_chunk_native(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w2_scale, global_num_experts, expert_map,

@@ -117,6 +117,12 @@ int moe_align_block_size(const void* topk_ids, int ids_int64, int64_t numel, int
                          int block_size, int32_t* sorted_ids, int64_t sorted_cap,
                          int32_t* expert_ids, int64_t expert_cap, int32_t* num_post_pad,
                          int32_t* status, void* stream);
+/* The same with clusters of at most cluster_limit CTAs (0: whatever the device runs).  Up to 1024 experts and 262144
+ * ids the sort takes a cluster of 8 or 16; where the device, or the partition of it that the process has, holds none of
+ * that size, a kernel with a cluster of 8 or of one CTA serves the call.  The outputs are the same, bit for bit. */
+int moe_align_block_size_ex(const void* topk_ids, int ids_int64, int64_t numel, int num_experts, int block_size,
+                            int32_t* sorted_ids, int64_t sorted_cap, int32_t* expert_ids, int64_t expert_cap,
+                            int32_t* num_post_pad, int cluster_limit, int32_t* status, void* stream);
 
 /*
  * In place: expert_ids[i] = expert_map[expert_ids[i]] for n block ids (ids outside
@@ -169,6 +175,9 @@ int moe_router_gemm(const void* x, int x_dtype, int64_t x_ld, const void* w, int
 /* The same with the device status word of the kernels that wait on barriers (may be NULL). */
 int moe_router_gemm_ex(const void* x, int x_dtype, int64_t x_ld, const void* w, int w_dtype, int64_t M, int N, int K,
                        float* out, int32_t* status, void* stream);
+/* The rule behind it (host only): columns of a tile and CTAs that share its K loop (a cluster), on a device or partition
+ * with `sms` multiprocessors whose largest cluster has largest_cluster CTAs. */
+int moe_router_gemm_tile(int64_t M, int N, int K, int sms, int largest_cluster, int* columns, int* split);
 
 /*
  * Router GEMM fused with the group-limited routing, for decode batches: one launch takes the hidden

@@ -202,3 +202,55 @@ def test_align_slices(numel, E, bs):
     ref = O.moe_align_block_size_oracle(ids.cpu(), bs, E)
     for g, r in zip(got, ref):
         assert torch.equal(g.cpu(), torch.as_tensor(r))
+
+
+@pytest.mark.parametrize("limit", [1, 8])
+@pytest.mark.parametrize("numel", [0, 1, 2049, 4097, 16385, 65537, 262144])
+@pytest.mark.parametrize("E,bs", [(5, 16), (256, 128), (1024, 7)])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_align_where_large_clusters_do_not_run(limit, numel, E, bs, dtype):
+    """A partition of the GPU may hold no cluster of 16, or none of 8: other kernels, the same outputs."""
+    ids = T.make_align_ids(numel, 1, E, DEV, skewed=E > 5, seed=numel).to(dtype)
+    if numel > 40:
+        ids[7], ids[numel // 2] = -1, -3
+    cap = numel + E * (bs - 1)
+    got = [torch.full((n,), -7, dtype=torch.int32, device=DEV) for n in (cap, -(-cap // bs), 1)]
+    _lib.check(_lib.lib().moe_align_block_size_ex(
+        ids.data_ptr(), int(dtype == torch.int64), numel, E, bs, got[0].data_ptr(), cap, got[1].data_ptr(), got[1].numel(),
+        got[2].data_ptr(), limit, _lib.status_word(DEV).data_ptr(), _lib.stream_of(ids)))
+    for g, r in zip(got, fg.moe_align_block_size(ids, bs, E)):
+        assert torch.equal(g[:r.numel()], r)
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("fmt", ["half", "fp8_block", "int8_weight", "fp8_row", "int8_row"])
+def test_layer_where_the_route_plan_does_not_run(fmt, monkeypatch):
+    """The plan of more than 2048 routes needs a cluster; without one the layer goes through the align kernels."""
+    M, E, k, H, I = 1100, 4, 2, 256, 128
+    x, w1, w2, tw, ti = _half_layer(M, E, k, H, I, torch.bfloat16)
+    kw = {}
+    if fmt == "half":
+        ref = O.fused_moe_half_oracle(x, w1, w2, tw, ti)
+    elif fmt == "fp8_block":
+        (w1, s1), (w2, s2) = T.make_fp8_block_weights(E, 2 * I, H, DEV, seed=1), T.make_fp8_block_weights(E, H, I, DEV, seed=2)
+        kw = dict(use_fp8_w8a8=True, block_shape=[128, 128], w1_scale=s1, w2_scale=s2)
+        ref = O.fused_moe_fp8_block_oracle(x, w1, w2, s1, s2, tw, ti)
+    else:
+        w1, s1 = T.make_int8_channel_weights(E, 2 * I, H, DEV, seed=1)
+        w2, s2 = T.make_int8_channel_weights(E, H, I, DEV, seed=2)
+        if fmt == "fp8_row":
+            w1, w2 = w1.to(torch.float8_e4m3fn), w2.to(torch.float8_e4m3fn)
+        option = {"int8_weight": "use_int8_w8a16", "fp8_row": "use_fp8_w8a8", "int8_row": "use_int8_w8a8"}[fmt]
+        kw = {"per_channel_quant": True, "w1_scale": s1, "w2_scale": s2, option: True}
+        ref = (O.fused_moe_w8a16_oracle(x, w1, w2, s1, s2, tw, ti) if fmt == "int8_weight" else
+               O.fused_moe_row_scaled_oracle(x, w1, w2, s1.reshape(E, -1), s2.reshape(E, -1), tw, ti, fmt=fmt[:-4], per_token=True))
+
+    class NoPlan:
+        fused_experts = staticmethod(lambda *a: None)
+
+    served = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+    monkeypatch.setattr(_lib, "host", lambda: NoPlan)
+    monkeypatch.setattr("flaggems_vllm_b200.fused_moe._workspace_bytes", lambda *a: None)
+    staged = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+    _parity(served, ref, fmt)
+    _parity(staged, ref, fmt)

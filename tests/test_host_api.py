@@ -203,6 +203,18 @@ def test_small_batch_slice_count_model():
                     assert 1 <= S <= 16 and (S >= need or need > 16) and S <= max(chunks, 1)
 
 
+@pytest.mark.parametrize("sms,largest", [(148, 8), (148, 4), (70, 8), (32, 2), (16, 1)])
+def test_router_tile_keeps_to_the_clusters_of_the_device(sms, largest):
+    columns, split = ctypes.c_int(), ctypes.c_int()
+    for M in (5, 64, 200, 1000, 8192):
+        for N, K in ((8, 4096), (33, 72), (128, 2048), (256, 7168), (1024, 512)):
+            _lib.check(_lib.lib().moe_router_gemm_tile(M, N, K, sms, largest, ctypes.addressof(columns), ctypes.addressof(split)))
+            assert columns.value in (32, 64, 128, 256) and 1 <= split.value <= min(largest, -(-K // 64))
+    _lib.check(_lib.lib().moe_router_gemm_tile(200, 256, 7168, sms, largest, ctypes.addressof(columns), ctypes.addressof(split)))
+    assert split.value == largest  # a small product wants every SM it can get
+    assert _lib.lib().moe_router_gemm_tile(200, 256, 7168, 0, 8, ctypes.addressof(columns), ctypes.addressof(split)) != 0
+
+
 def test_kernel_choice_at_the_benchmark_configurations(monkeypatch):
     """Host policy (no device work): which schedule serves the configurations of the benchmark plan."""
     from flaggems_vllm_b200 import fused_moe as fm
