@@ -81,6 +81,7 @@ SYMBOLS = {
     "moe_sum": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int, c_int64, c_void_p, c_int, c_int, c_void_p,
                         c_void_p, c_void_p]),
     "moe_layer_workspace": (c_int, [c_int, c_int, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "moe_layer_layout": (c_int, [c_int, c_int, c_int64, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "moe_layer": (c_int, [c_int, c_int, c_void_p, c_int64, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                           c_float, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
@@ -96,7 +97,7 @@ _status = {}
 # calls of entry points that enqueue a kernel; LAUNCHES adds those of the native host path (bench.py reports the
 # count of its timed region)
 _ctypes_launches = 0
-_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_router_gemm_tile", "moe_set_wait_limit_ns")
+_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_layer_layout", "moe_router_gemm_tile", "moe_set_wait_limit_ns")
 
 
 class _Counted:

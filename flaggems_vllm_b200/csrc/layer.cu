@@ -3,6 +3,8 @@
 // The launches of a decode step take a few microseconds each; made one by one from Python (a dozen allocations, a
 // ctypes call per launch) they cost the host more than the device.  Here the caller passes the workspaces and the
 // launches follow each other in native code.  No state is kept between calls.
+#include <cstring>
+
 #include "moe_common.cuh"
 
 namespace moe {
@@ -102,11 +104,16 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
 
 bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
 
-// Pieces of the four workspaces (plan; rows of GEMM1; intermediate; rows behind GEMM2), 256-byte aligned.
-struct Piece { int ws; int64_t at; };
-struct Layout {
-  int64_t rows_cap, tiles_cap;
+// Pieces of the four workspaces (plan; rows of GEMM1; intermediate; rows behind GEMM2): 256-byte aligned, with at
+// least kGap bytes that nobody writes behind each, so that a write past the end of a piece can be seen.
+constexpr int64_t kGap = 256;
+struct Piece { int64_t ws, at, bytes; };
+struct Pieces {
   Piece row_index, tiles, counts, row_weight, tmp_scales, x_rows, x_scales, tmp_q, act, act_q, act_scales, y, small_counters;
+};
+static_assert(sizeof(Pieces) == MOE_LAYER_PIECES * 3 * sizeof(int64_t), "moe_layer_layout hands the table out as it is");
+struct Layout : Pieces {
+  int64_t rows_cap, tiles_cap;
   int64_t bytes[4];
   int slices[2];         // gemm_small.cu: K slices of GEMM1, GEMM2
   int64_t ncounters[3];  // and its counters: units of GEMM1, of GEMM2, tokens of GEMM2
@@ -116,8 +123,8 @@ Layout layout(int mode, const Choice& c, int64_t M, int k, int E, int E_local, i
   Layout L = {};
   const int64_t numel = M * k;
   auto take = [&](int ws, int64_t bytes) {
-    const Piece p = {ws, L.bytes[ws]};
-    L.bytes[ws] += (bytes + 255) / 256 * 256;
+    const Piece p = {ws, L.bytes[ws], bytes};
+    if (bytes > 0) L.bytes[ws] += (bytes + 255) / 256 * 256 + kGap;
     return p;
   };
   const bool byte = mode != MOE_MODE_HALF && mode != MOE_MODE_W8A16, row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
@@ -159,12 +166,18 @@ Layout layout(int mode, const Choice& c, int64_t M, int k, int E, int E_local, i
 
 extern "C" int moe_layer_workspace(int mode, int act_dtype, int64_t num_tokens, int topk, int num_experts, int E_local, int H,
                                    int I, int activation, int64_t* bytes) {
+  return moe_layer_layout(mode, act_dtype, num_tokens, topk, num_experts, E_local, H, I, activation, bytes, nullptr);
+}
+
+extern "C" int moe_layer_layout(int mode, int act_dtype, int64_t num_tokens, int topk, int num_experts, int E_local, int H, int I,
+                                int activation, int64_t* bytes, int64_t* pieces) {
   using namespace moe;
   if (num_tokens <= 0 || num_tokens > 65535 || topk <= 0 || topk > 32 || E_local <= 0 || H <= 0 || I <= 0 || !bytes ||
       !plan_serves(num_tokens * topk, num_experts, E_local) || !sizes_served(mode, act_dtype, H, I, activation))
     return fail(MOE_E_SHAPE, "layer: mode, type or sizes are not served by this call");
   const Layout L = layout(mode, choose(mode, activation, num_tokens * topk, num_experts, H, I), num_tokens, topk, num_experts, E_local, H, I);
   for (int i = 0; i < 4; ++i) bytes[i] = L.bytes[i];
+  if (pieces) std::memcpy(pieces, static_cast<const Pieces*>(&L), sizeof(Pieces));
   return 0;
 }
 

@@ -45,8 +45,6 @@ _ALL_ACTIVATIONS = ("silu", "gelu", "relu2", "swigluoai", "swigluoai_uninterleav
 
 # bench.py sets this to a callable(name) to time the stages of a step
 STAGE_HOOK = None
-# the allocator function the native host path stands in for: whoever replaces torch.empty gets the Python path
-_TORCH_EMPTY = torch.empty
 
 
 def _no_mark(_name):
@@ -610,7 +608,7 @@ def fused_experts_impl(
     logger.debug("GEMS FUSED MOE")
     if hidden_states.is_cuda and STAGE_HOOK is None and gemm1_alpha is None and gemm1_beta is None \
             and gemm1_clamp_limit is None and ocp_mx_scheme is None and w1_zp is None and w2_zp is None \
-            and w1_bias is None and w2_bias is None and torch.empty is _TORCH_EMPTY:
+            and w1_bias is None and w2_bias is None:
         # the usual cases, checked, allocated and launched in one native call
         out = _lib.host().fused_experts(
             hidden_states, w1, w2, topk_weights, topk_ids, inplace, activation, apply_router_weight_on_input, use_fp8_w8a8,

@@ -449,6 +449,13 @@ int moe_ep_unpack(const float* side, int64_t rows, int groups, int k, int rank, 
  */
 int moe_layer_workspace(int mode, int act_dtype, int64_t num_tokens, int topk, int num_experts, int E_local, int H, int I,
                         int activation, int64_t bytes[4]);
+/* The same, and where the buffers lie in the workspaces: MOE_LAYER_PIECES entries of (workspace, offset, bytes; 0 bytes =
+ * not used) in the order row_index, tiles, counts, row_weight, tmp_scales, x_rows, x_scales, tmp_q, act, act_q,
+ * act_scales, y, small_counters.  Offsets are multiples of 256; nothing is written outside the pieces, and at
+ * least 256 bytes lie behind each.  pieces may be NULL. */
+#define MOE_LAYER_PIECES 13
+int moe_layer_layout(int mode, int act_dtype, int64_t num_tokens, int topk, int num_experts, int E_local, int H, int I,
+                     int activation, int64_t bytes[4], int64_t* pieces);
 int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tokens, int topk, const void* topk_ids, int ids_int64,
               const float* topk_weights, const void* w1, const float* w1_scale, const void* w2, const float* w2_scale,
               void* out, int num_experts, const int32_t* expert_map, int E_local, int H, int I, int weight_on_input,

@@ -1,11 +1,13 @@
 """Failure handling on a real GPU without faulting or hanging it: a bounded wait that is made
 to run out sets the status bit and the context stays usable."""
 
+import ctypes
+
 import pytest
 import torch
 
 import flaggems_vllm_b200 as fg
-from flaggems_vllm_b200 import _lib
+from flaggems_vllm_b200 import _lib, fused_moe
 from flaggems_vllm_b200 import testing as T
 
 pytestmark = pytest.mark.gpu
@@ -98,36 +100,92 @@ class _GuardedAllocator:
         return len(self.blocks)
 
 
-@pytest.mark.parametrize("mode", ["bf16", "fp8", "w8a16"])
-@pytest.mark.parametrize("M", [1, 5, 200, 1500])
-def test_guard_bands_around_every_workspace_stay_intact(monkeypatch, mode, M):
-    """All internal buffers of the layer (sorted ids, expert ids, quantised rows and scales, the
-    sorted copies, the intermediate, y, the row index, split-K partial sums) are allocated with guard
-    bands on both sides; after the layer every band still holds its pattern.  The sizes cover the
-    small-batch schedule, the 128-row kernels with row stores and the staged TMA output."""
+_MODES = {"bf16": _lib.MODE_HALF, "fp8": _lib.MODE_FP8_BLOCK, "w8a16": _lib.MODE_W8A16, "fp8_row": _lib.MODE_FP8_ROW,
+          "int8_row": _lib.MODE_INT8_ROW}
+
+
+def _layer_inputs(mode, M):
     E, H, I, k = 8, 512, 512, 2
     x = T.make_activations(M, H, DEV, seed=M)
     logits, _ = T.make_router_inputs(M, E, DEV, seed=M + 1)
     tw, ti = fg.grouped_topk(torch.softmax(logits, -1), 1, 1, k, True, 1.0, torch.zeros(E, device=DEV), 0)
-    kw = {}
     if mode == "bf16":
         w1 = T.make_half_weights(E, 2 * I, H, DEV, seed=1, std=H**-0.5)
         w2 = T.make_half_weights(E, H, I, DEV, seed=2, std=I**-0.5)
-    elif mode == "fp8":
+        return x, w1, w2, tw, ti, None, None
+    if mode == "fp8":
         w1, s1 = T.make_fp8_block_weights(E, 2 * I, H, DEV, seed=1)
         w2, s2 = T.make_fp8_block_weights(E, H, I, DEV, seed=2)
-        kw = dict(use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
-    else:
-        w1, s1 = T.make_int8_channel_weights(E, 2 * I, H, DEV, seed=1)
-        w2, s2 = T.make_int8_channel_weights(E, H, I, DEV, seed=2)
-        kw = dict(use_int8_w8a16=True, per_channel_quant=True, w1_scale=s1, w2_scale=s2)
-    ref = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+        return x, w1, w2, tw, ti, s1, s2
+    w1, s1 = T.make_int8_channel_weights(E, 2 * I, H, DEV, seed=1)
+    w2, s2 = T.make_int8_channel_weights(E, H, I, DEV, seed=2)
+    if mode == "fp8_row":
+        w1, w2 = w1.to(torch.float8_e4m3fn), w2.to(torch.float8_e4m3fn)
+    return x, w1, w2, tw, ti, s1, s2
+
+
+@pytest.mark.parametrize("mode", ["bf16", "fp8", "w8a16"])
+@pytest.mark.parametrize("M", [1, 5, 200, 1500])
+def test_guard_bands_around_every_workspace_stay_intact(monkeypatch, mode, M):
+    """The staged pipeline: all its buffers (sorted ids, expert ids, quantised rows and scales, the
+    sorted copies, the intermediate, y, the row index, split-K partial sums) are allocated with guard
+    bands on both sides; after the layer every band still holds its pattern.  The sizes cover the
+    small-batch schedule, the 128-row kernels with row stores and the staged TMA output."""
+    x, w1, w2, tw, ti, s1, s2 = _layer_inputs(mode, M)
+    ref, out = torch.empty_like(x), torch.empty_like(x)
+
+    def staged(result):
+        fused_moe.run_chunk(x, w1, w2, tw, ti, result, mode=_MODES[mode], w1_scale=s1, w2_scale=s2,
+                            global_num_experts=w1.shape[0], expert_map=None, apply_router_weight_on_input=False, keep={})
+
+    staged(ref)
     guard = _GuardedAllocator()
     monkeypatch.setattr(torch, "empty", guard)
     try:
-        out = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+        staged(out)
         torch.cuda.synchronize()
     finally:
         monkeypatch.undo()
     assert guard.check() >= 4
     assert torch.equal(out, ref) and fg.read_status(torch.device(DEV)) == 0
+
+
+def _native_layer(mode, M, weight_on_input, fill, stages=63):
+    """moe_layer on workspaces of the test's own, every byte of them `fill` before: (out, workspaces, pieces)."""
+    x, w1, w2, tw, ti, s1, s2 = _layer_inputs(mode, M)
+    (E, N, H), k, band = w1.shape, ti.shape[1], _GuardedAllocator.GUARD
+    sizes = (_MODES[mode], _lib.dtype_code(x.dtype), M, k, E, E, H, N // 2, _lib.ACT_SILU)
+    need, table = (ctypes.c_int64 * 4)(), (ctypes.c_int64 * (3 * 13))()
+    _lib.check(_lib.lib().moe_layer_layout(*sizes, ctypes.addressof(need), ctypes.addressof(table)))
+    pieces = [(table[3 * i], band + table[3 * i + 1], table[3 * i + 2]) for i in range(13)]
+    ws = [torch.full((n + 2 * band,), fill, dtype=torch.uint8, device=DEV) for n in need]
+    out = torch.empty_like(x)
+    kind = 1 if mode == "fp8_row" else 0
+    _lib.check(_lib.lib().moe_layer(
+        sizes[0], sizes[1], x.data_ptr(), M, k, ti.data_ptr(), 0, tw.data_ptr(), w1.data_ptr(), _lib.ptr(s1), w2.data_ptr(),
+        _lib.ptr(s2), out.data_ptr(), E, None, E, H, N // 2, int(weight_on_input), _lib.ACT_SILU, 0.0, 0.0, 0.0, kind, None, kind,
+        None, *[w.data_ptr() + band for w in ws], stages, _lib.status_word(DEV).data_ptr(), _lib.stream_of(x)))
+    torch.cuda.synchronize()
+    return out, ws, pieces
+
+
+@pytest.mark.parametrize("mode", list(_MODES))
+@pytest.mark.parametrize("M", [1, 5, 200, 1500])
+@pytest.mark.parametrize("weight_on_input", [False, True])
+def test_gaps_between_the_buffers_of_the_layer_call_stay_intact(mode, M, weight_on_input):
+    """The layer call keeps its buffers in four workspaces.  Every byte outside the buffers, 256 or more behind
+    each and 4 KB around the workspaces, still holds its pattern afterwards, and what the workspaces held before changes no
+    result.  The sizes cover the few-route plan and split-K schedule, occupied rows only, whole blocks and staged stores."""
+    out, ws, pieces = _native_layer(mode, M, weight_on_input, _GuardedAllocator.PATTERN)
+    for i, w in enumerate(ws):
+        outside = torch.ones(w.numel(), dtype=torch.bool, device=DEV)
+        used = [(at, n) for at_ws, at, n in pieces if at_ws == i and n > 0]
+        assert used and all(at % 256 == 0 for at, _ in used)
+        for at, n in used:
+            assert bool(outside[at:at + n].all()), "pieces overlap"
+            outside[at:at + n] = False
+        for at, n in used:
+            assert bool(outside[at + n:at + n + 256].all()), "no gap behind a piece"
+        assert bool((w[outside] == _GuardedAllocator.PATTERN).all()), f"a kernel wrote outside its buffer in workspace {i}"
+    assert torch.equal(out, _native_layer(mode, M, weight_on_input, 0xFF)[0])  # 0xFF: NaN in every float type
+    assert torch.isfinite(out).all() and fg.read_status(torch.device(DEV)) == 0

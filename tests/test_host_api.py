@@ -247,3 +247,17 @@ def test_kernel_choice_at_the_benchmark_configurations(monkeypatch):
     assert fm._choose_kernel(_lib.MODE_FP8_BLOCK, bf16, 7168, 2048, 65536, 256) == fm.KERNEL_TC_PAIR
     monkeypatch.setenv("FLAGGEMS_B200_GENERIC_GEMM", "1")
     assert fm._choose_kernel(_lib.MODE_FP8_BLOCK, bf16, 7168, 2048, 65536, 256) == fm.KERNEL_GENERIC
+
+
+@pytest.mark.parametrize("mode", [_lib.MODE_HALF, _lib.MODE_FP8_BLOCK, _lib.MODE_W8A16, _lib.MODE_FP8_ROW, _lib.MODE_INT8_ROW])
+@pytest.mark.parametrize("tokens", [1, 40, 1500])
+def test_layer_buffers_lie_apart(mode, tokens):
+    """Buffers of the layer call share four workspaces: aligned, inside them, at least 256 bytes between neighbours."""
+    need, table = (ctypes.c_int64 * 4)(), (ctypes.c_int64 * 39)()
+    _lib.check(_lib.lib().moe_layer_layout(mode, _lib.MOE_BF16, tokens, 2, 8, 8, 512, 512, _lib.ACT_SILU,
+                                           ctypes.addressof(need), ctypes.addressof(table)))
+    for ws in range(4):
+        used = sorted((table[i + 1], table[i + 2]) for i in range(0, 39, 3) if table[i] == ws and table[i + 2] > 0)
+        assert used
+        for (at, n), (after, _) in zip(used, used[1:] + [(need[ws], 0)]):
+            assert at % 256 == 0 and at + n + 256 <= after
