@@ -16,7 +16,8 @@ int plan_routes(const void* ids, int ids64, int64_t numel, int E, const int32_t*
 int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,
                         float* scales_t, cudaStream_t st);
 int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st);
-int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, cudaStream_t st);
+int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, int groups,
+                 int64_t rows_cap, float* scales_t, cudaStream_t st);
 int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
                  const void* tiles, const int32_t* rows, int64_t numel, int64_t rows_cap, int E, int K, int Nout, void* out,
                  float* out_scales_t, const float* row_weight, bool all_rows, bool staged, int32_t* status, cudaStream_t st);
@@ -247,7 +248,9 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
     } else {
       rc = scatter_rows(x, M, (int64_t)H * 2, topk, row_index, at(L.x_rows), st);
     }
-    if (!rc && c.zero_pad) rc = zero_padding(tiles, L.tiles_cap, counts, (int64_t)H * (block ? 1 : 2), at(L.x_rows), st);
+    if (!rc && c.zero_pad)
+      rc = zero_padding(tiles, L.tiles_cap, counts, (int64_t)H * (block ? 1 : 2), at(L.x_rows), block ? H / 128 : 0, L.rows_cap,
+                        block ? x_scales : nullptr, st);
     if (!rc && row_weight != nullptr) rc = scatter_floats(topk_weights, numel, 1, row_index, row_weight, st);
     if (rc) return rc;
   }

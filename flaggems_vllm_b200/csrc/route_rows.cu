@@ -13,20 +13,25 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Zeroes the padding rows of the plan's tiles, one block per (tile, eighth of its padding rows).  At prefill sizes the
-// GEMMs multiply those rows, and zeros cost the power-limited board less than stale bytes (DSV3 FP8, 8192 tokens:
-// 5430 -> 5050 us per layer).
+// Zeroes the padding rows of the plan's tiles and (1x128 scaled rows) their scales, one block per (tile, eighth of its
+// padding).  At prefill sizes the GEMMs multiply those rows.
 constexpr int kPadParts = 8;
 __global__ void __launch_bounds__(kThreads) zero_padding_kernel(const int4* __restrict__ tiles, const int32_t* __restrict__ counts,
-                                                                int row_vec, uint4* __restrict__ rows) {
+                                                                int row_vec, uint4* __restrict__ rows, int groups,
+                                                                int64_t scale_ld, float* __restrict__ scales_t) {
   pdl_wait();
   pdl_trigger();
   if ((int)blockIdx.x >= counts[0]) return;
   const int4 d = tiles[blockIdx.x];
-  for (int r = (d.y >> 16) + blockIdx.y; r < (d.y & 0xFFFF); r += kPadParts) {
-    uint4* p = rows + (int64_t)(d.x + r) * row_vec;
+  const int occupied = d.y >> 16, padding = (d.y & 0xFFFF) - occupied;
+  for (int r = blockIdx.y; r < padding; r += kPadParts) {
+    uint4* p = rows + (int64_t)(d.x + occupied + r) * row_vec;
     for (int i = threadIdx.x; i < row_vec; i += kThreads) p[i] = make_uint4(0, 0, 0, 0);
   }
+  if (scales_t == nullptr) return;
+  // zero times a stale scale is NaN where the workspace happened to hold one
+  for (int i = blockIdx.y * kThreads + threadIdx.x; i < padding * groups; i += kPadParts * kThreads)
+    scales_t[(int64_t)(i / padding) * scale_ld + d.x + occupied + i % padding] = 0.0f;
 }
 
 // Block (c, m): P x 2048 columns of token m, a warp per two neighbouring 128-groups, 8 elements per lane.  The arithmetic
@@ -188,9 +193,10 @@ bool whole_rows(int64_t M) { return M >= 4 * sm_count(); }
 }  // namespace
 
 // M <= 65535 for all of these (the second grid dimension): the layer call checks it.
-int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, cudaStream_t st) {
+int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, int groups,
+                 int64_t rows_cap, float* scales_t, cudaStream_t st) {
   return launch_pdl(zero_padding_kernel, dim3((unsigned)tiles_cap, kPadParts), kThreads, 0, 1, st, "zero padding rows",
-                    (const int4*)tiles, counts, (int)(row_bytes / 16), (uint4*)rows);
+                    (const int4*)tiles, counts, (int)(row_bytes / 16), (uint4*)rows, groups, rows_cap, scales_t);
 }
 
 int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,

@@ -189,3 +189,19 @@ def test_gaps_between_the_buffers_of_the_layer_call_stay_intact(mode, M, weight_
         assert bool((w[outside] == _GuardedAllocator.PATTERN).all()), f"a kernel wrote outside its buffer in workspace {i}"
     assert torch.equal(out, _native_layer(mode, M, weight_on_input, 0xFF)[0])  # 0xFF: NaN in every float type
     assert torch.isfinite(out).all() and fg.read_status(torch.device(DEV)) == 0
+
+
+@pytest.mark.parametrize("M", [600, 1500])
+def test_padding_rows_are_zero_whatever_the_workspaces_held(M):
+    """From 128 rows per expert on, the FP8 GEMMs multiply whole blocks: the padding rows of both operands are zeros,
+    with finite scales, although every byte of the workspaces was 0xFF (NaN) before."""
+    _, ws, pieces = _native_layer("fp8", M, False, 0xFF, stages=1 | 2 | 4)
+    view = lambda i, t: ws[pieces[i][0]][pieces[i][1]:pieces[i][1] + pieces[i][2]].view(t)
+    H = I = 512
+    x_rows, act = view(5, torch.uint8).view(-1, H), view(8, torch.uint8).view(-1, I)
+    x_scales, act_scales = (view(i, torch.float32).view(4, -1) for i in (6, 10))
+    tiles = view(1, torch.int32).view(-1, 4)[:int(view(2, torch.int32)[0])].tolist()
+    padding = [r for row0, n, _, _ in tiles for r in range(row0 + (n >> 16), row0 + (n & 0xFFFF))]
+    assert len(padding) > 8
+    assert bool((x_rows[padding] == 0).all()) and bool((x_scales[:, padding] == 0).all())
+    assert bool(((act[padding] & 0x7F) == 0).all()) and bool(torch.isfinite(act_scales[:, padding]).all())
