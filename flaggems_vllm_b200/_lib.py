@@ -24,6 +24,7 @@ _DTYPE_CODE = {torch.float32: MOE_F32, torch.float16: MOE_F16, torch.bfloat16: M
 SYMBOLS = {
     "moe_abi_version": (c_int, []),
     "moe_last_error": (c_char_p, []),
+    "moe_launch_count": (c_uint64, []),
     "moe_set_wait_limit_ns": (c_uint64, [c_uint64]),
     "moe_debug_wait_timeout": (c_int, [c_void_p, c_uint64, c_void_p, c_void_p]),
     "moe_grouped_topk": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int,
@@ -94,28 +95,6 @@ SYMBOLS = {
 
 _lib = None
 _status = {}
-# calls of entry points that enqueue a kernel; LAUNCHES adds those of the native host path (bench.py reports the
-# count of its timed region)
-_ctypes_launches = 0
-_NO_KERNEL = ("moe_abi_version", "moe_last_error", "moe_small_m_plan", "moe_layer_workspace", "moe_layer_layout", "moe_router_gemm_tile", "moe_set_wait_limit_ns")
-
-
-class _Counted:
-    """The library handle with a call counter in front of every kernel-launching entry point."""
-
-    def __init__(self, handle):
-        for name in SYMBOLS:
-            fn = getattr(handle, name)
-            setattr(self, name, fn if name in _NO_KERNEL else self._wrap(fn))
-
-    @staticmethod
-    def _wrap(fn):
-        def call(*args):
-            global _ctypes_launches
-            _ctypes_launches += 1
-            return fn(*args)
-
-        return call
 
 
 class MoeKernelError(RuntimeError):
@@ -135,7 +114,7 @@ def lib():
             fn = getattr(handle, name)
             fn.restype = res
             fn.argtypes = args
-        _lib = _Counted(handle)
+        _lib = handle
     return _lib
 
 
@@ -158,7 +137,7 @@ def host():
 
 def __getattr__(name):
     if name == "LAUNCHES":
-        return _ctypes_launches + (_host.launches() if _host is not None else 0)
+        return lib().moe_launch_count()  # kernels enqueued so far; bench.py reports the count of its timed region
     raise AttributeError(name)
 
 

@@ -70,12 +70,15 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
+static std::atomic<unsigned long long> g_launches{0};
+
 int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     snprintf(g_err, sizeof(g_err), "%s: %s", what, cudaGetErrorString(e));
     return (int)e;
   }
+  g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
 }
 }  // namespace moe
@@ -86,4 +89,5 @@ extern "C" unsigned long long moe_set_wait_limit_ns(unsigned long long ns) {
   if (ns != 0) moe::g_wait_limit_ns = ns;
   return old;
 }
+extern "C" unsigned long long moe_launch_count(void) { return moe::g_launches.load(std::memory_order_relaxed); }
 extern "C" const char* moe_last_error(void) { return moe::g_err; }

@@ -21,7 +21,6 @@
 namespace {
 
 std::atomic<int32_t*> g_status[64];        // status word of every device, registered by _lib.status_word
-std::atomic<long long> g_launches{0};      // kernels enqueued from here
 
 #define MOE_NONE Py_RETURN_NONE
 
@@ -74,7 +73,6 @@ PyObject* set_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
   g_status[dev].store(reinterpret_cast<int32_t*>(ptr));
   MOE_NONE;
 }
-PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 
 // The interpreter lock is given back for as long as a function allocates and launches: cudaMalloc may wait for the
 // device, and a launch waits when the stream's queue is full, while the work it waits for may need another thread
@@ -174,7 +172,6 @@ PyObject* fused_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
                    c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
   }
   if (rc != 0) MOE_NONE;
-  g_launches += 5;
   if (inplace) {
     Py_INCREF(a[0]);
     return a[0];
@@ -209,7 +206,6 @@ PyObject* grouped_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
                           ids.mutable_data_ptr<int32_t>(), c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
   }
   if (rc != 0) MOE_NONE;
-  ++g_launches;
   PyObject* r = PyTuple_New(2);
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(w));
   PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(ids));
@@ -249,7 +245,6 @@ PyObject* topk_route(PyObject*, PyObject* const* a, Py_ssize_t n) {
                         c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
   }
   if (rc != 0) MOE_NONE;
-  ++g_launches;
   Py_RETURN_TRUE;
 }
 
@@ -274,7 +269,6 @@ PyObject* router_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
                             out.mutable_data_ptr<float>(), status, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
   }
   if (rc != 0) MOE_NONE;
-  ++g_launches;
   return THPVariable_Wrap(out);
 }
 
@@ -303,7 +297,6 @@ PyObject* align(PyObject*, PyObject* const* a, Py_ssize_t n) {
                               c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream());
   }
   if (rc != 0) MOE_NONE;
-  ++g_launches;
   PyObject* r = PyTuple_New(3);
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(sorted));
   PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(experts));
@@ -323,7 +316,7 @@ PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
 
 #define MOE_FN(name) {#name, (PyCFunction)(void (*)(void))guarded<name>, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MOE_FN(set_status), MOE_FN(fused_experts), MOE_FN(grouped_topk), MOE_FN(topk_route),
-                         MOE_FN(router_gemm), MOE_FN(align), {"launches", launches, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                         MOE_FN(router_gemm), MOE_FN(align), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ext", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

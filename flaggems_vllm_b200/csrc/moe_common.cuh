@@ -14,7 +14,8 @@ namespace moe {
 
 // Records a host-side failure text for moe_last_error(); returns `code`.
 int fail(int code, const char* fmt, ...);
-// Checks the launch error of the kernel just enqueued; returns 0 or the cudaError_t.
+// Checks the launch error of the kernel just enqueued; returns 0 or the cudaError_t.  Called once per kernel: it counts
+// the launches that were accepted (moe_launch_count).
 int check_launch(const char* what);
 // Limit, in nanoseconds, of every bounded barrier wait of the kernels launched from now on
 // (moe_set_wait_limit_ns; 2 s unless changed).

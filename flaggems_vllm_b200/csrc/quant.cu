@@ -522,9 +522,12 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
         done = true;                                                                                                \
       }                                                                                                             \
     }                                                                                                               \
-    if (!done)                                                                                                      \
+    if (!done) {                                                                                                    \
       rowwise_quant_kernel<T, K><<<grid, 256, 0, st>>>((const T*)x, rows, cols, SIN, row_ids, valid_below,          \
                                                        indirect, (uint8_t*)q, scale_out);                                     \
+      const int rc = check_launch("rowwise_quant");                                                                 \
+      if (rc) return rc;                                                                                            \
+    }                                                                                                               \
   } while (0)
   switch (kind) {
     case 0: MOE_RQ(0, nullptr); break;
@@ -535,14 +538,18 @@ static int rowwise_quant_launch(const void* x, int64_t rows, int64_t cols, int k
       cudaError_t ce = cudaMemsetAsync(scale_out, 0, sizeof(float), st);
       if (ce != cudaSuccess) return fail((int)ce, "rowwise_quant: %s", cudaGetErrorString(ce));
       tensor_amax_kernel<T><<<grid, 256, 0, st>>>((const T*)x, rows, cols, row_ids, valid_below, indirect, (unsigned int*)scale_out);
+      int rc = check_launch("rowwise_quant (amax)");
+      if (rc) return rc;
       amax_to_scale_kernel<<<1, 1, 0, st>>>(scale_out);
+      rc = check_launch("rowwise_quant (scale)");
+      if (rc) return rc;
       MOE_RQ(3, scale_out);
       break;
     }
     default: return fail(MOE_E_BADARG, "rowwise_quant: unknown kind %d", kind);
   }
 #undef MOE_RQ
-  return check_launch("rowwise_quant");
+  return 0;
 }
 
 namespace moe {

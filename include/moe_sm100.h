@@ -59,6 +59,9 @@ enum { MOE_ACT_SILU = 0, MOE_ACT_SWIGLUOAI = 1 };
 
 int moe_abi_version(void);
 const char* moe_last_error(void);
+/* Kernels this library has enqueued in the process, whoever called (launches that a stream capture recorded count
+ * once; replays of the graph do not). */
+unsigned long long moe_launch_count(void);
 
 /*
  * Failure handling hooks; neither has a counterpart in the reference (its Triton kernels have no

@@ -254,3 +254,34 @@ def test_layer_where_the_route_plan_does_not_run(fmt, monkeypatch):
     staged = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
     _parity(served, ref, fmt)
     _parity(staged, ref, fmt)
+
+
+@pytest.mark.parametrize("fmt,M,kernels", [
+    ("half", 2, 3),        # split K: align, GEMM 1, GEMM 2 with the sum
+    ("half", 300, 5),      # plan, scatter, GEMM 1, GEMM 2, sum
+    ("fp8_block", 300, 6),  # the padding rows of whole blocks are cleared besides
+    ("int8_row", 300, 6),  # the intermediate has its own quantiser
+    ("align", 64, 1),
+    ("fp8_tensor_quant", 64, 3)])  # one scale for the tensor: its largest value, the scale, the quantiser
+def test_launch_count_is_the_number_of_kernels(fmt, M, kernels):
+    E, k, H, I = 4, 2, 256, 128
+    x, w1, w2, tw, ti = _half_layer(M, E, k, H, I, torch.bfloat16)
+    if fmt == "align":
+        call = lambda: fg.moe_align_block_size(ti, 16, E)
+    elif fmt == "fp8_tensor_quant":
+        q, sc = torch.empty(x.shape, dtype=torch.uint8, device=DEV), torch.empty(1, device=DEV)
+        call = lambda: _lib.check(_lib.lib().moe_rowwise_quant(x.data_ptr(), _lib.dtype_code(x.dtype), M, H, 3, None, None, 0,
+                                                               q.data_ptr(), sc.data_ptr(), _lib.stream_of(x)))
+    else:
+        kw = {}
+        if fmt == "fp8_block":
+            (w1, s1), (w2, s2) = T.make_fp8_block_weights(E, 2 * I, H, DEV), T.make_fp8_block_weights(E, H, I, DEV)
+            kw = dict(use_fp8_w8a8=True, block_shape=[128, 128], w1_scale=s1, w2_scale=s2)
+        elif fmt == "int8_row":
+            (w1, s1), (w2, s2) = T.make_int8_channel_weights(E, 2 * I, H, DEV), T.make_int8_channel_weights(E, H, I, DEV)
+            kw = dict(use_int8_w8a8=True, per_channel_quant=True, w1_scale=s1, w2_scale=s2)
+        call = lambda: fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+    call()
+    before = _lib.LAUNCHES
+    call()
+    assert _lib.LAUNCHES - before == kernels

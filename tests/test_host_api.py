@@ -29,6 +29,13 @@ def test_library_builds_and_exports_every_declared_symbol():
     assert handle.moe_abi_version() >= 1
 
 
+def test_a_refused_call_counts_no_launch():
+    before = _lib.LAUNCHES
+    assert _lib.lib().moe_align_block_size(None, 0, 4, 8, 16, None, 64, None, 4, None, None, None) != 0
+    assert _lib.lib().moe_layer_workspace(_lib.MODE_HALF, _lib.MOE_BF16, 0, 2, 8, 8, 512, 512, 0, None) != 0
+    assert _lib.LAUNCHES == before
+
+
 def _sig(fn):
     return [(n, p.kind, p.default) for n, p in inspect.signature(fn).parameters.items()]
 
