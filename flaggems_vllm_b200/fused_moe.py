@@ -714,6 +714,10 @@ def fused_experts_impl(
         w1c, w2c = _widen_int8(w1c, hidden_states.dtype), _widen_int8(w2c, hidden_states.dtype)
         mode = _lib.MODE_HALF
 
+    if expert_map is not None and expert_map.numel() < global_num_experts:
+        # the kernels look up every id below the expert count: ids beyond the map are not local
+        expert_map = torch.nn.functional.pad(expert_map, (0, global_num_experts - expert_map.numel()), value=-1)
+
     out_hidden_states = hidden_states if inplace else torch.empty_like(hidden_states)
     for chunk in range((num_tokens // CHUNK_SIZE) + 1):
         begin, end = chunk * CHUNK_SIZE, min((chunk + 1) * CHUNK_SIZE, num_tokens)

@@ -285,3 +285,20 @@ def test_launch_count_is_the_number_of_kernels(fmt, M, kernels):
     before = _lib.LAUNCHES
     call()
     assert _lib.LAUNCHES - before == kernels
+
+
+@pytest.mark.parametrize("M", [3, 300, 2500])
+@pytest.mark.parametrize("staged", [False, True])
+def test_expert_map_shorter_than_the_expert_count(M, staged, monkeypatch):
+    """Ids beyond the map have no local expert; the kernels, which look up every id below the count, get a map that long."""
+    E, k, H, I = 12, 3, 256, 128
+    x, w1, w2, tw, ti = _half_layer(M, E, k, H, I, torch.bfloat16)
+    emap = torch.tensor([-1, 1, 0, 3, -1, 2], dtype=torch.int32, device=DEV)
+    order = [2, 1, 5, 3]  # global expert of local expert 0, 1, 2, 3
+    keep = torch.isin(ti, torch.tensor(order, dtype=torch.int32, device=DEV))
+    ref = O.fused_moe_half_oracle(x, w1, w2, tw * keep, ti)
+    if staged:
+        monkeypatch.setenv("FLAGGEMS_B200_PRESORT", "auto")  # any of the switches takes the staged pipeline
+    out = fg.fused_experts_impl(x, w1[order].contiguous(), w2[order].contiguous(), tw, ti, global_num_experts=E, expert_map=emap)
+    _parity(out, ref, M)
+    assert bool((out[~keep.any(1)] == 0).all())
