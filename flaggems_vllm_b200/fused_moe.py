@@ -153,7 +153,6 @@ def _check_activation(activation, gemm1_alpha, gemm1_beta, gemm1_clamp_limit):
 
 
 SMALL_BLOCK_M = 8
-_small_scratch = {}
 
 
 def _small_eligible(mode, act_dtype, H, I, k) -> bool:
@@ -193,17 +192,6 @@ def _sm_count(dev) -> int:
     if idx not in _sm_counts:
         _sm_counts[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
     return _sm_counts[idx]
-
-
-def _small_counters(dev, n):
-    """Zeroed int32 words the small-batch kernels count arrivals in.  Every launch leaves them
-    zero, so one buffer per (device, stream) is zeroed once and reused."""
-    key = (dev.index, torch.cuda.current_stream(dev).cuda_stream)
-    buf = _small_scratch.get(key)
-    if buf is None or buf.numel() < n:
-        buf = torch.zeros(max(n, 1 << 16), dtype=torch.int32, device=dev)
-        _small_scratch[key] = buf
-    return buf
 
 
 def small_k_slices(mode, gemm1, K, N, blocks, sms) -> int:
@@ -271,7 +259,9 @@ def run_chunk_small(x, w1, w2, topk_weights, topk_ids, out, *, mode, w1_scale, w
 
     h1, part1, uc1, _ = plan(True, H, I)
     h2, part2, uc2, tc2 = plan(False, I, H)
-    counters = _small_counters(dev, uc1 + uc2 + tc2)
+    # arrival counts; the call's own: a buffer kept per stream would be shared by graphs captured on it and replayed
+    # side by side, and would keep the counts of a call that gave up on a wait
+    counters = torch.zeros(uc1 + uc2 + tc2, dtype=torch.int32, device=dev)
     partial = torch.empty(max(part1, part2, 1), dtype=torch.float32, device=dev)
     act = torch.empty((rows_cap, I), dtype=x.dtype, device=dev)
     y = torch.empty((numel, H), dtype=x.dtype, device=dev)

@@ -791,7 +791,7 @@ def test_layer_under_cuda_graph_replay_with_new_inputs():
 
 @pytest.mark.parametrize("case", ["bf16_small_batch", "w8a16_small_batch", "bf16_sorted_output"])
 def test_other_paths_under_cuda_graph_replay_with_new_inputs(case):
-    """The small-batch schedule (its counters clean themselves, its scratch is reused) and the
+    """The small-batch schedule (counters and scratch are part of the graph) and the
     staged-output GEMM 2 replay correctly from a CUDA graph when the inputs change."""
     E, H, I, k = 8, 512, 256, 2
     M = {"bf16_small_batch": 2, "w8a16_small_batch": 1, "bf16_sorted_output": 700}[case]
@@ -824,6 +824,30 @@ def test_other_paths_under_cuda_graph_replay_with_new_inputs(case):
         graph.replay()
         torch.cuda.synchronize()
         _assert_parity(out, oracle(x, tw, ti), f"{case} replay {seed}")
+
+
+def test_small_batch_graphs_captured_on_one_stream_replay_side_by_side(monkeypatch):
+    """Every call of the split-K schedule counts arrivals in words of its own."""
+    monkeypatch.setenv("FLAGGEMS_B200_SMALL_M", "1")
+    E, H, I, k, M = 8, 4096, 2048, 2, 4
+    w1 = T.make_half_weights(E, 2 * I, H, DEV, seed=1, std=H**-0.5)
+    w2 = T.make_half_weights(E, H, I, DEV, seed=2, std=I**-0.5)
+    xs = [T.make_activations(M, H, DEV, seed=s) for s in (3, 4)]
+    tw, ti = _route(M, E, k, torch.bfloat16)
+    expected = [fg.fused_experts_impl(x, w1, w2, tw, ti) for x in xs]
+    capture, graphs, outs = torch.cuda.Stream(), [], []
+    for x in xs:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=capture):
+            outs.append(fg.fused_experts_impl(x, w1, w2, tw, ti))
+        graphs.append(graph)
+    streams = [torch.cuda.Stream() for _ in xs]
+    for _ in range(20):
+        for graph, stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, e) for o, e in zip(outs, expected)) and _lib.read_status() == 0
 
 
 def test_empty_batch_and_single_token():
