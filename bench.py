@@ -782,11 +782,11 @@ def main():
         f1 = 2.0 * M * k * (2 * I) * H
         peak2x = 2.0 * peaks["bf16_tflops"]
         peak = fp8_peak if fp8_peak else peak2x
-        # DRAM traffic of one GEMM1 launch: ncu (dram__bytes_read+write) on the 32-expert /
-        # 1024-token capture gave 1.134 GB for 0.964 GB of algorithmic bytes (weights of the
-        # experts in use + e4m3 activations + scales + the e4m3 intermediate), a ratio of 1.18;
-        # both grow with the number of experts in use, so the full-size figure is that ratio
-        # times this launch's algorithmic bytes.
+        # DRAM traffic of one GEMM1 launch: ncu (dram__bytes_read+write, one pass) on this workload, 8192
+        # tokens and 256 experts, gave 10.12 GB for 7.713 GB of algorithmic bytes (weights of the experts in
+        # use + e4m3 activations + scales + the e4m3 intermediate), a ratio of 1.31 (the weights of an expert's
+        # second and third row block are not always still in L2, and the sorted rows are read eight
+        # times as often as the tokens); 32 experts and 1024 tokens give 1.31 too.
         _, ti0 = fg.grouped_topk(logits, c["n_group"], c["topk_group"], k, True, c["rsf"], bias, 1)
         e_act = int(torch.unique(ti0).numel())
         alg1 = e_act * (2 * I * H + (2 * I // 128) * (H // 128) * 4) + M * H + M * (H // 128) * 4 + M * k * I
@@ -795,7 +795,7 @@ def main():
                             "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                             "peak_fp8_measured": fp8_peak, "frac_vs_2x_bf16": ach / peak2x,
                             "frac_of_sustained": ach / (2.0 * peaks["bf16_tflops_sustained"]),
-                            "traffic": 1.18 * alg1, "traffic_source": "ncu small-case DRAM bytes scaled by algorithmic bytes (x1.18)",
+                            "traffic": 1.31 * alg1, "traffic_source": "ncu DRAM bytes of this launch over its algorithmic bytes (x1.31)",
                             "algorithmic_bytes": alg1,
                             "peak_source": ("torch._scaled_mm e4m3 8192^3, best of 10, CUDA events, measured in this run"
                                             if fp8_peak else f"2 x bf16_tflops of {peaks['source']} peaks"),

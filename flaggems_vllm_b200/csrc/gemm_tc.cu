@@ -289,7 +289,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #endif
   if constexpr (!GATHER && !PAIR && RB == 1) {
     // Route plan, occupied rows only: the other rows of a stage are multiplied all the same.  They start as zeros and
-    // stay zeros until a larger tile comes by, and zeros cost the tensor cores less energy than stale bytes.
+    // stay zeros until a larger tile comes by.  Without this: DSV3 FP8, 61 tokens 1005 -> 1103 us per layer, one of 8 ranks
+    // with 2000 tokens 319 -> 323; Mixtral shape, 300 tokens 520 -> 533.
     if (P.tiles != nullptr && !P.all_rows) {
       for (int i = threadIdx.x; i < STAGES * A_LOCAL_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(sA)[i] = make_uint4(0, 0, 0, 0);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -24,8 +24,9 @@
 //                swizzle of the raw tile makes its 16-byte loads conflict-free.
 // TMEM columns hold two elements of K each, so an MMA (16 elements) takes 8 columns of A.
 //
-// Bound at prefill (Qwen3 shape, 4096 tokens): L2 -> SM traffic, 10.8 TB/s in GEMM1 with the tensor pipe at 52 %; at decode
-// HBM, less the last partial wave.  Against gemm_w8.cu: 33 tokens 191 -> 146 us per layer, 4096 tokens 591 -> 465.
+// Bound at prefill (Qwen3 shape, 4096 tokens): cycles on the SM and not memory.  GEMM1 takes 330 thousand cycles at
+// 1.35 GHz and 334 at 1.58, GEMM2 217 and 223, the tensor pipe 53 and 44 % of them; which of the chains (converters, tile
+// boundary) is the long one is open.  At decode HBM, less the last partial wave.  Against gemm_w8.cu: 33 tokens 191 -> 146 us per layer, 4096 tokens 591 -> 465.
 #include "wt_common.cuh"
 
 namespace moe {

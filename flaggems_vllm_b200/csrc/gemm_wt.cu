@@ -7,8 +7,9 @@
 // DeepSeek-V3's prefill sizes, and every CTA fetches 48 KB of operands per 128-byte K block of a 128x256 tile.
 // Here the padding is to 16 (route plan, plan.cu), and the pair shares the token tile: each CTA fetches
 // its 16 KB of weights and HALF of the tokens (<= 16 KB) and the tensor cores read the other half from the peer.
-// At prefill sizes the board runs at its power limit, so operands not moved and padding not multiplied are
-// clock as well as cycles.
+// Bound at prefill: the clock that power leaves.  Mixtral shape, 16384 tokens: GEMM1 6.73 million cycles, 94 % of them
+// MMA, whether the clock in the kernel is 1.30 GHz (after a pause) or 1.10 (sustained); operands not moved and padding
+// not multiplied are clock as well as cycles.
 //
 // Both operands arrive by TMA: token rows were put into sorted order by the scatter kernels (route_rows.cu, quant.cu).  Every load
 // of both CTAs counts its bytes on the leader's barrier of the stage; the leader's MMA thread needs no other

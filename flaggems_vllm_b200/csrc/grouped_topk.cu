@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(128) grouped_topk_kernel(
 
 // The same routing for groups of 32 experts (DeepSeek-V3: 8 groups), one warp per GROUP and one CTA per token.  With a
 // warp per token eight double-precision sigmoids, eight group maxima and topk extractions follow each other in
-// one warp (13-15 us for one token); here every lane owns one expert and nothing is extracted: an expert's
+// one warp (8.5 us for one token under graph replay, 2.6 here); here every lane owns one expert and nothing is extracted: an expert's
 // rank in its group, and a candidate's rank among all groups' candidates, are counted against keys in shared memory.
 // Keys are unique, so the counted order is the extracted one, bit for bit.
 constexpr int kGroupWarps = 8;  // at most 8 groups

@@ -68,8 +68,13 @@ bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
 
 // The split-K weight streaming of gemm_small.cu: three launches instead of five, every SM busy however few tiles there
 // are, but one CTA needs more instructions per byte than the tile kernels.  So it is for calls whose launches count: up to
-// 8 routes that read up to 1 GB of weights (Mixtral shape: one token, 2 routes, 0.7 GB, 143 against 171 us with the tile
-// kernels; two tokens 230 against 225; four tokens 394 against 334; E8 H1024 I2048: four tokens 29 against 38).
+// 8 routes that read up to 1 GB of weights if no two share an expert, which the host cannot see.  us per layer, split K
+// against tile kernels, bf16:
+//   Mixtral shape    1 token  0.7 GB  137 : 168   2 tokens 1.4 GB  256 : 253 (one pair of experts 143 : 168)
+//                    3 tokens 2.1 GB  371 : 330 (143 : 169)       4 tokens 2.8 GB  483 : 438 (148 : 171)
+//   E8 H1024 I2048   1 token   25 MB   18 : 30    2 tokens          20 : 31    4 tokens 27 : 37
+//   E128 H2048 I768  1 token   75 MB   23 : 28
+// From 1.4 GB on, distinct experts lose what shared ones would win, and distinct is the usual case.
 constexpr int kSmallRoutes = 8;
 constexpr int64_t kSmallBytes = 1000000000;
 

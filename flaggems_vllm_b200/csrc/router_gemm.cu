@@ -89,8 +89,8 @@ __global__ void __launch_bounds__(kThreads) router_gemm_kernel(const XT* __restr
 // run-to-run deterministic and no partial ever goes to memory.  The product is small (256 x 7168
 // weights): what bounds it is how many SMs pull operands from L2 at once and the latency of one CTA's
 // K loop, hence the split.  Rows and columns beyond the matrix are zero-filled by TMA.
-// B200, K = 7168, N = 256, bf16, graph replay: 200 rows 54 -> 8.6 us (one CTA per column on CUDA cores before),
-// 64 rows 19 -> 6.6 us, 8192 rows 36 us.
+// B200, K = 7168, N = 256, bf16, graph replay: 200 rows 54 -> 8.6 us (the row-streaming kernel before), 64 rows
+// 19 -> 6.7 us, 8192 rows 36 us.
 constexpr int RBM = 128, RTHREADS = 192;
 template <int BN> struct RCfg {
   static constexpr int STAGE = (RBM + BN) * 128;
@@ -369,9 +369,10 @@ extern "C" int moe_router_gemm_ex(const void* x, int x_dtype, int64_t x_ld, cons
   if (K % 8 != 0 || x_ld % 8 != 0 || x_ld < K) return fail(MOE_E_SHAPE, "router_gemm: K and the row pitch must be multiples of 8");
   if (((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return fail(MOE_E_BADARG, "router_gemm: operands must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
-  // Half-precision products run on tcgen05 from five rows on (5 us whatever the row count up to 128, K = 7168; the
-  // row-streaming kernel takes 2.6 us for one row, 4.8 for two, 10 for eight, 19 for 64).  Below, the row-streaming
-  // kernel's reduction order is shared by the fused router (moe_router_gemm_grouped_topk) bit for bit.
+  // Half-precision products run on tcgen05 from five rows on (K = 7168, N = 256, graph replay: 6.5-6.9 us for 8 to 128
+  // rows, 7.7 for five; the row-streaming kernel 2.7 us for one row, 3.7 for two, 5.2 for four, 10 for eight, 19 for
+  // 64).  Below, the row-streaming kernel's reduction order is shared by the fused router
+  // (moe_router_gemm_grouped_topk) bit for bit.
   if (M > kRowStreamMax && x_dtype == w_dtype && (x_dtype == MOE_BF16 || x_dtype == MOE_F16) && M < (1ll << 31) - RBM && ((uintptr_t)out & 15) == 0) {
     if ((M + RBM - 1) / RBM > 65535) return fail(MOE_E_TOOBIG, "router_gemm: serves at most %d rows", 65535 * RBM);
     return x_dtype == MOE_BF16 ? dispatch_tc<__nv_bfloat16>(x, x_ld, w, M, N, K, out, status, st)

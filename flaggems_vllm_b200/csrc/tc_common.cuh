@@ -41,11 +41,9 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 // One lane of a converged warp.  The warp that feeds the tensor core runs its loop with all 32
-// lanes and only predicates the instructions on this lane: under a divergent `lane == 0` branch
-// the compiler cannot keep descriptors and addresses in uniform registers and moves each of them
-// there in front of every tcgen05.mma, which costs a warp that shares its scheduler with busy
-// ones several hundred cycles per K block (e4m3 128x256 tile with the fp32 fold beside it,
-// operands streaming from L2: 880 -> 612 cycles per 128-wide K block).
+// lanes and only predicates the instructions on this lane.  The same loop under a divergent
+// `lane == 0` branch is slower in a warp that shares its scheduler with busy ones: 880 against 612
+// cycles per 128-wide K block (e4m3 128x256 tile with the fp32 fold beside it, operands streaming from L2).
 __device__ __forceinline__ bool elect_lane() {
   uint32_t p;
   asm volatile(
@@ -132,7 +130,8 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* ba
       : "memory");
 }
 // The loads of a CTA pair: the data lands in this CTA, the bytes are counted on the barrier at this
-// offset in the pair's leader (clearing the peer bit of a shared-memory address names the even CTA).
+// offset in the pair's leader (clearing the peer bit of a shared-memory address names the even CTA: the value is
+// Sm100MmaPeerBitMask of CUTLASS, include/cute/arch/copy_sm100_tma.hpp).
 constexpr uint32_t LEADER_BAR_MASK = 0xFEFFFFFFu;
 __device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint64_t* bar, void* dst, int c0, int c1) {
   asm volatile(

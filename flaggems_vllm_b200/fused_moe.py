@@ -1,7 +1,16 @@
 """fused_experts_impl: the MoE layer on expert-sorted rows.
 
-Pipeline per chunk of at most 32768 tokens (the reference's chunk size,
-src/flaggems_vllm/ops/fused_moe.py:2399-2400):
+Chunks of at most 32768 tokens (the reference's chunk size,
+src/flaggems_vllm/ops/fused_moe.py:2399-2400) go through one native call (``moe_layer``, csrc/layer.cu):
+
+    route plan                    stable sort of routes by expert, tiles of the GEMMs
+    scatter                       token rows into sorted order, quantised on the way where the mode wants it
+    gemm1                         SiLU(x Wg^T) * (x Wu^T)   (+ 1x128 re-quant, FP8)
+    gemm2                         act W2^T, sorted order
+    combine                       fixed-order fp32 sum over the top-k routes, times the route weights
+
+What it does not serve (odd sizes, f32, other activations, more than 2^18 routes in a chunk, a partition of the GPU without
+the plan's cluster), kept intermediates and pinned kernels take the staged pipeline:
 
     moe_align_block_size          stable sort of routes by expert, 1 launch
     per_token_group_quant_fp8     FP8 mode only: activations -> e4m3 + 1x128 scales, once per token
@@ -66,8 +75,9 @@ def _choose_kernel(mode, act_dtype, H, I, numel, num_experts):
     kernel, FLAGGEMS_B200_TC_WIDE / FLAGGEMS_B200_TC_PAIR = 0/1 force the 256-row variants
     off/on (tests and experiments); otherwise:
 
-    * FP8 block scales: one CTA per 128-row block.  (The cta_group::2 pair loses there: the
-      per-K-block accumulator hand-off would cross two SMs; GEMM1 3.6 -> 4.2 ms at M=8192.)
+    * FP8 block scales: one CTA per 128-row block.  (The cta_group::2 pair loses there: 8192 tokens of the
+      DeepSeek-V3 shape, 966 cycles per K block and unit against 813 with nothing padded, and 256-row blocks pad
+      more: GEMM1 3.04 -> 3.49 ms.)
     * weight-only int8: the kernel that widens the weights in shared memory.
     * half precision with >= 256 rows per expert: the 256x256 single-CTA tile,
       which fetches each weight tile once per 256 rows.

@@ -441,9 +441,11 @@ int moe_ep_unpack(const float* side, int64_t rows, int groups, int k, int rank, 
 /*
  * The whole expert layer in one call: route plan, scatter (with the activation quantiser of the mode), GEMM1,
  * GEMM2, weighted sum over a token's routes (src/flaggems_vllm/ops/fused_moe.py:2314-2737).  Serves the modes
- * MOE_MODE_HALF (H % 64 == 0), MOE_MODE_FP8_BLOCK (SiLU), MOE_MODE_FP8_ROW and MOE_MODE_INT8_ROW (H % 128 == 0), f16 / bf16
- * activations, I % 128 == 0, topk <= 32, at most 1024 experts and 2^20 routes; moe_layer_workspace
- * writes the sizes in bytes of the four workspaces, or returns MOE_E_SHAPE for anything else.
+ * MOE_MODE_HALF (H % 64 == 0), MOE_MODE_FP8_BLOCK (SiLU), MOE_MODE_W8A16 (SiLU, H % 64 == 0), MOE_MODE_FP8_ROW and
+ * MOE_MODE_INT8_ROW (H % 128 == 0), f16 / bf16 activations, I % 128 == 0, at most 65535 tokens, topk <= 32, 1024 local
+ * experts and 2^18 routes, and on a device (or partition of one) that runs the route plan's cluster: none up to 2048
+ * routes, 8 CTAs up to 16384, 16 beyond.  moe_layer_workspace writes the sizes in bytes of the four workspaces, or returns
+ * MOE_E_SHAPE for anything else.
  *   x, out [num_tokens, H]; topk_ids, topk_weights [num_tokens, topk]; weights and scales as in moe_gemm1_ex /
  *   moe_gemm2; expert_map [num_experts] or NULL: local index of every expert, negative = not local;
  *   quant_kind1 / 2, quant_scale1 / 2: row-scaled modes, how the input and the intermediate are quantised

@@ -268,3 +268,14 @@ def test_layer_buffers_lie_apart(mode, tokens):
         assert used
         for (at, n), (after, _) in zip(used, used[1:] + [(need[ws], 0)]):
             assert at % 256 == 0 and at + n + 256 <= after
+
+
+@pytest.mark.parametrize("tokens,topk,experts,served", [
+    (32768, 8, 256, True), (32769, 8, 256, False), (32768, 9, 256, False), (65535, 4, 256, True), (65536, 1, 256, False),
+    (4096, 8, 1024, True), (4096, 8, 1025, False), (8, 32, 64, True), (8, 33, 64, False)])
+def test_layer_call_serves_what_its_declaration_says(tokens, topk, experts, served):
+    need = (ctypes.c_int64 * 4)()
+    for mode in (_lib.MODE_HALF, _lib.MODE_FP8_BLOCK, _lib.MODE_W8A16, _lib.MODE_FP8_ROW, _lib.MODE_INT8_ROW):
+        rc = _lib.lib().moe_layer_workspace(mode, _lib.MOE_BF16, tokens, topk, experts, experts, 256, 128, _lib.ACT_SILU,
+                                            ctypes.addressof(need))
+        assert (rc == 0) == served
