@@ -21,9 +21,8 @@
 //   warps 2-3   GEMM1: cp.async gather of the A rows
 //   warps 4-7   epilogue: accumulator -> channel scale -> SiLU*up / route weight -> store,
 //               two passes of 128 columns per tile
-//   warps 8-19  converters: raw int8 -> f16 / bf16 operand tile.  The conversion is integer-ALU
-//               work (about 1.5 byte-permute / logic instructions per weight), the limiter
-//               of this kernel, hence twelve warps of it.
+//   warps 8-19  converters: raw int8 -> f16 / bf16 operand tile, integer-ALU work (about 1.5
+//               byte-permute / logic instructions per weight); sixteen warps of it are 3-8 % slower.
 // Both TMEM accumulators are used, so the epilogue of one tile overlaps the K
 // loop of the next.  Every barrier wait is bounded; on expiry the kernel sets
 // MOE_ST_WAIT_TIMEOUT, leaves its loops, frees TMEM and returns.

@@ -3,7 +3,7 @@
 //     D[weight row, token] = (int8 W[row, :] widened exactly to f16 / bf16) . X[token, :],   channel scale at the end
 //
 // gemm_w8.cu widens the weights into shared memory, where every 128x256 tile moves 128 KB per 64 elements of K: raw
-// bytes in and out, widened bytes in and out, activations in and out; 1000 cycles for 512 cycles of MMA.  Here the
+// bytes in and out, widened bytes in and out, activations in and out; 1400 cycles for 512 cycles of MMA.  Here the
 // weights are the M operand, so their widened form can live in TENSOR MEMORY: converter warps read the raw bytes
 // (each byte once), widen them in registers and write them with tcgen05.st, and the MMA takes A from there
 // (tcgen05.mma with a TMEM A operand).  Shared memory only sees the raw bytes and the token rows.
@@ -24,9 +24,9 @@
 //                swizzle of the raw tile makes its 16-byte loads conflict-free.
 // TMEM columns hold two elements of K each, so an MMA (16 elements) takes 8 columns of A.
 //
-// Bound at prefill (Qwen3 shape, 4096 tokens): cycles on the SM and not memory.  GEMM1 takes 330 thousand cycles at
-// 1.35 GHz and 334 at 1.58, GEMM2 217 and 223, the tensor pipe 53 and 44 % of them; which of the chains (converters, tile
-// boundary) is the long one is open.  At decode HBM, less the last partial wave.  Against gemm_w8.cu: 33 tokens 191 -> 146 us per layer, 4096 tokens 591 -> 465.
+// Bound at prefill (Qwen3 shape, 4096 tokens): GEMM1 335 thousand cycles and GEMM2 220, whatever the clock, of which 294 and
+// 167 are left without widening and epilogue: the load streams through their rings (57 B per clock and SM in GEMM1).  At
+// decode HBM, less the last partial wave.  Against gemm_w8.cu: 33 tokens 191 -> 146 us per layer, 4096 tokens 591 -> 465.
 #include "wt_common.cuh"
 
 namespace moe {
