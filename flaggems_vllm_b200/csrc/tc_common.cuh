@@ -43,7 +43,7 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 // One lane of a converged warp.  The warp that feeds the tensor core runs its loop with all 32
 // lanes and only predicates the instructions on this lane.  The same loop under a divergent
 // `lane == 0` branch is slower in a warp that shares its scheduler with busy ones: 880 against 612
-// cycles per 128-wide K block (e4m3 128x256 tile with the fp32 fold beside it, operands streaming from L2).
+// cycles per 128-wide K block (stand-alone e4m3 128x256 tile with the fp32 fold beside it).
 __device__ __forceinline__ bool elect_lane() {
   uint32_t p;
   asm volatile(
