@@ -152,7 +152,7 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const Params P) {
   constexpr bool FP8 = MODE == MOE_MODE_FP8_BLOCK;
   constexpr bool W8 = MODE == MOE_MODE_W8A16;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = tc::align_1024(smem_raw);
   uint8_t* ring = smem;
   uint8_t* xs = smem + (size_t)STAGES * STAGE_BYTES;  // [ROWS][XPITCH]
   Smem* aux = reinterpret_cast<Smem*>(xs + ROWS * F::XPITCH);

@@ -34,18 +34,18 @@
 // back to the tensor core before its last FMAs.  The scales of the K blocks
 // in flight sit in a small shared-memory ring filled by the producer side, so
 // the consumers issue no global loads inside the K loop.
-// Bound (FP8, 2048 rows per expert): GEMM1 the fold's chain, 809 cycles per K block, 803 with one of its four MMAs, 586
-// without the fold; GEMM2, 16 K blocks per tile, the tile boundary (988 cycles per K block, 909 without the fold).
-// The clock those cycles run at is what power leaves, 1.0 to 1.4 GHz at prefill sizes.
+// Bound (FP8, 2048 rows per expert, cycles per K block, tile boundaries included): GEMM1 the fold's chain, 701 (620 without
+// the fold, whatever the number of MMAs or commits: the operand stream); GEMM2, 16 K blocks per tile, the chain and the tile
+// boundary, 836.  The chain is a consumer warp's instructions and their latencies, not the MMAs (the same with one of
+// the four) nor the loads (the same with none); before barriers, slots and descriptors were carried in registers it was
+// 811 and 900.  The clock those cycles run at is what power leaves: 1.4 GHz with 32 experts, 0.9 to 1.2 with 256, whose
+// weights come out of HBM; there time follows energy and 14 % fewer cycles are 3 to 8 % of the time.
 // Half mode: the whole K loop accumulates in TMEM; the two accumulators let
 // the epilogue of one tile overlap the main loop of the next.
 //
 // Every barrier wait is bounded (wall-clock limit); on expiry the kernel sets
 // MOE_ST_WAIT_TIMEOUT, leaves its loops, frees TMEM and returns.
 #include "tc_common.cuh"
-#ifdef MOE_TC_TRACE
-#include <cstdlib>
-#endif
 
 namespace moe {
 namespace tc {
@@ -89,7 +89,7 @@ struct SmemAux {
   uint64_t full[MAX_STAGES];       // this CTA's operands (and scales) of the stage have landed
   uint64_t empty[MAX_STAGES];      // the tensor core has finished reading the stage
   uint64_t peer_full[MAX_STAGES];  // pair leader only: the partner CTA's stage has landed
-  uint64_t tmem_full[2];
+  alignas(16) uint64_t tmem_full[2];  // the FP8 loops toggle between the two by address bit 3, and find tmem_empty 16 bytes on
   uint64_t tmem_empty[2];
   uint64_t xch_bar;
   uint32_t tmem_base;
@@ -99,9 +99,12 @@ struct SmemAux {
   // with cp.async and read by the consumers.  The ring is deeper than
   // STAGES + the two accumulators, so a slot is never rewritten before the
   // consumers have read it.
-  float sc_a[SCALE_SLOTS][BM];  // activation scale of each tile row
-  float sc_w[SCALE_SLOTS][4];   // weight scales of the two column halves
+  struct Slot {
+    float a[BM];  // activation scale of each tile row
+    float w[4];   // weight scales of the two column halves
+  } sc[SCALE_SLOTS];
 };
+static_assert(offsetof(SmemAux, tmem_full) % 16 == 0 && offsetof(SmemAux, tmem_empty) == offsetof(SmemAux, tmem_full) + 16, "barrier addresses");
 constexpr int OUT_STAGE_BYTES = BM * BN * 2;  // staged output tile of the TMAOUT variant
 template <bool PAIR, int RB, bool TMAOUT = false> constexpr size_t smem_bytes() {
   return TMAOUT ? (size_t)3 * Cfg<PAIR, RB>::STAGE_BYTES + sizeof(SmemAux) + 1024 + OUT_STAGE_BYTES + 1024
@@ -137,19 +140,7 @@ struct Params {
   int w_row0;   // GEMM2 over a window of the output columns: first weight row (output column) of the window
   bool all_rows;    // route plan: fetch whole 128-row blocks of A (their padding rows are zero) instead of the occupied rows
   bool wide_store;  // the output is 32-byte aligned: rows are written with 32-byte stores
-#ifdef MOE_TC_TRACE
-  long long* trace;  // [4 roles][64 K blocks][8 events] cycle stamps of CTA 0, third tile (experiment builds)
-#endif
 };
-#ifdef MOE_TC_TRACE
-#define MOE_TR(role, kb, ev) \
-  do { if (blockIdx.x == 0 && tile == tile0 + 2 * tile_step && P.trace && (kb) < 64) P.trace[((role) * 64 + (kb)) * 8 + (ev)] = clock64(); } while (0)
-#define MOE_TRN(role, slot, ev) \
-  do { if (blockIdx.x == 0 && tile == tile0 + 3 * tile_step && P.trace) P.trace[((role) * 64 + (slot)) * 8 + (ev)] = clock64(); } while (0)
-#else
-#define MOE_TR(role, kb, ev) do {} while (0)
-#define MOE_TRN(role, slot, ev) do {} while (0)
-#endif
 
 // Instruction descriptor: fp32 accumulator (bits 4-5 = 1), A/B element format
 // (bits 7-9 / 10-12: e4m3 = 0 for kind::f8f6f4; f16 = 0, bf16 = 1 for
@@ -231,14 +222,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   constexpr int A_LOCAL_BYTES = Cfg<PAIR, RB>::A_LOCAL;
   constexpr int B_LOCAL_BYTES = PAIR ? B_HALF_BYTES : B_STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_1024(smem_raw);
   uint8_t* sA = smem;
   uint8_t* sB = smem + (size_t)STAGES * A_LOCAL_BYTES;
   SmemAux* aux = reinterpret_cast<SmemAux*>(smem + (size_t)STAGES * Cfg<PAIR, RB>::STAGE_BYTES);
   // staged output tile: four sub-tiles of 128 rows x 64 columns (128 bytes per row), 1024-byte aligned
   [[maybe_unused]] uint8_t* s_out = smem + (((size_t)STAGES * Cfg<PAIR, RB>::STAGE_BYTES + sizeof(SmemAux) + 1023) & ~(size_t)1023);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // the compiler sees that `warp` is uniform
   constexpr int KBE = BYTE ? 128 : 64;  // elements of K per stage
   const int KB = (P.K + KBE - 1) / KBE;
   const int npp = min((int64_t)__ldcg(P.num_post_pad), P.rows_cap);
@@ -287,9 +278,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     e_next = expert_of(blk0);
   }
 
-#ifdef MOE_TC_TRACE
-  if (threadIdx.x == 0 && blockIdx.x == 0 && P.trace) { P.trace[2048] = clock64(); P.trace[2049] = (long long)now_ns(); P.trace[2052] = total_tiles; }
-#endif
   if constexpr (!GATHER && !PAIR && RB == 1) {
     // Route plan, occupied rows only: the other rows of a stage are multiplied all the same.  They start as zeros and
     // stay zeros until a larger tile comes by.  Without this: DSV3 FP8, 61 tokens 1005 -> 1103 us per layer, one of 8 ranks
@@ -341,7 +329,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const bool leader = elect_lane();
       if constexpr (!GATHER) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
-      uint32_t it = 0;
+      uint32_t s = 0, ph = 1;  // stage, and the parity its "empty" barrier is waited for with
       bool alive = true;
       constexpr bool EARLY = !GATHER && !PAIR && RB == 1;
       auto occupied_rows = [&](int blk) -> int {  // rows of A to fetch
@@ -374,27 +362,54 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         [[maybe_unused]] const int row0 = mb * BM;
         const int wrow0 = e * P.rows_w + P.w_row0;
         [[maybe_unused]] const int a_rows = occupied_rows(blk);
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          MOE_TR(0, kb, 0);
-          if (!mbar_wait(&aux->empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
-          MOE_TR(0, kb, 1);
-          if (!leader) continue;
-          if (early > 0) --early;
-          else load_weights(kb, s, a_rows, wrow0, nt);
-          if constexpr (!GATHER) {
-            uint8_t* dst = sA + (size_t)s * A_LOCAL_BYTES;
-            if (a_rows < RB * BM) {  // route plan, few rows: the rest of the stage keeps stale bytes, its results are never stored
-              int r = 0;
-              for (; a_rows - r >= 16; r += 16) tma_load_2d(&map_a16, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
-              if (r < a_rows) tma_load_2d(&map_a8, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
-            } else {
+        for (int kb = 0; kb < KB; ++kb) {
+          if (!mbar_wait_at(smem_u32(&aux->empty[s]), ph, P.status, P.wait_ns)) { alive = false; break; }
+          if (leader) {
+            if (early > 0) --early;
+            else load_weights(kb, (int)s, a_rows, wrow0, nt);
+            if constexpr (!GATHER) {
+              uint8_t* dst = sA + (size_t)s * A_LOCAL_BYTES;
+              if (a_rows < RB * BM) {  // route plan, few rows: the rest of the stage keeps stale bytes, its results are never stored
+                int r = 0;
+                for (; a_rows - r >= 16; r += 16) tma_load_2d(&map_a16, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
+                if (r < a_rows) tma_load_2d(&map_a8, &aux->full[s], dst + r * 128, kb * KBE, row0 + r);
+              } else {
 #pragma unroll
-              for (int j = 0; j < RB; ++j) tma_load_2d(&map_a, &aux->full[s], dst + j * A_STAGE_BYTES, kb * KBE, row0 + j * BM);
+                for (int j = 0; j < RB; ++j) tma_load_2d(&map_a, &aux->full[s], dst + j * A_STAGE_BYTES, kb * KBE, row0 + j * BM);
+              }
             }
           }
-          MOE_TR(0, kb, 2);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
+        }
+      }
+    } else if (FP8 && !PAIR && warp == 1) {
+      // ------------------------------------------------------------ MMA issuer, FP8: a fresh accumulator per K block
+      // Every barrier and descriptor is carried in a register: what stands between "accumulator released" and the MMAs is a
+      // fence.  (A loop that computed them took 118 cycles from one K block's commits to its next wait.)
+      constexpr uint32_t idesc = IDesc<FMT, AT, PAIR>::value;
+      const bool leader = elect_lane();
+      const uint64_t adesc0 = make_smem_desc(smem_u32(sA)), bdesc0 = make_smem_desc(smem_u32(sB));
+      const uint32_t full0 = smem_u32(&aux->full[0]);
+      constexpr uint32_t TO_EMPTY = (uint32_t)(offsetof(SmemAux, empty) - offsetof(SmemAux, full));
+      uint32_t full = full0, sph = 0, acc_empty = smem_u32(&aux->tmem_empty[0]), aph = 1, d = tmem_base;
+      uint64_t adesc = adesc0, bdesc = bdesc0;
+      bool alive = true;
+      for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
+        MOE_TILE_COORDS(tile)
+        if (e < 0 || e >= P.E) continue;
+#pragma unroll 1
+        for (int left = KB; left > 0; --left) {
+          if (!mbar_wait_at(full, sph, P.status, P.wait_ns) || !mbar_wait_at(acc_empty, aph, P.status, P.wait_ns)) { alive = false; break; }
+          if constexpr (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async writes -> tensor core reads
+          tc_fence_after();
+          tc_mma_block_f8(leader, d, adesc, bdesc, idesc, acc_empty - 16, full + TO_EMPTY);
+          d ^= BN;
+          acc_empty ^= 8;
+          aph ^= ((acc_empty >> 3) & 1) ^ 1;
+          full += 8;
+          adesc += (uint64_t)(A_LOCAL_BYTES >> 4);
+          bdesc += (uint64_t)(B_LOCAL_BYTES >> 4);
+          if (full == full0 + 8 * STAGES) { full = full0; adesc = adesc0; bdesc = bdesc0; sph ^= 1; }
         }
       }
     } else if (warp == 1 && cr == 0) {
@@ -404,58 +419,39 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t acc_it = 0;
       bool alive = true;
       if constexpr (!PAIR) {
-        // This thread shares its scheduler with two consumer warps that stream FMAs, and every
-        // instruction it needs between "accumulator released" and "MMAs issued" waits for an issue
-        // slot behind them.  So everything that does not depend on the release is done before the
-        // wait for it: stage index and phase are carried (no division), the descriptors are one
-        // add away from a base, and the operands' barrier (which completed long before) is waited
-        // for first.  After the release only the fence, the four MMAs and the commits remain.
         const bool leader = elect_lane();
         const uint64_t adesc0 = make_smem_desc(smem_u32(sA));
         const uint64_t bdesc0 = make_smem_desc(smem_u32(sB));
         uint32_t s = 0, sph = 0;
         for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
-          MOE_TRN(1, 61, 0);
           MOE_TILE_COORDS(tile)
           if (e < 0 || e >= P.E) continue;
-          MOE_TRN(1, 61, 1);
           for (int kb = 0; kb < KB; ++kb) {
             const uint32_t a = RB == 2 ? 0u : (acc_it & 1);
             const uint32_t aph = RB == 2 ? (acc_it & 1) : ((acc_it >> 1) & 1);
             const uint64_t bdesc = bdesc0 + (uint64_t)(s * (uint32_t)(B_LOCAL_BYTES >> 4));
             const uint64_t adesc = adesc0 + (uint64_t)(s * (uint32_t)(A_LOCAL_BYTES >> 4));
             const uint32_t d0 = tmem_base + a * BN;
-            MOE_TR(1, kb, 0);
             if (!mbar_wait(&aux->full[s], sph, P.status, P.wait_ns)) { alive = false; break; }
-            MOE_TR(1, kb, 1);
             if constexpr (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async writes -> tensor core reads
-            if (FP8 || kb == 0) {
+            if (kb == 0) {
               if (!mbar_wait(&aux->tmem_empty[a], aph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
             }
-            MOE_TR(1, kb, 2);
             tc_fence_after();
             if (leader) {
 #pragma unroll
             for (int j = 0; j < RB; ++j) {
               const uint64_t aj = adesc + (uint64_t)(j * (A_STAGE_BYTES >> 4));
               const uint32_t d = RB == 2 ? tmem_base + (uint32_t)j * BN : d0;
-              if (FP8) {
-                tc_mma_const<KIND, false>(d, aj, bdesc, idesc);
-              } else {
-                tc_mma<KIND>(d, aj, bdesc, idesc, kb > 0);
-              }
+              tc_mma<KIND>(d, aj, bdesc, idesc, kb > 0);
 #pragma unroll
               for (int k4 = 1; k4 < 4; ++k4)  // 32 bytes of K per instruction: start address advances by 32 B >> 4
                 tc_mma_const<KIND, true>(d, aj + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc);
             }
-            if (FP8 || kb == KB - 1) tc_commit(&aux->tmem_full[a]);
+            if (kb == KB - 1) tc_commit(&aux->tmem_full[a]);
             tc_commit(&aux->empty[s]);
             }
-            if (FP8 || kb == KB - 1) ++acc_it;
-            MOE_TR(1, kb, 3);
-            if (kb == 0) MOE_TRN(1, 61, 2);
-            if (kb == 1) MOE_TRN(1, 61, 3);
-            if (kb == 2) MOE_TRN(1, 61, 4);
+            if (kb == KB - 1) ++acc_it;
             if (++s == STAGES) { s = 0; sph ^= 1; }
           }
         }
@@ -555,9 +551,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % STAGES;
-          if (g == 0) MOE_TR(2, kb, 0);
           if (!mbar_wait(&aux->empty[s], ((it / STAGES) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
-          if (g == 0) MOE_TR(2, kb, 1);
           const uint32_t base = smem_u32(sA + (size_t)s * A_LOCAL_BYTES);
 #pragma unroll
           for (int j = 0; j < RPT; ++j) {
@@ -573,11 +567,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int slot = it % SCALE_SLOTS;
 #pragma unroll
             for (int j = 0; j < 2; ++j)
-              if (as_src[j] != nullptr) cp_async4(smem_u32(&aux->sc_a[slot][g + 64 * j]), as_src[j] + (int64_t)kb * P.a_scale_ld);
-            if (g < 2) cp_async4(smem_u32(&aux->sc_w[slot][g]), ws_src + kb);
+              if (as_src[j] != nullptr) cp_async4(smem_u32(&aux->sc[slot].a[g + 64 * j]), as_src[j] + (int64_t)kb * P.a_scale_ld);
+            if (g < 2) cp_async4(smem_u32(&aux->sc[slot].w[g]), ws_src + kb);
           }
           cp_async_arrive_noinc(&aux->full[s]);
-          if (g == 0) MOE_TR(2, kb, 2);
         }
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
@@ -598,8 +591,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const int s = it % STAGES;
           if (!mbar_wait(&aux->empty[s], ((it / STAGES) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           const int slot = it % SCALE_SLOTS;
-          cp_async16(smem_u32(&aux->sc_a[slot][4 * lane]), as_row + (int64_t)kb * P.a_scale_ld);
-          if (lane < 2) cp_async4(smem_u32(&aux->sc_w[slot][lane]), ws_src + kb);
+          cp_async16(smem_u32(&aux->sc[slot].a[4 * lane]), as_row + (int64_t)kb * P.a_scale_ld);
+          if (lane < 2) cp_async4(smem_u32(&aux->sc[slot].w[lane]), ws_src + kb);
           cp_async_arrive_noinc(&aux->full[s]);
         }
       }
@@ -612,8 +605,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int row = ((warp & 3) << 5) + lane;       // accumulator lane = tile row
     const uint32_t t_lane = tmem_base + ((uint32_t)((warp & 3) << 5) << 16) + (uint32_t)(h * (GEMM1 ? 64 : 128));
     constexpr uint32_t SECOND = GEMM1 ? 128 : 64;  // column distance of the group's second 64-column chunk
-    uint32_t acc_it = 0, tile_it = 0;
+    [[maybe_unused]] uint32_t acc_it = 0, tile_it = 0;
     bool alive = true;
+    // FP8: the accumulator, its barrier and phase, and the scale slot of the next K block
+    [[maybe_unused]] uint32_t t_acc = t_lane, acc_full = smem_u32(&aux->tmem_full[0]), acc_ph = 0, slot_at = 0;
+    [[maybe_unused]] const uint32_t row_at = smem_u32(aux) + 4 * (uint32_t)row, w_at = smem_u32(aux) + (GEMM1 ? 0u : 4u * (uint32_t)h);
     // releasing an accumulator: the pair's leader collects the arrivals of both CTAs
     auto release_acc = [&](uint32_t a) {
       tc_fence_before();
@@ -647,14 +643,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     };
     prefetch_tile(tile0);
     for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
-      if (threadIdx.x == 128) MOE_TRN(3, 61, 0);
       const int blk = nx_blk, nt = nx_nt, e = nx_e;
       const int64_t sid_first = nx_sid;
       [[maybe_unused]] const int mb = UNIT * blk + RB * cr;
       (void)blk;
       if (!FP8 || e < 0 || e >= P.E) prefetch_tile(tile + tile_step);  // half precision has no K loop here
       if (e < 0 || e >= P.E) continue;
-      if (threadIdx.x == 128) MOE_TRN(3, 61, 1);
       for (int sub = 0; sub < RB && alive; ++sub) {  // the 128-row blocks of this tile (two for wide tiles)
       const int64_t p = (int64_t)(mb + sub) * BM + row;
       int64_t sid = P.numel;
@@ -668,51 +662,70 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if constexpr (FP8) {
 #pragma unroll
         for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
-        // one K block: wait for its accumulator, fold it into acc, release it
-        auto fold_block = [&](float s_lo, float s_hi, [[maybe_unused]] int kb) {
-          const uint32_t a = acc_it & 1;
-          tc_fence_after();
-          const uint32_t t0 = t_lane + a * BN;
-          uint32_t ra[32], rb[32];
-          unsigned long long* acc2 = reinterpret_cast<unsigned long long*>(acc);
-          const unsigned long long lo2 = splat2(s_lo), hi2 = splat2(s_hi);
-          // The accumulator is held from the first load to the release, and the tensor core's next
-          // K block into it waits for that.  The second half is therefore reloaded into each
-          // 32-register staging set as soon as its FMAs have consumed it, under the FMAs of the
-          // other set, and the FMAs of the second half run after the release.  Packed pair FMAs:
-          // the fold's issue slots are what the MMA-issuing thread on the same scheduler competes with.
-          tmem_ld64_sync(t0, ra, rb);
-          if (threadIdx.x == 128) MOE_TR(3, kb, 2);
+        // Each K block: wait for its accumulator, fold it into acc, release it.  The accumulator is held from the first load
+        // to the release, and the tensor core's next K block into it waits for that.  The second half is therefore reloaded into
+        // each 32-register staging set as soon as its FMAs have consumed it, under the FMAs of the other set, and the FMAs of
+        // the second half run after the release; the probe for the next accumulator is in flight under them.  Packed pair
+        // FMAs: the fold's issue slots are what the MMA-issuing thread on the same scheduler competes with.
+        // Two warps per scheduler do not hide each other's latencies (both wait for the same barrier), so what is not an
+        // FMA counts: barrier, scale slot and accumulator are addresses carried in registers and toggled, the release is
+        // predicated and not branched around, nothing is asked per K block that can be asked per tile.  811 -> 701 cycles per K
+        // block of GEMM1 (2048 rows per expert), of which the FMAs are 256.
+        uint32_t ra[32], rb[32];
+        unsigned long long* acc2 = reinterpret_cast<unsigned long long*>(acc);
+        constexpr int SC = (int)offsetof(SmemAux, sc), SLOT = (int)sizeof(SmemAux::Slot);
+        float sa, w_lo, w_hi;
+        // scales from the shared-memory ring filled by the producer side: GEMM1 halves are (gate, up) -> w[0], w[1]; GEMM2 group
+        // h owns one weight block
+        auto next_scales = [&] {
+          sa = lds_f32<SC>(row_at + slot_at);
+          w_lo = lds_f32<SC + BM * 4>(w_at + slot_at);
+          w_hi = GEMM1 ? lds_f32<SC + BM * 4 + 4>(w_at + slot_at) : w_lo;
+          slot_at += SLOT;
+          if (slot_at == SCALE_SLOTS * SLOT) slot_at = 0;
+        };
+        prefetch_tile(tile + tile_step);
+        if (P.mul_weight && row_ok) rw = P.route_weight[sid];
+        alive = mbar_wait_at(acc_full, acc_ph, P.status, P.wait_ns);
+        if (!alive) break;
+        __syncwarp();
+        tc_fence_after();
+        next_scales();
+#pragma unroll 1
+        for (int left = KB; left > 0; --left) {
+          const unsigned long long lo2 = splat2(sa * w_lo), hi2 = GEMM1 ? splat2(sa * w_hi) : lo2;
+          tmem_ld64_sync(t_acc, ra, rb);
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma2(acc2[i], ra[2 * i], ra[2 * i + 1], lo2);
-          tmem_ld32_async(t0 + SECOND, ra);
+          tmem_ld32_async(t_acc + SECOND, ra);
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma2(acc2[16 + i], rb[2 * i], rb[2 * i + 1], lo2);
-          tmem_ld32_async(t0 + SECOND + 32, rb);
+          tmem_ld32_async(t_acc + SECOND + 32, rb);
           tmem_wait64(ra, rb);
-          release_acc(a);
-          if (threadIdx.x == 128) MOE_TR(3, kb, 3);
+          if constexpr (PAIR) {
+            release_acc((acc_full >> 3) & 1);
+          } else {
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_at<16>(acc_full, lane == 0);
+          }
+          t_acc ^= BN;
+          acc_full ^= 8;
+          acc_ph ^= ((acc_full >> 3) & 1) ^ 1;
+          bool ready = true;
+          if (left > 1) ready = mbar_try_at(acc_full, acc_ph);
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma2(acc2[32 + i], ra[2 * i], ra[2 * i + 1], hi2);
+          if (left > 1) {
+            if (!__all_sync(0xFFFFFFFFu, ready)) {
+              ready = mbar_wait_at(acc_full, acc_ph, P.status, P.wait_ns);
+              if (!__all_sync(0xFFFFFFFFu, ready)) { alive = false; break; }
+            }
+            tc_fence_after();
+            next_scales();
+          }
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma2(acc2[48 + i], rb[2 * i], rb[2 * i + 1], hi2);
-          ++acc_it;
-        };
-        // scales come from the shared-memory ring filled by the producer side:
-        // GEMM1 halves are (gate, up) -> sc_w[0], sc_w[1]; GEMM2 group h owns one weight block
-        for (int kb = 0; kb < KB; ++kb) {
-          const int slot = acc_it % SCALE_SLOTS;
-          if (threadIdx.x == 128) MOE_TR(3, kb, 0);
-          if (kb == (KB > 1 ? 1 : 0)) prefetch_tile(tile + tile_step);
-          if (!mbar_wait(&aux->tmem_full[acc_it & 1], (acc_it >> 1) & 1, P.status, P.wait_ns)) { alive = false; break; }
-          if (threadIdx.x == 128) MOE_TR(3, kb, 1);
-          if (threadIdx.x == 128 && kb == 0) MOE_TRN(3, 61, 2);
-          const float sa = aux->sc_a[slot][row];
-          const float s_lo = sa * aux->sc_w[slot][GEMM1 ? 0 : h];
-          const float s_hi = sa * aux->sc_w[slot][GEMM1 ? 1 : h];
-          fold_block(s_lo, s_hi, kb);
-          if (kb == 0 && P.mul_weight && row_ok) rw = P.route_weight[sid];  // sid arrived during the first fold
-          if (threadIdx.x == 128) MOE_TR(3, kb, 4);
         }
         if (!alive) break;
       } else {
@@ -736,7 +749,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
 
-      if (threadIdx.x == 128) MOE_TR(3, 60, 0);
       // ---------------------------------------------------------- tile epilogue
       if constexpr (ROW) {
 #pragma unroll
@@ -863,7 +875,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
-      if (threadIdx.x == 128) MOE_TR(3, 60, 1);
       }  // sub
       ++tile_it;
     }
@@ -883,9 +894,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     else
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
   }
-#ifdef MOE_TC_TRACE
-  if (threadIdx.x == 0 && blockIdx.x == 0 && P.trace) { P.trace[2050] = clock64(); P.trace[2051] = (long long)now_ns(); }
-#endif
 #undef MOE_TILE_COORDS
 }
 
@@ -1006,9 +1014,6 @@ int tc_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
     P.group_m = (int)(gm < 1 ? 1 : (gm > 16 ? 16 : gm));
   }
   P.wide_store = ((uintptr_t)out & 31) == 0;
-#ifdef MOE_TC_TRACE
-  { const char* t = getenv(gemm1 ? "MOE_TRACE1" : "MOE_TRACE2"); P.trace = t ? (long long*)strtoull(t, nullptr, 0) : nullptr; }
-#endif
 
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);

@@ -120,7 +120,7 @@ template <typename AT, bool GEMM1>
 __global__ void __launch_bounds__(THREADS, 1)
 w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Params P) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_1024(smem_raw);
   uint8_t* sA = smem;
   uint8_t* sB = sA + (size_t)SA * A_BYTES;
   uint8_t* sR = sB + (size_t)SB * B_BYTES;

@@ -94,7 +94,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   using C = Cfg<WIDE>;
   constexpr int RSTAGES = C::RSTAGES, TSTAGES = C::TSTAGES;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_1024(smem_raw);
   uint8_t* s_tok = smem + (size_t)RSTAGES * RAW_BYTES;
   uint8_t* s_out = s_tok + (size_t)TSTAGES * C::TOK_BYTES;
   Aux* aux = reinterpret_cast<Aux*>(s_out + (size_t)C::TILE * ((GEMM1 ? 64 : 128) * 2 + 16));

@@ -74,7 +74,7 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   using C = Cfg<GEMM1>;
   constexpr int STAGES = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_1024(smem_raw);
   uint8_t* s_out = smem + (size_t)STAGES * STAGE_BYTES;
   Aux* aux = reinterpret_cast<Aux*>(s_out + C::OUT_BYTES);
 

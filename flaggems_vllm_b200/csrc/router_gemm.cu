@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(RTHREADS, 1) router_tc_kernel(const __grid_con
   using namespace tc;
   using C = RCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_1024(smem_raw);
   RAux* aux = reinterpret_cast<RAux*>(smem + C::RING);
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();

@@ -89,22 +89,67 @@ __device__ __forceinline__ unsigned long long now_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-// Bounded wait: false when the limit ran out (status word is set).
+// Looked at now and then by a wait: true, with the status bit set, when `limit_ns` have passed since the first look (t0 = 0).
+__device__ __forceinline__ bool wait_expired(unsigned long long& t0, int32_t* status, unsigned long long limit_ns) {
+  const unsigned long long now = now_ns();
+  if (t0 == 0) t0 = now;
+  if (now - t0 <= limit_ns) return false;
+  set_status(status, MOE_ST_WAIT_TIMEOUT);
+  return true;
+}
+// Start of the operand rings: the first 1024-byte boundary of the dynamic shared memory.  An offset from the array, not a
+// pointer made from an integer: the compiler keeps knowing that it is shared memory (LDS and constant addresses; with
+// generic pointers the FP8 GEMM1 loop had 16 generic loads and 24 reads of the window base per K block).
+__device__ __forceinline__ uint8_t* align_1024(uint8_t* smem_raw) {
+  return smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+}
+// Bounded wait: false when the limit ran out (status word is set).  The clock is looked at every 1024 probes only, so a
+// wait that ends soon never reads it.
 // CLUSTER: the barrier is also arrived on by the partner CTA (acquire at cluster scope).
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int32_t* status,
                                           unsigned long long limit_ns = WAIT_LIMIT_NS) {
-  auto probe = [&]() { return CLUSTER ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity); };
-  if (probe()) return true;
-  const unsigned long long t0 = now_ns();
-  uint32_t spins = 0;
-  while (!probe()) {
-    if ((++spins & 0x3FF) == 0 && now_ns() - t0 > limit_ns) {
-      set_status(status, MOE_ST_WAIT_TIMEOUT);
-      return false;
-    }
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (uint32_t spins = 1; !(CLUSTER ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity)); ++spins) {
+    if ((spins & 0x3FF) == 0 && wait_expired(t0, status, limit_ns)) return false;
   }
   return true;
+}
+// The barrier operations on shared-memory addresses that a loop carries in registers: with the address taken from a
+// pointer in every K block, address arithmetic made up a good part of a consumer's instructions.
+__device__ __forceinline__ bool mbar_try_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity, int32_t* status, unsigned long long limit_ns) {
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (uint32_t spins = 1; !mbar_try_at(bar, parity); ++spins) {
+    if ((spins & 0x3FF) == 0 && wait_expired(t0, status, limit_ns)) return false;
+  }
+  return true;
+}
+// arrives on the barrier OFFSET bytes behind `bar` where `yes`, without a branch
+template <int OFFSET>
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar, bool yes) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%0 + %2];\n\t}" ::"r"(bar), "r"((uint32_t)yes), "n"(OFFSET)
+      : "memory");
+}
+template <int OFFSET>
+__device__ __forceinline__ float lds_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(addr), "n"(OFFSET) : "memory");
+  return v;
 }
 // The same bounded wait for warps that expect to wait long (an epilogue warp waiting for a
 // whole K loop): they sleep between probes, so their polling does not take issue slots from
@@ -198,6 +243,24 @@ __device__ __forceinline__ void tc_mma_const(uint32_t tmem_d, uint64_t adesc, ui
   else MOE_MMA_ASM("f16", "n", acc);
 }
 #undef MOE_MMA_ASM
+// A K block of e4m3 (four instructions, 32 bytes of K each) into a fresh accumulator, and the commits to the accumulator's
+// barrier and the stage's, by the lane where `yes`, in one statement: nothing is left between the wait and the issue.
+__device__ __forceinline__ void tc_mma_block_f8(bool yes, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                uint32_t acc_bar, uint32_t stage_bar) {
+  asm volatile(
+      "{\n\t.reg .pred l, f, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 l, %0, 0;\n\tsetp.ne.b32 f, 0, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 a1, %2, 2;\n\tadd.s64 a2, %2, 4;\n\tadd.s64 a3, %2, 6;\n\t"
+      "add.s64 b1, %3, 2;\n\tadd.s64 b2, %3, 4;\n\tadd.s64 b3, %3, 6;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%1], %2, %3, %4, f;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%1], a1, b1, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%1], a2, b2, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%1], a3, b3, %4, t;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+      ::"r"((uint32_t)yes), "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc_bar), "r"(stage_bar)
+      : "memory");
+}
 // Packed fp32 pair FMA: d = a * b + d on two lanes of a 64-bit register pair.  Half the issue
 // slots of two scalar FMAs, which matters for warps that share a scheduler with the thread
 // that feeds the tensor core.

@@ -117,6 +117,19 @@ def test_fp8_block_layer_tiles(M, E, k):
     assert torch.equal(fg.fused_experts_impl(x2, w1, w2, tw, ti, inplace=True, **kw), out)
 
 
+@pytest.mark.parametrize("M,E,k,H,I", [(16384, 8, 2, 128, 128), (2600, 4, 2, 384, 1664), (900, 32, 4, 640, 1152)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_fp8_block_layer_odd_k_blocks_and_several_tiles_per_cta(M, E, k, H, I, dtype):
+    """One K block or an odd number of them in a tile: the two accumulators, the stages and the scale slots do not start
+    the next tile of the CTA where they started this one."""
+    x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
+    w1, s1 = T.make_fp8_block_weights(E, 2 * I, H, DEV, seed=1)
+    w2, s2 = T.make_fp8_block_weights(E, H, I, DEV, seed=2)
+    tw, ti = _route(M, E, k)
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti, use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
+    _parity(out, O.fused_moe_fp8_block_oracle(x, w1, w2, s1, s2, tw, ti), (M, H, I))
+
+
 @pytest.mark.parametrize("M,E,k,H,I", [
     (1, 1, 1, 128, 64), (1, 8, 8, 256, 192), (8, 2, 1, 2176, 128), (4, 8, 2, 1024, 2048),
     (3, 4, 3, 128, 64)])  # nine routes: the tile kernels
