@@ -16,17 +16,23 @@
 // Warp roles (640 threads):
 //   warp 0       TMA: raw weights
 //   warp 1       MMA issuer
-//   warp 2       TMEM allocation: two accumulators of 160 columns, three A buffers of 64 columns
+//   warp 2       TMEM allocation: two accumulators of 160 (64) columns, three (six) A buffers of 64 columns
 //   warp 3       TMA: token rows
 //   warps 4-7    epilogue (drain_tile)
-//   warps 8-19   converters: three groups of four warps; group g owns A buffer g and every third K block, warp quarter
+//   warps 8-19   converters: three groups of four warps; group g owns every third A buffer and K block, warp quarter
 //                q the 32 weight rows = TMEM lanes 32 q...  A thread widens one row of 128 bytes; the 128-byte
 //                swizzle of the raw tile makes its 16-byte loads conflict-free.
 // TMEM columns hold two elements of K each, so an MMA (16 elements) takes 8 columns of A.
 //
-// Bound at prefill (Qwen3 shape, 4096 tokens): GEMM1 335 thousand cycles and GEMM2 220, whatever the clock, of which 294 and
-// 167 are left without widening and epilogue: the load streams through their rings (57 B per clock and SM in GEMM1).  At
-// decode HBM, less the last partial wave.  Against gemm_w8.cu: 33 tokens 191 -> 146 us per layer, 4096 tokens 591 -> 465.
+// Bound.  Decode: HBM, less the last partial wave; before, the MMA warp's chain of a K block, two waits, eight
+// instructions and two commits.  Now a K block is one wait, one statement of eight instructions and ONE commit (token rows and
+// widened weights of a K block share a stage index), the loops carry their addresses, and an epilogue warp stages 16 tokens
+// of its own rows instead of a tile of everybody's (no barriers, and room for twice the raw stages).  GEMM1 / GEMM2 back to
+// back, Qwen3 shape, us: 33 tokens 64.7 / 37.7 -> 59.7 / 31.9, 500 tokens 89 / 50 -> 78 / 42, 4096 tokens 228 / 128 -> 218 /
+// 122.  A second commit and wait per K block (token stages of half a K block, four blocks of them) measured 78.6 / 45.0 at 33
+// tokens and 247 / 136 at 4096.  Prefill: no single part.  Without the token loads 162 of 208 us of GEMM1 are left, with one
+// of the eight MMAs 171, without raw loads 179, without widening 186, without epilogue 195.
+// Against gemm_w8.cu: 33 tokens 191 -> 121 us per layer, 4096 tokens 591 -> 460.
 #include "wt_common.cuh"
 
 namespace moe {
@@ -35,8 +41,6 @@ using namespace wt;
 
 constexpr int THREADS = 640, EPI_THREADS = 128, GROUPS = 3;
 constexpr int RAW_BYTES = 128 * 128;
-constexpr int ACC_COLS = 160, A_COLS = 64, A_BASE = 2 * ACC_COLS;
-static_assert(A_BASE + GROUPS * A_COLS <= 512, "TMEM columns");
 constexpr int LAUNCH_REGS = 96, PRODUCER_REGS = 40, EPI_REGS = 144;  // converters keep what they were launched with
 static_assert(128 * PRODUCER_REGS + 128 * EPI_REGS + 384 * LAUNCH_REGS <= THREADS * LAUNCH_REGS, "register redistribution");
 
@@ -44,26 +48,30 @@ template <bool WIDE> struct Cfg {
   static constexpr int TILE = WIDE ? 160 : 64;     // most tokens of a tile
   static constexpr int SUB_BYTES = TILE * 128;     // 64 elements of K of the token rows
   static constexpr int TOK_BYTES = 2 * SUB_BYTES;
-  static constexpr int RSTAGES = WIDE ? 3 : 6, TSTAGES = WIDE ? 3 : 4;
-  // Every raw stage belongs to ONE converter group (as every A buffer does), which has seen the use before the one it waits
-  // for.  With five stages a group could wait two uses ahead of a late load: the parity wait lets it pass, it hands the
-  // stage back too early, and the launch fails, about once in a thousand layers.
-  static_assert(RSTAGES % GROUPS == 0, "raw stages per converter group");
+  // stages: a K block's token rows in shared memory and its widened weights in tensor memory; raw stages
+  static constexpr int STAGES = WIDE ? 3 : 6, RSTAGES = 6;
+  static constexpr int A_COLS = 64, A_BASE = 2 * TILE;  // TMEM: two accumulators, then the widened weights
+  static_assert(A_BASE + STAGES * A_COLS <= 512, "TMEM columns");
+  // Every stage belongs to ONE converter group, which has seen the use before the one it waits for.  With five raw
+  // stages a group could wait two uses ahead of a late load: the parity wait lets it pass, it hands the stage back too
+  // early, and the launch fails, about once in a thousand layers.
+  static_assert(RSTAGES % GROUPS == 0 && STAGES % GROUPS == 0, "stages per converter group");
 };
+// What one K block costs the MMA warp is what bounds this kernel, so a K block has one barrier to wait for and one to
+// commit to: ready[s] counts the token rows (bytes) and the four converter warps, done[s] frees both.
 struct Aux {
   uint64_t r_full[6], r_empty[6];
-  uint64_t t_full[4], t_empty[4];
-  uint64_t a_full[GROUPS], a_empty[GROUPS];
+  uint64_t ready[6], done[6];
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   uint32_t pad;
 };
-template <bool WIDE, bool GEMM1> constexpr size_t smem_bytes() {
+constexpr int OUT_TOKENS = 16, OUT_BYTES = OUT_TOKENS * (32 * 2 + 16);  // staging buffer of an epilogue warp (drain_tile)
+template <bool WIDE> constexpr size_t smem_bytes() {
   using C = Cfg<WIDE>;
-  return (size_t)C::RSTAGES * RAW_BYTES + (size_t)C::TSTAGES * C::TOK_BYTES + (size_t)C::TILE * ((GEMM1 ? 64 : 128) * 2 + 16) +
-         sizeof(Aux) + 1024;
+  return (size_t)C::RSTAGES * RAW_BYTES + (size_t)C::STAGES * C::TOK_BYTES + EPI_THREADS / 32 * OUT_BYTES + sizeof(Aux) + 1024;
 }
-static_assert(smem_bytes<true, false>() <= 232448 && smem_bytes<false, false>() <= 232448, "shared memory of one SM");
+static_assert(smem_bytes<true>() <= 232448 && smem_bytes<false>() <= 232448, "shared memory of one SM");
 
 __device__ __forceinline__ void tma_load_5d(const CUtensorMap* map, uint64_t* bar, void* dst, int c0, int c1, int c2, int c3, int c4) {
   asm volatile(
@@ -71,10 +79,28 @@ __device__ __forceinline__ void tma_load_5d(const CUtensorMap* map, uint64_t* ba
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
 }
-// A from tensor memory
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-               ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
+// A K block (128 elements, eight instructions) with A from tensor memory, and the commit to the stage's barrier, by the lane
+// where `yes`, in one statement
+template <int SUB_BYTES>
+__device__ __forceinline__ void mma_ts_block(bool yes, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc, uint32_t done) {
+  asm volatile(
+      "{\n\t.reg .pred l, p, t;\n\t.reg .b64 b1, b2, b3, b4, b5, b6, b7;\n\t.reg .b32 a1, a2, a3, a4, a5, a6, a7;\n\t"
+      "setp.ne.b32 l, %0, 0;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+      "add.s64 b1, %3, 2;\n\tadd.s64 b2, %3, 4;\n\tadd.s64 b3, %3, 6;\n\tadd.s64 b4, %3, %7;\n\t"
+      "add.s64 b5, b4, 2;\n\tadd.s64 b6, b4, 4;\n\tadd.s64 b7, b4, 6;\n\t"
+      "add.u32 a1, %2, 8;\n\tadd.u32 a2, %2, 16;\n\tadd.u32 a3, %2, 24;\n\tadd.u32 a4, %2, 32;\n\t"
+      "add.u32 a5, %2, 40;\n\tadd.u32 a6, %2, 48;\n\tadd.u32 a7, %2, 56;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, p;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], b1, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], b2, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], b3, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a4], b4, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a5], b5, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a6], b6, %4, t;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%1], [a7], b7, %4, t;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+      ::"r"((uint32_t)yes), "r"(d), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc), "r"(done), "n"(SUB_BYTES >> 4)
+      : "memory");
 }
 #define MOE_S8(a, o) "r"(a[o]), "r"(a[o + 1]), "r"(a[o + 2]), "r"(a[o + 3]), "r"(a[o + 4]), "r"(a[o + 5]), "r"(a[o + 6]), "r"(a[o + 7])
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&a)[32]) {
@@ -92,14 +118,14 @@ __global__ void __launch_bounds__(THREADS, 1)
 w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_b64,
                 const __grid_constant__ CUtensorMap map_b16, const __grid_constant__ CUtensorMap map_b8, const Params P) {
   using C = Cfg<WIDE>;
-  constexpr int RSTAGES = C::RSTAGES, TSTAGES = C::TSTAGES;
+  constexpr int RSTAGES = C::RSTAGES, STAGES = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_1024(smem_raw);
   uint8_t* s_tok = smem + (size_t)RSTAGES * RAW_BYTES;
-  uint8_t* s_out = s_tok + (size_t)TSTAGES * C::TOK_BYTES;
-  Aux* aux = reinterpret_cast<Aux*>(s_out + (size_t)C::TILE * ((GEMM1 ? 64 : 128) * 2 + 16));
+  uint8_t* s_out = s_tok + (size_t)STAGES * C::TOK_BYTES;
+  Aux* aux = reinterpret_cast<Aux*>(s_out + EPI_THREADS / 32 * OUT_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // the compiler sees that `warp` is uniform
   const int KB = (P.K + 127) / 128;
   const int item0 = blockIdx.x, step = gridDim.x;
   const int total = __ldcg(P.counts) * P.R;  // the route plan is older than the predecessor
@@ -107,8 +133,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < RSTAGES; ++s) { mbar_init(&aux->r_full[s], 1); mbar_init(&aux->r_empty[s], 4); }
-    for (int s = 0; s < TSTAGES; ++s) { mbar_init(&aux->t_full[s], 1); mbar_init(&aux->t_empty[s], 1); }
-    for (int g = 0; g < GROUPS; ++g) { mbar_init(&aux->a_full[g], 4); mbar_init(&aux->a_empty[g], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&aux->ready[s], 1 + 4); mbar_init(&aux->done[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&aux->tmem_full[a], 1); mbar_init(&aux->tmem_empty[a], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -142,7 +167,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (item + step < total) nx = fetch(item + step);
         const int wrow = GEMM1 ? it.rt * 8 : it.e * P.Nout + it.rt * 128;
         for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait(&aux->r_empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+          if (!mbar_wait_at(smem_u32(&aux->r_empty[s]), ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           if (leader) {
             mbar_expect_tx(&aux->r_full[s], RAW_BYTES);
             if constexpr (GEMM1) tma_load_5d(&map_w, &aux->r_full[s], smem + (size_t)s * RAW_BYTES, kb * 128, 0, 0, wrow, it.e);
@@ -160,20 +185,20 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const Item it = nx;
         if (item + step < total) nx = fetch(item + step);
         for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait(&aux->t_empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+          if (!mbar_wait_at(smem_u32(&aux->done[s]), ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           if (leader) {
-            mbar_expect_tx(&aux->t_full[s], (uint32_t)it.n * 256);  // both sub-tiles
+            mbar_expect_tx(&aux->ready[s], (uint32_t)it.n * 256);  // both sub-tiles
 #pragma unroll
             for (int sub = 0; sub < 2; ++sub) {
               uint8_t* dst = s_tok + (size_t)s * C::TOK_BYTES + sub * C::SUB_BYTES;
               const int k0 = kb * 128 + sub * 64;
               int r = 0;
-              for (; it.n - r >= 64; r += 64) tma_load_2d(&map_b64, &aux->t_full[s], dst + r * 128, k0, it.row0 + r);
-              for (; it.n - r >= 16; r += 16) tma_load_2d(&map_b16, &aux->t_full[s], dst + r * 128, k0, it.row0 + r);
-              if (r < it.n) tma_load_2d(&map_b8, &aux->t_full[s], dst + r * 128, k0, it.row0 + r);
+              for (; it.n - r >= 64; r += 64) tma_load_2d(&map_b64, &aux->ready[s], dst + r * 128, k0, it.row0 + r);
+              for (; it.n - r >= 16; r += 16) tma_load_2d(&map_b16, &aux->ready[s], dst + r * 128, k0, it.row0 + r);
+              if (r < it.n) tma_load_2d(&map_b8, &aux->ready[s], dst + r * 128, k0, it.row0 + r);
             }
           }
-          if (++s == TSTAGES) { s = 0; ph ^= 1; }
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
     } else if (warp == 1) {
@@ -182,74 +207,66 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       constexpr uint32_t fmt = std::is_same<AT, __nv_bfloat16>::value ? 1u : 0u;
       constexpr uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 4) << 24);
       const uint64_t b0 = make_smem_desc(smem_u32(s_tok));
-      uint32_t s = 0, ph = 0, g = 0, gph = 0, acc_it = 0;
+      const uint32_t ready0 = smem_u32(&aux->ready[0]), a0 = tmem_base + C::A_BASE;
+      constexpr uint32_t TO_DONE = (uint32_t)(offsetof(Aux, done) - offsetof(Aux, ready));
+      uint32_t ready = ready0, ph = 0, ta = a0, acc_it = 0;
+      uint64_t bd = b0;
       for (int item = item0; item < total && alive; item += step) {
         const Item it = nx;
         if (item + step < total) nx = fetch(item + step);
         const uint32_t idesc = idesc0 | ((uint32_t)(it.n >> 3) << 17);
-        const uint32_t a = acc_it & 1, d = tmem_base + a * ACC_COLS;
+        const uint32_t a = acc_it & 1, d = tmem_base + a * C::TILE;
         if (!mbar_wait(&aux->tmem_empty[a], ((acc_it >> 1) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+#pragma unroll 1
         for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait(&aux->t_full[s], ph, P.status, P.wait_ns) ||
-              !mbar_wait(&aux->a_full[g], gph, P.status, P.wait_ns)) { alive = false; break; }
+          if (!mbar_wait_at(ready, ph, P.status, P.wait_ns)) { alive = false; break; }
           tc_fence_after();
-          if (leader) {
-            const uint64_t bd = b0 + (uint64_t)(s * (C::TOK_BYTES >> 4));
-            const uint32_t ta = tmem_base + A_BASE + g * A_COLS;
-#pragma unroll
-            for (int k = 0; k < 8; ++k)  // 16 elements of K: 8 columns of A, 32 bytes of a token row
-              mma_ts(d, ta + k * 8, bd + (uint64_t)((k >> 2) * (C::SUB_BYTES >> 4) + (k & 3) * 2), idesc, (k > 0 || kb > 0) ? 1u : 0u);
-            tc_commit(&aux->a_empty[g]);
-            tc_commit(&aux->t_empty[s]);
-            if (kb == KB - 1) tc_commit(&aux->tmem_full[a]);
-          }
-          if (++s == TSTAGES) { s = 0; ph ^= 1; }
-          if (++g == GROUPS) { g = 0; gph ^= 1; }
+          mma_ts_block<C::SUB_BYTES>(leader, d, ta, bd, idesc, kb > 0, ready + TO_DONE);
+          ready += 8;
+          ta += C::A_COLS;
+          bd += (uint64_t)(C::TOK_BYTES >> 4);
+          if (ready == ready0 + 8 * STAGES) { ready = ready0; ta = a0; bd = b0; ph ^= 1; }
         }
+        if (leader && alive) tc_commit(&aux->tmem_full[a]);
         ++acc_it;
       }
     }
   } else if (warp < 8) {
     // -------------------------------------------------------------- epilogue
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPI_REGS));
-    const int wq = warp & 3, et = threadIdx.x - 128;
+    const int wq = warp & 3;
     const uint32_t t_lane = tmem_base + ((uint32_t)(wq << 5) << 16);
-    const uint32_t out_base = smem_u32(s_out);
+    const uint32_t out_base = smem_u32(s_out) + wq * OUT_BYTES;
     uint32_t acc_it = 0;
-    bool alive = true;
     Item nx = {};
     if (item0 < total) nx = fetch(item0);
-    // the tile loop runs to its end even after a wait has timed out: every epilogue thread reaches the barriers
     for (int item = item0; item < total; item += step) {
       const Item it = nx;
       if (item + step < total) nx = fetch(item + step);
       const uint32_t a = acc_it & 1;
-      asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory");  // the staging tile has been read
-      if (alive && !mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) alive = false;
-      if (alive) {
-        tc_fence_after();
-        drain_tile<FMT_W8, AT, GEMM1, true, 1, 1>(P, it, 0, t_lane + a * ACC_COLS, 0, wq, lane, out_base, [&] {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&aux->tmem_empty[a]);
-        });
-        ++acc_it;
-      }
-      asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory");  // the tile is staged
-      if (alive) store_rows<AT, GEMM1, 1, EPI_THREADS>(P, it, 0, s_out, et);
+      if (!mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) break;
+      tc_fence_after();
+      drain_tile<FMT_W8, AT, GEMM1, true, 1, 1, OUT_TOKENS>(P, it, 0, t_lane + a * C::TILE, 0, wq, lane, out_base, [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&aux->tmem_empty[a]);
+      });
+      ++acc_it;
     }
   } else {
     // -------------------------------------------------------------- converters
     const int grp = (warp - 8) >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
-    const uint32_t ta = tmem_base + ((uint32_t)(wq << 5) << 16) + A_BASE + grp * A_COLS;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(wq << 5) << 16) + C::A_BASE;
     // K blocks of all tiles in one sequence; this group takes every third of them
     const int tiles = item0 < total ? (total - item0 + step - 1) / step : 0;
     const int64_t blocks = (int64_t)tiles * KB;
-    uint32_t s = grp % RSTAGES, rph = 0, aph = 1;
+    uint32_t rs = grp, rph = 0, s = grp, ph = 1;
     for (int64_t j = grp; j < blocks; j += GROUPS) {
-      if (!mbar_wait(&aux->r_full[s], rph, P.status, P.wait_ns)) break;
-      const uint8_t* src = smem + (size_t)s * RAW_BYTES + row * 128;
+      if (!mbar_wait_at(smem_u32(&aux->r_full[rs]), rph, P.status, P.wait_ns)) break;
+      const uint8_t* src = smem + (size_t)rs * RAW_BYTES + row * 128;
+      const uint32_t ta = t_lane + s * C::A_COLS;
+      bool ok = true;
       uint4 raw[4];
       uint32_t w[32];
 #pragma unroll
@@ -266,22 +283,22 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         if (half == 0) {
           // the buffer's last MMA is over (the wait comes after the first half is widened)
-          if (!mbar_wait(&aux->a_empty[grp], aph, P.status, P.wait_ns)) { s = ~0u; break; }
+          ok = mbar_wait_at(smem_u32(&aux->done[s]), ph, P.status, P.wait_ns);
+          if (!ok) break;
           tc_fence_after();
         }
         tmem_st32(ta + half * 32, w);
       }
-      if (s == ~0u) break;
+      if (!ok) break;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&aux->r_empty[s]);
-        mbar_arrive(&aux->a_full[grp]);
-      }
-      aph ^= 1;
+      mbar_arrive_at<0>(smem_u32(&aux->r_empty[rs]), lane == 0);
+      mbar_arrive_at<0>(smem_u32(&aux->ready[s]), lane == 0);
+      rs += GROUPS;
+      if (rs >= RSTAGES) { rs -= RSTAGES; rph ^= 1; }
       s += GROUPS;
-      if (s >= RSTAGES) { s -= RSTAGES; rph ^= 1; }
+      if (s >= STAGES) { s -= STAGES; ph ^= 1; }
     }
   }
 
@@ -298,7 +315,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 template <typename AT, bool GEMM1, bool WIDE>
 static int launch(const CUtensorMap& mw, const CUtensorMap (&mb)[3], const Params& P, int64_t items, cudaStream_t st) {
   auto kern = w8t_gemm_kernel<AT, GEMM1, WIDE>;
-  constexpr size_t smem = smem_bytes<WIDE, GEMM1>();
+  constexpr size_t smem = smem_bytes<WIDE>();
   static const int regs = [&] {
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : 0;

@@ -82,8 +82,9 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
   const int64_t per_expert = numel / (E > 0 ? E : 1);
   Choice c = {};
   if (mode == MOE_MODE_W8A16) {
-    // Qwen3 shape: at 32 rows per expert the narrow tile is 3 % ahead, at 64 the wide one 15 %
-    c.wide = per_expert > 40;
+    // Qwen3 shape, GEMM1 + GEMM2 in us, narrow (more stages) against wide: 40 rows per expert 128 : 139, 50 rows 133 : 140,
+    // 62 rows 170 : 153 (every second expert has more than 64 rows: two tiles)
+    c.wide = per_expert > 52;
     c.gran = 16;
     c.tile = w8t_tile(c.wide);
     return c;

@@ -59,18 +59,25 @@ __device__ __forceinline__ Item fetch_item(const Params& P, int item) {
   return it;
 }
 
+// output columns of a warp's 32 weight rows
+template <bool GEMM1> __host__ __device__ constexpr int warp_cols() { return GEMM1 ? 16 : 32; }
+
 // Accumulator tile -> staged 16-bit rows [token][64 or 128 columns].  Warp quarter wq owns lanes 32 wq.., group h of
 // GROUPS the h-th part of the tile's tokens; CTAS CTAs hold 128 weight rows each.  t_acc: TMEM address of the tile in
 // the warp's lanes.  `release` runs when the whole accumulator is in registers or staged.  Rows are padded by
 // 16 bytes, which spreads the rows of a stmatrix over the banks.
+// WARP_TOKENS > 0 (one CTA, one group): the staging buffer at out_base is the warp's own and holds that many tokens of its 16
+// (GEMM1) or 32 columns; it goes to HBM whenever it is full, in whole sectors, without a barrier between the warps.
 // Rows of a thread: in 16-lane block rh (0, 1) of the warp's 32 lanes, lanes tr and tr + 8:
 //   GEMM1: output 64 cr + 8 (2 wq + rh) + tr of the row tile (gate in lane tr, up in lane tr + 8)
 //   GEMM2: output columns 128 cr + 32 wq + 16 rh + tr and + 8
-template <int FMT, typename AT, bool GEMM1, bool SILU, int CTAS, int GROUPS, typename Release>
+template <int FMT, typename AT, bool GEMM1, bool SILU, int CTAS, int GROUPS, int WARP_TOKENS, typename Release>
 __device__ __forceinline__ void drain_tile(const Params& P, const Item& it, int cr, uint32_t t_acc, int h, int wq, int lane,
                                            uint32_t out_base, Release release) {
   constexpr bool ROW = FMT == FMT_FP8ROW || FMT == FMT_I8ROW, CHANNEL = ROW || FMT == FMT_W8;
-  constexpr int PITCH = (GEMM1 ? 64 : 128) * 2 + 16;
+  constexpr bool WARP_STORE = WARP_TOKENS > 0;
+  static_assert(!WARP_STORE || (CTAS == 1 && GROUPS == 1 && (WARP_TOKENS == 16 || WARP_TOKENS == 32)), "a warp's own staging buffer");
+  constexpr int PITCH = (WARP_STORE ? warp_cols<GEMM1>() : (GEMM1 ? 64 : 128)) * 2 + 16;
   const int tr = lane >> 2, tq = lane & 3;
   const int nh = it.n / GROUPS, tok0 = h * nh;  // this group's tokens [tok0, tok0 + nh) of the tile
   const int nst = (nh + 31) >> 5;               // steps of 32 tokens
@@ -136,12 +143,35 @@ __device__ __forceinline__ void drain_tile(const Params& P, const Item& it, int 
             hi[rh][0] = v[1][0]; hi[rh][1] = v[1][1];
           }
         }
-        const uint32_t row = out_base + (uint32_t)(tok0 + st * 32 + c * 8 + (lane & 7)) * PITCH;
+        const uint32_t row = out_base + (uint32_t)((WARP_STORE ? c * 8 % (WARP_STORE ? WARP_TOKENS : 1) : tok0 + st * 32 + c * 8) + (lane & 7)) * PITCH;
+        const int wqs = WARP_STORE ? 0 : wq;
         if constexpr (GEMM1)
-          stmatrix_x2_trans(row + (uint32_t)((2 * wq + ((lane >> 3) & 1)) * 16), pack2<AT>(lo[0][0], lo[0][1]), pack2<AT>(lo[1][0], lo[1][1]));
+          stmatrix_x2_trans(row + (uint32_t)((2 * wqs + ((lane >> 3) & 1)) * 16), pack2<AT>(lo[0][0], lo[0][1]), pack2<AT>(lo[1][0], lo[1][1]));
         else
-          stmatrix_x4_trans(row + (uint32_t)(wq * 64 + (lane >> 3) * 16), pack2<AT>(lo[0][0], lo[0][1]), pack2<AT>(hi[0][0], hi[0][1]),
+          stmatrix_x4_trans(row + (uint32_t)(wqs * 64 + (lane >> 3) * 16), pack2<AT>(lo[0][0], lo[0][1]), pack2<AT>(hi[0][0], hi[0][1]),
                             pack2<AT>(lo[1][0], lo[1][1]), pack2<AT>(hi[1][0], hi[1][1]));
+      }
+      if constexpr (WARP_STORE) {
+        if ((c + 1) * 8 % WARP_TOKENS == 0) {
+          constexpr int LANES = warp_cols<GEMM1>() / 8;  // lanes of a row, 16 bytes each
+          const int col = it.rt * (GEMM1 ? 64 : 128) + wq * warp_cols<GEMM1>() + (lane % LANES) * 8;
+          const int first = st * 32 + (c + 1) * 8 - WARP_TOKENS, left = nh - first;
+          __syncwarp();
+          if (col < P.Nout) {
+#pragma unroll
+            for (int t0 = 0; t0 < WARP_TOKENS; t0 += 32 / LANES) {
+              const int tok = t0 + lane / LANES;
+              if (tok < left) {
+                uint4 v;
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                             : "r"(out_base + (uint32_t)(tok * PITCH + (lane % LANES) * 16)) : "memory");
+                *reinterpret_cast<uint4*>(reinterpret_cast<AT*>(P.out) + ((int64_t)it.row0 + first + tok) * P.Nout + col) = v;
+              }
+            }
+          }
+          __syncwarp();
+        }
       }
     }
   }

@@ -193,7 +193,8 @@ def test_layer_with_local_experts_and_weights_on_the_input(M):
 
 @pytest.mark.parametrize("M,E,k,H,I", [
     (20, 4, 2, 192, 128), (90, 3, 1, 256, 384),      # 64-token tiles: a last K block of 64, several tiles of one expert
-    (200, 2, 1, 320, 256), (1300, 4, 2, 128, 128)])  # 160-token tiles: even splits with remainders
+    (200, 2, 1, 320, 256), (1300, 4, 2, 128, 128),   # 160-token tiles: even splits with remainders
+    (208, 16, 4, 448, 1920), (212, 16, 4, 448, 1920), (1500, 16, 4, 448, 1920)])  # either tile's last and first; many tiles per CTA
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_int8_weight_layer_tiles(M, E, k, H, I, dtype):
     x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
