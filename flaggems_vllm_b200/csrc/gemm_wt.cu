@@ -39,46 +39,50 @@ namespace wt {
 using namespace tc;
 
 constexpr int WROWS = 128;   // weight rows per CTA
-constexpr int NTOK = 256;    // most tokens of a tile
 constexpr int A_BYTES = WROWS * 128;
-constexpr int B_BYTES = NTOK / 2 * 128;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 384;
 constexpr int CONS_THREADS = 256;
 // setmaxnreg moves registers inside the CTA's allocation: 128 x 56 + 256 x 224 = 384 x 168
 constexpr int LAUNCH_REGS = 168, PRODUCER_REGS = 56, CONSUMER_REGS = 224;
 static_assert(128 * PRODUCER_REGS + CONS_THREADS * CONSUMER_REGS <= THREADS * LAUNCH_REGS, "register redistribution");
 
-template <bool GEMM1> struct Cfg {
-  static constexpr int STAGES = GEMM1 ? 5 : 4;
+// NTOK: most tokens of a tile.  64: the ring is left to the weights, ten stages of 16 KB of them in flight instead of five while
+// they stream.  Qwen3 shape, e4m3, GEMM1 back to back in us, 256 against 64: 33 tokens 58.3 : 55.1, 500 tokens 69.4 : 65.2.  GEMM2
+// (six K blocks per tile) is 2 % slower with it (39.5 : 40.5) and has one kernel.
+template <bool GEMM1, int NTOK> struct Cfg {
+  static constexpr int STAGE_BYTES = A_BYTES + NTOK / 2 * 128;
+  static_assert(NTOK == 256 || (GEMM1 && NTOK == 64), "tile");
+  static constexpr int STAGES = NTOK <= 64 ? 10 : (GEMM1 ? 5 : 4);
   static constexpr int OUT_BYTES = NTOK * ((GEMM1 ? 64 : 128) * 2 + 16);  // staged rows, see drain_tile
 };
 struct Aux {
-  uint64_t full[6], empty[6];
+  uint64_t full[10], empty[10];
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   uint32_t pad;
 };
-template <bool GEMM1> constexpr size_t smem_bytes() {
-  return (size_t)Cfg<GEMM1>::STAGES * STAGE_BYTES + Cfg<GEMM1>::OUT_BYTES + sizeof(Aux) + 1024;
+template <bool GEMM1, int NTOK> constexpr size_t smem_bytes() {
+  using C = Cfg<GEMM1, NTOK>;
+  return (size_t)C::STAGES * C::STAGE_BYTES + C::OUT_BYTES + sizeof(Aux) + 1024;
 }
-static_assert(smem_bytes<true>() <= 232448 && smem_bytes<false>() <= 232448, "shared memory of one SM");
+static_assert(smem_bytes<true, 256>() <= 232448 && smem_bytes<false, 256>() <= 232448, "shared memory of one SM");
+static_assert(smem_bytes<true, 64>() <= 232448, "shared memory of one SM");
 
 // SILU: the activation of GEMM1 (false: swigluoai, which reads GEMM1's result rounded to the activation type)
-template <int FMT, typename AT, bool GEMM1, bool SILU>
+template <int FMT, typename AT, bool GEMM1, bool SILU, int NTOK>
 __global__ void __launch_bounds__(THREADS, 1)
 wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_b64,
                const __grid_constant__ CUtensorMap map_b16, const __grid_constant__ CUtensorMap map_b8, const Params P) {
   constexpr int KIND = FMT == FMT_HALF ? MMA_F16 : (FMT == FMT_I8ROW ? MMA_I8 : MMA_F8);
   constexpr int KBE = FMT == FMT_HALF ? 64 : 128;  // elements of K per stage
-  using C = Cfg<GEMM1>;
-  constexpr int STAGES = C::STAGES;
+  using C = Cfg<GEMM1, NTOK>;
+  constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_1024(smem_raw);
   uint8_t* s_out = smem + (size_t)STAGES * STAGE_BYTES;
   Aux* aux = reinterpret_cast<Aux*>(s_out + C::OUT_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // the compiler sees that `warp` is uniform
   const int KB = (P.K + KBE - 1) / KBE;
   const int cr = (int)cluster_ctarank();  // 0 leads
   const int item0 = blockIdx.x / 2, step = gridDim.x / 2;
@@ -139,7 +143,7 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const int nh = it.n >> 1;                 // this CTA's share of the token rows
         const int brow = it.row0 + cr * nh;
         for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait(&aux->empty[s], ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+          if (!mbar_wait_at(smem_u32(&aux->empty[s]), ph ^ 1, P.status, P.wait_ns)) { alive = false; break; }
           if (leader) {
             if (early > 0) --early;
             else load_weights(it, kb, s);
@@ -159,7 +163,10 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       constexpr uint32_t idesc0 =
           ((FMT == FMT_I8ROW ? 2u : 1u) << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(2 * WROWS >> 4) << 24);
       const uint64_t a0 = make_smem_desc(smem_u32(smem)), b0 = make_smem_desc(smem_u32(smem + A_BYTES));
-      uint32_t s = 0, ph = 0, acc_it = 0;
+      const uint32_t full0 = smem_u32(&aux->full[0]);
+      constexpr uint32_t TO_EMPTY = (uint32_t)(offsetof(Aux, empty) - offsetof(Aux, full));
+      uint32_t full = full0, ph = 0, acc_it = 0;
+      uint64_t ad = a0, bd = b0;
       bool alive = true;
       Item nx = {};
       if (item0 < total) nx = fetch(item0);
@@ -167,26 +174,20 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const Item it = nx;
         if (item + step < total) nx = fetch(item + step);
         const uint32_t idesc = idesc0 | ((uint32_t)(it.n >> 3) << 17);
+        const uint32_t a = acc_it & 1, d = tmem_base + a * NTOK;
+        if (!mbar_wait(&aux->tmem_empty[a], ((acc_it >> 1) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+#pragma unroll 1
         for (int kb = 0; kb < KB; ++kb) {
-          const uint32_t a = acc_it & 1;
-          if (!mbar_wait(&aux->full[s], ph, P.status, P.wait_ns)) { alive = false; break; }
-          if (kb == 0) {
-            if (!mbar_wait(&aux->tmem_empty[a], ((acc_it >> 1) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
-          }
+          if (!mbar_wait_at(full, ph, P.status, P.wait_ns)) { alive = false; break; }
           tc_fence_after();
-          if (leader) {
-            const uint64_t ad = a0 + (uint64_t)(s * (STAGE_BYTES >> 4)), bd = b0 + (uint64_t)(s * (STAGE_BYTES >> 4));
-            const uint32_t d = tmem_base + a * NTOK;
-#pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4)  // 32 bytes of K per instruction
-              tc_mma_pair<KIND>(d, ad + (uint64_t)(k4 * 2), bd + (uint64_t)(k4 * 2), idesc,
-                                (k4 > 0 || kb > 0) ? 1u : 0u);
-            if (kb == KB - 1) tc_commit_pair(&aux->tmem_full[a]);
-            tc_commit_pair(&aux->empty[s]);
-          }
-          if (kb == KB - 1) ++acc_it;
-          if (++s == STAGES) { s = 0; ph ^= 1; }
+          tc_mma_block_pair<KIND>(leader, d, ad, bd, idesc, kb > 0, full + TO_EMPTY);
+          full += 8;
+          ad += (uint64_t)(STAGE_BYTES >> 4);
+          bd += (uint64_t)(STAGE_BYTES >> 4);
+          if (full == full0 + 8 * STAGES) { full = full0; ad = a0; bd = b0; ph ^= 1; }
         }
+        if (leader && alive) tc_commit_pair(&aux->tmem_full[a]);
+        ++acc_it;
       }
     }
   } else {
@@ -237,10 +238,10 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 }
 
 // ------------------------------------------------------------------ host side
-template <int FMT, typename AT, bool GEMM1, bool SILU = true>
+template <int FMT, typename AT, bool GEMM1, bool SILU, int NTOK>
 static int launch(const CUtensorMap& mw, const CUtensorMap (&mb)[3], const Params& P, int grid, cudaStream_t st) {
-  auto kern = wt_gemm_kernel<FMT, AT, GEMM1, SILU>;
-  constexpr size_t smem = smem_bytes<GEMM1>();
+  auto kern = wt_gemm_kernel<FMT, AT, GEMM1, SILU, NTOK>;
+  constexpr size_t smem = smem_bytes<GEMM1, NTOK>();
   static const int regs = [&] {
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : 0;
@@ -262,8 +263,8 @@ bool wt_serves(int mode, int act_dtype, int H, int I) {
   return (mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW) && H % 128 == 0 && I % 128 == 0;
 }
 
-// a: [rows_cap, K] operand rows in the order of the route plan
-int wt_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
+// a: [rows_cap, K] operand rows in the order of the route plan, whose tiles have at most `tile_rows` rows
+int wt_gemm(bool gemm1, int mode, int tile_rows, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
             const void* tiles, int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K,
             int Nout, void* out, int act_kind, float alpha, float beta, float limit, int32_t* status,
             cudaStream_t st) {
@@ -288,28 +289,27 @@ int wt_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
   const int64_t items = tiles_cap * P.R;
   const int pairs = sm_count() / 2;
   const int grid = 2 * (int)(items < pairs ? items : pairs);
-  if (gemm1 && act_kind != MOE_ACT_SILU) {
-#define MOE_WT(F) \
-  (act_dtype == MOE_BF16 ? launch<F, __nv_bfloat16, true, false>(mw, mb, P, grid, st) : launch<F, __half, true, false>(mw, mb, P, grid, st))
-    switch (mode) {
-      case MOE_MODE_HALF: return MOE_WT(FMT_HALF);
-      case MOE_MODE_FP8_ROW: return MOE_WT(FMT_FP8ROW);
-      case MOE_MODE_INT8_ROW: return MOE_WT(FMT_I8ROW);
-      default: return fail(MOE_E_BADARG, "grouped GEMM: mode %d", mode);
+  // half precision comes with 96 rows per expert and more (layer.cu), never with 64-token tiles
+  auto go = [&](auto F, auto T) {
+    constexpr int FMT = decltype(F)::value;
+    using AT = decltype(T);
+    if (!gemm1) return launch<FMT, AT, false, true, 256>(mw, mb, P, grid, st);
+    auto sized = [&](auto N) {
+      constexpr int NTOK = decltype(N)::value;
+      return act_kind == MOE_ACT_SILU ? launch<FMT, AT, true, true, NTOK>(mw, mb, P, grid, st) : launch<FMT, AT, true, false, NTOK>(mw, mb, P, grid, st);
+    };
+    if constexpr (FMT != FMT_HALF) {
+      if (tile_rows <= 64) return sized(std::integral_constant<int, 64>());
     }
-#undef MOE_WT
-  }
-#define MOE_WT(F)                                                                                               \
-  (act_dtype == MOE_BF16 ? (gemm1 ? launch<F, __nv_bfloat16, true>(mw, mb, P, grid, st)                         \
-                                  : launch<F, __nv_bfloat16, false>(mw, mb, P, grid, st))                       \
-                         : (gemm1 ? launch<F, __half, true>(mw, mb, P, grid, st) : launch<F, __half, false>(mw, mb, P, grid, st)))
+    return sized(std::integral_constant<int, 256>());
+  };
+  auto typed = [&](auto F) { return act_dtype == MOE_BF16 ? go(F, __nv_bfloat16()) : go(F, __half()); };
   switch (mode) {
-    case MOE_MODE_HALF: return MOE_WT(FMT_HALF);
-    case MOE_MODE_FP8_ROW: return MOE_WT(FMT_FP8ROW);
-    case MOE_MODE_INT8_ROW: return MOE_WT(FMT_I8ROW);
+    case MOE_MODE_HALF: return typed(std::integral_constant<int, FMT_HALF>());
+    case MOE_MODE_FP8_ROW: return typed(std::integral_constant<int, FMT_FP8ROW>());
+    case MOE_MODE_INT8_ROW: return typed(std::integral_constant<int, FMT_I8ROW>());
     default: return fail(MOE_E_BADARG, "grouped GEMM: mode %d", mode);
   }
-#undef MOE_WT
 }
 
 }  // namespace moe

@@ -38,7 +38,7 @@ bool rowwise_scatter_serves(int kind, int64_t cols);
 int rowwise_scatter(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, int k, const int32_t* row_index, void* q,
                     float* scales, cudaStream_t st);
 bool wt_serves(int mode, int act_dtype, int H, int I);
-int wt_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
+int wt_gemm(bool gemm1, int mode, int tile_rows, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
             const void* tiles, int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K,
             int Nout, void* out, int act_kind, float alpha, float beta, float limit, int32_t* status,
             cudaStream_t st);
@@ -78,6 +78,8 @@ bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
 constexpr int kSmallRoutes = 8;
 constexpr int64_t kSmallBytes = 1000000000;
 
+bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
+
 Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
   const int64_t per_expert = numel / (E > 0 ? E : 1);
   Choice c = {};
@@ -100,7 +102,9 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
   c.pair = mode != MOE_MODE_FP8_BLOCK && !(mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && per_expert < 96);
   if (c.pair) {
     c.gran = mode == MOE_MODE_INT8_ROW ? 32 : 16;  // kind::i8 on a pair takes multiples of 32
-    c.tile = 256;
+    // Few rows: tiles of 64, whose GEMM1 has a deeper ring for the weights (gemm_wt.cu).  GEMM1 + GEMM2 in us, 256 against 64: 500
+    // tokens of the Qwen3 shape (31 rows per expert) 108.9 : 104.7, 1000 tokens 115 : 118 (every second expert takes two tiles)
+    c.tile = row_mode(mode) && per_expert <= 52 ? 64 : 256;
   } else {
     c.gran = c.tile = 128;
     c.zero_pad = per_expert >= 128;
@@ -108,8 +112,6 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
   }
   return c;
 }
-
-bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
 
 // Pieces of the four workspaces (plan; rows of GEMM1; intermediate; rows behind GEMM2): 256-byte aligned, with at
 // least kGap bytes that nobody writes behind each, so that a write past the end of a piece can be seen.
@@ -263,7 +265,7 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
   if (stages & 4) {
     rc = mode == MOE_MODE_W8A16 ? w8t_gemm(true, c.wide, act_dtype, at(L.x_rows), w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
                                            L.rows_cap, E_local, H, I, at(L.act), status, st)
-         : c.pair ? wt_gemm(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
+         : c.pair ? wt_gemm(true, mode, c.tile, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
                           L.rows_cap, E_local, H, I, at(L.act), activation, alpha, beta, limit, status, st)
                 : tc_gemm_plan(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, counts + 1, numel, L.rows_cap,
                                E_local, H, I, at(L.act), act_scales, row_weight, c.zero_pad, c.staged, status, st);
@@ -284,7 +286,7 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
   if (stages & 16) {
     rc = mode == MOE_MODE_W8A16 ? w8t_gemm(false, c.wide, act_dtype, act, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
                                            E_local, I, H, at(L.y), status, st)
-         : c.pair ? wt_gemm(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
+         : c.pair ? wt_gemm(false, mode, c.tile, act_dtype, act, act_scales, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
                           E_local, I, H, at(L.y), MOE_ACT_SILU, 0.0f, 0.0f, 0.0f, status, st)
                 : tc_gemm_plan(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, counts + 1, numel, L.rows_cap, E_local,
                                I, H, at(L.y), nullptr, nullptr, c.zero_pad, c.staged, status, st);

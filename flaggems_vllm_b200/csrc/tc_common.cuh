@@ -261,6 +261,30 @@ __device__ __forceinline__ void tc_mma_block_f8(bool yes, uint32_t tmem_d, uint6
       ::"r"((uint32_t)yes), "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc_bar), "r"(stage_bar)
       : "memory");
 }
+// A K block of a CTA pair (four instructions, 32 bytes of K each) and the commit to the stage's barrier in both CTAs, by the
+// lane where `yes`, in one statement; acc: the first instruction adds to the accumulator as well.
+template <int KIND>
+__device__ __forceinline__ void tc_mma_block_pair(bool yes, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool acc,
+                                                  uint32_t stage_bar) {
+#define MOE_MMA2_BLOCK(KINDSTR)                                                                                  \
+  asm volatile(                                                                                                  \
+      "{\n\t.reg .pred l, p, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"                                        \
+      "setp.ne.b32 l, %0, 0;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"                               \
+      "add.s64 a1, %2, 2;\n\tadd.s64 a2, %2, 4;\n\tadd.s64 a3, %2, 6;\n\t"                                       \
+      "add.s64 b1, %3, 2;\n\tadd.s64 b2, %3, 4;\n\tadd.s64 b3, %3, 6;\n\t"                                       \
+      "@l tcgen05.mma.cta_group::2.kind::" KINDSTR " [%1], %2, %3, %4, p;\n\t"                                    \
+      "@l tcgen05.mma.cta_group::2.kind::" KINDSTR " [%1], a1, b1, %4, t;\n\t"                                    \
+      "@l tcgen05.mma.cta_group::2.kind::" KINDSTR " [%1], a2, b2, %4, t;\n\t"                                    \
+      "@l tcgen05.mma.cta_group::2.kind::" KINDSTR " [%1], a3, b3, %4, t;\n\t"                                    \
+      "@l tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], %7;\n\t}" \
+      ::"r"((uint32_t)yes), "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)acc), "r"(stage_bar),   \
+        "h"((uint16_t)3)                                                                                         \
+      : "memory")
+  if constexpr (KIND == MMA_F8) MOE_MMA2_BLOCK("f8f6f4");
+  else if constexpr (KIND == MMA_I8) MOE_MMA2_BLOCK("i8");
+  else MOE_MMA2_BLOCK("f16");
+#undef MOE_MMA2_BLOCK
+}
 // Packed fp32 pair FMA: d = a * b + d on two lanes of a 64-bit register pair.  Half the issue
 // slots of two scalar FMAs, which matters for warps that share a scheduler with the thread
 // that feeds the tensor core.

@@ -24,7 +24,8 @@ def _parity(out, ref, what):
 
 
 @pytest.mark.parametrize("fmt", ["fp8", "int8"])
-@pytest.mark.parametrize("M,E,k,H,I", [(1, 8, 2, 256, 128), (129, 4, 2, 1152, 384), (700, 4, 2, 256, 640)])
+@pytest.mark.parametrize("M,E,k,H,I", [(1, 8, 2, 256, 128), (129, 4, 2, 1152, 384), (700, 4, 2, 256, 640),
+                                         (208, 16, 4, 1408, 1920), (212, 16, 4, 1408, 1920)])  # last of the 64-row tiles, first of the others
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_row_scaled_tensor_core_layer(fmt, M, E, k, H, I, dtype):
     x = T.make_activations(M, H, DEV, dtype=dtype)
