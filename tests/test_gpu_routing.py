@@ -117,6 +117,32 @@ def test_known_answer_inf_and_signed_zero(groups, keep):
     assert torch.equal(torch.signbit(w), torch.signbit(scores[:, :8]))
 
 
+@pytest.mark.parametrize("M", [296, 297, 1001])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("form", ["rows", "strided", "odd_offset"])
+def test_eight_groups_of_32_both_kernels(M, dtype, form):
+    """A CTA per token and a warp per token, either side of the rule; other strides and alignments, ties, -inf, padding."""
+    g = torch.Generator().manual_seed(M)
+    s = torch.randn((M, 256), generator=g)
+    s[: M // 3] = (s[: M // 3] * 2).round() / 2  # ties
+    s[M // 3: M // 2, ::3] = -float("inf")
+    s[M // 2] = -float("inf")
+    s = s.to(dtype).to(DEV)
+    bias = torch.randn((257,), generator=g).mul(0.1).to(dtype).to(DEV)
+    if form == "strided":
+        s = s.t().contiguous().t()
+    elif form == "odd_offset":
+        wide = torch.zeros((M, 259), dtype=dtype, device=DEV)
+        wide[:, 1:257] = s
+        s = wide[:, 1:257]
+    pad = (torch.arange(M, device=DEV) % 5 == 0)
+    for k, keep, sf in ((8, 4, 1), (1, 1, 0), (32, 3, 1), (30, 8, 0)):
+        b = bias[1:] if form == "odd_offset" else bias[:256].contiguous()
+        _check(s, 8, keep, k, sf == 1, 2.5, b, sf)  # raw scores of -inf do not renormalise to anything
+        if form != "strided":  # refused with a mask
+            _check(s, 8, keep, k, False, 1.0, b, sf, pad)
+
+
 @pytest.mark.parametrize("mode", ["mixed", "all", "none"])
 def test_padding_rows(mode):
     rows, E = 9, 256
