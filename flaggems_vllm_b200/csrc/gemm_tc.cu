@@ -138,7 +138,6 @@ struct Params {
   int n_tiles;  // column tiles per align block
   int group_m;  // align blocks per group of the tile order
   int w_row0;   // GEMM2 over a window of the output columns: first weight row (output column) of the window
-  bool all_rows;    // route plan: fetch whole 128-row blocks of A (their padding rows are zero) instead of the occupied rows
   bool wide_store;  // the output is 32-byte aligned: rows are written with 32-byte stores
 };
 
@@ -201,11 +200,15 @@ __device__ __forceinline__ int box_row(int nt, int c, int cr, int Nout) {
 // the next tile -- sat in those stores for ~5000 cycles per tile; staged, they are done after
 // sixteen conflict-free shared-memory stores.  Costs one pipeline stage of shared memory.
 //
+// BY_EXPERT (route plan, whole blocks): the blocks of an expert, which the plan knows, share its column tiles in the tile order.
+// Fixed groups of blocks start somewhere inside an expert and read its weights once per group: DSV3 FP8, 8192 tokens, the
+// layer 4799 -> 4719 us.  With few rows per expert the order is the same and the plan entries cost up to 1 %.
+//
 // Row-scaled formats (FMT_FP8ROW, FMT_I8ROW): one-byte operands like the block-scaled mode, but
 // nothing has to happen between K blocks, so the whole K loop accumulates in TMEM like half
 // precision (int8: exact int32 sums) and the epilogue multiplies by the row's and the channel's
 // scale.  Qwen3 shape, 500 tokens, e4m3: 5605 us for the two GEMMs on CUDA cores before.
-template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false>
+template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false, bool BY_EXPERT = false>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_a16,
@@ -216,6 +219,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   static_assert(!ROW || (!PAIR && RB == 1 && !SORTED), "row-scaled formats: the single-CTA kernel");
   static_assert(!TMAOUT || (!GEMM1 && !PAIR && RB == 1), "staged output: single-CTA GEMM2 only");
   static_assert(!SORTED || GEMM1, "pre-sorted A rows: GEMM1 only");
+  static_assert(!BY_EXPERT || (FP8 && !PAIR && RB == 1 && (GEMM1 ? SORTED : TMAOUT)), "expert order: the FP8 kernels of a route plan's whole blocks");
   constexpr bool GATHER = GEMM1 && !SORTED;  // A rows gathered inside the kernel
   static_assert(RB == 1 || (RB == 2 && !BYTE), "wide tiles: half precision only");
   constexpr int STAGES = TMAOUT ? 3 : Cfg<PAIR, RB>::STAGES;
@@ -257,32 +261,52 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     blk = first + within - nt * gsz;
   };
   auto expert_of = [&](int blk) -> int { return P.tiles != nullptr ? __ldcg(&P.tiles[blk].z) : P.expert_ids[blk]; };
+  // BY_EXPERT: plan entry of one of the blocks of the expert that the NEXT tile belongs to, loaded a whole tile before it is used
+  [[maybe_unused]] int2 ahead = make_int2(-1, 1 << 16);  // {expert, first block | blocks << 16}
+  [[maybe_unused]] auto look_ahead = [&](int tile) {
+    if (tile < total_tiles) ahead = __ldcg(reinterpret_cast<const int2*>(P.tiles + tile / P.n_tiles) + 1);
+  };
   // tile -> expert_ids index (blk), this CTA's 128-row block (mb), column tile (nt).  The expert of
   // the NEXT tile is fetched while the current one is worked on: a tile starts without waiting
   // for a global load (every role walks the same tile list with its own copy of e_next).
-#define MOE_TILE_COORDS(tile)                             \
-  int blk, nt;                                            \
-  tile_blk_nt((tile), blk, nt);                           \
-  [[maybe_unused]] const int mb = UNIT * blk + RB * cr;   \
-  const int e = e_next;                                   \
-  e_next = -1;                                            \
-  if ((tile) + tile_step < total_tiles) {                 \
-    int blk2, nt2;                                        \
-    tile_blk_nt((tile) + tile_step, blk2, nt2);           \
-    e_next = expert_of(blk2);                             \
-  }
   int e_next = -1;
-  if (tile0 < total_tiles) {
+  if constexpr (BY_EXPERT) {
+    look_ahead(tile0);
+  } else if (tile0 < total_tiles) {
     int blk0, nt0;
     tile_blk_nt(tile0, blk0, nt0);
     e_next = expert_of(blk0);
   }
+  auto coords = [&](int tile, int& blk, int& nt) -> int {
+    if constexpr (BY_EXPERT) {
+      const int first = ahead.y & 0xFFFF, blocks = (int)((uint32_t)ahead.y >> 16), within = tile - first * P.n_tiles;
+      const int e = ahead.x;
+      nt = within / blocks;
+      blk = first + within - nt * blocks;
+      look_ahead(tile + tile_step);
+      return e;
+    } else {
+      tile_blk_nt(tile, blk, nt);
+      const int e = e_next;
+      e_next = -1;
+      if (tile + tile_step < total_tiles) {
+        int blk2, nt2;
+        tile_blk_nt(tile + tile_step, blk2, nt2);
+        e_next = expert_of(blk2);
+      }
+      return e;
+    }
+  };
+#define MOE_TILE_COORDS(tile)                             \
+  int blk, nt;                                            \
+  const int e = coords((tile), blk, nt);                  \
+  [[maybe_unused]] const int mb = UNIT * blk + RB * cr;
 
-  if constexpr (!GATHER && !PAIR && RB == 1) {
+  if constexpr (!GATHER && !PAIR && RB == 1 && !BY_EXPERT) {
     // Route plan, occupied rows only: the other rows of a stage are multiplied all the same.  They start as zeros and
     // stay zeros until a larger tile comes by.  Without this: DSV3 FP8, 61 tokens 1005 -> 1103 us per layer, one of 8 ranks
     // with 2000 tokens 319 -> 323; Mixtral shape, 300 tokens 520 -> 533.
-    if (P.tiles != nullptr && !P.all_rows) {
+    if (P.tiles != nullptr) {
       for (int i = threadIdx.x; i < STAGES * A_LOCAL_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(sA)[i] = make_uint4(0, 0, 0, 0);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -333,7 +357,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       bool alive = true;
       constexpr bool EARLY = !GATHER && !PAIR && RB == 1;
       auto occupied_rows = [&](int blk) -> int {  // rows of A to fetch
-        if (EARLY && P.tiles != nullptr && !P.all_rows) return ((__ldcg(&P.tiles[blk].y) >> 16) + 7) & ~7;
+        if (EARLY && !BY_EXPERT && P.tiles != nullptr) return ((__ldcg(&P.tiles[blk].y) >> 16) + 7) & ~7;
         return RB * BM;
       };
       // the stage's byte count and its weight tile
@@ -348,9 +372,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       int early = 0;
       if constexpr (EARLY) {
         if (P.tiles != nullptr && tile0 < total_tiles) {
-          int blk, nt;
-          tile_blk_nt(tile0, blk, nt);
-          const int a_rows = occupied_rows(blk), wrow0 = e_next * P.rows_w + P.w_row0;
+          int blk, nt, e0;
+          if constexpr (BY_EXPERT) {  // as coords(), which moves on
+            const int first = ahead.y & 0xFFFF, blocks = (int)((uint32_t)ahead.y >> 16), within = tile0 - first * P.n_tiles;
+            nt = within / blocks;
+            blk = first + within - nt * blocks;
+            e0 = ahead.x;
+          } else {
+            tile_blk_nt(tile0, blk, nt);
+            e0 = e_next;
+          }
+          const int a_rows = occupied_rows(blk), wrow0 = e0 * P.rows_w + P.w_row0;
           for (; early < STAGES && early < KB; ++early)
             if (leader) load_weights(early, early, a_rows, wrow0, nt);
         }
@@ -641,21 +673,28 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
     };
-    prefetch_tile(tile0);
+    if constexpr (!BY_EXPERT) prefetch_tile(tile0);
     for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
-      const int blk = nx_blk, nt = nx_nt, e = nx_e;
-      const int64_t sid_first = nx_sid;
+      int blk = nx_blk, nt = nx_nt, e = nx_e;
+      [[maybe_unused]] int occupied = 0;
+      if constexpr (BY_EXPERT) {
+        e = coords(tile, blk, nt);
+        occupied = __ldcg(&P.tiles[blk].y) >> 16;  // first looked at behind the K loop
+      }
+      [[maybe_unused]] const int64_t sid_first = nx_sid;
       [[maybe_unused]] const int mb = UNIT * blk + RB * cr;
-      (void)blk;
-      if (!FP8 || e < 0 || e >= P.E) prefetch_tile(tile + tile_step);  // half precision has no K loop here
+      if constexpr (!BY_EXPERT) {
+        if (!FP8 || e < 0 || e >= P.E) prefetch_tile(tile + tile_step);  // half precision has no K loop here
+      }
       if (e < 0 || e >= P.E) continue;
       for (int sub = 0; sub < RB && alive; ++sub) {  // the 128-row blocks of this tile (two for wide tiles)
       const int64_t p = (int64_t)(mb + sub) * BM + row;
       int64_t sid = P.numel;
-      if (sub == 0) sid = sid_first;
+      if (BY_EXPERT) sid = p;
+      else if (sub == 0) sid = sid_first;
       else if (p < P.rows_cap) sid = (int64_t)P.sorted_ids[p];
-      const bool row_ok = sid >= 0 && sid < P.numel;
-      if (sid < 0 || sid > P.numel) set_status(P.status, MOE_ST_BAD_ROW);  // the pad value is numel; anything else outside is corrupt
+      const bool row_ok = BY_EXPERT ? row < occupied : sid >= 0 && sid < P.numel;
+      if (!BY_EXPERT && (sid < 0 || sid > P.numel)) set_status(P.status, MOE_ST_BAD_ROW);  // the pad value is numel; anything else outside is corrupt
       float acc[128];
       [[maybe_unused]] float as = 0.0f;  // row-scaled formats: activation scale of this row
       float rw = 1.0f;  // route weight of this row, fetched early: the epilogue must not wait for it
@@ -684,7 +723,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           slot_at += SLOT;
           if (slot_at == SCALE_SLOTS * SLOT) slot_at = 0;
         };
-        prefetch_tile(tile + tile_step);
+        if constexpr (!BY_EXPERT) prefetch_tile(tile + tile_step);
         if (P.mul_weight && row_ok) rw = P.route_weight[sid];
         alive = mbar_wait_at(acc_full, acc_ph, P.status, P.wait_ns);
         if (!alive) break;
@@ -803,7 +842,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           amax = fmaxf(amax, x[(1 - h) * BM + row]);
           const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
           const float inv_s = 1.0f / s;  // one reciprocal per row instead of 64 divisions
-          if (row_ok || (SORTED && P.tiles != nullptr && P.all_rows)) {  // zero rows stay zero for GEMM2
+          if (row_ok || BY_EXPERT) {  // zero rows stay zero for GEMM2
             uint4 pieces[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
@@ -898,10 +937,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ------------------------------------------------------------------ host side
-template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false>
+template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false, bool BY_EXPERT = false>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P, int grid, cudaStream_t st,
                   const CUtensorMap* mo = nullptr, const CUtensorMap* ms = nullptr) {
-  auto kern = tc_gemm_kernel<FMT, AT, GEMM1, PAIR, RB, SORTED, TMAOUT>;
+  auto kern = tc_gemm_kernel<FMT, AT, GEMM1, PAIR, RB, SORTED, TMAOUT, BY_EXPERT>;
   constexpr size_t smem = smem_bytes<PAIR, RB, TMAOUT>();
   static const int regs = [&] {
     cudaFuncAttributes fa;
@@ -1000,7 +1039,7 @@ int tc_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
 
   Params P;
   if (sorted && (topk <= 0 || a_tokens * topk != numel)) return fail(MOE_E_BADARG, "tensor-core GEMM1: tokens * topk != numel");
-  P.tiles = nullptr; P.all_rows = true;
+  P.tiles = nullptr;
   P.a_rows = (const uint8_t*)a; P.a_scale_ld = (gemm1 && !sorted) ? a_tokens : rows_cap; P.topk = gemm1 ? topk : 1;
   P.a_scales_t = a_scales_t; P.w_scale = w_scale; P.expert_ids = expert_ids; P.sorted_ids = sorted_ids;
   P.num_post_pad = npp; P.route_weight = route_weight; P.out = out; P.out_scales_t = out_scales_t; P.inv = nullptr;
@@ -1098,7 +1137,7 @@ int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float
   if (rc) return rc;
   Params P = {};
   P.a_rows = (const uint8_t*)a; P.a_scale_ld = rows_cap; P.topk = 1;
-  P.a_scales_t = a_scales_t; P.w_scale = w_scale; P.tiles = (const int4*)tiles; P.all_rows = all_rows;
+  P.a_scales_t = a_scales_t; P.w_scale = w_scale; P.tiles = (const int4*)tiles;
   P.route_weight = row_weight; P.mul_weight = row_weight != nullptr;  // sorted order: row p's weight
   P.num_post_pad = rows; P.out = out; P.out_scales_t = out_scales_t; P.status = status; P.wait_ns = wait_limit_ns();
   P.numel = rows_cap; P.rows_cap = rows_cap; P.E = E; P.K = K; P.Nout = Nout; P.rows_w = rows_w;
@@ -1109,6 +1148,15 @@ int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float
   const int64_t cap_tiles = (rows_cap / BM) * (int64_t)P.n_tiles;
   const int sms = sm_count();
   const int grid = (int)(cap_tiles < sms ? cap_tiles : sms);
+  // whole blocks: from 128 rows per expert on (layer.cu), where an expert has several
+  if (all_rows) {
+    if (!fp8 || !staged) return fail(MOE_E_SHAPE, "tensor-core GEMM over a route plan: whole blocks are FP8's, with staged stores");
+#define MOE_TCE(T)                                                                                                \
+  (gemm1 ? launch<FMT_FP8, T, true, false, 1, true, false, true>(ma, mb, P, grid, st, nullptr, ms)                \
+         : launch<FMT_FP8, T, false, false, 1, false, true, true>(ma, mb, P, grid, st, &mo, ms))
+    return act_dtype == MOE_BF16 ? MOE_TCE(__nv_bfloat16) : MOE_TCE(__half);
+#undef MOE_TCE
+  }
 #define MOE_TCP(F, T)                                                                                             \
   (gemm1 ? launch<F, T, true, false, 1, true>(ma, mb, P, grid, st, nullptr, ms)                                   \
          : (staged ? launch<F, T, false, false, 1, false, true>(ma, mb, P, grid, st, &mo, ms)                     \
