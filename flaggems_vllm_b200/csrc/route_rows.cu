@@ -40,8 +40,17 @@ __global__ void __launch_bounds__(kThreads) zero_padding_kernel(const int4* __re
     scales_t[(int64_t)(i / padding) * scale_ld + d.x + occupied + i % padding] = 0.0f;
 }
 
-// Block (c, m): P x 2048 columns of token m, a warp per two neighbouring 128-groups, 8 elements per lane.  The arithmetic
-// is that of the stand-alone quantiser (quant.cu), bit for bit.
+// v / s, correctly rounded, for |v| <= 448 s (1 + ulp) from the rounded reciprocal of s: one correction step by the exact
+// remainder (P. Markstein, Computation of elementary functions on the IBM RISC System/6000, 1990).  Where the quotient is
+// so small that the remainder is not exact it rounds to zero in e4m3 all the same: over every pair of finite bf16 or f16
+// values (amax, |v| <= amax) the e4m3 bytes are those of the division.  The sign is v's, of a zero too.
+__device__ __forceinline__ float div_by_scale(float v, float s, float inv) {
+  const float q = v * inv;
+  return copysignf(fmaf(fmaf(-q, s, v), inv, q), v);
+}
+
+// Block (c, m): P x blockDim.x / 8 128-groups of token m, eight lanes per group, 16 elements per lane.  The bytes and scales
+// are those of the stand-alone quantiser (quant.cu).  With a division per element the kernel was bound by its instructions.
 template <typename T, int P>
 __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* __restrict__ x, int groups, int k,
                                                                        const int32_t* __restrict__ row_index,
@@ -52,48 +61,60 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
   const int lane = threadIdx.x & 31;
   const int64_t m = blockIdx.y;
   const int row = lane < k ? row_index[m * k + lane] : -1;
-  if (__ballot_sync(0xFFFFFFFFu, row >= 0) == 0) return;  // no route of this token is local
+  uint32_t rows = __ballot_sync(0xFFFFFFFFu, row >= 0);
+  if (rows == 0) return;  // no route of this token is local
   const int64_t K = (int64_t)groups * 128;
-  const int g0 = (blockIdx.x * P * (kThreads / 32) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
-  constexpr int STEP = kThreads / 16;  // groups of one pass of the block
-  uint4 raw[P];
+  const int step = blockDim.x / 8;  // groups of one pass of the block
+  const int g0 = blockIdx.x * P * step + (threadIdx.x >> 3);
+  uint4 raw[P][2];
 #pragma unroll
   for (int u = 0; u < P; ++u) {
-    raw[u] = make_uint4(0, 0, 0, 0);
-    if (g0 + u * STEP < groups) raw[u] = *reinterpret_cast<const uint4*>(x + m * K + (int64_t)(g0 + u * STEP) * 128 + (lane & 15) * 8);
+    raw[u][0] = raw[u][1] = make_uint4(0, 0, 0, 0);
+    if (g0 + u * step < groups) {
+      const uint4* src = reinterpret_cast<const uint4*>(x + m * K + (int64_t)(g0 + u * step) * 128 + (lane & 7) * 16);
+      raw[u][0] = src[0];
+      raw[u][1] = src[1];
+    }
   }
-  uint2 packed[P];
+  uint4 packed[P];
   float scale[P];
 #pragma unroll
   for (int u = 0; u < P; ++u) {
-    const T* pv = reinterpret_cast<const T*>(&raw[u]);
-    float v[8], amax = 0.0f;
+    const T* pv = reinterpret_cast<const T*>(&raw[u][0]);
+    float v[16], amax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 16; ++i) {
       v[i] = ToF32<T>::get(pv[i]);
       amax = fmaxf(amax, fabsf(v[i]));
     }
 #pragma unroll
-    for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
-    const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
-    uint32_t lo = 0, hi = 0;
+    for (int off = 4; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
+    const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max), inv = 1.0f / s;
+    const bool finite = s < INFINITY;
+    uint32_t w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      lo |= (uint32_t)f32_to_fp8e4m3(fminf(fmaxf(v[i] / s, -kFp8Max), kFp8Max)) << (8 * i);
-      hi |= (uint32_t)f32_to_fp8e4m3(fminf(fmaxf(v[4 + i] / s, -kFp8Max), kFp8Max)) << (8 * i);
+      float d[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        d[j] = finite ? div_by_scale(v[4 * i + j], s, inv) : v[4 * i + j] / s;
+        d[j] = fminf(fmaxf(d[j], -kFp8Max), kFp8Max);
+      }
+      w[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(d[0], d[1]), __NV_SATFINITE, __NV_E4M3) |
+             (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(d[2], d[3]), __NV_SATFINITE, __NV_E4M3) << 16;
     }
-    packed[u] = make_uint2(lo, hi);
+    packed[u] = make_uint4(w[0], w[1], w[2], w[3]);
     scale[u] = s;
   }
-  for (int j = 0; j < k; ++j) {
-    const int r = __shfl_sync(0xFFFFFFFFu, row, j);
-    if (r < 0) continue;
+  while (rows != 0) {
+    const int64_t r = __shfl_sync(0xFFFFFFFFu, row, __ffs(rows) - 1);
+    rows &= rows - 1;
 #pragma unroll
     for (int u = 0; u < P; ++u) {
-      const int g = g0 + u * STEP;
+      const int g = g0 + u * step;
       if (g < groups) {
-        *reinterpret_cast<uint2*>(q + (int64_t)r * K + (int64_t)g * 128 + (lane & 15) * 8) = packed[u];
-        if ((lane & 15) == 0) scales_t[(int64_t)g * rows_cap + r] = scale[u];
+        *reinterpret_cast<uint4*>(q + r * K + (int64_t)g * 128 + (lane & 7) * 16) = packed[u];
+        if ((lane & 7) == 0) scales_t[(int64_t)g * rows_cap + r] = scale[u];
       }
     }
   }
@@ -209,13 +230,13 @@ int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const
                         float* scales_t, cudaStream_t st) {
   const int groups = H / 128;
   const bool whole = whole_rows(M);
-  const int per_block = whole ? 64 : 16;
+  const int threads = whole ? kThreads : kThreads / 2, per_block = whole ? 64 : 16;
   const dim3 grid((unsigned)((groups + per_block - 1) / per_block), (unsigned)M);
-#define MOE_SCATTER(T, P)                                                                                                     \
-  launch_pdl(scatter_quant_group_kernel<T, P>, grid, kThreads, 0, 1, st, "scatter (1x128 quantised)", (const T*)x, groups, k, \
+#define MOE_SCATTER(T, P)                                                                                                   \
+  launch_pdl(scatter_quant_group_kernel<T, P>, grid, threads, 0, 1, st, "scatter (1x128 quantised)", (const T*)x, groups, k, \
              row_index, rows_cap, (uint8_t*)q, scales_t)
-  if (dtype == MOE_BF16) return whole ? MOE_SCATTER(__nv_bfloat16, 4) : MOE_SCATTER(__nv_bfloat16, 1);
-  return whole ? MOE_SCATTER(__half, 4) : MOE_SCATTER(__half, 1);
+  if (dtype == MOE_BF16) return whole ? MOE_SCATTER(__nv_bfloat16, 2) : MOE_SCATTER(__nv_bfloat16, 1);
+  return whole ? MOE_SCATTER(__half, 2) : MOE_SCATTER(__half, 1);
 #undef MOE_SCATTER
 }
 

@@ -1,6 +1,8 @@
 """The newer kernels at the sizes where they can go wrong: edges of tiles, remainders, the smallest and the
 largest of the range that their dispatch rule sends them."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -129,6 +131,40 @@ def test_fp8_block_layer_odd_k_blocks_and_several_tiles_per_cta(M, E, k, H, I, d
     tw, ti = _route(M, E, k)
     out = fg.fused_experts_impl(x, w1, w2, tw, ti, use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
     _parity(out, O.fused_moe_fp8_block_oracle(x, w1, w2, s1, s2, tw, ti), (M, H, I))
+
+
+@pytest.mark.parametrize("M", [3, 700])  # a block per 16 groups of a token, a block per token
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_scattered_fp8_rows_are_the_quantisers(M, dtype):
+    """Bytes and scales of the sorted rows against the stand-alone quantiser: zeros of either sign, subnormals, the type's
+    largest, infinities and NaN among them, and every magnitude in between."""
+    E, k, H, I = 4, 2, 8320, 128
+    x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
+    x *= torch.logspace(-30 if dtype == torch.bfloat16 else -6, 4, H // 128, device=DEV).repeat_interleave(128).to(dtype)
+    big = torch.finfo(dtype).max
+    for i, v in enumerate((0.0, -0.0, torch.finfo(dtype).tiny / 4, big, -big, float("inf"), -float("inf"), float("nan"))):
+        x[i % M, 128 * i + i:128 * i + 128:7] = v
+    x[M - 1, -128:] = -0.0
+    ti = torch.stack([torch.arange(M, device=DEV) % E, (torch.arange(M, device=DEV) + 1) % E], 1).to(torch.int32)
+    tw = torch.ones(M, k, device=DEV)
+    w1, s1 = T.make_fp8_block_weights(E, 2 * I, H, DEV, seed=1)
+    w2, s2 = T.make_fp8_block_weights(E, H, I, DEV, seed=2)
+    sizes = (_lib.MODE_FP8_BLOCK, _lib.dtype_code(dtype), M, k, E, E, H, I, _lib.ACT_SILU)
+    need, table = (ctypes.c_int64 * 4)(), (ctypes.c_int64 * (3 * 13))()
+    _lib.check(_lib.lib().moe_layer_layout(*sizes, ctypes.addressof(need), ctypes.addressof(table)))
+    ws = [torch.zeros(n, dtype=torch.uint8, device=DEV) for n in need]
+    out = torch.empty_like(x)
+    _lib.check(_lib.lib().moe_layer(
+        sizes[0], sizes[1], x.data_ptr(), M, k, ti.data_ptr(), 0, tw.data_ptr(), w1.data_ptr(), s1.data_ptr(), w2.data_ptr(),
+        s2.data_ptr(), out.data_ptr(), E, None, E, H, I, 0, _lib.ACT_SILU, 0.0, 0.0, 0.0, 0, None, 0, None,
+        *[w.data_ptr() for w in ws], 1 | 2, _lib.status_word(torch.device(DEV)).data_ptr(), _lib.stream_of(x)))
+    piece = lambda i, t: ws[table[3 * i]][table[3 * i + 1]:table[3 * i + 1] + table[3 * i + 2]].view(t)
+    rows = piece(0, torch.int32).view(M, k).long()
+    q, s = fg.per_token_group_quant_fp8(x, 128)
+    got, scales = piece(5, torch.uint8).view(-1, H), piece(6, torch.float32).view(H // 128, -1)
+    for j in range(k):
+        assert torch.equal(got[rows[:, j]], q.view(torch.uint8))
+        assert torch.equal(scales[:, rows[:, j]].t().contiguous().view(torch.int32), s.view(torch.int32))
 
 
 @pytest.mark.parametrize("M,E,k,H,I", [
