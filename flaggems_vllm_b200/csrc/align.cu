@@ -309,22 +309,25 @@ align_cluster_kernel(const IdT* __restrict__ ids, int numel, int E, int block_si
 
 // The usual sizes (at most 1024 experts, 262144 ids): one pass over the ids with the ranks in registers, padding slots
 // written by a warp per expert and the unused tail by everybody, so no slot is written twice and the only
-// barriers are those of the scan.  B200, 256 experts, block 128, graph replay, 65536 ids: 11.3 us uniform and 10.5 with
-// half of them on four experts; the kernels above took 26 and 20.
-template <typename IdT, int CTAS, int ROUNDS>
-__device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int numel, int E, int block_size,
+// barriers are those of the scan.  B200, 256 experts, block 128, 65536 ids with half of them on four experts: 8.0 us back to
+// back; the kernels above took 20.  Bound: the chain, in cycles of a cold call: ids 3200, ranks 2500, prefix and exchange 3000,
+// scan 1300, scatter of the ids 2600 (32 sectors per warp store), padding and tail 2900.
+template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
+__device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int numel, int E, int block_size, int block_shift,
                                                 int32_t* __restrict__ sorted_ids, int sorted_cap,
                                                 int32_t* __restrict__ expert_ids, int expert_cap,
                                                 int32_t* __restrict__ num_post_pad, int32_t* __restrict__ status) {
   using namespace sorting;
   extern __shared__ __align__(16) int32_t sort_smem[];
-  const Shared sh = carve(sort_smem, E);
+  const Shared sh = carve<CTAS>(sort_smem, E);
+  // blocks of n ids, rounded down; a shift where the block size is a power of two
+  auto blocks = [&](int n) { return block_shift >= 0 ? n >> block_shift : n / block_size; };
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int rank = 0;
   if constexpr (CTAS > 1) rank = (int)cg::this_cluster().block_rank();
   bool bad = false;
   int packed[ROUNDS], first, end;
-  rank_ids<CTAS, ROUNDS>(numel, E, sh, [&](int i) -> int {
+  rank_ids<CTAS, ROUNDS, MASKS>(numel, E, sh, [&](int i) -> int {
     const long long e = (long long)ids[i];
     if (e >= E) bad = true;  // negative ids mean "no route" (padding rows, other ranks' slots)
     return e >= 0 && e < E ? (int)e : -1;
@@ -332,12 +335,11 @@ __device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int
   if (bad) set_status(status, MOE_ST_BAD_EXPERT_ID);
   int before = 0, all = 0, padded = 0;
   if (tid < E) {
-    all = count_all<CTAS>(sh, tid, before);
-    padded = (all + block_size - 1) / block_size * block_size;
+    all = count_all<CTAS>(sh, tid, E, rank, before);
+    padded = blocks(all + block_size - 1) * block_size;
   }
-  if constexpr (CTAS > 1) cg::this_cluster().barrier_arrive();  // this CTA has read its peers' totals
-  unsigned long long sum;
-  const int start = (int)scan_cta((unsigned long long)padded, sum);
+  unsigned sum;
+  const int start = (int)scan_cta((unsigned)padded, sum);
   const int total = (int)sum;
   if (tid < E) {
     sh.base[tid] = start;
@@ -361,7 +363,8 @@ __device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int
     if (s0 == s1) continue;
     for (int p = s0 + sh.count[e] + lane; p < s1; p += 32)
       if (p < sorted_cap) sorted_ids[p] = numel;
-    for (int b = s0 / block_size + lane; b < s1 / block_size; b += 32)
+    const int b1 = blocks(s1);
+    for (int b = blocks(s0) + lane; b < b1; b += 32)
       if (b < expert_cap) expert_ids[b] = e;
   }
   // what no expert uses
@@ -371,14 +374,13 @@ __device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int
   for (int i = rank * kThreads + tid; i < whole; i += CTAS * kThreads)
     reinterpret_cast<int4*>(sorted_ids + quads)[i] = make_int4(numel, numel, numel, numel);
   for (int p = quads + 4 * whole + rank * kThreads + tid; p < sorted_cap; p += CTAS * kThreads) sorted_ids[p] = numel;
-  for (int b = total / block_size + rank * kThreads + tid; b < expert_cap; b += CTAS * kThreads) expert_ids[b] = -1;
-  if constexpr (CTAS > 1) cg::this_cluster().barrier_wait();  // no CTA leaves while its totals may still be read
+  for (int b = blocks(total) + rank * kThreads + tid; b < expert_cap; b += CTAS * kThreads) expert_ids[b] = -1;
 }
-template <typename IdT, int CTAS, int ROUNDS>
+template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
 __global__ void __launch_bounds__(sorting::kThreads)
-align_sort_kernel(const IdT* ids, int numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
+align_sort_kernel(const IdT* ids, int numel, int E, int block_size, int block_shift, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
                   int expert_cap, int32_t* npp, int32_t* status) {
-  align_sort_body<IdT, CTAS, ROUNDS>(ids, numel, E, block_size, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status);
+  align_sort_body<IdT, CTAS, ROUNDS, MASKS>(ids, numel, E, block_size, block_shift, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status);
 }
 
 // A cluster at any size: even a call of a few ids writes tens of thousands of sentinels.  False where no such cluster can
@@ -387,15 +389,18 @@ template <typename IdT>
 bool launch_align_sort(const void* ids, int numel, int E, int block_size, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
                        int expert_cap, int32_t* npp, int32_t* status, int limit, cudaStream_t st, int* rc) {
   using namespace sorting;
+  const int block_shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz((unsigned)block_size) : -1;
   auto launch = [&](auto kern, int ctas) {
     if (ctas > limit || !cluster_fits(kern, ctas, E)) return false;
-    *rc = launch_cluster(kern, ctas, E, st, "align (sort)", (const IdT*)ids, numel, E, block_size, sorted_ids, sorted_cap, expert_ids,
-                         expert_cap, npp, status);
+    *rc = launch_cluster(kern, ctas, E, st, "align (sort)", (const IdT*)ids, numel, E, block_size, block_shift, sorted_ids, sorted_cap,
+                         expert_ids, expert_cap, npp, status);
     return true;
   };
-  if (numel <= capacity(kSmall, 2)) return launch(align_sort_kernel<IdT, kSmall, 2>, kSmall);
-  if (numel <= capacity(kLarge, 4)) return launch(align_sort_kernel<IdT, kLarge, 4>, kLarge);
-  return launch(align_sort_kernel<IdT, kLarge, 16>, kLarge);
+#define MOE_ALIGN(C, R) (by_masks(E) ? launch(align_sort_kernel<IdT, C, R, true>, C) : launch(align_sort_kernel<IdT, C, R, false>, C))
+  if (numel <= capacity(kSmall, 2)) return MOE_ALIGN(kSmall, 2);
+  if (numel <= capacity(kLarge, 4)) return MOE_ALIGN(kLarge, 4);
+  return MOE_ALIGN(kLarge, 16);
+#undef MOE_ALIGN
 }
 
 template <typename IdT>

@@ -16,20 +16,20 @@
 namespace moe {
 namespace {
 
-template <typename IdT, int CTAS, int ROUNDS>
+template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
 __device__ __forceinline__ void plan_body(const IdT* __restrict__ ids, int numel, int E, const int32_t* __restrict__ emap,
-                                          int E_local, int gran, int tile_rows, int32_t* __restrict__ row_index, int rows_cap,
+                                          int E_local, int gran_shift, int tile_rows, int32_t* __restrict__ row_index, int rows_cap,
                                           int4* __restrict__ tiles, int tiles_cap, int32_t* __restrict__ counts,
                                           int32_t* __restrict__ status) {
   using namespace sorting;
   extern __shared__ __align__(16) int32_t sort_smem[];
-  const Shared sh = carve(sort_smem, E_local);
+  const Shared sh = carve<CTAS>(sort_smem, E_local);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int rank = 0;
   if constexpr (CTAS > 1) rank = (int)cg::this_cluster().block_rank();
   bool bad = false;
   int packed[ROUNDS], first, end;
-  rank_ids<CTAS, ROUNDS>(numel, E_local, sh, [&](int i) -> int {
+  rank_ids<CTAS, ROUNDS, MASKS>(numel, E_local, sh, [&](int i) -> int {
     const long long e = (long long)ids[i];
     if (e < 0 || e >= E) {
       if (e >= E) bad = true;  // negative ids mean "no route" (padding rows, other ranks' slots)
@@ -40,29 +40,25 @@ __device__ __forceinline__ void plan_body(const IdT* __restrict__ ids, int numel
     return m >= 0 && m < E_local ? m : -1;
   }, packed, first, end);
   if (bad) set_status(status, MOE_ST_BAD_EXPERT_ID);
-  int before = 0, all = 0, padded = 0, q = 0;
+  // rows of an expert in units of the granule, and the tiles they are cut into; both fit 16 bits (launch_plan)
+  auto units_of = [&](int n) { return (n + (1 << gran_shift) - 1) >> gran_shift; };
+  auto tiles_of = [&](int units) { return ((units << gran_shift) + tile_rows - 1) / tile_rows; };
+  int before = 0, all = 0;
+  unsigned mine = 0, sum;
   if (tid < E_local) {
-    all = count_all<CTAS>(sh, tid, before);
-    padded = (all + gran - 1) / gran * gran;
-    q = (padded + tile_rows - 1) / tile_rows;
+    all = count_all<CTAS>(sh, tid, E_local, rank, before);
+    const int units = units_of(all);
+    mine = (unsigned)units | (unsigned)tiles_of(units) << 16;
   }
-  if constexpr (CTAS > 1) cg::this_cluster().barrier_arrive();  // this CTA has read its peers' totals
-  unsigned long long sum;
-  const unsigned long long base = scan_cta(((unsigned long long)q << 32) | (unsigned)padded, sum);
+  const unsigned base = scan_cta(mine, sum);
   if (tid < E_local) {
-    const int row0 = (int)(base & 0xFFFFFFFFull), at = (int)(base >> 32);
-    sh.place[tid] = row0 + before;
-    if (q > 0 && (CTAS == 1 || tid % CTAS == rank)) {
-      const int size = ((padded / gran + q - 1) / q) * gran;  // even split, in multiples of gran rows
-      for (int t = 0; t < q; ++t) {
-        const int r = min(padded, t * size), n = min(size, padded - r), occupied = max(0, min(n, all - r));
-        if (at + t < tiles_cap) tiles[at + t] = make_int4(row0 + r, max(n, 0) | (occupied << 16), tid, at | (q << 16));
-      }
-    }
+    sh.base[tid] = (int)base;
+    sh.count[tid] = all;
+    sh.place[tid] = (int)((base & 0xFFFFu) << gran_shift) + before;
   }
   if (rank == 0 && tid == 0) {
-    counts[0] = min((int)(sum >> 32), tiles_cap);
-    counts[1] = min((int)(sum & 0xFFFFFFFFull), rows_cap);
+    counts[0] = min((int)(sum >> 16), tiles_cap);
+    counts[1] = min((int)((sum & 0xFFFFu) << gran_shift), rows_cap);
   }
   __syncthreads();
 #pragma unroll
@@ -75,14 +71,27 @@ __device__ __forceinline__ void plan_body(const IdT* __restrict__ ids, int numel
       row_index[i] = -1;
     }
   }
-  if constexpr (CTAS > 1) cg::this_cluster().barrier_wait();  // no CTA leaves while its totals may still be read
+  // The tiles, an even split in multiples of the granule.  A warp per expert, which may have many; in one CTA (2048 ids at
+  // most) the experts do not have enough tiles for that, and a warp would come to eight of them in turn: a thread each.
+  constexpr bool BY_WARP = CTAS > 1;
+  for (int e = BY_WARP ? rank * kWarps + warp : tid; e < E_local; e += BY_WARP ? CTAS * kWarps : kThreads) {
+    const int n_all = sh.count[e];
+    if (n_all == 0) continue;
+    const unsigned at0 = (unsigned)sh.base[e];
+    const int row0 = (int)((at0 & 0xFFFFu) << gran_shift), at = (int)(at0 >> 16), units = units_of(n_all), q = tiles_of(units);
+    const int padded = units << gran_shift, size = ((units + q - 1) / q) << gran_shift;
+    for (int t = BY_WARP ? lane : 0; t < q; t += BY_WARP ? 32 : 1) {
+      const int r = min(padded, t * size), n = min(size, padded - r), occupied = max(0, min(n, n_all - r));
+      if (at + t < tiles_cap) tiles[at + t] = make_int4(row0 + r, max(n, 0) | (occupied << 16), e, at | (q << 16));
+    }
+  }
 }
 
-template <typename IdT, int CTAS, int ROUNDS>
+template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
 __global__ void __launch_bounds__(sorting::kThreads) plan_kernel(const IdT* ids, int numel, int E, const int32_t* emap, int E_local,
-                                                                 int gran, int tile_rows, int32_t* row_index, int rows_cap,
+                                                                 int gran_shift, int tile_rows, int32_t* row_index, int rows_cap,
                                                                  int4* tiles, int tiles_cap, int32_t* counts, int32_t* status) {
-  plan_body<IdT, CTAS, ROUNDS>(ids, numel, E, emap, E_local, gran, tile_rows, row_index, rows_cap, tiles, tiles_cap, counts, status);
+  plan_body<IdT, CTAS, ROUNDS, MASKS>(ids, numel, E, emap, E_local, gran_shift, tile_rows, row_index, rows_cap, tiles, tiles_cap, counts, status);
 }
 
 // Up to 32 ids: one warp, everything in registers and votes, no shared memory and no barrier (one token of 8 routes:
@@ -132,15 +141,21 @@ int launch_plan(const void* ids, int numel, int E, const int32_t* emap, int E_lo
   if (numel <= kWarpIds && (kWarpIds + gran - 1) / gran * gran <= tile_rows)
     return launch_pdl(plan_warp_kernel<IdT>, dim3(1), 32, 0, 1, st, "route plan (warp)", (const IdT*)ids, numel, E, emap, E_local, gran,
                       row_index, rows_cap, tiles, tiles_cap, counts, status);
-#define MOE_PLAN(C, R)                                                                                                   \
-  launch_cluster(plan_kernel<IdT, C, R>, C, E_local, st, "route plan", (const IdT*)ids, numel, E, emap, E_local, gran, tile_rows, \
-                 row_index, rows_cap, tiles, tiles_cap, counts, status)
+  // the kernel counts rows in granules and tiles in 16 bits each
+  if (gran < 16 || (gran & (gran - 1)) != 0 || rows_cap / gran > 65535 || tiles_cap > 65535)
+    return fail(MOE_E_SHAPE, "route plan: granules of %d rows, at most 65535 of them and of tiles", gran);
+  const int gran_shift = __builtin_ctz((unsigned)gran);
+#define MOE_PLAN_B(C, R, B)                                                                                                    \
+  launch_cluster(plan_kernel<IdT, C, R, B>, C, E_local, st, "route plan", (const IdT*)ids, numel, E, emap, E_local, gran_shift, \
+                 tile_rows, row_index, rows_cap, tiles, tiles_cap, counts, status)
+#define MOE_PLAN(C, R) (by_masks(E_local) ? MOE_PLAN_B(C, R, true) : MOE_PLAN_B(C, R, false))
   // one CTA while a warp sees at most two rounds of ids: no cluster barriers
   if (numel <= capacity(1, 2)) return MOE_PLAN(1, 2);
   if (numel <= capacity(kSmall, 2)) return MOE_PLAN(kSmall, 2);
   if (numel <= capacity(kLarge, 4)) return MOE_PLAN(kLarge, 4);
   return MOE_PLAN(kLarge, 16);
 #undef MOE_PLAN
+#undef MOE_PLAN_B
 }
 }  // namespace
 
@@ -157,9 +172,9 @@ bool plan_serves(int64_t numel, int E, int E_local) {
   using namespace sorting;
   if (E <= 0 || E_local <= 0 || E_local > kMaxExperts || numel <= 0 || numel > capacity(kLarge, 16)) return false;
   if (numel <= capacity(1, 2)) return true;
-  if (numel <= capacity(kSmall, 2)) return cluster_fits(plan_kernel<int32_t, kSmall, 2>, kSmall, E_local);
-  if (numel <= capacity(kLarge, 4)) return cluster_fits(plan_kernel<int32_t, kLarge, 4>, kLarge, E_local);
-  return cluster_fits(plan_kernel<int32_t, kLarge, 16>, kLarge, E_local);
+  if (numel <= capacity(kSmall, 2)) return cluster_fits(plan_kernel<int32_t, kSmall, 2, false>, kSmall, E_local);
+  if (numel <= capacity(kLarge, 4)) return cluster_fits(plan_kernel<int32_t, kLarge, 4, false>, kLarge, E_local);
+  return cluster_fits(plan_kernel<int32_t, kLarge, 16, false>, kLarge, E_local);
 }
 
 int plan_routes(const void* ids, int ids64, int64_t numel, int E, const int32_t* emap, int E_local, int gran, int tile_rows,

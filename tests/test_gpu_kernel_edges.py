@@ -255,6 +255,31 @@ def test_align_slices(numel, E, bs):
         assert torch.equal(g.cpu(), torch.as_tensor(r))
 
 
+@pytest.mark.parametrize("E", [511, 512])
+@pytest.mark.parametrize("numel", [33, 2048, 2049, 16384, 16385, 65537])
+def test_sorted_ids_either_side_of_the_lane_masks(E, numel):
+    """Up to 511 experts the lanes of an expert are found by lane masks, beyond by votes: align, and the route plan of a layer
+    whose tiles, rows and combine follow it."""
+    ids = T.make_align_ids(numel, 1, E, DEV, skewed=numel % 2 == 1, seed=numel)
+    ids[5], ids[numel // 2] = -1, E - 1
+    got = fg.moe_align_block_size(ids, 32, E)
+    ref = O.moe_align_block_size_oracle(ids.cpu(), 32, E)
+    for g, r in zip(got, ref):
+        assert torch.equal(g.cpu(), torch.as_tensor(r))
+    H = I = 128
+    k = 1 if numel % 2 else 2
+    M = numel // k
+    ti = ids[:M * k].view(M, k).contiguous()
+    if k == 2:
+        ti[:, 1] = (ti[:, 0].clamp(min=0) + 1) % E
+    x, w1, w2, tw, _ = _half_layer(M, E, k, H, I, torch.bfloat16)
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti)
+    keep = ti >= 0
+    rows = torch.arange(0, M, max(1, M // 300), device=DEV)  # the oracle on some of the tokens
+    ref = O.fused_moe_half_oracle(x[rows], w1, w2, (tw * keep)[rows], ti.clamp(min=0)[rows])
+    _parity(out[rows], ref, (M, E))
+
+
 @pytest.mark.parametrize("limit", [1, 8])
 @pytest.mark.parametrize("numel", [0, 1, 2049, 4097, 16385, 65537, 262144])
 @pytest.mark.parametrize("E,bs", [(5, 16), (256, 128), (1024, 7)])
