@@ -30,6 +30,8 @@ template <typename XT, typename WT, int ROWS, int COLS>
 __global__ void __launch_bounds__(kThreads) router_gemm_kernel(const XT* __restrict__ x, int64_t x_ld,
                                                                 const WT* __restrict__ w, int64_t M, int N, int K,
                                                                 float* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   const int n0 = blockIdx.x * COLS;
   const int64_t m0 = (int64_t)blockIdx.y * ROWS;
   const int rows = (int)min((int64_t)ROWS, M - m0);
@@ -89,8 +91,9 @@ __global__ void __launch_bounds__(kThreads) router_gemm_kernel(const XT* __restr
 // run-to-run deterministic and no partial ever goes to memory.  The product is small (256 x 7168
 // weights): what bounds it is how many SMs pull operands from L2 at once and the latency of one CTA's
 // K loop, hence the split.  Rows and columns beyond the matrix are zero-filled by TMA.
-// B200, K = 7168, N = 256, bf16, graph replay: 200 rows 54 -> 8.6 us (the row-streaming kernel before), 64 rows
-// 19 -> 6.7 us, 8192 rows 36 us.
+// Launched so that the next kernel's set-up (barriers, TMEM, the launch itself) overlaps this one's end: back to back,
+// K = 7168, N = 256, bf16, us, before and with it and all partial sums of an element in flight: 8 rows 8.9 -> 6.1, 64 rows
+// 8.3 -> 6.1, 200 rows 10.3 -> 7.1, 1000 rows 12.4 -> 11.1, 8192 rows 39.5 -> 34.0.
 constexpr int RBM = 128, RTHREADS = 192;
 template <int BN> struct RCfg {
   static constexpr int STAGE = (RBM + BN) * 128;
@@ -135,6 +138,8 @@ __global__ void __launch_bounds__(RTHREADS, 1) router_tc_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = aux->tmem_base;
+  pdl_wait();  // the operands and the output may be the kernel's in front
+  pdl_trigger();
   if (warp == 0) {
     const bool leader = elect_lane();
     for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
@@ -203,10 +208,16 @@ __global__ void __launch_bounds__(RTHREADS, 1) router_tc_kernel(const __grid_con
       const int64_t m = m0 + row;
       if (m >= M || n0 + c >= N) continue;
       float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      for (int r = 0; r < split; ++r) {
-        const float4 v = *reinterpret_cast<const float4*>(
-            cluster.map_shared_rank(reinterpret_cast<float*>(smem), r) + (size_t)row * (BN + 4) + c);
-        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+      for (int r0 = 0; r0 < split; r0 += 8) {  // eight CTAs' partial sums in flight, added in rank order
+        float4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (r0 + j < split)
+            v[j] = *reinterpret_cast<const float4*>(
+                cluster.map_shared_rank(reinterpret_cast<float*>(smem), r0 + j) + (size_t)row * (BN + 4) + c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (r0 + j < split) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
       }
       float* o = out + m * N + n0 + c;
       if (N % 4 == 0) {
@@ -239,23 +250,11 @@ int launch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int 
   rc = tc::make_map(&mw, w, dt, 2, (uint64_t)N, (uint64_t)K, BN, true);
   if (rc) return rc;
   auto kern = router_tc_kernel<T, BN>;
-  rc = allow_smem((const void*)kern, (int)C::SMEM);
+  rc = allow_smem((const void*)kern, (int)C::SMEM, split > 8);
   if (rc) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((N + BN - 1) / BN * split), (unsigned)((M + RBM - 1) / RBM));
-  cfg.blockDim = dim3(RTHREADS);
-  cfg.dynamicSmemBytes = C::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)split;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, mx, mw, M, N, (K + 63) / 64, split, out, status, wait_limit_ns());
-  if (ce != cudaSuccess) return fail((int)ce, "router_gemm (tcgen05): %s", cudaGetErrorString(ce));
-  return check_launch("router_gemm (tcgen05)");
+  const dim3 grid((unsigned)((N + BN - 1) / BN * split), (unsigned)((M + RBM - 1) / RBM));
+  return launch_pdl(kern, grid, RTHREADS, C::SMEM, split, st, "router_gemm (tcgen05)", mx, mw, M, N, (K + 63) / 64, split, out, status,
+                    wait_limit_ns());
 }
 
 // Column tile and K split.  A CTA's K loop advances by the larger of its operand bytes (an SM takes about 64 bytes
@@ -264,13 +263,14 @@ int launch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int 
 // round starts (128 CTAs in clusters of 8, one per SM, took two rounds); narrow tiles run two CTAs per SM, which
 // then share its bandwidth.  Of a whole GPU's 148 SMs it is 112 and 132 and not what the occupancy query gives (120 and
 // 132 on one GPU; which SMs are fused off differs), so that the order of the sums is one on every B200; a
-// partition has its share.  `largest`: most CTAs of a cluster.
+// partition has its share.  `largest`: most CTAs of a cluster.  Tiles of 256 columns are nowhere the fastest (four stages):
+// 8192 x 256 x 7168, us, 256 columns and two CTAs in K 40.4, 128 columns undivided 34.0.
 void pick_tc(int64_t M, int N, int K, int sms, int largest, int& bn, int& split) {
   const int kb = (K + 63) / 64;
   const int64_t mt = (M + RBM - 1) / RBM;
   double best = 0.0;
   bn = 0;
-  for (int b = 32; b <= 256; b *= 2) {
+  for (int b = 32; b <= 128; b *= 2) {
     if (b > 32 && b / 2 >= N) break;
     for (int s = 1; s <= 8 && s <= kb && s <= largest; s *= 2) {
       const double reach = (s == 8 ? 112.0 : (s == 4 ? 132.0 : 148.0)) * sms / 148.0;
@@ -294,8 +294,7 @@ bool split_fits(int bn, int split) {
   switch (bn) {
     case 32: return split_fits<T, 32>(split);
     case 64: return split_fits<T, 64>(split);
-    case 128: return split_fits<T, 128>(split);
-    default: return split_fits<T, 256>(split);
+    default: return split_fits<T, 128>(split);
   }
 }
 
@@ -309,8 +308,7 @@ int dispatch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, in
   switch (bn) {
     case 32: return launch_tc<T, 32>(x, x_ld, w, M, N, K, split, out, status, st);
     case 64: return launch_tc<T, 64>(x, x_ld, w, M, N, K, split, out, status, st);
-    case 128: return launch_tc<T, 128>(x, x_ld, w, M, N, K, split, out, status, st);
-    default: return launch_tc<T, 256>(x, x_ld, w, M, N, K, split, out, status, st);
+    default: return launch_tc<T, 128>(x, x_ld, w, M, N, K, split, out, status, st);
   }
 }
 
@@ -318,19 +316,15 @@ template <typename XT, typename WT>
 int launch_rows(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int K, float* out, cudaStream_t st) {
   // one token: its row and one weight row per CTA, several loads in flight; more tokens than fill one tile of
   // rows: four columns per CTA, so that a token row is fetched from L2 once per four columns
-  if (M == 1)
-    router_gemm_kernel<XT, WT, 1, 1><<<dim3((unsigned)N, 1), kThreads, 0, st>>>((const XT*)x, x_ld, (const WT*)w, M, N, K, out);
-  else if (M == 2)
-    router_gemm_kernel<XT, WT, 2, 1><<<dim3((unsigned)N, 1), kThreads, 0, st>>>((const XT*)x, x_ld, (const WT*)w, M, N, K, out);
-  else if (M <= kRowStreamMax)
-    router_gemm_kernel<XT, WT, kRowStreamMax, 1><<<dim3((unsigned)N, 1), kThreads, 0, st>>>((const XT*)x, x_ld, (const WT*)w, M, N, K, out);
-  else if (M <= 2 * kRows)
-    router_gemm_kernel<XT, WT, kRows, 1><<<dim3((unsigned)N, (unsigned)((M + kRows - 1) / kRows)), kThreads, 0, st>>>(
-        (const XT*)x, x_ld, (const WT*)w, M, N, K, out);
-  else
-    router_gemm_kernel<XT, WT, kRows, 4><<<dim3((unsigned)((N + 3) / 4), (unsigned)((M + kRows - 1) / kRows)), kThreads, 0, st>>>(
-        (const XT*)x, x_ld, (const WT*)w, M, N, K, out);
-  return check_launch("router_gemm");
+#define MOE_ROWS(ROWS, COLS)                                                                                              \
+  launch_pdl(router_gemm_kernel<XT, WT, ROWS, COLS>, dim3((unsigned)((N + COLS - 1) / COLS), (unsigned)((M + ROWS - 1) / ROWS)), \
+             kThreads, 0, 1, st, "router_gemm", (const XT*)x, x_ld, (const WT*)w, M, N, K, out)
+  if (M == 1) return MOE_ROWS(1, 1);
+  if (M == 2) return MOE_ROWS(2, 1);
+  if (M <= kRowStreamMax) return MOE_ROWS(kRowStreamMax, 1);
+  if (M <= 2 * kRows) return MOE_ROWS(kRows, 1);
+  return MOE_ROWS(kRows, 4);
+#undef MOE_ROWS
 }
 
 template <typename XT>
