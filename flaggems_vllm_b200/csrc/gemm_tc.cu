@@ -1116,18 +1116,18 @@ int tc_gemm(bool gemm1, int mode, int act_dtype, const void* a, const float* a_s
 #undef MOE_TC_LAUNCH2
 }
 
-// The same GEMMs over the blocks of a route plan made with 128-row tiles (plan.cu): A rows (GEMM1: scattered token
+// The FP8 GEMMs over the blocks of a route plan made with 128-row tiles (plan.cu): A rows (GEMM1: scattered token
 // rows, GEMM2: the intermediate) in sorted order, results in sorted order.  all_rows: the padding rows of A are zero,
 // fetch whole blocks.
-int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
+int tc_gemm_plan(bool gemm1, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
                  const void* tiles, const int32_t* rows, int64_t numel, int64_t rows_cap, int E, int K, int Nout, void* out,
                  float* out_scales_t, const float* row_weight, bool all_rows, bool staged, int32_t* status, cudaStream_t st) {
   using namespace tc;
-  const bool fp8 = mode == MOE_MODE_FP8_BLOCK;
-  const int eb = fp8 ? 1 : 2, rows_w = gemm1 ? 2 * Nout : Nout;
+  constexpr int eb = 1;
+  const int rows_w = gemm1 ? 2 * Nout : Nout;
   if ((int64_t)E * rows_w >= (1ll << 31) || rows_cap >= (1ll << 31)) return fail(MOE_E_TOOBIG, "tensor-core GEMM: extent exceeds int32 coordinates");
   const CUtensorMapDataType half_t = act_dtype == MOE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const CUtensorMapDataType dt = fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : half_t;
+  const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   CUtensorMap ma, mb, mo, ms[2];
   int rc = make_map(&ma, a, dt, eb, (uint64_t)rows_cap, (uint64_t)K, BM, false);
   if (!rc) rc = make_map(&ms[0], a, dt, eb, (uint64_t)rows_cap, (uint64_t)K, 16, false);
@@ -1149,22 +1149,15 @@ int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float
   const int sms = sm_count();
   const int grid = (int)(cap_tiles < sms ? cap_tiles : sms);
   // whole blocks: from 128 rows per expert on (layer.cu), where an expert has several
-  if (all_rows) {
-    if (!fp8 || !staged) return fail(MOE_E_SHAPE, "tensor-core GEMM over a route plan: whole blocks are FP8's, with staged stores");
-#define MOE_TCE(T)                                                                                                \
-  (gemm1 ? launch<FMT_FP8, T, true, false, 1, true, false, true>(ma, mb, P, grid, st, nullptr, ms)                \
-         : launch<FMT_FP8, T, false, false, 1, false, true, true>(ma, mb, P, grid, st, &mo, ms))
-    return act_dtype == MOE_BF16 ? MOE_TCE(__nv_bfloat16) : MOE_TCE(__half);
-#undef MOE_TCE
-  }
-#define MOE_TCP(F, T)                                                                                             \
-  (gemm1 ? launch<F, T, true, false, 1, true>(ma, mb, P, grid, st, nullptr, ms)                                   \
-         : (staged ? launch<F, T, false, false, 1, false, true>(ma, mb, P, grid, st, &mo, ms)                     \
-                   : launch<F, T, false, false, 1>(ma, mb, P, grid, st, nullptr, ms)))
-  if (fp8) return act_dtype == MOE_BF16 ? MOE_TCP(FMT_FP8, __nv_bfloat16) : MOE_TCP(FMT_FP8, __half);
-  if (mode == MOE_MODE_HALF) return act_dtype == MOE_BF16 ? MOE_TCP(FMT_HALF, __nv_bfloat16) : MOE_TCP(FMT_HALF, __half);
+  if (all_rows && !staged) return fail(MOE_E_SHAPE, "tensor-core GEMM over a route plan: whole blocks go with staged stores");
+#define MOE_TCP(T)                                                                                                                \
+  (gemm1 ? (all_rows ? launch<FMT_FP8, T, true, false, 1, true, false, true>(ma, mb, P, grid, st, nullptr, ms)                     \
+                     : launch<FMT_FP8, T, true, false, 1, true>(ma, mb, P, grid, st, nullptr, ms))                                 \
+         : (all_rows ? launch<FMT_FP8, T, false, false, 1, false, true, true>(ma, mb, P, grid, st, &mo, ms)                        \
+            : staged ? launch<FMT_FP8, T, false, false, 1, false, true>(ma, mb, P, grid, st, &mo, ms)                              \
+                     : launch<FMT_FP8, T, false, false, 1>(ma, mb, P, grid, st, nullptr, ms)))
+  return act_dtype == MOE_BF16 ? MOE_TCP(__nv_bfloat16) : MOE_TCP(__half);
 #undef MOE_TCP
-  return fail(MOE_E_SHAPE, "tensor-core GEMM over a route plan: FP8 block scales and half precision");
 }
 
 }  // namespace moe

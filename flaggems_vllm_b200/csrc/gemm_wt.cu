@@ -46,13 +46,13 @@ constexpr int CONS_THREADS = 256;
 constexpr int LAUNCH_REGS = 168, PRODUCER_REGS = 56, CONSUMER_REGS = 224;
 static_assert(128 * PRODUCER_REGS + CONS_THREADS * CONSUMER_REGS <= THREADS * LAUNCH_REGS, "register redistribution");
 
-// NTOK: most tokens of a tile.  64: the ring is left to the weights, ten stages of 16 KB of them in flight instead of five while
-// they stream.  Qwen3 shape, e4m3, GEMM1 back to back in us, 256 against 64: 33 tokens 58.3 : 55.1, 500 tokens 69.4 : 65.2.  GEMM2
-// (six K blocks per tile) is 2 % slower with it (39.5 : 40.5) and has one kernel.
+// NTOK: most tokens of a tile.  With few rows per expert the weights stream, and what they need is bytes in flight: small tiles
+// leave the ring to them, ten (64 tokens) or eight and seven (128) stages of 16 KB of weights instead of five and four.
+// layer.cu has the figures.
 template <bool GEMM1, int NTOK> struct Cfg {
   static constexpr int STAGE_BYTES = A_BYTES + NTOK / 2 * 128;
-  static_assert(NTOK == 256 || (GEMM1 && NTOK == 64), "tile");
-  static constexpr int STAGES = NTOK <= 64 ? 10 : (GEMM1 ? 5 : 4);
+  static_assert(NTOK == 256 || NTOK == 128 || NTOK == 64, "tile");
+  static constexpr int STAGES = NTOK <= 64 ? 10 : (NTOK <= 128 ? (GEMM1 ? 8 : 7) : (GEMM1 ? 5 : 4));
   static constexpr int OUT_BYTES = NTOK * ((GEMM1 ? 64 : 128) * 2 + 16);  // staged rows, see drain_tile
 };
 struct Aux {
@@ -66,7 +66,8 @@ template <bool GEMM1, int NTOK> constexpr size_t smem_bytes() {
   return (size_t)C::STAGES * C::STAGE_BYTES + C::OUT_BYTES + sizeof(Aux) + 1024;
 }
 static_assert(smem_bytes<true, 256>() <= 232448 && smem_bytes<false, 256>() <= 232448, "shared memory of one SM");
-static_assert(smem_bytes<true, 64>() <= 232448, "shared memory of one SM");
+static_assert(smem_bytes<true, 64>() <= 232448 && smem_bytes<false, 64>() <= 232448, "shared memory of one SM");
+static_assert(smem_bytes<true, 128>() <= 232448 && smem_bytes<false, 128>() <= 232448, "shared memory of one SM");
 
 // SILU: the activation of GEMM1 (false: swigluoai, which reads GEMM1's result rounded to the activation type)
 template <int FMT, typename AT, bool GEMM1, bool SILU, int NTOK>
@@ -289,19 +290,19 @@ int wt_gemm(bool gemm1, int mode, int tile_rows, int act_dtype, const void* a, c
   const int64_t items = tiles_cap * P.R;
   const int pairs = sm_count() / 2;
   const int grid = 2 * (int)(items < pairs ? items : pairs);
-  // half precision comes with 96 rows per expert and more (layer.cu), never with 64-token tiles
+  // the kernel of the plan's tiles: 64 (half precision), 128 or 256 rows (layer.cu); the other activation has one
   auto go = [&](auto F, auto T) {
     constexpr int FMT = decltype(F)::value;
     using AT = decltype(T);
-    if (!gemm1) return launch<FMT, AT, false, true, 256>(mw, mb, P, grid, st);
+    if (gemm1 && act_kind != MOE_ACT_SILU) return launch<FMT, AT, true, false, 256>(mw, mb, P, grid, st);
     auto sized = [&](auto N) {
       constexpr int NTOK = decltype(N)::value;
-      return act_kind == MOE_ACT_SILU ? launch<FMT, AT, true, true, NTOK>(mw, mb, P, grid, st) : launch<FMT, AT, true, false, NTOK>(mw, mb, P, grid, st);
+      return gemm1 ? launch<FMT, AT, true, true, NTOK>(mw, mb, P, grid, st) : launch<FMT, AT, false, true, NTOK>(mw, mb, P, grid, st);
     };
-    if constexpr (FMT != FMT_HALF) {
+    if constexpr (FMT == FMT_HALF) {
       if (tile_rows <= 64) return sized(std::integral_constant<int, 64>());
     }
-    return sized(std::integral_constant<int, 256>());
+    return tile_rows <= 128 ? sized(std::integral_constant<int, 128>()) : sized(std::integral_constant<int, 256>());
   };
   auto typed = [&](auto F) { return act_dtype == MOE_BF16 ? go(F, __nv_bfloat16()) : go(F, __half()); };
   switch (mode) {

@@ -18,7 +18,7 @@ int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const
 int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st);
 int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, int groups,
                  int64_t rows_cap, float* scales_t, cudaStream_t st);
-int tc_gemm_plan(bool gemm1, int mode, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
+int tc_gemm_plan(bool gemm1, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
                  const void* tiles, const int32_t* rows, int64_t numel, int64_t rows_cap, int E, int K, int Nout, void* out,
                  float* out_scales_t, const float* row_weight, bool all_rows, bool staged, int32_t* status, cudaStream_t st);
 int small_align(const void* ids, int ids64, int numel, int E, int32_t* sorted_ids, int rows_cap, int32_t* expert_ids, int32_t* npp,
@@ -52,7 +52,7 @@ namespace {
 // Which grouped GEMM serves the call and how the plan cuts the rows for it.
 struct Choice {
   bool small;       // gemm_small.cu: blocks of 8 routes, K split over the chip; no scatter, the sum inside GEMM2
-  bool pair;        // gemm_wt.cu: weights as the M operand of a CTA pair; else gemm_tc.cu: 128 tokens as M
+  bool pair;        // gemm_wt.cu: weights as the M operand of a CTA pair; else gemm_tc.cu (FP8 block scales): 128 tokens as M
   bool wide;        // weight-only int8 (gemm_w8t.cu): tiles of up to 160 tokens instead of 64
   int gran, tile;   // row granule and most rows of a tile
   bool zero_pad;    // gemm_tc.cu: zero the padding rows and fetch whole blocks
@@ -96,15 +96,15 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
     c.small = true;
     return c;
   }
-  // FP8 block scales: tokens as M (gemm_wt.cu says why).  Half precision: up to 96 rows per expert the weights are
-  // streamed and both kernels wait for memory (the single-CTA kernel is a few per cent ahead); above, the pair's finer
-  // row padding counts (Mixtral shape, 1024 tokens: 1047 -> 887 us).
-  c.pair = mode != MOE_MODE_FP8_BLOCK && !(mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && per_expert < 96);
+  // FP8 block scales: tokens as M (gemm_wt.cu says why).  All else: the pair, in tiles whose kernel has the deepest ring that still
+  // holds an expert's rows.  us per layer, Mixtral shape, bf16, tokens as M (before) / pair in tiles of 64 / 128 / 256:
+  //   rows per expert   5: 449 / 429 / 436 / 473    37: 465 / 440 / 447 / 484    57: 467 / 448 / 453 / 490    65: 480 / 485 / 458 / 494
+  //                    75: 485 / 558 / 459 / 499   105: 516 / 593 / 473 / 515   120: 543 / 617 / 515 / 519   140: 557 / 771 / 624 / 532
+  // e4m3 per channel, Qwen3 shape, 64 / 128 / 256: 31 rows per expert 136 / 135 / 139, 62 rows 159 / 155 / 158, 100 rows 197 / 177 / 177
+  c.pair = mode != MOE_MODE_FP8_BLOCK;
   if (c.pair) {
     c.gran = mode == MOE_MODE_INT8_ROW ? 32 : 16;  // kind::i8 on a pair takes multiples of 32
-    // Few rows: tiles of 64, whose GEMM1 has a deeper ring for the weights (gemm_wt.cu).  GEMM1 + GEMM2 in us, 256 against 64: 500
-    // tokens of the Qwen3 shape (31 rows per expert) 108.9 : 104.7, 1000 tokens 115 : 118 (every second expert takes two tiles)
-    c.tile = row_mode(mode) && per_expert <= 52 ? 64 : 256;
+    c.tile = mode == MOE_MODE_HALF && per_expert <= 58 ? 64 : (per_expert <= 120 ? 128 : 256);
   } else {
     c.gran = c.tile = 128;
     c.zero_pad = per_expert >= 128;
@@ -267,7 +267,7 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
                                            L.rows_cap, E_local, H, I, at(L.act), status, st)
          : c.pair ? wt_gemm(true, mode, c.tile, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, L.tiles_cap, counts, row_weight,
                           L.rows_cap, E_local, H, I, at(L.act), activation, alpha, beta, limit, status, st)
-                : tc_gemm_plan(true, mode, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, counts + 1, numel, L.rows_cap,
+                : tc_gemm_plan(true, act_dtype, at(L.x_rows), x_scales, w1, w1_scale, tiles, counts + 1, numel, L.rows_cap,
                                E_local, H, I, at(L.act), act_scales, row_weight, c.zero_pad, c.staged, status, st);
     if (rc) return rc;
   }
@@ -288,7 +288,7 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
                                            E_local, I, H, at(L.y), status, st)
          : c.pair ? wt_gemm(false, mode, c.tile, act_dtype, act, act_scales, w2, w2_scale, tiles, L.tiles_cap, counts, nullptr, L.rows_cap,
                           E_local, I, H, at(L.y), MOE_ACT_SILU, 0.0f, 0.0f, 0.0f, status, st)
-                : tc_gemm_plan(false, mode, act_dtype, act, act_scales, w2, w2_scale, tiles, counts + 1, numel, L.rows_cap, E_local,
+                : tc_gemm_plan(false, act_dtype, act, act_scales, w2, w2_scale, tiles, counts + 1, numel, L.rows_cap, E_local,
                                I, H, at(L.y), nullptr, nullptr, c.zero_pad, c.staged, status, st);
     if (rc) return rc;
   }
