@@ -67,16 +67,15 @@ bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
 }
 
 // The split-K weight streaming of gemm_small.cu: three launches instead of five, every SM busy however few tiles there
-// are, but one CTA needs more instructions per byte than the tile kernels.  So it is for calls whose launches count: up to
-// 8 routes that read up to 1 GB of weights if no two share an expert, which the host cannot see.  us per layer, split K
-// against tile kernels, bf16:
-//   Mixtral shape    1 token  0.7 GB  137 : 168   2 tokens 1.4 GB  256 : 253 (one pair of experts 143 : 168)
-//                    3 tokens 2.1 GB  371 : 330 (143 : 169)       4 tokens 2.8 GB  483 : 438 (148 : 171)
-//   E8 H1024 I2048   1 token   25 MB   18 : 30    2 tokens          20 : 31    4 tokens 27 : 37
-//   E128 H2048 I768  1 token   75 MB   23 : 28
-// From 1.4 GB on, distinct experts lose what shared ones would win, and distinct is the usual case.
-constexpr int kSmallRoutes = 8;
-constexpr int64_t kSmallBytes = 1000000000;
+// are, but one CTA needs more instructions per byte than the pair.  So it is for the calls whose launches count: up to four
+// routes and 200 MB of weights if no two share an expert, which the host cannot see.  us per layer (graph replay), bf16,
+// split K against the pair in tiles of 64:
+//   E8 H1024 I2048    1 token (25 MB, 2 routes) 17.5 : 19.9    2 tokens (50 MB) 21.0 : 22.6    3 tokens (6 routes) 28.9 : 25.7
+//   E8 H2048 I4096    1 token (101 MB, 2 routes) 29.9 : 34.7   2 tokens (201 MB) 43.1 : 43.5   4 tokens (8 routes) 78.6 : 61.8
+//   E128 H2048 I768   1 token (75 MB, 8 routes) 29.1 : 28.7    E64 H2048 I1408  1 token (104 MB, 6 routes) 33.5 : 31.7
+//   E16 H5120 I8192   1 token (252 MB, 1 route) 59.5 : 58.2    Mixtral shape    1 token (705 MB, 2 routes) 141.1 : 127.2
+constexpr int kSmallRoutes = 4;
+constexpr int64_t kSmallBytes = 200000000;
 
 bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
 
