@@ -14,8 +14,9 @@ int plan_routes(const void* ids, int ids64, int64_t numel, int E, const int32_t*
                 int32_t* row_index, int64_t rows_cap, void* tiles, int64_t tiles_cap, int32_t* counts, int32_t* status,
                 cudaStream_t st);
 int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,
-                        float* scales_t, cudaStream_t st);
-int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st);
+                        float* scales_t, bool early, cudaStream_t st);
+int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, bool early,
+                 cudaStream_t st);
 int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, int64_t row_bytes, void* rows, int groups,
                  int64_t rows_cap, float* scales_t, cudaStream_t st);
 int tc_gemm_plan(bool gemm1, int act_dtype, const void* a, const float* a_scales_t, const void* w, const float* w_scale,
@@ -31,12 +32,12 @@ int small_gemm(bool pdl, int gemm1, int mode, int act_dtype, const void* a, int6
                int32_t* unit_counters, int32_t* token_counters, int32_t* status, cudaStream_t st);
 int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_index, float* dst, cudaStream_t st);
 int combine_rows(const void* y, int dtype, const float* weight, const int32_t* row_index, int64_t M, int k, int64_t H, void* out,
-                 cudaStream_t st);
+                 bool early, cudaStream_t st);
 int rowwise_quant(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, const float* scale_in,
                   const int32_t* row_ids, int64_t valid_below, const int32_t* indirect, void* q, float* scale_out, cudaStream_t st);
 bool rowwise_scatter_serves(int kind, int64_t cols);
 int rowwise_scatter(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, int k, const int32_t* row_index, void* q,
-                    float* scales, cudaStream_t st);
+                    float* scales, bool early, cudaStream_t st);
 bool wt_serves(int mode, int act_dtype, int H, int I);
 int wt_gemm(bool gemm1, int mode, int tile_rows, int act_dtype, const void* a, const float* a_scales, const void* w, const float* w_scale,
             const void* tiles, int64_t tiles_cap, const int32_t* counts, const float* row_weight, int64_t rows_cap, int E, int K,
@@ -240,20 +241,21 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
     if (rc) return rc;
   }
   if (stages & 2) {
+    const bool early = (stages & 1) != 0 && M < 4 * sm_count();  // the kernel in front is this call's route plan, x is older
     if (block) {
-      rc = scatter_quant_group(x, act_dtype, M, H, topk, row_index, L.rows_cap, at(L.x_rows), x_scales, st);
+      rc = scatter_quant_group(x, act_dtype, M, H, topk, row_index, L.rows_cap, at(L.x_rows), x_scales, early, st);
     } else if (row) {
       const bool per_row = quant_kind1 == 0 || quant_kind1 == 1;
       if (rowwise_scatter_serves(quant_kind1, H)) {
-        rc = rowwise_scatter(x, act_dtype, M, H, quant_kind1, topk, row_index, at(L.x_rows), x_scales, st);
+        rc = rowwise_scatter(x, act_dtype, M, H, quant_kind1, topk, row_index, at(L.x_rows), x_scales, early, st);
       } else {
         float* sc = (float*)at(L.tmp_scales);
         rc = rowwise_quant(x, act_dtype, M, H, quant_kind1, quant_scale1, nullptr, 0, nullptr, at(L.tmp_q), sc, st);
-        if (!rc) rc = scatter_rows(at(L.tmp_q), M, H, topk, row_index, at(L.x_rows), st);
+        if (!rc) rc = scatter_rows(at(L.tmp_q), M, H, topk, row_index, at(L.x_rows), false, st);  // behind the quantiser of its rows
         if (!rc) rc = scatter_floats(sc, numel, per_row ? topk : (int)numel, row_index, x_scales, st);
       }
     } else {
-      rc = scatter_rows(x, M, (int64_t)H * 2, topk, row_index, at(L.x_rows), st);
+      rc = scatter_rows(x, M, (int64_t)H * 2, topk, row_index, at(L.x_rows), early, st);
     }
     if (!rc && c.zero_pad)
       rc = zero_padding(tiles, L.tiles_cap, counts, (int64_t)H * (block ? 1 : 2), at(L.x_rows), block ? H / 128 : 0, L.rows_cap,
@@ -292,6 +294,6 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
     if (rc) return rc;
   }
   if (stages & 32)
-    rc = combine_rows(at(L.y), act_dtype, weight_on_input ? nullptr : topk_weights, row_index, M, topk, H, out, st);
+    rc = combine_rows(at(L.y), act_dtype, weight_on_input ? nullptr : topk_weights, row_index, M, topk, H, out, (stages & 16) != 0, st);
   return rc;
 }

@@ -353,13 +353,22 @@ __global__ void __launch_bounds__(256) rowwise_quant_kernel(const T* __restrict_
 // long rows) hold the row in registers (CH pieces of 8 elements each), so it is read once, with all loads in
 // flight, and written with 8-byte stores.  The kernel above reads every row twice, 64 bytes per warp and
 // instruction (500 x 2048 and 4000 x 768: 29 us for both).
-// SCATTER: row r goes to the rows `indirect`[r k + j], j < k (negative: none), its scale with it.
-template <typename T, int KIND, int TPR, int CH, bool SCATTER = false>
+// SCATTER: row r goes to the rows `indirect`[r k + j], j < k (negative: none), its scale with it.  EARLY (a CTA per row): the row
+// is read before the predecessor, which makes `indirect`, has ended (route_rows.cu says when that is allowed).
+template <typename T, int KIND, int TPR, int CH, bool SCATTER = false, bool EARLY = false>
 __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restrict__ x, int64_t rows, int cols,
                                                                 const float* __restrict__ scale_in,
                                                                 const int32_t* __restrict__ row_ids, int64_t valid_below,
                                                                 const int32_t* __restrict__ indirect,
                                                                 uint8_t* __restrict__ q, float* __restrict__ scale_out, int k = 1) {
+  static_assert(!EARLY || (SCATTER && TPR == 256), "early: one row per CTA");
+  uint4 raw[CH];
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if ((int)threadIdx.x + c * TPR < cols / 8)
+        raw[c] = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)blockIdx.x * cols) + threadIdx.x + c * TPR);
+  }
   pdl_wait();
   pdl_trigger();
   constexpr int RPC = 256 / TPR;  // rows per CTA
@@ -378,10 +387,11 @@ __global__ void __launch_bounds__(256) rowwise_quant_vec_kernel(const T* __restr
       if (lane < k) dst = indirect[idx * k + lane];
       if (__ballot_sync(0xFFFFFFFFu, dst >= 0) == 0) continue;  // no route of this token is local
     }
-    uint4 raw[CH];
+    if constexpr (!EARLY) {
 #pragma unroll
-    for (int c = 0; c < CH; ++c)
-      if (t + c * TPR < pieces) raw[c] = reinterpret_cast<const uint4*>(x + r * cols)[t + c * TPR];
+      for (int c = 0; c < CH; ++c)
+        if (t + c * TPR < pieces) raw[c] = reinterpret_cast<const uint4*>(x + r * cols)[t + c * TPR];
+    }
     float scale;
     if constexpr (KIND == 0 || KIND == 1) {
       float amax = 0.0f, nan_term = 0.0f;
@@ -578,19 +588,21 @@ bool rowwise_scatter_serves(int kind, int64_t cols) { return (kind == 0 || kind 
 
 template <typename T>
 static int rowwise_scatter_launch(const void* x, int64_t rows, int cols, int kind, int k, const int32_t* row_index, void* q,
-                                  float* scales, cudaStream_t st) {
-#define MOE_RS(K, CH)                                                                                                       \
-  launch_pdl(rowwise_quant_vec_kernel<T, K, 256, CH, true>, dim3((unsigned)rows), 256, 0, 1, st, "scatter (row quantised)", \
+                                  float* scales, bool early, cudaStream_t st) {
+#define MOE_RS_E(K, CH, E)                                                                                                     \
+  launch_pdl(rowwise_quant_vec_kernel<T, K, 256, CH, true, E>, dim3((unsigned)rows), 256, 0, 1, st, "scatter (row quantised)", \
              (const T*)x, rows, cols, (const float*)nullptr, (const int32_t*)nullptr, (int64_t)0, row_index, (uint8_t*)q, scales, k)
+#define MOE_RS(K, CH) (early ? MOE_RS_E(K, CH, true) : MOE_RS_E(K, CH, false))
   if (cols <= 2048) return kind == 0 ? MOE_RS(0, 1) : MOE_RS(1, 1);
   return kind == 0 ? MOE_RS(0, 4) : MOE_RS(1, 4);
 #undef MOE_RS
+#undef MOE_RS_E
 }
 
 int rowwise_scatter(const void* x, int x_dtype, int64_t rows, int64_t cols, int kind, int k, const int32_t* row_index, void* q,
-                    float* scales, cudaStream_t st) {
-  return x_dtype == MOE_BF16 ? rowwise_scatter_launch<__nv_bfloat16>(x, rows, (int)cols, kind, k, row_index, q, scales, st)
-                             : rowwise_scatter_launch<__half>(x, rows, (int)cols, kind, k, row_index, q, scales, st);
+                    float* scales, bool early, cudaStream_t st) {
+  return x_dtype == MOE_BF16 ? rowwise_scatter_launch<__nv_bfloat16>(x, rows, (int)cols, kind, k, row_index, q, scales, early, st)
+                             : rowwise_scatter_launch<__half>(x, rows, (int)cols, kind, k, row_index, q, scales, early, st);
 }
 }  // namespace moe
 

@@ -7,7 +7,7 @@
 //   combine   out[token] = sum over its routes, in slot order, of weight * y[row], fp32.
 // Bound: memory only where a launch is long; else the chain of a block (row index, rows, store) with too few bytes in flight.
 // DSV3 FP8, 8192 tokens: combine 179 us for 1.06 GB (5.9 TB/s; a copy runs at 6.5), clearing the padding 23 us, the
-// quantising scatter 125 us for 0.60 GB (4.8 TB/s, issue slots 65 % busy: its divisions).  Qwen3 shape, 4096 tokens, 151 MB
+// quantising scatter 125 us for 0.60 GB while it divided every element (issue slots 65 % busy).  Qwen3 shape, 4096 tokens, 151 MB
 // each: scatter 25 us, combine 29 us (5.2 TB/s; registers let 23 % of an SM's warps in, and 7 of 10 wait for a load).
 // 1024 tokens of DSV3 width: combine 29 us for 125 MB (4.3 TB/s).
 #include "moe_common.cuh"
@@ -49,20 +49,28 @@ __device__ __forceinline__ float div_by_scale(float v, float s, float inv) {
   return copysignf(fmaf(fmaf(-q, s, v), inv, q), v);
 }
 
+// EARLY (below): the token is read and quantised while the route plan is still being made.
 // Block (c, m): P x blockDim.x / 8 128-groups of token m, eight lanes per group, 16 elements per lane.  The bytes and scales
 // are those of the stand-alone quantiser (quant.cu).  With a division per element the kernel was bound by its instructions.
-template <typename T, int P>
+template <typename T, int P, bool EARLY>
 __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* __restrict__ x, int groups, int k,
                                                                        const int32_t* __restrict__ row_index,
                                                                        int64_t rows_cap, uint8_t* __restrict__ q,
                                                                        float* __restrict__ scales_t) {
-  pdl_wait();
-  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t m = blockIdx.y;
-  const int row = lane < k ? row_index[m * k + lane] : -1;
-  uint32_t rows = __ballot_sync(0xFFFFFFFFu, row >= 0);
-  if (rows == 0) return;  // no route of this token is local
+  int row = -1;
+  uint32_t rows = 0;
+  auto fetch_rows = [&] {
+    pdl_wait();
+    pdl_trigger();
+    if (lane < k) row = row_index[m * k + lane];
+    rows = __ballot_sync(0xFFFFFFFFu, row >= 0);
+  };
+  if constexpr (!EARLY) {
+    fetch_rows();
+    if (rows == 0) return;  // no route of this token is local
+  }
   const int64_t K = (int64_t)groups * 128;
   const int step = blockDim.x / 8;  // groups of one pass of the block
   const int g0 = blockIdx.x * P * step + (threadIdx.x >> 3);
@@ -72,8 +80,8 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
     raw[u][0] = raw[u][1] = make_uint4(0, 0, 0, 0);
     if (g0 + u * step < groups) {
       const uint4* src = reinterpret_cast<const uint4*>(x + m * K + (int64_t)(g0 + u * step) * 128 + (lane & 7) * 16);
-      raw[u][0] = src[0];
-      raw[u][1] = src[1];
+      raw[u][0] = EARLY ? __ldcg(src) : src[0];
+      raw[u][1] = EARLY ? __ldcg(src + 1) : src[1];
     }
   }
   uint4 packed[P];
@@ -106,6 +114,7 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
     packed[u] = make_uint4(w[0], w[1], w[2], w[3]);
     scale[u] = s;
   }
+  if constexpr (EARLY) fetch_rows();
   while (rows != 0) {
     const int64_t r = __shfl_sync(0xFFFFFFFFu, row, __ffs(rows) - 1);
     rows &= rows - 1;
@@ -121,17 +130,19 @@ __global__ void __launch_bounds__(kThreads) scatter_quant_group_kernel(const T* 
 }
 
 // Rows of `vec` 16-byte pieces copied as they are; block (c, m): 512 pieces of token m, two per thread.
+template <bool EARLY>
 __global__ void __launch_bounds__(kThreads) scatter_rows_kernel(const uint4* __restrict__ x, int vec, int k,
                                                                 const int32_t* __restrict__ row_index,
                                                                 uint4* __restrict__ out) {
-  pdl_wait();
-  pdl_trigger();
+  if constexpr (!EARLY) pdl_wait();
   const int64_t m = blockIdx.y;
   const int c = blockIdx.x * 2 * kThreads + threadIdx.x;
   uint4 v[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
-    if (c + i * kThreads < vec) v[i] = x[m * vec + c + i * kThreads];
+    if (c + i * kThreads < vec) v[i] = __ldcg(x + m * vec + c + i * kThreads);
+  if constexpr (EARLY) pdl_wait();
+  pdl_trigger();
   for (int j = 0; j < k; ++j) {
     const int64_t r = row_index[m * k + j];
     if (r < 0) continue;
@@ -154,17 +165,18 @@ __global__ void scatter_floats_kernel(const float* __restrict__ src, int64_t num
 
 // Block (c, m): blockDim x P 16-byte pieces of token m's output row, P per thread, P x U route rows in flight.  The slots
 // without a row are skipped before the loads, so a token with one local route of eight costs one round.
-template <typename T, bool WEIGHTED, int P, int U>
+template <typename T, bool WEIGHTED, int P, int U, bool EARLY>
 __global__ void __launch_bounds__(kThreads) combine_kernel(const T* __restrict__ y, const float* __restrict__ weight,
                                                            const int32_t* __restrict__ row_index, int k, int vec,
                                                            T* __restrict__ out) {
-  pdl_wait();
-  pdl_trigger();
+  if constexpr (!EARLY) pdl_wait();
   constexpr int V = 16 / sizeof(T);
   const int64_t m = blockIdx.y;
   const int lane = threadIdx.x & 31, c0 = blockIdx.x * P * blockDim.x + threadIdx.x;
-  const int row = lane < k ? row_index[m * k + lane] : -1;
-  const float wl = WEIGHTED && lane < k ? weight[m * k + lane] : 1.0f;
+  const int row = lane < k ? __ldcg(row_index + m * k + lane) : -1;
+  const float wl = WEIGHTED && lane < k ? __ldcg(weight + m * k + lane) : 1.0f;
+  if constexpr (EARLY) pdl_wait();
+  pdl_trigger();
   uint32_t left = __ballot_sync(0xFFFFFFFFu, row >= 0);
   float acc[P][V];
 #pragma unroll
@@ -213,6 +225,14 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const T* __restrict__
   }
 }
 
+// What a kernel may read before pdl_wait().  A kernel of the layer call starts when its predecessor has passed its own wait, so
+// what is older than the predecessor is complete: for the scatter behind the route plan the tokens, for the combine behind
+// GEMM2 the plan and the route weights.  All of it is read past L1.  `early` says that the predecessor is the one of the same
+// layer call; the scatters take it below four tokens per SM only: beyond, few blocks fit beside the plan, and a token without a
+// local route would be read for nothing.
+// us per call, before and with it: DSV3 FP8, 1 token 79.6, 78.6; Qwen3 e4m3 per channel, 500 tokens 135.9, 134.6; from a
+// few hundred us of weights on nothing either way.
+//
 // From four tokens per SM on, a block takes a whole row: its dependent chain (row index, rows, store) is walked once per
 // token instead of once per quarter of it (DSV3 FP8, one of 8 ranks, 2000 tokens: layer 308 -> 300 us; 8192 tokens: the
 // same).  Below, quarters spread a token over more SMs.
@@ -227,23 +247,26 @@ int zero_padding(const void* tiles, int64_t tiles_cap, const int32_t* counts, in
 }
 
 int scatter_quant_group(const void* x, int dtype, int64_t M, int H, int k, const int32_t* row_index, int64_t rows_cap, void* q,
-                        float* scales_t, cudaStream_t st) {
+                        float* scales_t, bool early, cudaStream_t st) {
   const int groups = H / 128;
   const bool whole = whole_rows(M);
   const int threads = whole ? kThreads : kThreads / 2, per_block = whole ? 64 : 16;
   const dim3 grid((unsigned)((groups + per_block - 1) / per_block), (unsigned)M);
-#define MOE_SCATTER(T, P)                                                                                                   \
-  launch_pdl(scatter_quant_group_kernel<T, P>, grid, threads, 0, 1, st, "scatter (1x128 quantised)", (const T*)x, groups, k, \
+#define MOE_SCATTER(T, P, E)                                                                                                   \
+  launch_pdl(scatter_quant_group_kernel<T, P, E>, grid, threads, 0, 1, st, "scatter (1x128 quantised)", (const T*)x, groups, k, \
              row_index, rows_cap, (uint8_t*)q, scales_t)
-  if (dtype == MOE_BF16) return whole ? MOE_SCATTER(__nv_bfloat16, 2) : MOE_SCATTER(__nv_bfloat16, 1);
-  return whole ? MOE_SCATTER(__half, 2) : MOE_SCATTER(__half, 1);
+#define MOE_SCATTER_T(T) (whole ? MOE_SCATTER(T, 2, false) : early ? MOE_SCATTER(T, 1, true) : MOE_SCATTER(T, 1, false))
+  return dtype == MOE_BF16 ? MOE_SCATTER_T(__nv_bfloat16) : MOE_SCATTER_T(__half);
+#undef MOE_SCATTER_T
 #undef MOE_SCATTER
 }
 
-int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, cudaStream_t st) {
+int scatter_rows(const void* x, int64_t M, int64_t row_bytes, int k, const int32_t* row_index, void* out, bool early,
+                 cudaStream_t st) {
   const int vec = (int)(row_bytes / 16);
-  return launch_pdl(scatter_rows_kernel, dim3((unsigned)((vec + 2 * kThreads - 1) / (2 * kThreads)), (unsigned)M), kThreads, 0, 1, st,
-                    "scatter", (const uint4*)x, vec, k, row_index, (uint4*)out);
+  const dim3 grid((unsigned)((vec + 2 * kThreads - 1) / (2 * kThreads)), (unsigned)M);
+  return launch_pdl(early ? scatter_rows_kernel<true> : scatter_rows_kernel<false>, grid, kThreads, 0, 1, st, "scatter",
+                    (const uint4*)x, vec, k, row_index, (uint4*)out);
 }
 
 int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_index, float* dst, cudaStream_t st) {
@@ -253,16 +276,18 @@ int scatter_floats(const float* src, int64_t numel, int div, const int32_t* row_
 }
 
 int combine_rows(const void* y, int dtype, const float* weight, const int32_t* row_index, int64_t M, int k, int64_t H, void* out,
-                 cudaStream_t st) {
+                 bool early, cudaStream_t st) {
   const int vec = (int)(H / 8);
   const int P = whole_rows(M) ? 4 : 1;
   // equal blocks of whole warps: H = 7168 is 4 x 224 pieces, not 3.5 x 256
   const int blocks = (vec + P * kThreads - 1) / (P * kThreads);
   const int threads = ((vec + P * blocks - 1) / (P * blocks) + 31) / 32 * 32;
   const dim3 grid((unsigned)blocks, (unsigned)M);
-#define MOE_COMBINE_P(T, W, P, U) \
-  launch_pdl(combine_kernel<T, W, P, U>, grid, threads, 0, 1, st, "combine", (const T*)y, weight, row_index, k, vec, (T*)out)
-#define MOE_COMBINE(T, W) (P == 4 ? MOE_COMBINE_P(T, W, 4, 4) : MOE_COMBINE_P(T, W, 1, 8))
+#define MOE_COMBINE_P(T, W, P, U, E) \
+  launch_pdl(combine_kernel<T, W, P, U, E>, grid, threads, 0, 1, st, "combine", (const T*)y, weight, row_index, k, vec, (T*)out)
+#define MOE_COMBINE(T, W)                                                                    \
+  (P == 4 ? (early ? MOE_COMBINE_P(T, W, 4, 4, true) : MOE_COMBINE_P(T, W, 4, 4, false))     \
+          : (early ? MOE_COMBINE_P(T, W, 1, 8, true) : MOE_COMBINE_P(T, W, 1, 8, false)))
   if (dtype == MOE_BF16) return weight != nullptr ? MOE_COMBINE(__nv_bfloat16, true) : MOE_COMBINE(__nv_bfloat16, false);
   return weight != nullptr ? MOE_COMBINE(__half, true) : MOE_COMBINE(__half, false);
 #undef MOE_COMBINE_P

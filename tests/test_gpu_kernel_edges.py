@@ -280,6 +280,46 @@ def test_sorted_ids_either_side_of_the_lane_masks(E, numel):
     _parity(out[rows], ref, (M, E))
 
 
+@pytest.mark.parametrize("M", [5, 591, 592])  # 148 multiprocessors: the last size that reads tokens early, the first that does not
+@pytest.mark.parametrize("fmt", ["half", "fp8_block", "fp8_channel"])
+def test_tokens_and_weights_written_right_before_the_layer(fmt, M):
+    """The scatter reads its tokens and the combine its plan and weights before their predecessors have ended.  Layers in place,
+    one behind the other, each on what the last one wrote, equal layers with a synchronisation between, bit for bit."""
+    E, k, H, I = 8, 2, 1024, 512
+    kw = {}
+    w1f, w2f = torch.randn(E, 2 * I, H, device=DEV) * 4 * H**-0.5, torch.randn(E, H, I, device=DEV) * 4 * I**-0.5
+    if fmt == "half":
+        w1, w2 = w1f.bfloat16(), w2f.bfloat16()
+    elif fmt == "fp8_block":
+        (w1, s1), (w2, s2) = (T.make_fp8_block_weights(E, n, kk, DEV, seed=n, std=4 * kk**-0.5) for n, kk in ((2 * I, H), (H, I)))
+        kw = dict(use_fp8_w8a8=True, block_shape=[128, 128], w1_scale=s1, w2_scale=s2)
+    else:
+        s1, s2 = w1f.abs().amax(-1) / 448.0, w2f.abs().amax(-1) / 448.0
+        w1, w2 = (w1f / s1[..., None]).to(torch.float8_e4m3fn), (w2f / s2[..., None]).to(torch.float8_e4m3fn)
+        kw = dict(use_fp8_w8a8=True, per_channel_quant=True, w1_scale=s1, w2_scale=s2)
+    routes = [_route(M, E, k, seed=i) for i in range(4)]
+    xs = [T.make_activations(M, H, DEV, seed=i) for i in range(8)]
+    want = []
+    for x in xs:
+        for tw, ti in routes:
+            torch.cuda.synchronize()
+            x = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+        want.append(x)
+    torch.cuda.synchronize()
+    x, tw, ti = torch.empty_like(xs[0]), torch.empty_like(routes[0][0]), torch.empty_like(routes[0][1])
+    got = []
+    for src in xs:
+        x.copy_(src)
+        for a, b in routes:
+            ti.copy_(b)
+            tw.copy_(a)
+            fg.fused_experts_impl(x, w1, w2, tw, ti, inplace=True, **kw)
+        got.append(x.clone())
+    assert _lib.read_status() == 0
+    for g, w in zip(got, want):
+        assert w.float().norm() > 0 and torch.equal(g, w)
+
+
 @pytest.mark.parametrize("limit", [1, 8])
 @pytest.mark.parametrize("numel", [0, 1, 2049, 4097, 16385, 65537, 262144])
 @pytest.mark.parametrize("E,bs", [(5, 16), (256, 128), (1024, 7)])
