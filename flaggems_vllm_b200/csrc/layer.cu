@@ -69,14 +69,17 @@ bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
 
 // The split-K weight streaming of gemm_small.cu: three launches instead of five, every SM busy however few tiles there
 // are, but one CTA needs more instructions per byte than the pair.  So it is for the calls whose launches count: up to four
-// routes and 200 MB of weights if no two share an expert, which the host cannot see.  us per layer (graph replay), bf16,
-// split K against the pair in tiles of 64:
-//   E8 H1024 I2048    1 token (25 MB, 2 routes) 17.5 : 19.9    2 tokens (50 MB) 21.0 : 22.6    3 tokens (6 routes) 28.9 : 25.7
-//   E8 H2048 I4096    1 token (101 MB, 2 routes) 29.9 : 34.7   2 tokens (201 MB) 43.1 : 43.5   4 tokens (8 routes) 78.6 : 61.8
-//   E128 H2048 I768   1 token (75 MB, 8 routes) 29.1 : 28.7    E64 H2048 I1408  1 token (104 MB, 6 routes) 33.5 : 31.7
+// routes and 210 MB of weights if no two share an expert, which the host cannot see, and up to eight routes and 102 MB.  bf16,
+// split K against the pair in tiles of 64, us per layer under graph replay, and in brackets per call, where the host's five
+// launches (about 31 us) are a floor for the pair:
+//   E8 H1024 I2048    1 token (25 MB, 2 routes) 17.5 : 19.9    2 tokens (50 MB) 21.0 : 22.6
+//                     3 tokens (75 MB, 6 routes) 28.9 : 25.7 (30.2 : 31.7)    4 tokens (101 MB, 8 routes) (29.4 : 31.5)
+//   E8 H2048 I4096    1 token (101 MB, 2 routes) 29.9 : 34.7   2 tokens (201 MB, 4 routes) 43.1 : 43.5 (44.8 : 45.7)
+//                     3 tokens (302 MB, 6 routes) (60.0 : 55.6)   4 tokens (403 MB, 8 routes) 78.6 : 61.8 (73.3 : 61.4)
+//   E128 H2048 I768   1 token (75 MB, 8 routes) 29.1 : 28.7 (30.2 : 31.3)
+//   E64 H2048 I1408   1 token (104 MB, 6 routes) 33.5 : 31.7 (34.7 : 33.2)
 //   E16 H5120 I8192   1 token (252 MB, 1 route) 59.5 : 58.2    Mixtral shape    1 token (705 MB, 2 routes) 141.1 : 127.2
-constexpr int kSmallRoutes = 4;
-constexpr int64_t kSmallBytes = 200000000;
+constexpr int64_t kSmallBytes4 = 210000000, kSmallBytes8 = 102000000;
 
 bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
 
@@ -91,7 +94,7 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
     c.tile = w8t_tile(c.wide);
     return c;
   }
-  if (mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && numel <= kSmallRoutes && numel * 6 * H * I <= kSmallBytes &&
+  if (mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && numel <= 8 && numel * 6 * H * I <= (numel <= 4 ? kSmallBytes4 : kSmallBytes8) &&
       H % 128 == 0 && I % 64 == 0) {
     c.small = true;
     return c;
