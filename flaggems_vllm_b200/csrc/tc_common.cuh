@@ -98,8 +98,7 @@ __device__ __forceinline__ bool wait_expired(unsigned long long& t0, int32_t* st
   return true;
 }
 // Start of the operand rings: the first 1024-byte boundary of the dynamic shared memory.  An offset from the array, not a
-// pointer made from an integer: the compiler keeps knowing that it is shared memory (LDS and constant addresses; with
-// generic pointers the FP8 GEMM1 loop had 16 generic loads and 24 reads of the window base per K block).
+// pointer made from an integer: the compiler keeps knowing that it is shared memory.
 __device__ __forceinline__ uint8_t* align_1024(uint8_t* smem_raw) {
   return smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
 }
