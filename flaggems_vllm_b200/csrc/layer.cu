@@ -68,18 +68,18 @@ bool sizes_served(int mode, int act_dtype, int H, int I, int act_kind) {
 }
 
 // The split-K weight streaming of gemm_small.cu: three launches instead of five, every SM busy however few tiles there
-// are, but one CTA needs more instructions per byte than the pair.  So it is for the calls whose launches count: up to four
-// routes and 210 MB of weights if no two share an expert, which the host cannot see, and up to eight routes and 102 MB.  bf16,
-// split K against the pair in tiles of 64, us per layer under graph replay, and in brackets per call, where the host's five
-// launches (about 31 us) are a floor for the pair:
-//   E8 H1024 I2048    1 token (25 MB, 2 routes) 17.5 : 19.9    2 tokens (50 MB) 21.0 : 22.6
-//                     3 tokens (75 MB, 6 routes) 28.9 : 25.7 (30.2 : 31.7)    4 tokens (101 MB, 8 routes) (29.4 : 31.5)
-//   E8 H2048 I4096    1 token (101 MB, 2 routes) 29.9 : 34.7   2 tokens (201 MB, 4 routes) 43.1 : 43.5 (44.8 : 45.7)
-//                     3 tokens (302 MB, 6 routes) (60.0 : 55.6)   4 tokens (403 MB, 8 routes) 78.6 : 61.8 (73.3 : 61.4)
-//   E128 H2048 I768   1 token (75 MB, 8 routes) 29.1 : 28.7 (30.2 : 31.3)
-//   E64 H2048 I1408   1 token (104 MB, 6 routes) 33.5 : 31.7 (34.7 : 33.2)
-//   E16 H5120 I8192   1 token (252 MB, 1 route) 59.5 : 58.2    Mixtral shape    1 token (705 MB, 2 routes) 141.1 : 127.2
-constexpr int64_t kSmallBytes4 = 210000000, kSmallBytes8 = 102000000;
+// are, but one CTA needs more instructions per byte than the pair.  It serves up to 8 routes that read up to 1 GB of weights if
+// no two share an expert, which the host cannot see.  us per layer, bf16, split K against the pair in tiles of 64:
+//   Mixtral shape    1 token  0.7 GB  137 : 127   2 tokens 1.4 GB  256 : 253 (against tokens as M; one pair of experts 143 : 168)
+//   E8 H1024 I2048   1 token   25 MB   17 : 20    2 tokens          21 : 23    3 tokens 29 : 26    4 tokens 27 : 30
+//   E8 H2048 I4096   1 token  101 MB   30 : 35    2 tokens 201 MB   43 : 44    4 tokens 403 MB     79 : 62
+//   E128 H2048 I768  1 token   75 MB   29 : 29    E64 H2048 I1408   1 token 104 MB 34 : 32
+// The times cross between 100 MB and 0.7 GB, but the line is not drawn there: the results are not the same.  Here the K slices' sums
+// are added in fp32 and the activation is expf and a true division; the pair accumulates all of K in tensor memory and takes
+// the fast exponential (Mixtral shape, one token: outputs up to 3.4e-3 apart).  Up to 1 GB a call keeps the former; beyond,
+// distinct experts, the usual case, lose more than that is worth.
+constexpr int kSmallRoutes = 8;
+constexpr int64_t kSmallBytes = 1000000000;
 
 bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
 
@@ -94,7 +94,7 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
     c.tile = w8t_tile(c.wide);
     return c;
   }
-  if (mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && numel <= 8 && numel * 6 * H * I <= (numel <= 4 ? kSmallBytes4 : kSmallBytes8) &&
+  if (mode == MOE_MODE_HALF && act_kind == MOE_ACT_SILU && numel <= kSmallRoutes && numel * 6 * H * I <= kSmallBytes &&
       H % 128 == 0 && I % 64 == 0) {
     c.small = true;
     return c;

@@ -279,3 +279,20 @@ def test_layer_call_serves_what_its_declaration_says(tokens, topk, experts, serv
         rc = _lib.lib().moe_layer_workspace(mode, _lib.MOE_BF16, tokens, topk, experts, experts, 256, 128, _lib.ACT_SILU,
                                             ctypes.addressof(need))
         assert (rc == 0) == served
+
+
+def _layer_pieces(mode, tokens, topk, E, H, I, act=_lib.ACT_SILU):
+    need, table = (ctypes.c_int64 * 4)(), (ctypes.c_int64 * 39)()
+    _lib.check(_lib.lib().moe_layer_layout(mode, _lib.MOE_BF16, tokens, topk, E, E, H, I, act, ctypes.addressof(need),
+                                           ctypes.addressof(table)))
+    return [table[i + 2] for i in range(0, 39, 3)]
+
+
+@pytest.mark.parametrize("tokens,topk,E,H,I,split", [
+    (1, 2, 8, 4096, 14336, True), (2, 2, 8, 4096, 14336, False),                                   # 0.70 GB, 1.41 GB
+    (1, 1, 16, 5120, 8192, True), (3, 1, 16, 5120, 8192, True), (4, 1, 16, 5120, 8192, False),     # 0.25, 0.75, 1.01 GB
+    (1, 6, 64, 2048, 1408, True), (3, 2, 8, 2048, 4096, True), (4, 2, 8, 2048, 4096, True),
+    (8, 1, 8, 256, 128, True), (9, 1, 8, 256, 128, False), (1, 8, 128, 2048, 768, True)])
+def test_few_routes_of_half_precision_keep_k_slices_summed_in_fp32(tokens, topk, E, H, I, split):
+    """Up to eight routes and 1 GB of weights: the schedule that adds its K slices' sums in fp32 (only it has counters)."""
+    assert (_layer_pieces(_lib.MODE_HALF, tokens, topk, E, H, I)[12] > 0) == split
