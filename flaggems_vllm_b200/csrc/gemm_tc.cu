@@ -673,8 +673,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
     };
+    // Staged output: the warps meet twice per tile around the staging buffer, also a warp whose wait has timed out.
+    [[maybe_unused]] auto meet = [&] { asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory"); };
     if constexpr (!BY_EXPERT) prefetch_tile(tile0);
-    for (int tile = tile0; tile < total_tiles && alive; tile += tile_step) {
+    for (int tile = tile0; tile < total_tiles && (alive || TMAOUT); tile += tile_step) {
       int blk = nx_blk, nt = nx_nt, e = nx_e;
       [[maybe_unused]] int occupied = 0;
       if constexpr (BY_EXPERT) {
@@ -687,6 +689,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (!FP8 || e < 0 || e >= P.E) prefetch_tile(tile + tile_step);  // half precision has no K loop here
       }
       if (e < 0 || e >= P.E) continue;
+      if constexpr (TMAOUT) {
+        if (!alive) {
+          if constexpr (FP8 && !BY_EXPERT) prefetch_tile(tile + tile_step);
+          meet();
+          meet();
+          continue;
+        }
+      }
       for (int sub = 0; sub < RB && alive; ++sub) {  // the 128-row blocks of this tile (two for wide tiles)
       const int64_t p = (int64_t)(mb + sub) * BM + row;
       int64_t sid = P.numel;
@@ -725,9 +735,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         };
         if constexpr (!BY_EXPERT) prefetch_tile(tile + tile_step);
         if (P.mul_weight && row_ok) rw = P.route_weight[sid];
-        alive = mbar_wait_at(acc_full, acc_ph, P.status, P.wait_ns);
-        if (!alive) break;
-        __syncwarp();
+        if (!warp_agrees(mbar_wait_at(acc_full, acc_ph, P.status, P.wait_ns))) {
+          alive = false;
+          if constexpr (TMAOUT) { meet(); meet(); }
+          break;
+        }
+        __syncwarp();  // without it the compiler spills registers
         tc_fence_after();
         next_scales();
 #pragma unroll 1
@@ -756,9 +769,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma2(acc2[32 + i], ra[2 * i], ra[2 * i + 1], hi2);
           if (left > 1) {
-            if (!__all_sync(0xFFFFFFFFu, ready)) {
+            if (!warp_agrees(ready)) {
               ready = mbar_wait_at(acc_full, acc_ph, P.status, P.wait_ns);
-              if (!__all_sync(0xFFFFFFFFu, ready)) { alive = false; break; }
+              if (!warp_agrees(ready)) { alive = false; break; }
             }
             tc_fence_after();
             next_scales();
@@ -766,7 +779,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 16; ++i) fma2(acc2[48 + i], rb[2 * i], rb[2 * i + 1], hi2);
         }
-        if (!alive) break;
+        if (!alive) {
+          if constexpr (TMAOUT) { meet(); meet(); }
+          break;
+        }
       } else {
         const uint32_t a = RB == 2 ? 0u : (acc_it & 1);
         const uint32_t aph = RB == 2 ? (acc_it & 1) : ((acc_it >> 1) & 1);
@@ -775,7 +791,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (row_ok) as = GEMM1 ? P.a_scales_t[sid / P.topk] : P.a_scales_t[p];
         }
         if (sub == 0) {
-          if (!mbar_wait(&aux->tmem_full[a], aph, P.status, P.wait_ns)) { alive = false; break; }
+          if (!warp_agrees(mbar_wait(&aux->tmem_full[a], aph, P.status, P.wait_ns))) {
+            alive = false;
+            if constexpr (TMAOUT) { meet(); meet(); }
+            break;
+          }
           tc_fence_after();
         }
         const uint32_t t0 = t_lane + (RB == 2 ? (uint32_t)sub : a) * BN;
@@ -838,7 +858,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           float* x = &aux->xch[tile_it & 1][0][0];
           x[h * BM + row] = amax;
           mbar_arrive(&aux->xch_bar);
-          if (!mbar_wait(&aux->xch_bar, tile_it & 1, P.status, P.wait_ns)) { alive = false; break; }
+          if (!warp_agrees(mbar_wait(&aux->xch_bar, tile_it & 1, P.status, P.wait_ns))) { alive = false; break; }
           amax = fmaxf(amax, x[(1 - h) * BM + row]);
           const float s = fmaxf(amax, kQuantEps) * (1.0f / kFp8Max);
           const float inv_s = 1.0f / s;  // one reciprocal per row instead of 64 divisions
@@ -873,7 +893,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       } else if constexpr (TMAOUT) {
         // the previous tile's bulk stores have finished reading the staging buffer
         if (threadIdx.x == 128) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory");
+        meet();
 #pragma unroll
         for (int c = 0; c < 16; ++c) {  // 16-byte chunk c of this thread's 128 columns -> sub-tile 2h + c/8, chunk c%8
           const uint4 piece = make_uint4(pack2<AT>(acc[c * 8 + 0] * rw, acc[c * 8 + 1] * rw),
@@ -885,7 +905,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         if (row_ok && h == 0 && P.inv != nullptr) P.inv[sid] = (int32_t)p;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> TMA reads
-        asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory");
+        meet();
         if (threadIdx.x == 128) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {

@@ -311,7 +311,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       if (!alive) continue;
       const uint32_t a = acc_it & 1;
-      if (!mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) { alive = false; continue; }
+      if (!warp_agrees(mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns))) { alive = false; continue; }
       tc_fence_after();
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
@@ -380,8 +380,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (e < 0 || e >= P.E) continue;
       for (int kb = 0; kb < KB; ++kb, ++it) {
         const int sr = it % SR, sb = it % SB;
-        if (!mbar_wait(&aux->r_full[sr], (it / SR) & 1, P.status, P.wait_ns)) { alive = false; break; }
-        if (!mbar_wait(&aux->b_empty[sb], ((it / SB) & 1) ^ 1, P.status, P.wait_ns)) { alive = false; break; }
+        if (!warp_agrees(mbar_wait(&aux->r_full[sr], (it / SR) & 1, P.status, P.wait_ns))) { alive = false; break; }
+        if (!warp_agrees(mbar_wait(&aux->b_empty[sb], ((it / SB) & 1) ^ 1, P.status, P.wait_ns))) { alive = false; break; }
         const uint8_t* raw = sR + (size_t)sr * RAW_BYTES;
         uint8_t* dst = sB + (size_t)sb * B_BYTES;
         // 1024 chunks of 16 int8; chunk q = 16 K elements (q & 3) of weight row q >> 2.  A warp

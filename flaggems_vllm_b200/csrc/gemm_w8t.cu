@@ -244,7 +244,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       const Item it = nx;
       if (item + step < total) nx = fetch(item + step);
       const uint32_t a = acc_it & 1;
-      if (!mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) break;
+      if (!warp_agrees(mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns))) break;
       tc_fence_after();
       drain_tile<FMT_W8, AT, GEMM1, true, 1, 1, OUT_TOKENS>(P, it, 0, t_lane + a * C::TILE, 0, wq, lane, out_base, [&] {
         tc_fence_before();
@@ -263,7 +263,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int64_t blocks = (int64_t)tiles * KB;
     uint32_t rs = grp, rph = 0, s = grp, ph = 1;
     for (int64_t j = grp; j < blocks; j += GROUPS) {
-      if (!mbar_wait_at(smem_u32(&aux->r_full[rs]), rph, P.status, P.wait_ns)) break;
+      if (!warp_agrees(mbar_wait_at(smem_u32(&aux->r_full[rs]), rph, P.status, P.wait_ns))) break;
       const uint8_t* src = smem + (size_t)rs * RAW_BYTES + row * 128;
       const uint32_t ta = t_lane + s * C::A_COLS;
       bool ok = true;
@@ -283,7 +283,7 @@ w8t_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         if (half == 0) {
           // the buffer's last MMA is over (the wait comes after the first half is widened)
-          ok = mbar_wait_at(smem_u32(&aux->done[s]), ph, P.status, P.wait_ns);
+          ok = warp_agrees(mbar_wait_at(smem_u32(&aux->done[s]), ph, P.status, P.wait_ns));
           if (!ok) break;
           tc_fence_after();
         }

@@ -217,7 +217,7 @@ wt_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       if (item + step < total) nx = fetch(item + step);
       const uint32_t a = acc_it & 1;
       asm volatile("bar.sync 2, %0;" ::"n"(CONS_THREADS) : "memory");  // the staging tile has been read
-      if (alive && !mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns)) alive = false;
+      if (alive) alive = warp_agrees(mbar_wait_idle(&aux->tmem_full[a], (acc_it >> 1) & 1, P.status, P.wait_ns));
       if (alive) {
         tc_fence_after();
         drain_tile<FMT, AT, GEMM1, SILU, 2, 2, 0>(P, it, cr, t_lane + a * NTOK, h, wq, lane, out_base, [&] { release_acc(a); });

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(RTHREADS, 1) router_tc_kernel(const __grid_con
     if (leader) tc_commit(&aux->done);
   } else {
     // every MMA has finished reading the ring: it now holds the partial tile
-    const bool ok = mbar_wait(&aux->done, 0, status, wait_ns);
+    const bool ok = warp_agrees(mbar_wait(&aux->done, 0, status, wait_ns));
     tc_fence_after();
     const int row = ((warp & 3) << 5) + lane;
     const uint32_t t0 = tmem + ((uint32_t)((warp & 3) << 5) << 16);

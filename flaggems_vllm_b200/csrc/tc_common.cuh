@@ -150,6 +150,10 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
   asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(addr), "n"(OFFSET) : "memory");
   return v;
 }
+// The answer of a wait for the whole warp.  A wait gives up by the clock, which lanes may read on either side of the limit: what
+// the warp does as one behind it (tensor memory loads and stores, mma.sync, __syncwarp, named barriers) has to see one answer.
+// All lanes call it.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xFFFFFFFFu, ok); }
 // The same bounded wait for warps that expect to wait long (an epilogue warp waiting for a
 // whole K loop): they sleep between probes, so their polling does not take issue slots from
 // the warps that feed the tensor core.

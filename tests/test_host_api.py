@@ -296,3 +296,25 @@ def _layer_pieces(mode, tokens, topk, E, H, I, act=_lib.ACT_SILU):
 def test_few_routes_of_half_precision_keep_k_slices_summed_in_fp32(tokens, topk, E, H, I, split):
     """Up to eight routes and 1 GB of weights: the schedule that adds its K slices' sums in fp32 (only it has counters)."""
     assert (_layer_pieces(_lib.MODE_HALF, tokens, topk, E, H, I)[12] > 0) == split
+
+
+def test_warps_agree_on_a_wait_before_they_act_as_one():
+    """A bounded wait gives up by the clock, and lanes may read it on either side of the limit.  Where a warp goes on with
+    instructions that it executes as one (tensor memory, mma.sync, barriers), the lanes vote on the answer first."""
+    csrc = os.path.join(ROOT, "flaggems_vllm_b200", "csrc")
+    # barriers that consumers, converters and epilogues wait for; the issuing warps wait for others
+    waits = {"gemm_tc.cu": ("tmem_full", "acc_full", "xch_bar"), "gemm_wt.cu": ("tmem_full",), "gemm_w8t.cu": ("tmem_full", "r_full", r"done\[s\]\), ph,"),
+             "gemm_w8.cu": ("tmem_full", "r_full", "b_empty"), "router_gemm.cu": ("done",)}
+    for name, barriers in waits.items():
+        lines = open(os.path.join(csrc, name)).read().split("\n")
+        for barrier in barriers:
+            found = [i for i, line in enumerate(lines) if re.search(r"mbar_wait\w*(<\w+>)?\([^;]*\b" + barrier, line)]
+            assert found, (name, barrier)
+            for i in found:
+                voted = "warp_agrees(mbar_wait" in lines[i] or "warp_agrees(ready)" in lines[i + 1]
+                assert voted, f"{name}:{i + 1}: {lines[i].strip()}"
+    # a warp that has given up still meets the others at the named barriers of the tiles and units that are left; the split-K
+    # kernel's lanes go on without waiting
+    tc, small = (open(os.path.join(csrc, n)).read() for n in ("gemm_tc.cu", "gemm_small.cu"))
+    assert "(alive || TMAOUT); tile += tile_step" in tc and "for (int u = u_begin; u < u_end; ++u)" in small
+    assert "if (alive) alive = mbar_wait(&aux->full[st]" in small
