@@ -45,6 +45,8 @@
 //
 // Every barrier wait is bounded (wall-clock limit); on expiry the kernel sets
 // MOE_ST_WAIT_TIMEOUT, leaves its loops, frees TMEM and returns.
+#include <algorithm>
+
 #include "tc_common.cuh"
 
 namespace moe {
@@ -136,7 +138,7 @@ struct Params {
   int Nout;     // output columns (I for GEMM1, H for GEMM2)
   int rows_w;   // weight rows per expert (2I or H)
   int n_tiles;  // column tiles per align block
-  int group_m;  // align blocks per group of the tile order
+  int group_m;  // align blocks per group of the tile order; BY_EXPERT: most blocks of an expert in a group
   int w_row0;   // GEMM2 over a window of the output columns: first weight row (output column) of the window
   bool wide_store;  // the output is 32-byte aligned: rows are written with 32-byte stores
 };
@@ -202,7 +204,8 @@ __device__ __forceinline__ int box_row(int nt, int c, int cr, int Nout) {
 //
 // BY_EXPERT (route plan, whole blocks): the blocks of an expert, which the plan knows, share its column tiles in the tile order.
 // Fixed groups of blocks start somewhere inside an expert and read its weights once per group: DSV3 FP8, 8192 tokens, the
-// layer 4799 -> 4719 us.  With few rows per expert the order is the same and the plan entries cost up to 1 %.
+// layer 4799 -> 4719 us.  With few rows per expert the order is the same and the plan entries cost up to 1 %.  At most `group_m`
+// blocks make a pass over the column tiles together: their rows are read again for every column tile and have to stay in L2.
 //
 // Row-scaled formats (FMT_FP8ROW, FMT_I8ROW): one-byte operands like the block-scaled mode, but
 // nothing has to happen between K blocks, so the whole K loop accumulates in TMEM like half
@@ -266,6 +269,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   [[maybe_unused]] auto look_ahead = [&](int tile) {
     if (tile < total_tiles) ahead = __ldcg(reinterpret_cast<const int2*>(P.tiles + tile / P.n_tiles) + 1);
   };
+  // tile of the expert whose plan entry is `ahead`: its blocks in as few groups of up to group_m as hold them, of one size
+  [[maybe_unused]] auto expert_tile = [&](int tile, int& blk, int& nt) {
+    int first = ahead.y & 0xFFFF, blocks = (int)((uint32_t)ahead.y >> 16), within = tile - first * P.n_tiles;
+    if (blocks > P.group_m) {
+      const int parts = (blocks + P.group_m - 1) / P.group_m, size = (blocks + parts - 1) / parts;
+      const int part = within / (size * P.n_tiles);
+      first += part * size;
+      within -= part * size * P.n_tiles;
+      blocks = min(blocks - part * size, size);
+    }
+    nt = within / blocks;
+    blk = first + within - nt * blocks;
+  };
   // tile -> expert_ids index (blk), this CTA's 128-row block (mb), column tile (nt).  The expert of
   // the NEXT tile is fetched while the current one is worked on: a tile starts without waiting
   // for a global load (every role walks the same tile list with its own copy of e_next).
@@ -279,10 +295,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   auto coords = [&](int tile, int& blk, int& nt) -> int {
     if constexpr (BY_EXPERT) {
-      const int first = ahead.y & 0xFFFF, blocks = (int)((uint32_t)ahead.y >> 16), within = tile - first * P.n_tiles;
       const int e = ahead.x;
-      nt = within / blocks;
-      blk = first + within - nt * blocks;
+      expert_tile(tile, blk, nt);
       look_ahead(tile + tile_step);
       return e;
     } else {
@@ -374,9 +388,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (P.tiles != nullptr && tile0 < total_tiles) {
           int blk, nt, e0;
           if constexpr (BY_EXPERT) {  // as coords(), which moves on
-            const int first = ahead.y & 0xFFFF, blocks = (int)((uint32_t)ahead.y >> 16), within = tile0 - first * P.n_tiles;
-            nt = within / blocks;
-            blk = first + within - nt * blocks;
+            expert_tile(tile0, blk, nt);
             e0 = ahead.x;
           } else {
             tile_blk_nt(tile0, blk, nt);
@@ -1162,8 +1174,12 @@ int tc_gemm_plan(bool gemm1, int act_dtype, const void* a, const float* a_scales
   P.num_post_pad = rows; P.out = out; P.out_scales_t = out_scales_t; P.status = status; P.wait_ns = wait_limit_ns();
   P.numel = rows_cap; P.rows_cap = rows_cap; P.E = E; P.K = K; P.Nout = Nout; P.rows_w = rows_w;
   P.n_tiles = gemm1 ? Nout / 128 : (Nout + BN - 1) / BN;
+  // Blocks that share a pass over the column tiles.  Whole blocks: 16 MB of rows (18 blocks at K = 7168, 64 at 2048).  K 7168,
+  // I 2048, us per layer, groups of 16 across experts / 16 MB / 32 / 64 / an expert's blocks all together: 128 blocks per expert (4
+  // experts) 3545 / 3297 / 3425 / 3537 / 3878, 96 blocks 2619 / 2475 / 2462 / 2560 / 2843, 64 blocks 1813 / 1660 / 1691 / 1699 / 1741;
+  // 32 experts, half of the routes on four of them (128 blocks each) 6864 / 6388 / 6585 / 6639 / 6951.
   const int64_t gm = numel / E / BM + 1;
-  P.group_m = (int)(gm > 16 ? 16 : gm);
+  P.group_m = all_rows ? std::max(16, (16 << 20) / (BM * K)) : (int)(gm > 16 ? 16 : gm);
   P.wide_store = ((uintptr_t)out & 31) == 0;
   const int64_t cap_tiles = (rows_cap / BM) * (int64_t)P.n_tiles;
   const int sms = sm_count();

@@ -418,3 +418,22 @@ def test_expert_map_shorter_than_the_expert_count(M, staged, monkeypatch):
     out = fg.fused_experts_impl(x, w1[order].contiguous(), w2[order].contiguous(), tw, ti, global_num_experts=E, expert_map=emap)
     _parity(out, ref, M)
     assert bool((out[~keep.any(1)] == 0).all())
+
+
+def test_fp8_expert_of_more_blocks_than_a_group_of_the_tile_order():
+    """K = 7168: 18 blocks of 128 rows share a pass over the column tiles.  Experts of 41 (three groups of 14, 14, 13), 19 (10 and
+    9), 18, one and no blocks; rows do not depend on the order, bit for bit."""
+    counts, H, I = (41 * 128 - 5, 18 * 128 + 1, 18 * 128, 3, 0), 7168, 256
+    ids = torch.cat([torch.full((n,), e, dtype=torch.int32, device=DEV) for e, n in enumerate(counts)])
+    ids = ids[torch.randperm(ids.numel(), generator=torch.Generator().manual_seed(3)).to(DEV)][:, None].contiguous()
+    M, E = ids.shape[0], len(counts)
+    x = T.make_activations(M, H, DEV, seed=4)
+    tw = torch.rand((M, 1), device=DEV) + 0.5
+    w1, s1 = T.make_fp8_block_weights(E, 2 * I, H, DEV, seed=1)
+    w2, s2 = T.make_fp8_block_weights(E, H, I, DEV, seed=2)
+    kw = dict(use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
+    out = fg.fused_experts_impl(x, w1, w2, tw, ids, **kw)
+    _parity(out, O.fused_moe_fp8_block_oracle(x, w1, w2, s1, s2, tw, ids), counts)
+    for m0 in range(0, M, 2000):  # at most nine blocks per expert
+        part = slice(m0, m0 + 2000)
+        assert torch.equal(fg.fused_experts_impl(x[part], w1, w2, tw[part], ids[part], **kw), out[part])
