@@ -83,12 +83,42 @@ constexpr int64_t kSmallBytes = 1000000000;
 
 bool row_mode(int mode) { return mode == MOE_MODE_FP8_ROW || mode == MOE_MODE_INT8_ROW; }
 
-Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
+// Most rows of a pair's tile.  Small tiles leave shared memory to the ring and stream an even load's weights fastest; an expert
+// with more rows than a tile reads its weights once more per tile, while HBM idles.  The host sees the mean load only (and that
+// no expert has more rows than there are tokens), so the lines lie where skewed routing is no slower than under the
+// schedule that was there before either tile: half precision tokens as M below 96 rows per expert and 256 from there on, else 256.
+// us per layer (graph replay); even: uniform routing, zipf: popularity 1 / rank, hot: every token takes expert 0:
+//   bf16 E8 k2 H4096 I14336      before    64    128    256          bf16 E64 k6 H2048 I1408   before    64    128    256
+//     112 tokens (28 rows) even     455   428    437    475            200 tokens (18)  zipf      189   190    183    192
+//                          hot      462   434    440    476            400 (37)         zipf      201   201    193    199
+//     150 (37)             even     457   430    442    478            600 (56)         zipf      209   219    201    207
+//                          hot      469   474    448    482            900 (84)         zipf      238   248    217    220
+//     232 (58)             even     464   471    447    486            1200 (112)       even      227   246    213    220
+//                          hot      477   522    455    499                             zipf      240   284    245    234
+//     350 (87)             even     483   527    457    493
+//                          zipf     640   590    520    504          e4m3, E128 k8 H2048 I768
+//     400 (100)            even     519   539    465    509            1000 (62)        even      153          146    148
+//                          hot      548   634    558    514                             zipf      158          153    152
+//     440 (110)            even     522   548    472    509            1500 (93)        even      171          165    165
+//                          hot      538   592    571    541                             zipf      178          179    172
+//     480 (120)            zipf     528   622    542    527            1900 (118)       hot4      200          197    192
+// The other activation has GEMM1 in tiles of 256 only, so half of the gain: bf16 232 tokens even 497 / 522 / 461 / 481 and hot 510 / 528 /
+// 471 / 494, 300 tokens hot 517 / 572 / 547 / 506; int8 rows 256 is ahead from 31 rows per expert on (142 / - / 140 / 138).
+int pair_tile(int mode, int act_kind, int64_t M, int64_t per_expert) {
+  const bool half = mode == MOE_MODE_HALF;
+  if (act_kind != MOE_ACT_SILU) return half && per_expert <= 64 ? 128 : 256;
+  if (half) return M <= 128 && per_expert <= 32 ? 64 : (per_expert <= 100 ? 128 : 256);
+  return per_expert <= 64 ? 128 : 256;
+}
+
+Choice choose(int mode, int act_kind, int64_t M, int topk, int E, int H, int I) {
+  const int64_t numel = M * topk;
   const int64_t per_expert = numel / (E > 0 ? E : 1);
   Choice c = {};
   if (mode == MOE_MODE_W8A16) {
     // Qwen3 shape, GEMM1 + GEMM2 in us, narrow (more stages) against wide: 40 rows per expert 128 : 139, 50 rows 133 : 140,
-    // 62 rows 170 : 153 (every second expert has more than 64 rows: two tiles)
+    // 62 rows 170 : 153 (every second expert has more than 64 rows: two tiles).  Half of the routes on four experts, 51 rows: the
+    // layer 173 us, 190 when it was wide from 40 rows on.
     c.wide = per_expert > 52;
     c.gran = 16;
     c.tile = w8t_tile(c.wide);
@@ -99,15 +129,11 @@ Choice choose(int mode, int act_kind, int64_t numel, int E, int H, int I) {
     c.small = true;
     return c;
   }
-  // FP8 block scales: tokens as M (gemm_wt.cu says why).  All else: the pair, in tiles whose kernel has the deepest ring that still
-  // holds an expert's rows.  us per layer, Mixtral shape, bf16, tokens as M (before) / pair in tiles of 64 / 128 / 256:
-  //   rows per expert   5: 449 / 429 / 436 / 473    37: 465 / 440 / 447 / 484    57: 467 / 448 / 453 / 490    65: 480 / 485 / 458 / 494
-  //                    75: 485 / 558 / 459 / 499   105: 516 / 593 / 473 / 515   120: 543 / 617 / 515 / 519   140: 557 / 771 / 624 / 532
-  // e4m3 per channel, Qwen3 shape, 64 / 128 / 256: 31 rows per expert 136 / 135 / 139, 62 rows 159 / 155 / 158, 100 rows 197 / 177 / 177
+  // FP8 block scales: tokens as M (gemm_wt.cu says why).  All else: the pair, in tiles of pair_tile() rows.
   c.pair = mode != MOE_MODE_FP8_BLOCK;
   if (c.pair) {
     c.gran = mode == MOE_MODE_INT8_ROW ? 32 : 16;  // kind::i8 on a pair takes multiples of 32
-    c.tile = mode == MOE_MODE_HALF && per_expert <= 58 ? 64 : (per_expert <= 120 ? 128 : 256);
+    c.tile = pair_tile(mode, act_kind, M, per_expert);
   } else {
     c.gran = c.tile = 128;
     c.zero_pad = per_expert >= 128;
@@ -187,7 +213,7 @@ extern "C" int moe_layer_layout(int mode, int act_dtype, int64_t num_tokens, int
   if (num_tokens <= 0 || num_tokens > 65535 || topk <= 0 || topk > 32 || E_local <= 0 || H <= 0 || I <= 0 || !bytes ||
       !plan_serves(num_tokens * topk, num_experts, E_local) || !sizes_served(mode, act_dtype, H, I, activation))
     return fail(MOE_E_SHAPE, "layer: mode, type or sizes are not served by this call");
-  const Layout L = layout(mode, choose(mode, activation, num_tokens * topk, num_experts, H, I), num_tokens, topk, num_experts, E_local, H, I);
+  const Layout L = layout(mode, choose(mode, activation, num_tokens, topk, num_experts, H, I), num_tokens, topk, num_experts, E_local, H, I);
   for (int i = 0; i < 4; ++i) bytes[i] = L.bytes[i];
   if (pieces) std::memcpy(pieces, static_cast<const Pieces*>(&L), sizeof(Pieces));
   return 0;
@@ -211,7 +237,7 @@ extern "C" int moe_layer(int mode, int act_dtype, const void* x, int64_t num_tok
   const bool row = row_mode(mode), block = mode == MOE_MODE_FP8_BLOCK;
   if (mode != MOE_MODE_HALF && (!w1_scale || !w2_scale)) return fail(MOE_E_BADARG, "layer: weight scales missing");
   cudaStream_t st = (cudaStream_t)stream;
-  const Choice c = choose(mode, activation, numel, num_experts, H, I);
+  const Choice c = choose(mode, activation, M, topk, num_experts, H, I);
   const Layout L = layout(mode, c, M, topk, num_experts, E_local, H, I);
   void* const base[4] = {ws_plan, ws_x, ws_act, ws_y};
   auto at = [&](const Piece& p) -> void* { return (uint8_t*)base[p.ws] + p.at; };

@@ -318,3 +318,21 @@ def test_warps_agree_on_a_wait_before_they_act_as_one():
     tc, small = (open(os.path.join(csrc, n)).read() for n in ("gemm_tc.cu", "gemm_small.cu"))
     assert "(alive || TMAOUT); tile += tile_step" in tc and "for (int u = u_begin; u < u_end; ++u)" in small
     assert "if (alive) alive = mbar_wait(&aux->full[st]" in small
+
+
+@pytest.mark.parametrize("mode,act,E,topk,tokens,tile", [
+    # half precision: 64-row tiles while no expert can have more than two of them, 256 beyond 100 rows per expert
+    ("half", "silu", 8, 2, 100, 64), ("half", "silu", 8, 2, 128, 64), ("half", "silu", 8, 2, 129, 128), ("half", "silu", 4, 2, 65, 64),
+    ("half", "silu", 4, 2, 66, 128), ("half", "silu", 64, 6, 128, 64), ("half", "silu", 64, 6, 129, 128), ("half", "silu", 8, 2, 403, 128),
+    ("half", "silu", 8, 2, 404, 256), ("half", "silu", 8, 2, 16384, 256),
+    ("half", "swigluoai", 8, 2, 9, 128), ("half", "swigluoai", 8, 2, 259, 128), ("half", "swigluoai", 8, 2, 260, 256),
+    ("fp8_row", "silu", 128, 8, 33, 128), ("fp8_row", "silu", 128, 8, 1039, 128), ("fp8_row", "silu", 128, 8, 1040, 256),
+    ("int8_row", "silu", 128, 8, 1039, 128), ("int8_row", "silu", 128, 8, 1040, 256),
+    ("fp8_row", "swigluoai", 128, 8, 100, 256), ("int8_row", "swigluoai", 128, 8, 1500, 256)])
+def test_pair_tiles_where_their_lines_lie(mode, act, E, topk, tokens, tile):
+    """The lines that hold under skewed routing, which the host cannot see: read from the room for tiles in the plan."""
+    code = {"half": _lib.MODE_HALF, "fp8_row": _lib.MODE_FP8_ROW, "int8_row": _lib.MODE_INT8_ROW}[mode]
+    H = 512
+    pieces = _layer_pieces(code, tokens, topk, E, H, 256, _lib.ACT_SILU if act == "silu" else _lib.ACT_SWIGLUOAI)
+    rows, used = pieces[11] // (2 * H), min(tokens * topk, E)
+    assert {t for t in (64, 128, 256) if rows // t + used + 1 == pieces[1] // 16} == {tile}
