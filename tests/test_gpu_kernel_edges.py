@@ -437,3 +437,44 @@ def test_fp8_expert_of_more_blocks_than_a_group_of_the_tile_order():
     for m0 in range(0, M, 2000):  # at most nine blocks per expert
         part = slice(m0, m0 + 2000)
         assert torch.equal(fg.fused_experts_impl(x[part], w1, w2, tw[part], ids[part], **kw), out[part])
+
+
+def _fixed_routes(counts, k, seed):
+    """Expert e gets counts[e] routes of sum / k tokens, no token the same expert twice: slot j deals out the j-th part of a list."""
+    flat = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts)])
+    M = flat.numel() // k
+    assert flat.numel() == M * k and max(counts) <= M
+    ids = flat.view(k, M).t()[torch.randperm(M, generator=torch.Generator().manual_seed(seed))].contiguous().to(DEV)
+    return torch.rand((M, k), generator=torch.Generator().manual_seed(seed)).to(DEV) + 0.5, ids
+
+
+@pytest.mark.parametrize("fmt,k,counts", [
+    ("half", 2, (128, 65, 62, 1, 0, 0, 0, 0)), ("half", 1, (64, 1, 0, 63)),                # tiles of 64 rows: two full ones, 65 rows, one
+    ("half", 2, (129, 128, 1, 0, 0, 0, 0, 0)), ("half", 1, (128, 129, 257, 1, 0, 64, 65, 56)), ("half", 1, (380, 3, 0, 0)),  # 128 rows
+    ("half", 1, (256, 257, 486, 1)), ("half", 1, (404, 4, 0, 0)),                          # 256 rows
+    ("fp8", 1, (128, 129, 257, 1, 0, 64, 65, 56, 0, 0, 0, 0)), ("fp8", 1, (256, 257, 486, 1)),
+    ("int8", 1, (128, 129, 257, 1, 0, 64, 65, 56, 0, 0, 0, 0)), ("int8", 1, (256, 257, 486, 1))])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_pair_tiles_full_and_one_row_over(fmt, k, counts, dtype):
+    """Experts that fill a tile of the CTA pair exactly, have one row more, one row and none, in each tile size; rings and
+    accumulators wrap from tile to tile.  A row does not depend on the tile it is in, bit for bit: half the tokens at a time,
+    in tiles of other rows and, where the line is crossed, of another size."""
+    E, H, I = len(counts), 4224, 2560
+    tw, ti = _fixed_routes(counts, k, sum(counts))
+    M = ti.shape[0]
+    x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
+    w1 = T.make_half_weights(E, 2 * I, H, DEV, seed=1, dtype=dtype, std=H**-0.5)
+    w2 = T.make_half_weights(E, H, I, DEV, seed=2, dtype=dtype, std=I**-0.5)
+    if fmt == "half":
+        kw, ref = {}, O.fused_moe_half_oracle(x, w1, w2, tw, ti)
+    else:
+        top = 448.0 if fmt == "fp8" else 127.0
+        s1, s2 = w1.float().abs().amax(-1) / top, w2.float().abs().amax(-1) / top
+        cast = (lambda w: w.to(torch.float8_e4m3fn)) if fmt == "fp8" else (lambda w: w.round().to(torch.int8))
+        w1, w2 = cast(w1.float() / s1[..., None]), cast(w2.float() / s2[..., None])
+        kw = {"use_fp8_w8a8" if fmt == "fp8" else "use_int8_w8a8": True, "per_channel_quant": True, "w1_scale": s1, "w2_scale": s2}
+        ref = O.fused_moe_row_scaled_oracle(x, w1, w2, s1, s2, tw, ti, fmt=fmt, per_token=True)
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+    _parity(out, ref, (fmt, counts))
+    for part in (slice(0, M // 2), slice(M // 2, M)):
+        assert torch.equal(fg.fused_experts_impl(x[part], w1, w2, tw[part], ti[part], **kw), out[part])
