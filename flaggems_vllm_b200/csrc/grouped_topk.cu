@@ -249,13 +249,13 @@ __global__ void __launch_bounds__(32 * kGroupWarps) grouped_topk_g32_kernel(
   }
 }
 
-// Eight groups of 32 experts again, for many tokens: a warp per token, lane l owns the experts 8 l to 8 l + 7, so four
-// neighbouring lanes are a group.  The kernel above spends eight warps and three barriers on a token to keep its chain short;
-// with several tokens per SM what counts is the instructions per token.  Here a group's two largest come out of the lanes'
-// own eight values and two shuffles, and a round of the top-k extraction is one warp-wide maximum and one vote: the lowest lane
-// that holds the maximum holds the lowest expert.  Same keys, same order, same arithmetic as above, bit for bit.
-template <typename ST, typename BT>
-__global__ void __launch_bounds__(128) grouped_topk_8x32_kernel(
+// Groups of 32 experts again, for many tokens: a warp per token, lane l owns the N neighbouring experts from N l on (N groups:
+// 2, 4 or 8), so 32 / N neighbouring lanes are a group.  The kernel above spends N warps and three barriers on a token to keep its
+// chain short; with several tokens per SM what counts is the instructions per token.  Here a group's two largest come out of
+// the lanes' own values and a few shuffles, and a round of the top-k extraction is one warp-wide maximum and one vote: the lowest
+// lane that holds the maximum holds the lowest expert.  Same keys, same order, same arithmetic as above, bit for bit.
+template <typename ST, typename BT, int N>
+__global__ void __launch_bounds__(128) grouped_topk_warp32_kernel(
     const ST* __restrict__ scores, int64_t stride0, int64_t stride1, const BT* __restrict__ bias,
     const uint8_t* __restrict__ is_padding, int64_t M, int topk_group, int topk, int renormalize, float scaling,
     int scoring_func, float* __restrict__ out_w, int32_t* __restrict__ out_ids) {
@@ -270,36 +270,37 @@ __global__ void __launch_bounds__(128) grouped_topk_8x32_kernel(
     if (lane < topk) { w_row[lane] = 0.0f; id_row[lane] = -1; }
     return;
   }
-  float u[8], b[8];
-  const ST* row = scores + token * stride0 + (int64_t)(8 * lane) * stride1;
-  if (stride1 == 1 && ((uintptr_t)row & 15) == 0) {
-    load8<ST>(row, u);
+  constexpr int SHIFT = N == 8 ? 2 : (N == 4 ? 3 : 4);  // 32 / N = 1 << SHIFT lanes per group
+  float u[N], b[N];
+  const ST* row = scores + token * stride0 + (int64_t)(N * lane) * stride1;
+  if (N == 8 && stride1 == 1 && ((uintptr_t)row & 15) == 0) {
+    if constexpr (N == 8) load8<ST>(row, u);
   } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) u[j] = ToF32<ST>::get(row[(int64_t)j * stride1]);
+    for (int j = 0; j < N; ++j) u[j] = ToF32<ST>::get(row[(int64_t)j * stride1]);
   }
-  if (((uintptr_t)bias & 15) == 0) {
-    load8<BT>(bias + 8 * lane, b);
+  if (N == 8 && ((uintptr_t)bias & 15) == 0) {
+    if constexpr (N == 8) load8<BT>(bias + 8 * lane, b);
   } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = ToF32<BT>::get(bias[8 * lane + j]);
+    for (int j = 0; j < N; ++j) b[j] = ToF32<BT>::get(bias[N * lane + j]);
   }
   // order-preserving image of u + bias; a sum is no NaN with all bits set, so 0 is free to mean "consumed"
-  uint32_t v[8];
+  uint32_t v[N];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < N; ++j) {
     if (scoring_func == 1) u[j] = (float)(1.0 / (1.0 + exp(-(double)u[j])));
     v[j] = ordered_bits(u[j] + b[j]);
   }
   {
     uint32_t top1 = 0, top2 = 0;  // of this lane, then of its group
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < N; ++j) {
       top2 = max(top2, min(top1, v[j]));
       top1 = max(top1, v[j]);
     }
 #pragma unroll
-    for (int off = 1; off <= 2; off <<= 1) {
+    for (int off = 1; off <= (1 << SHIFT) / 2; off <<= 1) {
       const uint32_t o1 = __shfl_xor_sync(0xFFFFFFFFu, top1, off), o2 = __shfl_xor_sync(0xFFFFFFFFu, top2, off);
       top2 = max(max(top2, o2), min(top1, o1));
       top1 = max(top1, o1);
@@ -307,20 +308,20 @@ __global__ void __launch_bounds__(128) grouped_topk_8x32_kernel(
     const uint32_t mine = ordered_bits(from_ordered_bits(top1) + from_ordered_bits(top2));
     int rank = 0;  // of this lane's group
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-      const uint32_t other = __shfl_sync(0xFFFFFFFFu, mine, 4 * g);
-      rank += other > mine || (other == mine && g < (lane >> 2));
+    for (int g = 0; g < N; ++g) {
+      const uint32_t other = __shfl_sync(0xFFFFFFFFu, mine, g << SHIFT);
+      rank += other > mine || (other == mine && g < (lane >> SHIFT));
     }
     // experts of dropped groups rank as -inf (still ordered by index)
     if (rank >= topk_group) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = ordered_bits(__int_as_float(0xff800000));
+      for (int j = 0; j < N; ++j) v[j] = ordered_bits(__int_as_float(0xff800000));
     }
   }
   auto largest = [&] {
     uint32_t m = v[0];
 #pragma unroll
-    for (int j = 1; j < 8; ++j) m = max(m, v[j]);
+    for (int j = 1; j < N; ++j) m = max(m, v[j]);
     return m;
   };
   uint32_t best = largest();
@@ -333,16 +334,16 @@ __global__ void __launch_bounds__(128) grouped_topk_8x32_kernel(
     int at = 0;
     if (lane == owner) {
 #pragma unroll
-      for (int j = 7; j >= 0; --j)
+      for (int j = N - 1; j >= 0; --j)
         if (v[j] == top) { at = j; wsel = u[j]; }
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < N; ++j)
         if (j == at) v[j] = 0;
       best = largest();
     }
     wsel = __shfl_sync(0xFFFFFFFFu, wsel, owner);
     at = __shfl_sync(0xFFFFFFFFu, at, owner);
-    if (lane == t) { my_w = wsel; my_id = 8 * owner + at; }
+    if (lane == t) { my_w = wsel; my_id = N * owner + at; }
   }
   float sum = lane < topk ? my_w : 0.0f;
 #pragma unroll
@@ -510,11 +511,20 @@ int launch_vpt(const ST* scores, int64_t s0, int64_t s1, const BT* bias, const u
                                         scoring, w, ids);
     return check_launch("grouped_topk (wide router)");
   }
-  // Eight groups of 32: a warp per token from two tokens per SM on.  us back to back, CTA per token against warp per token:
-  // 1 token 3.4 : 4.0, 148 3.4 : 4.2, 300 4.4 : 4.2, 600 6.3 : 5.3, 2000 9.9 : 6.0, 8192 33.7 : 13.6.
-  if (n_group == 8 && E == 256 && M > 2 * (int64_t)sm_count() && M < (1ll << 31))
-    return launch_pdl(grouped_topk_8x32_kernel<ST, BT>, dim3((unsigned)((M + 3) / 4)), 128, 0, 1, st, "grouped_topk (8 groups of 32)",
-                      scores, s0, s1, bias, pad, M, topk_group, topk, renorm, scaling, scoring, w, ids);
+  // Groups of 32: a warp per token where a warp per group and token would be more than 28 warps per SM.  us, CTA per token : warp
+  // per token (f32 logits, sigmoid, top 8; 50 calls in a graph):
+  //   8 groups   148 tokens 2.5 : 4.2   400 3.5 : 3.9    600 6.0 : 4.1   2000 9.6 : 5.3   8192 33.3 : 12.8
+  //   4 groups   148        2.1 : 3.0   1000 3.2 : 3.3                   2000 5.2 : 3.8   8192 14.7 : 9.1
+  //   2 groups   148        2.0 : 2.3   1000 2.5 : 2.5                   2000 4.2 : 2.9   8192 10.1 : 6.7
+  if (E == 32 * n_group && M * n_group > 28 * (int64_t)sm_count() && M < (1ll << 31)) {
+#define MOE_TOPK_WARP(N)                                                                                                          \
+  launch_pdl(grouped_topk_warp32_kernel<ST, BT, N>, dim3((unsigned)((M + 3) / 4)), 128, 0, 1, st, "grouped_topk (groups of 32)", \
+             scores, s0, s1, bias, pad, M, topk_group, topk, renorm, scaling, scoring, w, ids)
+    if (n_group == 8) return MOE_TOPK_WARP(8);
+    if (n_group == 4) return MOE_TOPK_WARP(4);
+    if (n_group == 2) return MOE_TOPK_WARP(2);
+#undef MOE_TOPK_WARP
+  }
   // groups of exactly 32 experts whose candidates fit the CTA
   if (E == 32 * n_group && n_group <= kGroupWarps && topk * n_group <= E && M < (1ll << 31)) {
     return launch_pdl(grouped_topk_g32_kernel<ST, BT>, dim3((unsigned)M), E, 0, 1, st, "grouped_topk (warp per group)", scores, s0,

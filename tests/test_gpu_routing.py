@@ -143,6 +143,35 @@ def test_eight_groups_of_32_both_kernels(M, dtype, form):
             _check(s, 8, keep, k, False, 1.0, b, sf, pad)
 
 
+@pytest.mark.parametrize("groups", [2, 4, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("form", ["rows", "strided", "odd_offset"])
+def test_groups_of_32_a_warp_per_token_is_a_cta_per_token(groups, dtype, form):
+    """Up to 28 group warps per SM a CTA serves a token, beyond a warp: the same ids and weights, bit for bit, at any group count."""
+    few = 28 * torch.cuda.get_device_properties(0).multi_processor_count // groups
+    M, E = few + 1, 32 * groups
+    g = torch.Generator().manual_seed(groups)
+    s = torch.randn((M, E), generator=g)
+    s[: M // 3] = (s[: M // 3] * 2).round() / 2  # ties
+    s[M // 3: M // 2, ::3] = -float("inf")
+    s[M // 2] = -float("inf")
+    s = s.to(dtype).to(DEV)
+    bias = torch.randn((E + 1,), generator=g).mul(0.1).to(dtype).to(DEV)
+    b = bias[:E].contiguous()
+    if form == "strided":
+        s = s.t().contiguous().t()
+    elif form == "odd_offset":
+        wide = torch.zeros((M, E + 3), dtype=dtype, device=DEV)
+        wide[:, 1:E + 1] = s
+        s, b = wide[:, 1:E + 1], bias[1:]
+    pad = (torch.arange(M, device=DEV) % 5 == 0)
+    for k, keep, sf in ((8, max(1, groups // 2), 1), (1, 1, 0), (32, groups, 1), (30, groups, 0)):
+        for mask in (None, pad) if form != "strided" else (None,):  # a mask wants rows
+            w, ids = _check(s, groups, keep, k, sf == 1 and mask is None, 2.5, b, sf, mask)
+            w0, ids0 = fg.grouped_topk(s[:few], groups, keep, k, sf == 1 and mask is None, 2.5, b, sf, None if mask is None else mask[:few])
+            assert torch.equal(ids[:few], ids0) and torch.equal(w[:few].view(torch.int32), w0.view(torch.int32))
+
+
 @pytest.mark.parametrize("mode", ["mixed", "all", "none"])
 def test_padding_rows(mode):
     rows, E = 9, 256
