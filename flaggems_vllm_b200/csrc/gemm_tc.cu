@@ -202,7 +202,8 @@ __device__ __forceinline__ int box_row(int nt, int c, int cr, int Nout) {
 // the next tile -- sat in those stores for ~5000 cycles per tile; staged, they are done after
 // sixteen conflict-free shared-memory stores.  Costs one pipeline stage of shared memory.
 //
-// BY_EXPERT (route plan, whole blocks): the blocks of an expert, which the plan knows, share its column tiles in the tile order.
+// PLAN: 0 the blocks of moe_align_block_size; over a route plan made with 128-row tiles (FP8) 1 the occupied rows, 2 whole blocks.
+// BY_EXPERT (2): the blocks of an expert, which the plan knows, share its column tiles in the tile order.
 // Fixed groups of blocks start somewhere inside an expert and read its weights once per group: DSV3 FP8, 8192 tokens, the
 // layer 4799 -> 4719 us.  With few rows per expert the order is the same and the plan entries cost up to 1 %.  At most `group_m`
 // blocks make a pass over the column tiles together: their rows are read again for every column tile and have to stay in L2.
@@ -211,7 +212,7 @@ __device__ __forceinline__ int box_row(int nt, int c, int cr, int Nout) {
 // nothing has to happen between K blocks, so the whole K loop accumulates in TMEM like half
 // precision (int8: exact int32 sums) and the epilogue multiplies by the row's and the channel's
 // scale.  Qwen3 shape, 500 tokens, e4m3: 5605 us for the two GEMMs on CUDA cores before.
-template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false, bool BY_EXPERT = false>
+template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false, int PLAN = 0>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_a16,
@@ -222,7 +223,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   static_assert(!ROW || (!PAIR && RB == 1 && !SORTED), "row-scaled formats: the single-CTA kernel");
   static_assert(!TMAOUT || (!GEMM1 && !PAIR && RB == 1), "staged output: single-CTA GEMM2 only");
   static_assert(!SORTED || GEMM1, "pre-sorted A rows: GEMM1 only");
-  static_assert(!BY_EXPERT || (FP8 && !PAIR && RB == 1 && (GEMM1 ? SORTED : TMAOUT)), "expert order: the FP8 kernels of a route plan's whole blocks");
+  constexpr bool BY_EXPERT = PLAN == 2;
+  static_assert(PLAN == 0 || (FP8 && !PAIR && RB == 1 && (!GEMM1 || SORTED)), "route plan: the single-CTA FP8 kernels over sorted rows");
+  static_assert(!BY_EXPERT || GEMM1 || TMAOUT, "whole blocks go with staged stores");
   constexpr bool GATHER = GEMM1 && !SORTED;  // A rows gathered inside the kernel
   static_assert(RB == 1 || (RB == 2 && !BYTE), "wide tiles: half precision only");
   constexpr int STAGES = TMAOUT ? 3 : Cfg<PAIR, RB>::STAGES;
@@ -263,7 +266,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     nt = within / gsz;
     blk = first + within - nt * gsz;
   };
-  auto expert_of = [&](int blk) -> int { return P.tiles != nullptr ? __ldcg(&P.tiles[blk].z) : P.expert_ids[blk]; };
+  auto expert_of = [&](int blk) -> int { return PLAN != 0 ? __ldcg(&P.tiles[blk].z) : P.expert_ids[blk]; };
   // BY_EXPERT: plan entry of one of the blocks of the expert that the NEXT tile belongs to, loaded a whole tile before it is used
   [[maybe_unused]] int2 ahead = make_int2(-1, 1 << 16);  // {expert, first block | blocks << 16}
   [[maybe_unused]] auto look_ahead = [&](int tile) {
@@ -316,14 +319,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int e = coords((tile), blk, nt);                  \
   [[maybe_unused]] const int mb = UNIT * blk + RB * cr;
 
-  if constexpr (!GATHER && !PAIR && RB == 1 && !BY_EXPERT) {
-    // Route plan, occupied rows only: the other rows of a stage are multiplied all the same.  They start as zeros and
-    // stay zeros until a larger tile comes by.  Without this: DSV3 FP8, 61 tokens 1005 -> 1103 us per layer, one of 8 ranks
-    // with 2000 tokens 319 -> 323; Mixtral shape, 300 tokens 520 -> 533.
-    if (P.tiles != nullptr) {
-      for (int i = threadIdx.x; i < STAGES * A_LOCAL_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(sA)[i] = make_uint4(0, 0, 0, 0);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
+  if constexpr (PLAN == 1) {
+    // Occupied rows only: the other rows of a stage are multiplied all the same.  They start as zeros and stay zeros
+    // until a larger tile comes by.  Without this: DSV3 FP8, 61 tokens 1005 -> 1103 us per layer, one of 8 ranks with 2000
+    // tokens 319 -> 323.
+    for (int i = threadIdx.x; i < STAGES * A_LOCAL_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(sA)[i] = make_uint4(0, 0, 0, 0);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -369,10 +370,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
       uint32_t s = 0, ph = 1;  // stage, and the parity its "empty" barrier is waited for with
       bool alive = true;
-      constexpr bool EARLY = !GATHER && !PAIR && RB == 1;
-      auto occupied_rows = [&](int blk) -> int {  // rows of A to fetch
-        if (EARLY && !BY_EXPERT && P.tiles != nullptr) return ((__ldcg(&P.tiles[blk].y) >> 16) + 7) & ~7;
-        return RB * BM;
+      auto occupied_rows = [&]([[maybe_unused]] int blk) -> int {  // rows of A to fetch
+        if constexpr (PLAN == 1) return ((__ldcg(&P.tiles[blk].y) >> 16) + 7) & ~7;
+        else return RB * BM;
       };
       // the stage's byte count and its weight tile
       auto load_weights = [&](int kb, int s, int a_rows, int wrow0, int nt) {
@@ -384,8 +384,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       };
       // route plan: the weights of the first stages do not wait for the kernel in front
       int early = 0;
-      if constexpr (EARLY) {
-        if (P.tiles != nullptr && tile0 < total_tiles) {
+      if constexpr (PLAN != 0) {
+        if (tile0 < total_tiles) {
           int blk, nt, e0;
           if constexpr (BY_EXPERT) {  // as coords(), which moves on
             expert_tile(tile0, blk, nt);
@@ -668,18 +668,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // wait for the tensor core anyway), so a tile starts folding without integer divisions or a
     // dependent global load in front of it.
     int nx_blk = 0, nx_nt = 0, nx_e = -1;
-    int64_t nx_sid = P.numel;
+    [[maybe_unused]] int nx_occupied = 0;
+    [[maybe_unused]] int64_t nx_sid = P.numel;
     auto prefetch_tile = [&](int t) {
       nx_e = -1;
       nx_sid = P.numel;
       if (t < total_tiles) {
         tile_blk_nt(t, nx_blk, nx_nt);
-        const int64_t pn = (int64_t)(UNIT * nx_blk + RB * cr) * BM + row;
-        if (P.tiles != nullptr) {  // rows leave in sorted order, weighted by the combine
+        if constexpr (PLAN != 0) {  // rows leave in sorted order, weighted by the combine
           const int4 d = __ldcg(P.tiles + nx_blk);
+          nx_occupied = d.y >> 16;
           nx_e = d.z;
-          if (row < (d.y >> 16)) nx_sid = pn;
         } else {
+          const int64_t pn = (int64_t)(UNIT * nx_blk + RB * cr) * BM + row;
           nx_e = P.expert_ids[nx_blk];
           if (pn < P.rows_cap) nx_sid = (int64_t)P.sorted_ids[pn];
         }
@@ -690,7 +691,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if constexpr (!BY_EXPERT) prefetch_tile(tile0);
     for (int tile = tile0; tile < total_tiles && (alive || TMAOUT); tile += tile_step) {
       int blk = nx_blk, nt = nx_nt, e = nx_e;
-      [[maybe_unused]] int occupied = 0;
+      [[maybe_unused]] int occupied = nx_occupied;
       if constexpr (BY_EXPERT) {
         e = coords(tile, blk, nt);
         occupied = __ldcg(&P.tiles[blk].y) >> 16;  // first looked at behind the K loop
@@ -712,11 +713,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       for (int sub = 0; sub < RB && alive; ++sub) {  // the 128-row blocks of this tile (two for wide tiles)
       const int64_t p = (int64_t)(mb + sub) * BM + row;
       int64_t sid = P.numel;
-      if (BY_EXPERT) sid = p;
+      if (PLAN != 0) sid = p;
       else if (sub == 0) sid = sid_first;
       else if (p < P.rows_cap) sid = (int64_t)P.sorted_ids[p];
-      const bool row_ok = BY_EXPERT ? row < occupied : sid >= 0 && sid < P.numel;
-      if (!BY_EXPERT && (sid < 0 || sid > P.numel)) set_status(P.status, MOE_ST_BAD_ROW);  // the pad value is numel; anything else outside is corrupt
+      const bool row_ok = PLAN != 0 ? row < occupied : sid >= 0 && sid < P.numel;
+      if (PLAN == 0 && (sid < 0 || sid > P.numel)) set_status(P.status, MOE_ST_BAD_ROW);  // the pad value is numel; anything else outside is corrupt
       float acc[128];
       [[maybe_unused]] float as = 0.0f;  // row-scaled formats: activation scale of this row
       float rw = 1.0f;  // route weight of this row, fetched early: the epilogue must not wait for it
@@ -915,7 +916,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           uint8_t* dst = s_out + (size_t)(2 * h + (c >> 3)) * (BM * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4);
           *reinterpret_cast<uint4*>(dst) = piece;
         }
-        if (row_ok && h == 0 && P.inv != nullptr) P.inv[sid] = (int32_t)p;
+        if (PLAN == 0 && row_ok && h == 0 && P.inv != nullptr) P.inv[sid] = (int32_t)p;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> TMA reads
         meet();
         if (threadIdx.x == 128) {
@@ -969,10 +970,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ------------------------------------------------------------------ host side
-template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false, bool BY_EXPERT = false>
+template <int FMT, typename AT, bool GEMM1, bool PAIR, int RB, bool SORTED = false, bool TMAOUT = false, int PLAN = 0>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P, int grid, cudaStream_t st,
                   const CUtensorMap* mo = nullptr, const CUtensorMap* ms = nullptr) {
-  auto kern = tc_gemm_kernel<FMT, AT, GEMM1, PAIR, RB, SORTED, TMAOUT, BY_EXPERT>;
+  auto kern = tc_gemm_kernel<FMT, AT, GEMM1, PAIR, RB, SORTED, TMAOUT, PLAN>;
   constexpr size_t smem = smem_bytes<PAIR, RB, TMAOUT>();
   static const int regs = [&] {
     cudaFuncAttributes fa;
@@ -985,7 +986,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& P,
   if (rc) return rc;
   const CUtensorMap &m_out = mo != nullptr ? *mo : ma, &m16 = ms != nullptr ? ms[0] : ma, &m8 = ms != nullptr ? ms[1] : ma;
   const char* what = GEMM1 ? "gemm1 (tcgen05)" : "gemm2 (tcgen05)";
-  if (P.tiles != nullptr) return launch_pdl(kern, dim3((unsigned)grid), THREADS, smem, 1, st, what, ma, mb, m_out, m16, m8, P);
+  if (PLAN != 0) return launch_pdl(kern, dim3((unsigned)grid), THREADS, smem, 1, st, what, ma, mb, m_out, m16, m8, P);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(THREADS);
@@ -1187,11 +1188,11 @@ int tc_gemm_plan(bool gemm1, int act_dtype, const void* a, const float* a_scales
   // whole blocks: from 128 rows per expert on (layer.cu), where an expert has several
   if (all_rows && !staged) return fail(MOE_E_SHAPE, "tensor-core GEMM over a route plan: whole blocks go with staged stores");
 #define MOE_TCP(T)                                                                                                                \
-  (gemm1 ? (all_rows ? launch<FMT_FP8, T, true, false, 1, true, false, true>(ma, mb, P, grid, st, nullptr, ms)                     \
-                     : launch<FMT_FP8, T, true, false, 1, true>(ma, mb, P, grid, st, nullptr, ms))                                 \
-         : (all_rows ? launch<FMT_FP8, T, false, false, 1, false, true, true>(ma, mb, P, grid, st, &mo, ms)                        \
-            : staged ? launch<FMT_FP8, T, false, false, 1, false, true>(ma, mb, P, grid, st, &mo, ms)                              \
-                     : launch<FMT_FP8, T, false, false, 1>(ma, mb, P, grid, st, nullptr, ms)))
+  (gemm1 ? (all_rows ? launch<FMT_FP8, T, true, false, 1, true, false, 2>(ma, mb, P, grid, st, nullptr, ms)                        \
+                     : launch<FMT_FP8, T, true, false, 1, true, false, 1>(ma, mb, P, grid, st, nullptr, ms))                       \
+         : (all_rows ? launch<FMT_FP8, T, false, false, 1, false, true, 2>(ma, mb, P, grid, st, &mo, ms)                           \
+            : staged ? launch<FMT_FP8, T, false, false, 1, false, true, 1>(ma, mb, P, grid, st, &mo, ms)                           \
+                     : launch<FMT_FP8, T, false, false, 1, false, false, 1>(ma, mb, P, grid, st, nullptr, ms)))
   return act_dtype == MOE_BF16 ? MOE_TCP(__nv_bfloat16) : MOE_TCP(__half);
 #undef MOE_TCP
 }
