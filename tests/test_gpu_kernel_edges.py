@@ -167,6 +167,44 @@ def test_scattered_fp8_rows_are_the_quantisers(M, dtype):
         assert torch.equal(scales[:, rows[:, j]].t().contiguous().view(torch.int32), s.view(torch.int32))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_scattered_fp8_bytes_are_those_of_the_division(dtype):
+    """Every pair of finite magnitudes (amax of the 128-group, |v| <= amax) of the type, about 5e8 of them, either sign: a group
+    holds an amax and 127 of its values.  The kernel multiplies by a reciprocal and corrects; torch divides."""
+    H, I, chunk = 7168, 128, 8192
+    top = 0x7F7F if dtype == torch.bfloat16 else 0x7BFF  # bits of the largest finite value
+    per_amax = torch.arange(1, top + 1, device=DEV).div(127, rounding_mode="floor") + 1  # groups for the values 0 .. amax
+    amax = torch.repeat_interleave(torch.arange(1, top + 1, device=DEV), per_amax)
+    first = torch.arange(amax.numel(), device=DEV) - torch.repeat_interleave(per_amax.cumsum(0) - per_amax, per_amax)
+    sizes = (_lib.MODE_FP8_BLOCK, _lib.dtype_code(dtype), chunk, 1, 1, 1, H, I, _lib.ACT_SILU)
+    need, table = (ctypes.c_int64 * 4)(), (ctypes.c_int64 * (3 * 13))()
+    _lib.check(_lib.lib().moe_layer_layout(*sizes, ctypes.addressof(need), ctypes.addressof(table)))
+    ws = [torch.zeros(n, dtype=torch.uint8, device=DEV) for n in need]
+    ids, one = torch.zeros(chunk, dtype=torch.int32, device=DEV), torch.ones(chunk, device=DEV)
+    w = torch.zeros(16, device=DEV)  # not read: the first two steps only
+    piece = lambda i, t: ws[table[3 * i]][table[3 * i + 1]:table[3 * i + 1] + table[3 * i + 2]].view(t)
+    lane, pairs = torch.arange(128, device=DEV), 0
+    for g0 in range(0, amax.numel(), chunk * (H // 128)):
+        a, f = amax[g0:g0 + chunk * (H // 128)], first[g0:g0 + chunk * (H // 128)]
+        bits = torch.minimum(f[:, None] * 127 + (lane - 1), a[:, None])
+        bits[:, 0] = a
+        pairs += int((f[:, None] * 127 + (lane[1:] - 1) <= a[:, None]).sum())
+        bits |= ((lane + f[:, None]) % 2) << 15
+        x = torch.zeros((chunk * (H // 128), 128), dtype=dtype, device=DEV)
+        x[:a.numel()] = torch.where(bits >= 0x8000, bits - 0x10000, bits).to(torch.int16).view(dtype)
+        _lib.check(_lib.lib().moe_layer(
+            sizes[0], sizes[1], x.data_ptr(), chunk, 1, ids.data_ptr(), 0, one.data_ptr(), w.data_ptr(), w.data_ptr(), w.data_ptr(),
+            w.data_ptr(), x.data_ptr(), 1, None, 1, H, I, 0, _lib.ACT_SILU, 0.0, 0.0, 0.0, 0, None, 0, None,
+            *[t.data_ptr() for t in ws], 1 | 2, _lib.status_word(torch.device(DEV)).data_ptr(), _lib.stream_of(x)))
+        v = x.float()
+        s = v.abs().amax(-1, keepdim=True).clamp(min=1e-10) * (1.0 / 448.0)
+        want = (v / s).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+        got = piece(5, torch.uint8).view(-1, 128)[:want.shape[0]]  # one expert: the rows are the tokens, in order
+        assert torch.equal(got, want)
+        assert torch.equal(piece(6, torch.float32).view(H // 128, -1)[:, :chunk].t().reshape(-1, 1), s)
+    assert pairs == top * (top + 1) // 2 + top
+
+
 @pytest.mark.parametrize("M,E,k,H,I", [
     (1, 1, 1, 128, 64), (1, 8, 8, 256, 192), (8, 2, 1, 2176, 128), (4, 8, 2, 1024, 2048),
     (3, 4, 3, 128, 64)])  # nine routes: the tile kernels
