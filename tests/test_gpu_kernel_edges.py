@@ -516,3 +516,28 @@ def test_pair_tiles_full_and_one_row_over(fmt, k, counts, dtype):
     _parity(out, ref, (fmt, counts))
     for part in (slice(0, M // 2), slice(M // 2, M)):
         assert torch.equal(fg.fused_experts_impl(x[part], w1, w2, tw[part], ti[part], **kw), out[part])
+
+
+@pytest.mark.parametrize("fmt", ["fp8", "half", "fp8_row"])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_scatter_and_combine_either_side_of_four_tokens_per_sm(fmt, inplace):
+    """Parts of a token per block and the plan not waited for, below; a block per token, from there on: the same rows, bit for bit."""
+    M, E, k, H, I = 4 * torch.cuda.get_device_properties(0).multi_processor_count, 16, 3, 1152, 128
+    x = T.make_activations(M, H, DEV, seed=M)
+    tw, ti = _route(M, E, k)
+    if fmt == "half":
+        w1, w2 = (T.make_half_weights(E, n, K, DEV, seed=n, std=K**-0.5) for n, K in ((2 * I, H), (H, I)))
+        kw, ref = {}, O.fused_moe_half_oracle(x, w1, w2, tw, ti)
+    elif fmt == "fp8":
+        (w1, s1), (w2, s2) = (T.make_fp8_block_weights(E, n, K, DEV, seed=n) for n, K in ((2 * I, H), (H, I)))
+        kw = dict(use_fp8_w8a8=True, w1_scale=s1, w2_scale=s2, block_shape=[128, 128])
+        ref = O.fused_moe_fp8_block_oracle(x, w1, w2, s1, s2, tw, ti)
+    else:
+        w1f, w2f = torch.randn(E, 2 * I, H, device=DEV) * H**-0.5, torch.randn(E, H, I, device=DEV) * I**-0.5
+        s1, s2 = w1f.abs().amax(-1) / 448.0, w2f.abs().amax(-1) / 448.0
+        w1, w2 = (w1f / s1[..., None]).to(torch.float8_e4m3fn), (w2f / s2[..., None]).to(torch.float8_e4m3fn)
+        kw = dict(use_fp8_w8a8=True, per_channel_quant=True, w1_scale=s1, w2_scale=s2)
+        ref = O.fused_moe_row_scaled_oracle(x, w1, w2, s1, s2, tw, ti, fmt="fp8", per_token=True)
+    out = fg.fused_experts_impl(x.clone(), w1, w2, tw, ti, inplace=inplace, **kw)
+    _parity(out, ref, fmt)
+    assert torch.equal(fg.fused_experts_impl(x[:M - 1].clone(), w1, w2, tw[:M - 1], ti[:M - 1], inplace=inplace, **kw), out[:M - 1])
