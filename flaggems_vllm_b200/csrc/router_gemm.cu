@@ -91,9 +91,13 @@ __global__ void __launch_bounds__(kThreads) router_gemm_kernel(const XT* __restr
 // run-to-run deterministic and no partial ever goes to memory.  The product is small (256 x 7168
 // weights): what bounds it is how many SMs pull operands from L2 at once and the latency of one CTA's
 // K loop, hence the split.  Rows and columns beyond the matrix are zero-filled by TMA.
-// Launched so that the next kernel's set-up (barriers, TMEM, the launch itself) overlaps this one's end: back to back,
-// K = 7168, N = 256, bf16, us, before and with it and all partial sums of an element in flight: 8 rows 8.9 -> 6.1, 64 rows
-// 8.3 -> 6.1, 200 rows 10.3 -> 7.1, 1000 rows 12.4 -> 11.1, 8192 rows 39.5 -> 34.0.
+// Launched so that its set-up (barriers, TMEM, the launch itself) overlaps the end of the kernel in front.  What that is worth
+// depends on the neighbours; us per call, K = 7168, N = 256, bf16, ordinary launch : this one (neighbour subtracted):
+//                                               64 rows     200 rows     1000 rows    2000 rows    8192 rows
+//   back to back, stream                        8.3 : 6.0   10.3 : 7.2   12.9 : 10.4  15.1 : 12.4  39.0 : 34.1
+//   behind an elementwise kernel, stream        8.2 : 6.2   10.3 : 8.2   13.1 : 11.3  14.9 : 13.5  40.1 : 34.8
+//   back to back, graph                         6.6 : 5.4    8.3 : 6.4   10.7 : 9.3   12.6 : 11.8  36.3 : 34.3
+//   behind an elementwise kernel, graph         6.7 : 6.7    8.3 : 8.5   10.8 : 11.0  12.8 : 13.0  40.7 : 39.0
 constexpr int RBM = 128, RTHREADS = 192;
 template <int BN> struct RCfg {
   static constexpr int STAGE = (RBM + BN) * 128;
@@ -208,17 +212,20 @@ __global__ void __launch_bounds__(RTHREADS, 1) router_tc_kernel(const __grid_con
       const int64_t m = m0 + row;
       if (m >= M || n0 + c >= N) continue;
       float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      for (int r0 = 0; r0 < split; r0 += 8) {  // eight CTAs' partial sums in flight, added in rank order
-        float4 v[8];
+      auto add_all = [&](auto ranks) {  // all ranks' partial sums in flight, added in rank order
+        constexpr int R = decltype(ranks)::value;
+        float4 v[R];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (r0 + j < split)
-            v[j] = *reinterpret_cast<const float4*>(
-                cluster.map_shared_rank(reinterpret_cast<float*>(smem), r0 + j) + (size_t)row * (BN + 4) + c);
+        for (int j = 0; j < R; ++j)
+          v[j] = *reinterpret_cast<const float4*>(
+              cluster.map_shared_rank(reinterpret_cast<float*>(smem), j) + (size_t)row * (BN + 4) + c);
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (r0 + j < split) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
-      }
+        for (int j = 0; j < R; ++j) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
+      };
+      // a loop for each split: one for eight with a test per rank took 0.7 us more at 2000 rows (split 4)
+      if (split == 8) add_all(std::integral_constant<int, 8>());
+      else if (split == 4) add_all(std::integral_constant<int, 4>());
+      else add_all(std::integral_constant<int, 2>());
       float* o = out + m * N + n0 + c;
       if (N % 4 == 0) {
         *reinterpret_cast<float4*>(o) = sum;

@@ -541,3 +541,15 @@ def test_scatter_and_combine_either_side_of_four_tokens_per_sm(fmt, inplace):
     out = fg.fused_experts_impl(x.clone(), w1, w2, tw, ti, inplace=inplace, **kw)
     _parity(out, ref, fmt)
     assert torch.equal(fg.fused_experts_impl(x[:M - 1].clone(), w1, w2, tw[:M - 1], ti[:M - 1], inplace=inplace, **kw), out[:M - 1])
+
+
+@pytest.mark.parametrize("M,N,K,split", [(200, 256, 7168, 8), (1000, 256, 7168, 4), (4000, 256, 7168, 2), (8192, 256, 7168, 1), (4100, 130, 2040, 2)])
+def test_router_gemm_adds_the_partial_sums_of_each_split(M, N, K, split):
+    columns, s = ctypes.c_int(), ctypes.c_int()
+    _lib.check(_lib.lib().moe_router_gemm_tile(M, N, K, 148, 8, ctypes.addressof(columns), ctypes.addressof(s)))
+    assert s.value == split  # on a device of 148 multiprocessors
+    x = T.make_activations(M, K, DEV, seed=M)
+    w = torch.randn((N, K), generator=torch.Generator(device=DEV).manual_seed(N), device=DEV).to(torch.bfloat16)
+    out = fg.router_gemm(x, w)
+    ref = x.double() @ w.double().t()
+    assert float((out.double() - ref).norm() / ref.norm()) < 4e-6 and _lib.read_status() == 0
