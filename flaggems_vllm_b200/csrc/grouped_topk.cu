@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(128) grouped_topk_kernel(
 // rank in its group, and a candidate's rank among all groups' candidates, are counted against keys in shared memory.
 // Keys are unique, so the counted order is the extracted one, bit for bit.
 constexpr int kGroupWarps = 8;  // at most 8 groups
+constexpr size_t kG32Smem = 32 * kGroupWarps * (2 * sizeof(uint64_t) + sizeof(float)) + 512;  // its static shared memory, rounded up
 template <typename ST, typename BT>
 __global__ void __launch_bounds__(32 * kGroupWarps) grouped_topk_g32_kernel(
     const ST* __restrict__ scores, int64_t stride0, int64_t stride1, const BT* __restrict__ bias,
@@ -518,8 +519,8 @@ int launch_vpt(const ST* scores, int64_t s0, int64_t s1, const BT* bias, const u
   //   2 groups   148        2.0 : 2.3   1000 2.5 : 2.5                   2000 4.2 : 2.9   8192 10.1 : 6.7
   if (E == 32 * n_group && M * n_group > 28 * (int64_t)sm_count() && M < (1ll << 31)) {
 #define MOE_TOPK_WARP(N)                                                                                                          \
-  launch_pdl(grouped_topk_warp32_kernel<ST, BT, N>, dim3((unsigned)((M + 3) / 4)), 128, 0, 1, st, "grouped_topk (groups of 32)", \
-             scores, s0, s1, bias, pad, M, topk_group, topk, renorm, scaling, scoring, w, ids)
+  launch_pdl_spread(grouped_topk_warp32_kernel<ST, BT, N>, dim3((unsigned)((M + 3) / 4)), 128, 0, st, "grouped_topk (groups of 32)", \
+                    scores, s0, s1, bias, pad, M, topk_group, topk, renorm, scaling, scoring, w, ids)
     if (n_group == 8) return MOE_TOPK_WARP(8);
     if (n_group == 4) return MOE_TOPK_WARP(4);
     if (n_group == 2) return MOE_TOPK_WARP(2);
@@ -527,8 +528,8 @@ int launch_vpt(const ST* scores, int64_t s0, int64_t s1, const BT* bias, const u
   }
   // groups of exactly 32 experts whose candidates fit the CTA
   if (E == 32 * n_group && n_group <= kGroupWarps && topk * n_group <= E && M < (1ll << 31)) {
-    return launch_pdl(grouped_topk_g32_kernel<ST, BT>, dim3((unsigned)M), E, 0, 1, st, "grouped_topk (warp per group)", scores, s0,
-                      s1, bias, pad, n_group, topk_group, topk, renorm, scaling, scoring, w, ids);
+    return launch_pdl_spread(grouped_topk_g32_kernel<ST, BT>, dim3((unsigned)M), E, kG32Smem, st, "grouped_topk (warp per group)",
+                             scores, s0, s1, bias, pad, n_group, topk_group, topk, renorm, scaling, scoring, w, ids);
   }
   const int warps = 4;
   dim3 grid((unsigned)((M + warps - 1) / warps)), block(warps * 32);

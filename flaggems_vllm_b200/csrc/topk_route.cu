@@ -129,8 +129,8 @@ int launch_vpt(const LT* logits, const float* bias, const uint8_t* pad, int64_t 
   const int warps = 4;
   dim3 grid((unsigned)((M + warps - 1) / warps));
 #define MOE_TR_LAUNCH(V) \
-  launch_pdl(topk_route_kernel<LT, IT, V>, grid, warps * 32, 0, 1, st, "topk_route", logits, bias, pad, M, E, topk, sigmoid, renorm, \
-             scale, w, ids, src)
+  launch_pdl_spread(topk_route_kernel<LT, IT, V>, grid, warps * 32, 0, st, "topk_route", logits, bias, pad, M, E, topk, sigmoid, \
+                    renorm, scale, w, ids, src)
   if (E <= 32) return MOE_TR_LAUNCH(1);
   if (E <= 64) return MOE_TR_LAUNCH(2);
   if (E <= 128) return MOE_TR_LAUNCH(4);

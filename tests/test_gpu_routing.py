@@ -377,3 +377,27 @@ def test_fp32_router_gemm_under_graph_replay():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, fg.fp32_router_gemm(x, w))
+
+
+@pytest.mark.parametrize("per_sm", [1, 2, 5, 11, 16, 17])
+@pytest.mark.parametrize("M_off", [0, 1])
+def test_routing_that_starts_while_the_router_runs(per_sm, M_off):
+    """grouped_topk and topk_softmax right behind router_gemm, which lets them start early, at block counts either side of a whole
+    number per multiprocessor (blocks of four tokens): the same as behind a synchronisation."""
+    M = 4 * per_sm * torch.cuda.get_device_properties(0).multi_processor_count + M_off
+    x = T.make_activations(M, 1024, DEV, seed=M)
+    gate, bias = T.make_half_weights(1, 256, 1024, DEV, seed=2)[0], T.make_router_inputs(1, 256, DEV)[1]
+    outs = []
+    for wait in (False, True):
+        logits = fg.router_gemm(x, gate)
+        if wait:
+            torch.cuda.synchronize()
+        w, ids = fg.grouped_topk(logits, 8, 4, 8, True, 2.5, bias, 1)
+        logits2 = fg.router_gemm(x, gate[:128])
+        if wait:
+            torch.cuda.synchronize()
+        sw, si, sr = torch.empty((M, 8), device=DEV), *(torch.empty((M, 8), dtype=torch.int32, device=DEV) for _ in range(2))
+        fg.topk_softmax(sw, si, sr, logits2, True)
+        outs.append((w, ids, sw, si))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
