@@ -94,10 +94,10 @@ __global__ void __launch_bounds__(kThreads) router_gemm_kernel(const XT* __restr
 // Launched so that its set-up (barriers, TMEM, the launch itself) overlaps the end of the kernel in front.  What that is worth
 // depends on the neighbours; us per call, K = 7168, N = 256, bf16, ordinary launch : this one (neighbour subtracted):
 //                                               64 rows     200 rows     1000 rows    2000 rows    8192 rows
-//   back to back, stream                        8.3 : 6.0   10.3 : 7.2   12.9 : 10.4  15.1 : 12.4  39.0 : 34.1
-//   behind an elementwise kernel, stream        8.2 : 6.2   10.3 : 8.2   13.1 : 11.3  14.9 : 13.5  40.1 : 34.8
-//   back to back, graph                         6.6 : 5.4    8.3 : 6.4   10.7 : 9.3   12.6 : 11.8  36.3 : 34.3
-//   behind an elementwise kernel, graph         6.7 : 6.7    8.3 : 8.5   10.8 : 11.0  12.8 : 13.0  40.7 : 39.0
+//   back to back, stream                        8.3 : 6.0   10.3 : 7.1   12.4 : 10.2  14.7 : 12.3  39.0 : 35.4
+//   behind an elementwise kernel, stream        8.2 : 6.2   10.3 : 8.2   13.0 : 11.4  14.4 : 13.2  39.6 : 36.9
+//   back to back, graph                         6.5 : 5.4    8.5 : 6.5   10.6 : 9.2   12.5 : 11.8  36.2 : 33.9
+//   behind an elementwise kernel, graph         7.0 : 6.5    8.4 : 8.7   10.8 : 11.1  12.8 : 12.7  39.5 : 38.9
 constexpr int RBM = 128, RTHREADS = 192;
 template <int BN> struct RCfg {
   static constexpr int STAGE = (RBM + BN) * 128;
@@ -270,14 +270,16 @@ int launch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, int 
 // round starts (128 CTAs in clusters of 8, one per SM, took two rounds); narrow tiles run two CTAs per SM, which
 // then share its bandwidth.  Of a whole GPU's 148 SMs it is 112 and 132 and not what the occupancy query gives (120 and
 // 132 on one GPU; which SMs are fused off differs), so that the order of the sums is one on every B200; a
-// partition has its share.  `largest`: most CTAs of a cluster.  Tiles of 256 columns are nowhere the fastest (four stages):
-// 8192 x 256 x 7168, us, 256 columns and two CTAs in K 40.4, 128 columns undivided 34.0.
+// partition has its share.  `largest`: most CTAs of a cluster.  N = 256, K = 7168, bf16, us back to back, with tiles of 256 columns :
+// up to 128 : 128 with the split of the 256: 2600 rows 17.1 : 26.7 : 21.8, 4000 rows 18.2 : 19.4 : 23.5, 6000 rows 29.6 : 39.4 : 36.7,
+// 8192 rows 36.4 : 33.6 : 39.6.  Where narrower tiles were ahead they divided K less, and one accumulator over all of K = 7168 is twice
+// as far from 64-bit arithmetic as two (relative 7.9e-6 against 3.8e-6).
 void pick_tc(int64_t M, int N, int K, int sms, int largest, int& bn, int& split) {
   const int kb = (K + 63) / 64;
   const int64_t mt = (M + RBM - 1) / RBM;
   double best = 0.0;
   bn = 0;
-  for (int b = 32; b <= 128; b *= 2) {
+  for (int b = 32; b <= 256; b *= 2) {
     if (b > 32 && b / 2 >= N) break;
     for (int s = 1; s <= 8 && s <= kb && s <= largest; s *= 2) {
       const double reach = (s == 8 ? 112.0 : (s == 4 ? 132.0 : 148.0)) * sms / 148.0;
@@ -301,7 +303,8 @@ bool split_fits(int bn, int split) {
   switch (bn) {
     case 32: return split_fits<T, 32>(split);
     case 64: return split_fits<T, 64>(split);
-    default: return split_fits<T, 128>(split);
+    case 128: return split_fits<T, 128>(split);
+    default: return split_fits<T, 256>(split);
   }
 }
 
@@ -315,7 +318,8 @@ int dispatch_tc(const void* x, int64_t x_ld, const void* w, int64_t M, int N, in
   switch (bn) {
     case 32: return launch_tc<T, 32>(x, x_ld, w, M, N, K, split, out, status, st);
     case 64: return launch_tc<T, 64>(x, x_ld, w, M, N, K, split, out, status, st);
-    default: return launch_tc<T, 128>(x, x_ld, w, M, N, K, split, out, status, st);
+    case 128: return launch_tc<T, 128>(x, x_ld, w, M, N, K, split, out, status, st);
+    default: return launch_tc<T, 256>(x, x_ld, w, M, N, K, split, out, status, st);
   }
 }
 
