@@ -312,7 +312,7 @@ align_cluster_kernel(const IdT* __restrict__ ids, int numel, int E, int block_si
 // barriers are those of the scan.  B200, 256 experts, block 128, 65536 ids with half of them on four experts: 8.0 us back to
 // back; the kernels above took 20.  Bound: the chain, in cycles of a cold call: ids 3200, ranks 2500, prefix and exchange 3000,
 // scan 1300, scatter of the ids 2600 (32 sectors per warp store), padding and tail 2900.
-template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
+template <typename IdT, int CTAS, int ROUNDS, int LANES>
 __device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int numel, int E, int block_size, int block_shift,
                                                 int32_t* __restrict__ sorted_ids, int sorted_cap,
                                                 int32_t* __restrict__ expert_ids, int expert_cap,
@@ -327,7 +327,7 @@ __device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int
   if constexpr (CTAS > 1) rank = (int)cg::this_cluster().block_rank();
   bool bad = false;
   int packed[ROUNDS], first, end;
-  rank_ids<CTAS, ROUNDS, MASKS>(numel, E, sh, [&](int i) -> int {
+  rank_ids<CTAS, ROUNDS, LANES>(numel, E, sh, [&](int i) -> int {
     const long long e = (long long)ids[i];
     if (e >= E) bad = true;  // negative ids mean "no route" (padding rows, other ranks' slots)
     return e >= 0 && e < E ? (int)e : -1;
@@ -376,11 +376,11 @@ __device__ __forceinline__ void align_sort_body(const IdT* __restrict__ ids, int
   for (int p = quads + 4 * whole + rank * kThreads + tid; p < sorted_cap; p += CTAS * kThreads) sorted_ids[p] = numel;
   for (int b = blocks(total) + rank * kThreads + tid; b < expert_cap; b += CTAS * kThreads) expert_ids[b] = -1;
 }
-template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
+template <typename IdT, int CTAS, int ROUNDS, int LANES>
 __global__ void __launch_bounds__(sorting::kThreads)
 align_sort_kernel(const IdT* ids, int numel, int E, int block_size, int block_shift, int32_t* sorted_ids, int sorted_cap, int32_t* expert_ids,
                   int expert_cap, int32_t* npp, int32_t* status) {
-  align_sort_body<IdT, CTAS, ROUNDS, MASKS>(ids, numel, E, block_size, block_shift, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status);
+  align_sort_body<IdT, CTAS, ROUNDS, LANES>(ids, numel, E, block_size, block_shift, sorted_ids, sorted_cap, expert_ids, expert_cap, npp, status);
 }
 
 // A cluster at any size: even a call of a few ids writes tens of thousands of sentinels.  False where no such cluster can
@@ -396,7 +396,9 @@ bool launch_align_sort(const void* ids, int numel, int E, int block_size, int32_
                          expert_ids, expert_cap, npp, status);
     return true;
   };
-#define MOE_ALIGN(C, R) (by_masks(E) ? launch(align_sort_kernel<IdT, C, R, true>, C) : launch(align_sort_kernel<IdT, C, R, false>, C))
+#define MOE_ALIGN(C, R)                                                                      \
+  (lanes_by(E) == ONE_FIRST   ? launch(align_sort_kernel<IdT, C, R, ONE_FIRST>, C)           \
+   : lanes_by(E) == LANE_BITS ? launch(align_sort_kernel<IdT, C, R, LANE_BITS>, C) : launch(align_sort_kernel<IdT, C, R, VOTES>, C))
   if (numel <= capacity(kSmall, 2)) return MOE_ALIGN(kSmall, 2);
   if (numel <= capacity(kLarge, 4)) return MOE_ALIGN(kLarge, 4);
   return MOE_ALIGN(kLarge, 16);

@@ -16,7 +16,7 @@
 namespace moe {
 namespace {
 
-template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
+template <typename IdT, int CTAS, int ROUNDS, int LANES>
 __device__ __forceinline__ void plan_body(const IdT* __restrict__ ids, int numel, int E, const int32_t* __restrict__ emap,
                                           int E_local, int gran_shift, int tile_rows, int32_t* __restrict__ row_index, int rows_cap,
                                           int4* __restrict__ tiles, int tiles_cap, int32_t* __restrict__ counts,
@@ -29,7 +29,7 @@ __device__ __forceinline__ void plan_body(const IdT* __restrict__ ids, int numel
   if constexpr (CTAS > 1) rank = (int)cg::this_cluster().block_rank();
   bool bad = false;
   int packed[ROUNDS], first, end;
-  rank_ids<CTAS, ROUNDS, MASKS>(numel, E_local, sh, [&](int i) -> int {
+  rank_ids<CTAS, ROUNDS, LANES>(numel, E_local, sh, [&](int i) -> int {
     const long long e = (long long)ids[i];
     if (e < 0 || e >= E) {
       if (e >= E) bad = true;  // negative ids mean "no route" (padding rows, other ranks' slots)
@@ -87,11 +87,11 @@ __device__ __forceinline__ void plan_body(const IdT* __restrict__ ids, int numel
   }
 }
 
-template <typename IdT, int CTAS, int ROUNDS, bool MASKS>
+template <typename IdT, int CTAS, int ROUNDS, int LANES>
 __global__ void __launch_bounds__(sorting::kThreads) plan_kernel(const IdT* ids, int numel, int E, const int32_t* emap, int E_local,
                                                                  int gran_shift, int tile_rows, int32_t* row_index, int rows_cap,
                                                                  int4* tiles, int tiles_cap, int32_t* counts, int32_t* status) {
-  plan_body<IdT, CTAS, ROUNDS, MASKS>(ids, numel, E, emap, E_local, gran_shift, tile_rows, row_index, rows_cap, tiles, tiles_cap, counts, status);
+  plan_body<IdT, CTAS, ROUNDS, LANES>(ids, numel, E, emap, E_local, gran_shift, tile_rows, row_index, rows_cap, tiles, tiles_cap, counts, status);
 }
 
 // Up to 32 ids: one warp, everything in registers and votes, no shared memory and no barrier (one token of 8 routes:
@@ -148,7 +148,9 @@ int launch_plan(const void* ids, int numel, int E, const int32_t* emap, int E_lo
 #define MOE_PLAN_B(C, R, B)                                                                                                    \
   launch_cluster(plan_kernel<IdT, C, R, B>, C, E_local, st, "route plan", (const IdT*)ids, numel, E, emap, E_local, gran_shift, \
                  tile_rows, row_index, rows_cap, tiles, tiles_cap, counts, status)
-#define MOE_PLAN(C, R) (by_masks(E_local) ? MOE_PLAN_B(C, R, true) : MOE_PLAN_B(C, R, false))
+#define MOE_PLAN(C, R)                                                                                       \
+  (lanes_by(E_local) == ONE_FIRST   ? MOE_PLAN_B(C, R, ONE_FIRST)                                            \
+   : lanes_by(E_local) == LANE_BITS ? MOE_PLAN_B(C, R, LANE_BITS) : MOE_PLAN_B(C, R, VOTES))
   // one CTA while a warp sees at most two rounds of ids: no cluster barriers
   if (numel <= capacity(1, 2)) return MOE_PLAN(1, 2);
   if (numel <= capacity(kSmall, 2)) return MOE_PLAN(kSmall, 2);
@@ -172,9 +174,9 @@ bool plan_serves(int64_t numel, int E, int E_local) {
   using namespace sorting;
   if (E <= 0 || E_local <= 0 || E_local > kMaxExperts || numel <= 0 || numel > capacity(kLarge, 16)) return false;
   if (numel <= capacity(1, 2)) return true;
-  if (numel <= capacity(kSmall, 2)) return cluster_fits(plan_kernel<int32_t, kSmall, 2, false>, kSmall, E_local);
-  if (numel <= capacity(kLarge, 4)) return cluster_fits(plan_kernel<int32_t, kLarge, 4, false>, kLarge, E_local);
-  return cluster_fits(plan_kernel<int32_t, kLarge, 16, false>, kLarge, E_local);
+  if (numel <= capacity(kSmall, 2)) return cluster_fits(plan_kernel<int32_t, kSmall, 2, VOTES>, kSmall, E_local);
+  if (numel <= capacity(kLarge, 4)) return cluster_fits(plan_kernel<int32_t, kLarge, 4, VOTES>, kLarge, E_local);
+  return cluster_fits(plan_kernel<int32_t, kLarge, 16, VOTES>, kLarge, E_local);
 }
 
 int plan_routes(const void* ids, int ids64, int64_t numel, int E, const int32_t* emap, int E_local, int gran, int tile_rows,

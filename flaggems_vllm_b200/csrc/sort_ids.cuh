@@ -1,7 +1,7 @@
 // Stable counting sort of expert ids, the part that moe_align_block_size (align.cu) and the route plan (plan.cu)
 // share.  One CTA of 1024 threads, or a cluster of 8 or 16 that exchange their per-expert counts through distributed shared
 // memory.  Every warp owns a contiguous slice of the ids, at most ROUNDS x 32 of them: all loads are issued first,
-// then the slice's ids are ranked round by round (votes, running counts of the slice in shared memory) and
+// then the slice's ids are ranked round by round (lane bits or votes, running counts of the slice in shared memory) and
 // (expert, rank) stay in registers.  The position of an id is then
 //     expert base + ids of that expert in earlier CTAs + in earlier warps + rank,
 // its place in a stable sort.  Bound: the latency of this chain; ids are read once.  What it was before lane masks for votes,
@@ -26,8 +26,13 @@ constexpr int kNone = 0x7FF;  // expert field of an id that gets no place
 constexpr int kSmall = 8, kLarge = 16;
 // ids a launch with this many CTAs and rounds sorts
 constexpr int64_t capacity(int ctas, int rounds) { return (int64_t)ctas * kWarps * rounds * 32; }
-// Lanes of a warp with the same expert: up to 511 experts from a word of lane bits per expert (and warp), else by votes
-constexpr bool by_masks(int E) { return E < 512; }
+// Lanes of a warp with the same expert.  LANE_BITS: from a word of lane bits per expert and warp; its lanes queue for it, which
+// costs most in a warp that has one expert alone.  Few experts make such warps likely, so below 16 that is asked first (ONE_FIRST):
+// 262144 ids of 8 experts, in order: lane bits 16.5 us, asked first 9.7; drawn: 11.8, 12.3 (votes of four bits: 12.3, 13.8).
+// VOTES: from 512 experts on, where the words would not fit.
+constexpr int ONE_FIRST = 0, LANE_BITS = 1, VOTES = 2;
+constexpr int lanes_by(int E) { return E < 16 ? ONE_FIRST : (E < 512 ? LANE_BITS : VOTES); }
+constexpr bool by_masks(int E) { return lanes_by(E) != VOTES; }
 inline size_t smem_bytes(int E, int ctas) {
   return ((size_t)kWarps * E * (by_masks(E) ? 2 : 1) + ((size_t)ctas + 3) * E + 1) * 4;
 }
@@ -70,7 +75,7 @@ __device__ __forceinline__ unsigned peers(int v) {
 // `expert(i)`: expert of id i in [0, E), or -1.  Returns with packed[r] = rank << 11 | expert (or kNone) of id
 // first + 32 r + lane < end, hist filled and every CTA's totals in everybody's `total` (each CTA writes its own into all of
 // them: a remote store waits for nothing, the barrier behind them for all of them).
-template <int CTAS, int ROUNDS, bool MASKS, typename Expert>
+template <int CTAS, int ROUNDS, int LANES, typename Expert>
 __device__ __forceinline__ void rank_ids(int numel, int E, Shared sh, Expert expert, int (&packed)[ROUNDS], int& first, int& end) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();
@@ -92,7 +97,7 @@ __device__ __forceinline__ void rank_ids(int numel, int E, Shared sh, Expert exp
   const int slices = min(kWarps, (per_cta + per_warp - 1) / per_warp);  // warps that own ids
   for (int i = tid; i < slices * E; i += kThreads) {
     sh.hist[i] = 0;
-    if constexpr (MASKS) sh.mask[i] = 0;
+    if constexpr (LANES != VOTES) sh.mask[i] = 0;
   }
   __syncthreads();
   int32_t* h = sh.hist + (size_t)warp * E;
@@ -105,20 +110,22 @@ __device__ __forceinline__ void rank_ids(int numel, int E, Shared sh, Expert exp
     }
     const int e = packed[r];
     unsigned same = 0;
-    if constexpr (MASKS) {
+    if constexpr (LANES == VOTES) {
+      same = peers<kBits>(e >= 0 ? e : E);  // E itself stands for "none"
+    } else if (LANES == ONE_FIRST && __all_sync(0xFFFFFFFFu, e == __shfl_sync(0xFFFFFFFFu, e, 0))) {
+      same = e >= 0 ? 0xFFFFFFFFu : 0u;
+    } else {
       if (e >= 0) atomicOr(&mask[e], 1u << lane);
       __syncwarp();
       if (e >= 0) same = mask[e];
       __syncwarp();
-    } else {
-      same = peers<kBits>(e >= 0 ? e : E);  // E itself stands for "none"
     }
     const int leader = __ffs(same) - 1;
     int old = 0;
     if (e >= 0 && lane == leader) {
       old = h[e];
       h[e] = old + __popc(same);
-      if constexpr (MASKS) mask[e] = 0;
+      if constexpr (LANES != VOTES) mask[e] = 0;
     }
     old = __shfl_sync(0xFFFFFFFFu, old, leader & 31);
     packed[r] = e >= 0 ? ((old + __popc(same & ((1u << lane) - 1u))) << 11) | e : kNone;

@@ -139,3 +139,22 @@ def test_cuda_graph_capture_of_empty_and_nonempty():
         os_, oe, on = O.moe_align_block_size_oracle(fresh, 64, 256)
         assert np.array_equal(s.cpu().numpy(), os_) and np.array_equal(e.cpu().numpy(), oe)
         assert int(n.item()) == int(on[0])
+
+
+@pytest.mark.parametrize("E", [1, 7, 8, 15, 16, 511, 512])
+@pytest.mark.parametrize("numel", [31, 2049, 16385, 262144])
+@pytest.mark.parametrize("order", ["drawn", "sorted", "one"])
+def test_either_side_of_the_ways_to_find_the_lanes_of_an_expert(E, numel, order):
+    """Lane bits, below 16 experts behind a test for a warp of one expert, up to 511; votes from 512 on.  Whole warps of one expert,
+    and ids without an expert between them."""
+    g = torch.Generator().manual_seed(E + numel)
+    ids = torch.randint(0, E, (numel,), generator=g)
+    if order == "sorted":
+        ids = ids.sort().values
+    elif order == "one":
+        ids[:] = E - 1
+    if E % 2:
+        ids[torch.randint(0, numel, (numel // 7 + 1,), generator=g)] = -1
+    else:  # some warps without any, most whole
+        ids[(torch.arange(numel) // 40) % 9 == 4] = -1
+    _check(ids.to(torch.int32).view(-1, 1).to(DEV), 48, E)
