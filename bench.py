@@ -783,10 +783,9 @@ def main():
         peak2x = 2.0 * peaks["bf16_tflops"]
         peak = fp8_peak if fp8_peak else peak2x
         # DRAM traffic of one GEMM1 launch: ncu (dram__bytes_read+write, one pass) on this workload, 8192
-        # tokens and 256 experts, gave 10.12 GB for 7.713 GB of algorithmic bytes (weights of the experts in
-        # use + e4m3 activations + scales + the e4m3 intermediate), a ratio of 1.31 (the weights of an expert's
-        # second and third row block are not always still in L2, and the sorted rows are read eight
-        # times as often as the tokens); 32 experts and 1024 tokens give 1.31 too.
+        # tokens and 256 experts, gave 8.66 + 0.17 GB for 7.713 GB of algorithmic bytes (weights of the experts in
+        # use + e4m3 activations + scales + the e4m3 intermediate), a ratio of 1.145 (the sorted rows are
+        # read eight times as often as the tokens); 32 experts and 1024 tokens give 1.10.
         _, ti0 = fg.grouped_topk(logits, c["n_group"], c["topk_group"], k, True, c["rsf"], bias, 1)
         e_act = int(torch.unique(ti0).numel())
         alg1 = e_act * (2 * I * H + (2 * I // 128) * (H // 128) * 4) + M * H + M * (H // 128) * 4 + M * k * I
@@ -795,7 +794,7 @@ def main():
                             "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                             "peak_fp8_measured": fp8_peak, "frac_vs_2x_bf16": ach / peak2x,
                             "frac_of_sustained": ach / (2.0 * peaks["bf16_tflops_sustained"]),
-                            "traffic": 1.31 * alg1, "traffic_source": "ncu DRAM bytes of this launch over its algorithmic bytes (x1.31)",
+                            "traffic": 1.145 * alg1, "traffic_source": "ncu DRAM bytes of this launch over its algorithmic bytes (x1.145)",
                             "algorithmic_bytes": alg1,
                             "peak_source": ("torch._scaled_mm e4m3 8192^3, best of 10, CUDA events, measured in this run"
                                             if fp8_peak else f"2 x bf16_tflops of {peaks['source']} peaks"),

@@ -30,9 +30,9 @@
 // of its own rows instead of a tile of everybody's (no barriers, and room for twice the raw stages).  GEMM1 / GEMM2 back to
 // back, Qwen3 shape, us: 33 tokens 64.7 / 37.7 -> 59.7 / 31.9, 500 tokens 89 / 50 -> 78 / 42, 4096 tokens 228 / 128 -> 218 /
 // 122.  A second commit and wait per K block (token stages of half a K block, four blocks of them) measured 78.6 / 45.0 at 33
-// tokens and 247 / 136 at 4096.  Prefill: no single part.  Without the token loads 162 of 208 us of GEMM1 are left, with one
-// of the eight MMAs 171, without raw loads 179, without widening 186, without epilogue 195.
-// Against gemm_w8.cu: 33 tokens 191 -> 121 us per layer, 4096 tokens 591 -> 460.
+// tokens and 247 / 136 at 4096.  Prefill: no single part.  Copies that skip work, on a GPU where GEMM1 takes 208 us: without the
+// token loads 162, with one of the eight MMAs 171, without raw loads 179, without widening 186, without epilogue 195.
+// Against gemm_w8.cu: 33 tokens 191 -> 118 us per layer, 4096 tokens 591 -> 455.
 #include "wt_common.cuh"
 
 namespace moe {

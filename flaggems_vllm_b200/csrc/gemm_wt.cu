@@ -18,7 +18,7 @@
 // Warp roles (384 threads):
 //   warp 0      TMA producer (both CTAs; the whole warp runs the loop, one elected lane issues)
 //   warp 1      MMA issuer (leader CTA; likewise)
-//   warp 2      TMEM allocation: two accumulators of 256 columns, so that a tile's epilogue overlaps the next tile's
+//   warp 2      TMEM allocation: two accumulators of up to 256 columns, so that a tile's epilogue overlaps the next tile's
 //               main loop (the whole K loop of a tile accumulates in TMEM)
 //   warps 4-11  consumers: warp w owns accumulator lanes 32 (w mod 4)..., group h = (w - 4) / 4 the h-th half
 //               of the tile's tokens
