@@ -555,3 +555,31 @@ def test_router_gemm_adds_the_partial_sums_of_each_split(M, N, K, columns, split
     out = fg.router_gemm(x, w)
     ref = x.double() @ w.double().t()
     assert float((out.double() - ref).norm() / ref.norm()) < 4e-6 and _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("fmt,counts", [
+    ("half", (128, 129, 3, 0)), ("half", (64, 64, 64, 67)),                   # 65 and 64 rows per expert: tiles of 256 and of 128
+    ("half", (257, 256, 300, 1)), ("int8", (31, 64, 65, 0)), ("int8", (256, 257, 288, 1)), ("fp8", (128, 129, 257, 1))])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_other_activation_in_the_pair_tiles(fmt, counts, dtype):
+    """GEMM1 has the 256-row kernel for it, GEMM2 the kernel of the plan's tiles; a row is the same in another batch, bit for bit."""
+    E, H, I = len(counts), 1152, 1664
+    tw, ti = _fixed_routes(counts, 1, 7)
+    M = ti.shape[0]
+    x = T.make_activations(M, H, DEV, seed=M, dtype=dtype)
+    kw = dict(activation="swigluoai_uninterleave", gemm1_alpha=1.702, gemm1_beta=1.0, gemm1_clamp_limit=7.0)
+    w1 = T.make_half_weights(E, 2 * I, H, DEV, seed=1, dtype=dtype, std=H**-0.5)
+    w2 = T.make_half_weights(E, H, I, DEV, seed=2, dtype=dtype, std=I**-0.5)
+    if fmt == "half":
+        ref = O.fused_moe_half_oracle(x, w1, w2, tw, ti, act_fn=lambda z: O.swigluoai_oracle(z, 1.702, 1.0, 7.0))
+    else:
+        top = 448.0 if fmt == "fp8" else 127.0
+        s1, s2 = w1.float().abs().amax(-1) / top, w2.float().abs().amax(-1) / top
+        cast = (lambda w: w.to(torch.float8_e4m3fn)) if fmt == "fp8" else (lambda w: w.round().to(torch.int8))
+        w1, w2 = cast(w1.float() / s1[..., None]), cast(w2.float() / s2[..., None])
+        kw |= {"use_fp8_w8a8" if fmt == "fp8" else "use_int8_w8a8": True, "per_channel_quant": True, "w1_scale": s1, "w2_scale": s2}
+        ref = O.fused_moe_row_scaled_oracle(x, w1, w2, s1, s2, tw, ti, fmt=fmt, per_token=True, activation="swigluoai_uninterleave")
+    out = fg.fused_experts_impl(x, w1, w2, tw, ti, **kw)
+    _parity(out, ref, (fmt, counts))
+    half = slice(0, M // 2)
+    assert torch.equal(fg.fused_experts_impl(x[half], w1, w2, tw[half], ti[half], **kw), out[half])
